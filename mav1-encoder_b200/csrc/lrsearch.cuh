@@ -39,13 +39,8 @@
 
 namespace lrs {
 
-using flt::LrBlock;
-using flt::lr_block_setup;
-using flt::lr_src;
-
 constexpr int THREADS = 256;
 constexpr int CACHE = 40;       // candidate SSEs a unit keeps from the first pass and the speculative pass
-constexpr int ROWBUF = 4 * 96;  // samples of one block row of a unit (4 rows of at most 95)
 
 // What the first pass leaves for the serial choice, per unit.
 struct Fit {
@@ -105,58 +100,141 @@ __device__ void unit_geom(const FrameParams *fp, int plane, int ur, int uc, Geom
   g->c1 = c0 < c1 ? c1 : 0;
 }
 
-// A unit's samples staged in shared memory: the CDEF output, the deblocked
-// frame and the source over the unit plus 3 samples on every side (clamped to
-// the plane), which covers every tap the filters read for the unit's blocks
-// (get_source_sample moves a row at most to the block's own 3-row margin).
-// A unit spans at most 103 x 95 samples (the last unit row or column takes
-// the remainder, and unit rows are offset by 8 luma rows).
-constexpr int WP = 104, WH = 112;
-
-struct Win {
-  uint8_t cd[WH * WP], db[WH * WP], sr[WH * WP];
-  int x0, y0;
+// A unit's samples in shared memory. A unit is cut into the stripes its rows
+// fall in (a luma unit is one stripe, the last row of units up to two; a
+// chroma unit two, up to four): `tap` holds, per stripe, the samples
+// get_source_sample( ) returns over the stripe's rows and columns plus 3 on
+// every side, with the clamps to the plane and the stripe's CDEF / deblocked
+// choice already made, so the filters read it with plain indices. `src` holds
+// the unit's source samples. Every other array of a pass is laid out behind
+// them; Dims are the largest unit of the frame, so shared memory is no larger
+// than the frame's units need (64 x 64 units: 93 KB, two CTAs per SM; the
+// largest unit, 95 x 103, takes 222 KB).
+constexpr int MAX_SEGS = 4, MAX_UNIT_W = 95, MAX_UNIT_H = 103;
+struct Dims {
+  int w, h;                 // largest width and height
+  int rows6, rows2, odd;    // largest h + 6 segs, h + 2 segs, h / 2 + 2 segs
 };
+// units of 64 samples: a luma unit of up to 103 rows has two stripes, a chroma
+// unit of up to 99 rows four
+constexpr Dims MAX_DIMS = {MAX_UNIT_W, MAX_UNIT_H, 99 + 6 * 4, 103 + 2 * 2, 99 / 2 + 2 * 4};
+HD int align16(int x) { return (x + 15) & ~15; }
+struct Layout {
+  int tap_p, src_p;                         // row pitches
+  int tap, src;                             // byte offsets
+  int p1, b1, p2, b2, ab1, ab2, fd, sgr_end;  // self-guided pass
+  int hv, phi, wiener_end;                  // Wiener fit
+};
+HD Layout layout_of(const Dims &d) {
+  Layout l;
+  l.tap_p = (d.w + 6 + 3) & ~3;
+  l.src_p = (d.w + 3) & ~3;
+  l.tap = 0;
+  l.src = align16(d.rows6 * l.tap_p);
+  int base = align16(l.src + d.h * l.src_p);
+  int n1 = d.rows2 * (d.w + 2), n2 = d.odd * (d.w + 2);
+  l.p1 = base;
+  l.b1 = align16(l.p1 + 4 * n1);
+  l.p2 = align16(l.b1 + 2 * n1);
+  l.b2 = align16(l.p2 + 4 * n2);
+  l.ab1 = align16(l.b2 + 2 * n2);
+  l.ab2 = align16(l.ab1 + 4 * n1);
+  l.fd = align16(l.ab2 + 4 * n2);
+  l.sgr_end = align16(l.fd + 4 * d.h * d.w);
+  int nv = d.rows6 * d.w, nh = d.h * (d.w + 6);
+  l.hv = base;
+  l.phi = align16(l.hv + 8 * (nv > nh ? nv : nh));
+  l.wiener_end = l.phi + 2 * 4 * d.w * 4 * 8;
+  return l;
+}
+HD int smem_fit(const Layout &l) { return l.sgr_end > l.wiener_end ? l.sgr_end : l.wiener_end; }
+HD int smem_sse(const Layout &l) { return l.p1; }
 
-struct WinSrc {
-  const Win *w;
-  HD int tap(const LrBlock *lb, int x, int y) const {
-    x = imax(0, imin(lb->planeEndX, x));
-    y = imax(0, imin(lb->planeEndY, y));
-    const uint8_t *b = w->cd;
-    if (y < lb->stripeStart) {
-      y = imax(lb->stripeStart - 2, y);
-      b = w->db;
-    } else if (y > lb->stripeEnd) {
-      y = imin(lb->stripeEnd + 2, y);
-      b = w->db;
+// The largest unit of the planes of a frame (the last unit of a row or column
+// takes the remainder; unit rows start 8 luma rows early).
+inline Dims unit_dims(const FrameParams &fp) {
+  Dims d = {1, 1, 1, 1, 1};
+  for (int p = 0; p < 3; p++) {
+    int sub = p > 0, size = fp.lr_unit_size[p], off = 8 >> sub, stripe = 64 >> sub;
+    int pw = (fp.frame_w + sub) >> sub, ph = (fp.frame_h + sub) >> sub;
+    int rows = fp.lr_unit_rows[p], cols = fp.lr_unit_cols[p];
+    d.w = imax(d.w, cols <= 1 ? pw : imax(size, pw - size * (cols - 1)));
+    // the first row of units starts mid-stripe, later ones on a stripe when the size is a multiple of it
+    int hs[2] = {rows <= 1 ? ph : size - off, rows <= 1 ? 0 : imax(size, ph - size * (rows - 1) + off)};
+    for (int k = 0; k < 2; k++) {
+      int h = hs[k], slack = k == 0 ? off : size % stripe ? stripe - 1 : 0;
+      int segs = (h + slack + stripe - 1) / stripe;
+      d.h = imax(d.h, h);
+      d.rows6 = imax(d.rows6, h + 6 * segs);
+      d.rows2 = imax(d.rows2, h + 2 * segs);
+      d.odd = imax(d.odd, h / 2 + 2 * segs);
     }
-    return b[(y - w->y0) * WP + (x - w->x0)];
   }
-  HD int own(int x, int y) const { return w->cd[(y - w->y0) * WP + (x - w->x0)]; }
-  HD int src(int x, int y) const { return w->sr[(y - w->y0) * WP + (x - w->x0)]; }
-};
+  return d;
+}
 
-// Copies the unit's window into shared memory (the whole CTA).
-__device__ void stage_window(const FrameParams *fp, const Geom &g, const uint8_t *cdef, const uint8_t *dbk,
-                             const uint8_t *src, Win &w) {
-  const int sub = g.plane > 0, bw = MI_SIZE >> sub;
+// The unit a CTA works on: its plane samples x0 .. x0 + w - 1, rows y0 .. y0 +
+// h - 1, cut into stripes: segment s covers rows y0 + seg[s] .. y0 + seg[s + 1]
+// - 1. Row i of the unit (segment s) is row i + 6 s + 3 of `tap`.
+struct Area {
+  int plane, x0, y0, w, h, nseg, seg[MAX_SEGS + 1];
+  unsigned inv_w, inv_w2, inv_w6;  // 2^24 / d rounded up, d = w, w + 2, w + 6 (quotient())
+};
+// k / d for d's rounded-up reciprocal inv = ceil(2^24 / d): exact while k < 2^24 / d (here k < 14,000 and d < 104; the
+// product stays below 2^32, k / d being at most 127).
+__device__ __forceinline__ int quotient(int k, unsigned inv) { return (int)((unsigned)k * inv >> 24); }
+
+__device__ __forceinline__ int seg_of(const Area &a, int row) {
+  int s = 0;
+  while (s + 1 < a.nseg && row >= a.seg[s + 1]) s++;
+  return s;
+}
+
+// Finds the unit's area (one thread).
+__device__ void unit_area(const FrameParams *fp, const Geom &g, Area *a) {
+  const int sub = g.plane > 0, bw = MI_SIZE >> sub, stripe = 64 >> sub, off = 8 >> sub;
   const int endX = ((fp->frame_w + sub) >> sub) - 1, endY = ((fp->frame_h + sub) >> sub) - 1;
-  const int x0 = imax(0, ((g.c0 * MI_SIZE) >> sub) - 3), y0 = imax(0, ((g.r0 * MI_SIZE) >> sub) - 3);
-  const int x1 = imin(endX, ((g.c1 - 1) * MI_SIZE >> sub) + bw - 1 + 3);
-  const int y1 = imin(endY, ((g.r1 - 1) * MI_SIZE >> sub) + bw - 1 + 3);
-  const int nx = imin(WP, x1 - x0 + 1), ny = imin(WH, y1 - y0 + 1);
-  const int stride = fp->stride[g.plane], off = fp->offset[g.plane];
-  if (threadIdx.x == 0) {
-    w.x0 = x0;
-    w.y0 = y0;
+  a->plane = g.plane;
+  a->x0 = (g.c0 * MI_SIZE) >> sub;
+  a->y0 = (g.r0 * MI_SIZE) >> sub;
+  a->w = g.c1 > g.c0 ? imax(0, imin(endX, ((g.c1 - 1) * MI_SIZE >> sub) + bw - 1) - a->x0 + 1) : 0;
+  a->h = g.r1 > g.r0 && a->w > 0 ? imax(0, imin(endY, ((g.r1 - 1) * MI_SIZE >> sub) + bw - 1) - a->y0 + 1) : 0;
+  a->nseg = 0;
+  for (int row = 0; row < a->h && a->nseg < MAX_SEGS;) {
+    a->seg[a->nseg++] = row;
+    row += stripe - (a->y0 + row + off) % stripe;
   }
-  for (int i = threadIdx.x; i < nx * ny; i += blockDim.x) {
-    int r = i / nx, c = i - r * nx;
-    int o = off + (y0 + r) * stride + x0 + c, k = r * WP + c;
-    w.cd[k] = cdef[o];
-    w.db[k] = dbk[o];
-    w.sr[k] = src[o];
+  a->seg[a->nseg] = a->h;
+  a->inv_w = ((1u << 24) + imax(a->w, 1) - 1) / imax(a->w, 1);
+  a->inv_w2 = ((1u << 24) + a->w + 1) / (a->w + 2);
+  a->inv_w6 = ((1u << 24) + a->w + 5) / (a->w + 6);
+}
+
+// Fills `tap` and `src` (the whole CTA).
+__device__ void stage_unit(const FrameParams *fp, const Area &a, const uint8_t *cdef, const uint8_t *dbk,
+                           const uint8_t *src, const Layout &l, uint8_t *smem) {
+  const int p = a.plane, sub = p > 0, stride = fp->stride[p], off = fp->offset[p];
+  const int endX = ((fp->frame_w + sub) >> sub) - 1, endY = ((fp->frame_h + sub) >> sub) - 1;
+  const int nrow = a.h ? a.h + 6 * a.nseg : 0, W6 = a.w + 6;
+  for (int k = threadIdx.x; k < nrow * W6; k += THREADS) {
+    int tr = quotient(k, a.inv_w6), c = k - tr * W6, s = 0;
+    while (s + 1 < a.nseg && tr >= a.seg[s + 1] + 6 * (s + 1)) s++;
+    int row = a.y0 + tr - 6 * s - 3;                                  // plane row asked for
+    int st = ((a.y0 + a.seg[s] + (8 >> sub)) / (64 >> sub)) * (64 >> sub) - (8 >> sub), en = st + (64 >> sub) - 1;
+    int x = imax(0, imin(endX, a.x0 + c - 3)), y = imax(0, imin(endY, row));
+    const uint8_t *b = cdef;
+    if (y < st) {
+      y = imax(st - 2, y);
+      b = dbk;
+    } else if (y > en) {
+      y = imin(en + 2, y);
+      b = dbk;
+    }
+    smem[l.tap + tr * l.tap_p + c] = b[off + y * stride + x];
+  }
+  for (int k = threadIdx.x; k < a.h * a.w; k += THREADS) {
+    int r = quotient(k, a.inv_w), c = k - r * a.w;
+    smem[l.src + r * l.src_p + c] = src[off + (a.y0 + r) * stride + a.x0 + c];
   }
   __syncthreads();
 }
@@ -261,66 +339,93 @@ HD int unit_bits(int plane, const LrUnit &u, int refW[2][3], int refX[2]) {
 HD long long rd(const FrameParams *fp, long long sse, int bits) { return sse * 16 + (long long)fp->lambda * bits; }
 
 // ---- CTA-wide helpers ------------------------------------------------------------------
+constexpr int WARPS = THREADS / 32;
 struct Shared {
-  Win win;
-  double phi[2][ROWBUF][4];  // per sample of a block row: phi[0..nc) and the target
   double acc[12];
   double f[7], g[7];
-  long long red[THREADS / 32];
+  long long red[2][WARPS][12];  // a sum's per-warp parts, in turn
   Geom geom;
+  Area area;
   int stop;
+  uint16_t atab[256];           // self-guided a2 of z (lr_box)
   // k_lr_spec: the unit's candidate cache (Fit::taps / sse / n), kept by thread 0
   int ctaps[CACHE][6];
   long long csse[CACHE];
-  int cn;
-  // k_lr_select: the unit's first-pass results, and a cache lookup's result
+  int cn, found;
+  // k_lr_select: the unit's first-pass results; a candidate neither pass cached
   Fit fit;
-  int found;
+  int miss_unit;                // its unit, or -1: the scan is done
+  int miss_taps[6];
 };
 
+// Sum of a 32-bit value over the warp, in 64 bits.
+__device__ __forceinline__ long long warp_sum(int v) {
+  int hi = __reduce_add_sync(0xffffffffu, v >> 16), lo = __reduce_add_sync(0xffffffffu, v & 0xffff);
+  return ((long long)hi << 16) + lo;
+}
+
 // Sum of v over the CTA (every thread gets it).
-__device__ long long cta_sum(long long v, Shared &sh) {
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+__device__ long long cta_sum(int v, Shared &sh) {
+  long long s = warp_sum(v);
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) sh.red[0][threadIdx.x >> 5][0] = s;
   __syncthreads();
-  long long s = 0;
-  for (int w = 0; w < THREADS / 32; w++) s += sh.red[w];
-  __syncthreads();
+  s = 0;
+  for (int w = 0; w < WARPS; w++) s += sh.red[0][w][0];
   return s;
 }
 
-struct SseSink {
-  const Win *w;
-  long long sse;
-  HD void operator()(int x, int y, int v) {
-    int d = v - (int)w->sr[(y - w->y0) * WP + (x - w->x0)];
-    sse += d * d;
+// SSE of the unit's CDEF output against the source.
+__device__ long long none_sse(const Layout &l, const uint8_t *smem, Shared &sh) {
+  const Area &a = sh.area;
+  int e = 0;
+  for (int k = threadIdx.x; k < a.h * a.w; k += THREADS) {
+    int r = quotient(k, a.inv_w), c = k - r * a.w;
+    int d = (int)smem[l.tap + (r + 6 * seg_of(a, r) + 3) * l.tap_p + c + 3] - (int)smem[l.src + r * l.src_p + c];
+    e += d * d;
   }
-};
+  return cta_sum(e, sh);
+}
 
-// SSE of a unit filtered with u against the source (unit_sse), from the
-// staged window: a thread per 4x4 block of the unit.
-__device__ long long unit_sse(const FrameParams *fp, const Geom &g, const LrUnit &u, Shared &sh) {
-  int nc = g.c1 - g.c0, nb = (g.r1 - g.r0) * nc;
-  WinSrc in{&sh.win};
-  SseSink sink{&sh.win, 0};
-  for (int b = threadIdx.x; b < nb; b += THREADS) {
-    LrBlock lb;
-    if (!lr_block_setup(fp, g.plane, g.r0 + b / nc, g.c0 + b % nc, &lb)) continue;
-    if (u.type == RESTORE_WIENER) {
-      flt::lr_wiener_to(&lb, in, &u, sink);
-    } else if (u.type == RESTORE_SGRPROJ) {
-      int flt0[16], flt1[16];
-      flt::lr_box(&lb, in, u.set, 0, flt0);
-      flt::lr_box(&lb, in, u.set, 1, flt1);
-      flt::lr_sgr_project(&lb, in, &u, flt0, flt1, sink);
-    } else {
-      for (int i = 0; i < lb.h; i++)
-        for (int j = 0; j < lb.w; j++) sink(lb.x + j, lb.y + i, in.own(lb.x + j, lb.y + i));
-    }
-  }
-  return cta_sum(sink.sse, sh);
+// SSE of the unit filtered with Wiener taps tt (pass 0 vertical j 0..2, pass 1
+// horizontal) against the source: flt::lr_wiener_to's sums and clips. A warp
+// takes 16 rows of 32 columns, a lane a column: it keeps the last 7 rows'
+// horizontal sums in registers, so a row costs 7 samples read and 8 multiplies
+// instead of every 4x4 block filtering 10 rows for 4 (a 64 x 64 unit: 8 tasks,
+// one a warp).
+constexpr int SSE_ROWS = 16;
+__device__ __noinline__ long long wiener_unit_sse(const Layout &l, const uint8_t *smem, const int *tt, Shared &sh) {
+  const Area &a = sh.area;
+  const int v0 = tt[0], v1 = tt[1], v2 = tt[2], v3 = 128 - 2 * (v0 + v1 + v2);
+  const int h0 = tt[3], h1 = tt[4], h2 = tt[5], h3 = 128 - 2 * (h0 + h1 + h2);
+  const int offset = 1 << (8 + FILTER_BITS - 3 - 1), limit = (1 << (8 + 1 + FILTER_BITS - 3)) - 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cols = (a.w + 31) >> 5;
+  int e = 0, task = 0;
+  for (int s = 0; s < a.nseg; s++)
+    for (int r0 = a.seg[s]; r0 < a.seg[s + 1]; r0 += SSE_ROWS)
+      for (int cg = 0; cg < cols; cg++, task++) {
+        if (task % WARPS != warp) continue;
+        int x = cg * 32 + lane, r1 = imin(r0 + SSE_ROWS, a.seg[s + 1]);
+        if (x >= a.w) continue;
+        const uint8_t *t = smem + l.tap + (r0 + 6 * s) * l.tap_p + x;
+        const uint8_t *sr = smem + l.src + r0 * l.src_p + x;
+        auto hsum = [&](const uint8_t *q) {
+          int v = h3 * q[3] + h0 * (q[0] + q[6]) + h1 * (q[1] + q[5]) + h2 * (q[2] + q[4]);
+          return clip3(-offset, limit - offset, round2(v, 3));
+        };
+        int b0 = hsum(t), b1 = hsum(t + l.tap_p), b2 = hsum(t + 2 * l.tap_p), b3 = hsum(t + 3 * l.tap_p),
+            b4 = hsum(t + 4 * l.tap_p), b5 = hsum(t + 5 * l.tap_p);
+        t += 6 * l.tap_p;
+        for (int r = r0; r < r1; r++, t += l.tap_p, sr += l.src_p) {
+          int b6 = hsum(t);
+          int v = v3 * b3 + v0 * (b0 + b6) + v1 * (b1 + b5) + v2 * (b2 + b4);
+          int d = clip3(0, 255, round2(v, 11)) - (int)*sr;
+          e += d * d;
+          b0 = b1; b1 = b2; b2 = b3; b3 = b4; b4 = b5; b5 = b6;
+        }
+      }
+  return cta_sum(e, sh);
 }
 
 HD LrUnit wiener_unit(const int w[2][3]) {
@@ -333,82 +438,131 @@ HD LrUnit wiener_unit(const int w[2][3]) {
 
 // wiener_fit (lr_search.c:142-193): four alternating separable least-squares
 // solves, then the taps in coded units.
-__device__ void wiener_fit(const FrameParams *fp, const Geom &g, Shared &sh, int out[2][3]) {
-  const int plane = g.plane, first = plane ? 1 : 0, nc = 3 - first, nacc = nc * nc + nc;
-  const int sub = plane > 0, bwf = MI_SIZE >> sub;
-  const WinSrc in{&sh.win};
-  if (threadIdx.x < 7) {
-    sh.f[threadIdx.x] = threadIdx.x == 3 ? 1.0 : 0.0;
-    sh.g[threadIdx.x] = threadIdx.x == 3 ? 1.0 : 0.0;
+//
+// What a sample's 7 values Z[kk] are: the rows (columns) around it filtered by
+// the other direction's current taps. A filtered row is the same for the 7
+// samples that use it, so each is formed once (hv, in the reference's order of
+// additions) instead of once per use. The first solve's taps are the identity:
+// its sums are whole numbers, exact in any order, and every thread adds its
+// own. The later sums follow the reference's order: one lane per accumulator
+// of warp 0 adds a block row's products while the other warps form the next
+// row's; that chain of 4,096 dependent double additions a solve bounds the fit.
+__device__ void wiener_solve(Shared &sh, int first, int nc, int vertical) {
+  double M[3][3] = {{0}}, V[3] = {0}, x[3] = {0, 0, 0};
+  for (int a = 0; a < nc; a++) {
+    for (int b = 0; b < nc; b++) M[a][b] = sh.acc[a * nc + b];
+    V[a] = sh.acc[nc * nc + a];
   }
-  if (threadIdx.x == 0) sh.stop = 0;
+  for (int a = 0; a < nc; a++) M[a][a] = dadd(M[a][a], 1e-3);
+  if (!solve(nc, M, V, x)) {
+    sh.stop = 1;
+    return;
+  }
+  double *dst = vertical ? sh.f : sh.g;
+  double sum = 0.0;
+  for (int k = 0; k < 3; k++) {
+    double v = k < first ? 0.0 : x[k - first];
+    dst[k] = dst[6 - k] = v;
+    sum = dadd(sum, v);
+  }
+  dst[3] = dsub(1.0, dmul(2.0, sum));
+}
+
+__device__ void wiener_fit(const Layout &l, uint8_t *smem, Shared &sh, int out[2][3]) {
+  const Area &a = sh.area;
+  const int plane = a.plane, first = plane ? 1 : 0, nc = 3 - first, nacc = nc * nc + nc;
+  const int lb = plane ? 1 : 2, bwf = 1 << lb;  // block width and height of a 4x4 luma block in this plane
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double *hv = (double *)(smem + l.hv);
+  double(*phi)[4] = (double(*)[4])(smem + l.phi);  // two buffers of a block row's samples
+  const int rowbuf = bwf * a.w;
+  if (tid < 7) sh.f[tid] = sh.g[tid] = tid == 3 ? 1.0 : 0.0;
+  if (tid == 0) sh.stop = 0;
   __syncthreads();
-  for (int iter = 0; iter < 4 && !sh.stop; iter++) {
+  {  // first solve: the taps are the identity, every sum a whole number
+    int part[12];
+    for (int k = 0; k < 12; k++) part[k] = 0;
+    for (int k = tid; k < a.h * a.w; k += THREADS) {
+      int r = quotient(k, a.inv_w), c = k - r * a.w;
+      const uint8_t *t = smem + l.tap + (r + 6 * seg_of(a, r)) * l.tap_p + c + 3;
+      int z3 = t[3 * l.tap_p], ph[4];
+      for (int kk = 0; kk < 3; kk++) ph[kk] = (int)t[kk * l.tap_p] + t[(6 - kk) * l.tap_p] - 2 * z3;
+      ph[3] = (int)smem[l.src + r * l.src_p + c] - z3;
+      for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 4; j++) part[i * 4 + j] += ph[i] * ph[j];
+    }
+    for (int k = 0; k < 12; k++) {
+      long long v = warp_sum(part[k]);
+      if (lane == 0) sh.red[0][warp][k] = v;
+    }
+    __syncthreads();
+    if (tid < nacc) {
+      int i = first + (tid < nc * nc ? tid / nc : tid - nc * nc), j = tid < nc * nc ? first + tid % nc : 3;
+      long long v = 0;
+      for (int w = 0; w < WARPS; w++) v += sh.red[0][w][i * 4 + j];
+      sh.acc[tid] = (double)v;
+    }
+    __syncthreads();
+    if (tid == 0) wiener_solve(sh, first, nc, 1);
+    __syncthreads();
+  }
+  for (int iter = 1; iter < 4 && !sh.stop; iter++) {
     const int vertical = !(iter & 1);
+    {  // the filtered rows (vertical solve: hv[tap row][column]) or columns (hv[row][column - 3 .. + 3])
+      const double *q = vertical ? sh.g : sh.f;
+      const double q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5], q6 = q[6];
+      const int n = vertical ? (a.h + 6 * a.nseg) * a.w : a.h * (a.w + 6);
+      for (int k = tid; k < n; k += THREADS) {
+        int r = quotient(k, vertical ? a.inv_w : a.inv_w6), c = k - r * (vertical ? a.w : a.w + 6);
+        const uint8_t *t = smem + l.tap + (vertical ? r : r + 6 * seg_of(a, r)) * l.tap_p + c;
+        const int st = vertical ? 1 : l.tap_p;
+        double s = dadd(0.0, dmul(q0, (double)t[0]));
+        s = dadd(s, dmul(q1, (double)t[st]));
+        s = dadd(s, dmul(q2, (double)t[2 * st]));
+        s = dadd(s, dmul(q3, (double)t[3 * st]));
+        s = dadd(s, dmul(q4, (double)t[4 * st]));
+        s = dadd(s, dmul(q5, (double)t[5 * st]));
+        s = dadd(s, dmul(q6, (double)t[6 * st]));
+        hv[k] = s;
+      }
+    }
+    __syncthreads();
+    const int steps = (a.h + bwf - 1) >> lb;  // block rows
+    const int ia = lane < nc * nc ? lane / nc : lane - nc * nc, ib = lane < nc * nc ? lane % nc : 3;
     double acc = 0.0;  // lane L < nacc of warp 0: M[L / nc][L % nc], then V[L - nc * nc]
-    for (int r = g.r0; r < g.r1; r++) {
-      // the block row's samples in the reference's order: blocks left to
-      // right, each block's rows, each row's samples
-      LrBlock lb0;
-      lr_block_setup(fp, plane, r, g.c0, &lb0);
-      const int h = lb0.h;
-      int wsum = 0;
-      for (int c = g.c0; c < g.c1; c++) wsum += imin(bwf, lb0.planeEndX - ((c * MI_SIZE) >> sub) + 1);
-      const int npx = h * wsum;
-      const int buf = r & 1;
-      for (int k = threadIdx.x; k < npx; k += THREADS) {
-        // k -> (block column, row, column): full blocks are bwf wide, only the
-        // plane's last column of blocks can be narrower
-        int cb = k / (bwf * h);
-        int rem = k - cb * bwf * h;
-        LrBlock lb;
-        lr_block_setup(fp, plane, r, g.c0 + cb, &lb);
-        int i = rem / lb.w, j = rem - i * lb.w;
-        double Z[7];
-        for (int kk = 0; kk < 7; kk++) {
-          double s = 0.0;
-          for (int t = 0; t < 7; t++) {
-            int sv = vertical ? in.tap(&lb, lb.x + j + t - 3, lb.y + i + kk - 3)
-                              : in.tap(&lb, lb.x + j + kk - 3, lb.y + i + t - 3);
-            s = dadd(s, dmul(vertical ? sh.g[t] : sh.f[t], (double)sv));
-          }
-          Z[kk] = s;
+    for (int step = 0; step <= steps; step++) {
+      if (warp > 0 && step < steps) {
+        // block row `step` in the reference's order: blocks left to right,
+        // each block's rows, each row's samples
+        const int i0 = step << lb, h = imin(bwf, a.h - i0), s = seg_of(a, i0);
+        double(*ph)[4] = phi + (step & 1) * rowbuf;
+        for (int k = tid - 32; k < h * a.w; k += THREADS - 32) {
+          int i = quotient(k, a.inv_w), x = k - i * a.w, cb = x >> lb, lbw = imin(bwf, a.w - (cb << lb));
+          int o = (cb << lb) * h + i * lbw + x - (cb << lb);
+          const double *z = vertical ? hv + (i0 + i + 6 * s) * a.w + x : hv + (i0 + i) * (a.w + 6) + x;
+          const int st = vertical ? a.w : 1;
+          double z3 = z[3 * st], two = dmul(2.0, z3);
+          for (int kk = first; kk < 3; kk++) ph[o][kk - first] = dsub(dadd(z[kk * st], z[(6 - kk) * st]), two);
+          ph[o][3] = dsub((double)smem[l.src + (i0 + i) * l.src_p + x], z3);
         }
-        for (int kk = first; kk < 3; kk++) sh.phi[buf][k][kk - first] = dsub(dadd(Z[kk], Z[6 - kk]), dmul(2.0, Z[3]));
-        sh.phi[buf][k][3] = dsub((double)in.src(lb.x + j, lb.y + i), Z[3]);
+      } else if (warp == 0 && step > 0 && lane < nacc) {
+        const int h = imin(bwf, a.h - ((step - 1) << lb)), n = h * a.w;
+        double(*ph)[4] = phi + ((step - 1) & 1) * rowbuf;
+        int k = 0;
+        for (; k + 8 <= n; k += 8) {
+          double m[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) m[q] = dmul(ph[k + q][ia], ph[k + q][ib]);
+#pragma unroll
+          for (int q = 0; q < 8; q++) acc = dadd(acc, m[q]);
+        }
+        for (; k < n; k++) acc = dadd(acc, dmul(ph[k][ia], ph[k][ib]));
       }
       __syncthreads();
-      if (threadIdx.x < nacc) {
-        int L = threadIdx.x;
-        int a = L < nc * nc ? L / nc : L - nc * nc;
-        int b = L < nc * nc ? L % nc : 3;
-        for (int k = 0; k < npx; k++) acc = dadd(acc, dmul(sh.phi[buf][k][a], sh.phi[buf][k][b]));
-      }
-      // the next row writes the other buffer; this one is read until the
-      // barrier after that row's samples
     }
-    if (threadIdx.x < nacc) sh.acc[threadIdx.x] = acc;
+    if (tid < nacc) sh.acc[tid] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double M[3][3] = {{0}}, V[3] = {0}, x[3] = {0, 0, 0};
-      for (int a = 0; a < nc; a++) {
-        for (int b = 0; b < nc; b++) M[a][b] = sh.acc[a * nc + b];
-        V[a] = sh.acc[nc * nc + a];
-      }
-      for (int a = 0; a < nc; a++) M[a][a] = dadd(M[a][a], 1e-3);
-      if (!solve(nc, M, V, x)) {
-        sh.stop = 1;
-      } else {
-        double *dst = vertical ? sh.f : sh.g;
-        double sum = 0.0;
-        for (int k = 0; k < 3; k++) {
-          double v = k < first ? 0.0 : x[k - first];
-          dst[k] = dst[6 - k] = v;
-          sum = dadd(sum, v);
-        }
-        dst[3] = dsub(1.0, dmul(2.0, sum));
-      }
-    }
+    if (tid == 0) wiener_solve(sh, first, nc, vertical);
     __syncthreads();
   }
   for (int pass = 0; pass < 2; pass++) {
@@ -421,54 +575,182 @@ __device__ void wiener_fit(const FrameParams *fp, const Geom &g, Shared &sh, int
   __syncthreads();
 }
 
-// sgr_fit (lr_search.c:196-240): least-squares projection weights of set
-// `set`. The sums are integer-valued and exact in int64; the closing double
-// arithmetic follows the reference's operations.
-__device__ void sgr_fit(const FrameParams *fp, const Geom &g, int set, Shared &sh, int xqd[2]) {
-  const int r0 = T(Sgr_Params)[set][0], r1 = T(Sgr_Params)[set][2];
-  const int ncols = g.c1 - g.c0, nb = (g.r1 - g.r0) * ncols;
-  const WinSrc in{&sh.win};
-  long long h00 = 0, h01 = 0, h11 = 0, c0 = 0, c1 = 0;
-  for (int b = threadIdx.x; b < nb; b += THREADS) {
-    LrBlock lb;
-    if (!lr_block_setup(fp, g.plane, g.r0 + b / ncols, g.c0 + b % ncols, &lb)) continue;
-    int flt0[16], flt1[16];
-    flt::lr_box(&lb, in, set, 0, flt0);
-    flt::lr_box(&lb, in, set, 1, flt1);
-    for (int i = 0; i < lb.h; i++)
-      for (int j = 0; j < lb.w; j++) {
-        long long u = (long long)in.own(lb.x + j, lb.y + i) << SGRPROJ_RST_BITS;
-        long long s = ((long long)in.src(lb.x + j, lb.y + i) << SGRPROJ_RST_BITS) - u;
-        long long f0 = r0 ? flt0[i * 4 + j] - u : 0, f1 = r1 ? flt1[i * 4 + j] - u : 0;
-        h00 += f0 * f0;
-        h01 += f0 * f1;
-        h11 += f1 * f1;
-        c0 += f0 * s;
-        c1 += f1 * s;
+// ---- self-guided sets ------------------------------------------------------------------
+// flt::lr_box over a whole unit. A position's box sums do not depend on the
+// set, so p = n * sum(c^2) - sum(c)^2 and sum(c) of the 5x5 and 3x3 boxes are
+// formed once per unit (p1 / b1: 3x3, rows -1 .. rows of each stripe; p2 / b2:
+// 5x5, which only odd rows need); a set turns them into (a2, b2) per position,
+// and a sample combines its neighbours'. All in 32 bits: a2 <= 256, b2 <=
+// 65,088 (255 * 6375 * 164 >> 12), so a sample's sums stay below 2^23.
+__device__ void sgr_boxes(const Layout &l, uint8_t *smem, Shared &sh) {
+  const Area &a = sh.area;
+  const int W2 = a.w + 2;
+  uint32_t *p1 = (uint32_t *)(smem + l.p1), *p2 = (uint32_t *)(smem + l.p2);
+  uint16_t *b1 = (uint16_t *)(smem + l.b1), *b2 = (uint16_t *)(smem + l.b2);
+  for (int k = threadIdx.x; k < (a.h + 2 * a.nseg) * W2; k += THREADS) {
+    int r = quotient(k, a.inv_w2), c = k - r * W2, s = 0;
+    while (s + 1 < a.nseg && r >= a.seg[s + 1] + 2 * (s + 1)) s++;
+    int i = r - 2 * s - a.seg[s] - 1;  // row of the stripe, -1 .. rows
+    // the position is tap row (stripe base + i + 3), tap column c + 2
+    const uint8_t *t = smem + l.tap + (a.seg[s] + 6 * s + i + 3) * l.tap_p + c + 2;
+    int q = 0, m = 0;
+    for (int dy = -1; dy <= 1; dy++)
+      for (int dx = -1; dx <= 1; dx++) {
+        int v = t[dy * l.tap_p + dx];
+        q += v * v;
+        m += v;
       }
-  }
-  double H00 = (double)cta_sum(h00, sh), H01 = (double)cta_sum(h01, sh), H11 = (double)cta_sum(h11, sh);
-  double C0 = (double)cta_sum(c0, sh), C1 = (double)cta_sum(c1, sh);
-  double a = 0.0, bb = 0.0;
-  if (r0 && r1) {
-    double det = dsub(dmul(H00, H11), dmul(H01, H01));
-    if (fabs(det) > 1e-9) {
-      a = ddiv(dsub(dmul(C0, H11), dmul(C1, H01)), det);
-      bb = ddiv(dsub(dmul(C1, H00), dmul(C0, H01)), det);
+    p1[k] = (uint32_t)(q * 9 - m * m);
+    b1[k] = (uint16_t)m;
+    if (i & 1) {
+      for (int dy = -2; dy <= 2; dy++)
+        for (int dx = -2; dx <= 2; dx++) {
+          if (dy >= -1 && dy <= 1 && dx >= -1 && dx <= 1) continue;
+          int v = t[dy * l.tap_p + dx];
+          q += v * v;
+          m += v;
+        }
+      int k2 = (a.seg[s] / 2 + 2 * s + ((i + 1) >> 1)) * W2 + c;
+      p2[k2] = (uint32_t)(q * 25 - m * m);
+      b2[k2] = (uint16_t)m;
     }
-  } else if (r0) {
-    if (H00 > 0) a = ddiv(C0, H00);
-  } else if (r1) {
-    if (H11 > 0) bb = ddiv(C1, H11);
   }
-  int w0 = (int)lround_away(dmul(a, (double)(1 << SGRPROJ_PRJ_BITS)));
-  int w2 = (int)lround_away(dmul(bb, (double)(1 << SGRPROJ_PRJ_BITS)));
-  if (!r0) w0 = 0;
-  xqd[0] = imax(T(Sgrproj_Xqd_Min)[0], imin(T(Sgrproj_Xqd_Max)[0], w0));
-  if (!r1)
-    xqd[1] = imax(T(Sgrproj_Xqd_Min)[1], imin(T(Sgrproj_Xqd_Max)[1], (1 << SGRPROJ_PRJ_BITS) - xqd[0]));
-  else
-    xqd[1] = imax(T(Sgrproj_Xqd_Min)[1], imin(T(Sgrproj_Xqd_Max)[1], (1 << SGRPROJ_PRJ_BITS) - xqd[0] - w2));
+  for (int z = threadIdx.x; z < 256; z += THREADS)
+    sh.atab[z] = (uint16_t)(z == 0 ? 1 : z == 255 ? 256 : ((z << SGRPROJ_SGR_BITS) + (z / 2)) / (z + 1));
+  __syncthreads();
+}
+
+// (a2, b2) of positions 0 .. n - 1 of one box size.
+__device__ __forceinline__ void sgr_ab(const uint32_t *p, const uint16_t *b, uint32_t *ab, int n, int boxN, int eps,
+                                       const uint16_t *atab) {
+  const int n2e = boxN * boxN * eps;
+  const unsigned s = ((1 << SGRPROJ_MTABLE_BITS) + n2e / 2) / n2e;
+  const unsigned oneOverN = ((1 << SGRPROJ_RECIP_BITS) + (boxN / 2)) / boxN;
+  for (int k = threadIdx.x; k < n; k += THREADS) {
+    unsigned long long z = ((unsigned long long)p[k] * s + (1u << (SGRPROJ_MTABLE_BITS - 1))) >> SGRPROJ_MTABLE_BITS;
+    unsigned a2 = atab[z > 255 ? 255 : (unsigned)z];
+    unsigned b2 = ((1u << SGRPROJ_SGR_BITS) - a2) * b[k] * oneOverN;
+    ab[k] = a2 | ((b2 + (1u << (SGRPROJ_RECIP_BITS - 1))) >> SGRPROJ_RECIP_BITS) << 16;
+  }
+}
+
+// sgr_fit (lr_search.c:196-240) and the SSE of the fitted set, for sets s0 ..
+// s1 - 1. The fit's sums are whole numbers and exact in 64 bits; the closing
+// double arithmetic follows the reference's operations. With weights w0, w2
+// and w1 = 128 - w0 - w2 the projection w1 u + w0 F0 + w2 F1 is 128 u +
+// w0 (F0 - u) + w2 (F1 - u): the differences the fit forms are kept (fd) and
+// give the SSE without filtering again.
+__device__ void sgr_sets(const Layout &l, uint8_t *smem, int s0, int s1, Fit &F, Shared &sh) {
+  const Area &a = sh.area;
+  const int W2 = a.w + 2, n1 = (a.h + 2 * a.nseg) * W2, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t *p1 = (const uint32_t *)(smem + l.p1), *p2 = (const uint32_t *)(smem + l.p2);
+  const uint16_t *b1 = (const uint16_t *)(smem + l.b1), *b2 = (const uint16_t *)(smem + l.b2);
+  uint32_t *ab1 = (uint32_t *)(smem + l.ab1), *ab2 = (uint32_t *)(smem + l.ab2), *fd = (uint32_t *)(smem + l.fd);
+  sgr_boxes(l, smem, sh);
+  const int n2 = a.nseg ? (a.seg[a.nseg - 1] / 2 + 2 * (a.nseg - 1) + (a.h - a.seg[a.nseg - 1] + 1) / 2 + 1) * W2 : 0;
+  for (int set = s0; set < s1; set++) {
+    const int r0 = T(Sgr_Params)[set][0], r1 = T(Sgr_Params)[set][2];
+    // the first filter's box is 5x5 and the second's 3x3 in every set that has them
+    if (r0) sgr_ab(p2, b2, ab2, n2, 25, T(Sgr_Params)[set][1], sh.atab);
+    if (r1) sgr_ab(p1, b1, ab1, n1, 9, T(Sgr_Params)[set][3], sh.atab);
+    __syncthreads();
+    int h00 = 0, h01 = 0, h11 = 0, c0 = 0, c1 = 0;
+    for (int k = tid; k < a.h * a.w; k += THREADS) {
+      int r = quotient(k, a.inv_w), x = k - r * a.w, s = seg_of(a, r), i = r - a.seg[s];
+      int own = smem[l.tap + (r + 6 * s + 3) * l.tap_p + x + 3];
+      int u = own << SGRPROJ_RST_BITS, sd = ((int)smem[l.src + r * l.src_p + x] << SGRPROJ_RST_BITS) - u;
+      int d0 = 0, d1 = 0;
+      if (r0) {
+        // odd rows carry the sums: an odd row uses its own, an even row the two around it
+        const uint32_t *q = ab2 + (a.seg[s] / 2 + 2 * s + ((i + 1) >> 1)) * W2 + x;
+        unsigned l0 = q[0], m0 = q[1], e0 = q[2];
+        unsigned A = 6 * (m0 & 0xffff) + 5 * ((l0 & 0xffff) + (e0 & 0xffff)), B = 6 * (m0 >> 16) + 5 * ((l0 >> 16) + (e0 >> 16));
+        int sh0 = SGRPROJ_SGR_BITS + 4 - SGRPROJ_RST_BITS;
+        if (!(i & 1)) {
+          unsigned l1 = q[W2], m1 = q[W2 + 1], e1 = q[W2 + 2];
+          A += 6 * (m1 & 0xffff) + 5 * ((l1 & 0xffff) + (e1 & 0xffff));
+          B += 6 * (m1 >> 16) + 5 * ((l1 >> 16) + (e1 >> 16));
+          sh0++;
+        }
+        d0 = (int)((A * own + B + (1u << (sh0 - 1))) >> sh0) - u;
+      }
+      if (r1) {
+        const uint32_t *q = ab1 + (r + 2 * s) * W2 + x;
+        unsigned A = 0, B = 0;
+#pragma unroll
+        for (int dy = 0; dy < 3; dy++)
+#pragma unroll
+          for (int dx = 0; dx < 3; dx++) {
+            unsigned v = q[dy * W2 + dx], wgt = dy == 1 || dx == 1 ? 4 : 3;
+            A += wgt * (v & 0xffff);
+            B += wgt * (v >> 16);
+          }
+        constexpr int sh1 = SGRPROJ_SGR_BITS + 5 - SGRPROJ_RST_BITS;
+        d1 = (int)((A * own + B + (1u << (sh1 - 1))) >> sh1) - u;
+      }
+      fd[k] = (uint32_t)(d0 & 0xffff) | (uint32_t)d1 << 16;
+      h00 += d0 * d0;
+      h01 += d0 * d1;
+      h11 += d1 * d1;
+      c0 += d0 * sd;
+      c1 += d1 * sd;
+    }
+    const int par = set & 1;
+    {
+      long long v0 = warp_sum(h00), v1 = warp_sum(h01), v2 = warp_sum(h11), v3 = warp_sum(c0), v4 = warp_sum(c1);
+      if (lane == 0) {
+        long long *o = sh.red[par][warp];
+        o[0] = v0; o[1] = v1; o[2] = v2; o[3] = v3; o[4] = v4;
+      }
+    }
+    __syncthreads();
+    long long sum[5] = {0, 0, 0, 0, 0};
+    for (int w = 0; w < WARPS; w++)
+      for (int k = 0; k < 5; k++) sum[k] += sh.red[par][w][k];
+    double H00 = (double)sum[0], H01 = (double)sum[1], H11 = (double)sum[2], C0 = (double)sum[3], C1 = (double)sum[4];
+    double fa = 0.0, fb = 0.0;
+    if (r0 && r1) {
+      double det = dsub(dmul(H00, H11), dmul(H01, H01));
+      if (fabs(det) > 1e-9) {
+        fa = ddiv(dsub(dmul(C0, H11), dmul(C1, H01)), det);
+        fb = ddiv(dsub(dmul(C1, H00), dmul(C0, H01)), det);
+      }
+    } else if (r0) {
+      if (H00 > 0) fa = ddiv(C0, H00);
+    } else if (r1) {
+      if (H11 > 0) fb = ddiv(C1, H11);
+    }
+    int w0 = (int)lround_away(dmul(fa, (double)(1 << SGRPROJ_PRJ_BITS)));
+    int w2 = (int)lround_away(dmul(fb, (double)(1 << SGRPROJ_PRJ_BITS)));
+    if (!r0) w0 = 0;
+    const int x0 = imax(T(Sgrproj_Xqd_Min)[0], imin(T(Sgrproj_Xqd_Max)[0], w0));
+    const int x1 = imax(T(Sgrproj_Xqd_Min)[1],
+                        imin(T(Sgrproj_Xqd_Max)[1], (1 << SGRPROJ_PRJ_BITS) - x0 - (r1 ? w2 : 0)));
+    const int x2 = (1 << SGRPROJ_PRJ_BITS) - x0 - x1;
+    int e = 0;
+    for (int k = tid; k < a.h * a.w; k += THREADS) {
+      int r = quotient(k, a.inv_w), x = k - r * a.w, s = seg_of(a, r);
+      int u = (int)smem[l.tap + (r + 6 * s + 3) * l.tap_p + x + 3] << SGRPROJ_RST_BITS;
+      int d0 = (int)(int16_t)(fd[k] & 0xffff), d1 = (int)fd[k] >> 16;
+      int v = (u << SGRPROJ_PRJ_BITS) + x0 * d0 + x2 * d1;
+      int d = clip3(0, 255, round2(v, SGRPROJ_RST_BITS + SGRPROJ_PRJ_BITS)) - (int)smem[l.src + r * l.src_p + x];
+      e += d * d;
+    }
+    long long ew = warp_sum(e);
+    if (lane == 0) sh.red[par][warp][5] = ew;
+    if (tid == 0) {
+      F.xqd[set][0] = x0;
+      F.xqd[set][1] = x1;
+    }
+    // the next set's barriers order these parts; the one after it writes this
+    // buffer again only after this set's SSE has been read
+    __syncthreads();
+    if (tid == 0) {
+      long long t = 0;
+      for (int w = 0; w < WARPS; w++) t += sh.red[par][w][5];
+      F.sgr_sse[set] = t;
+    }
+  }
 }
 
 HD void taps_of(const LrUnit &u, int *t) {
@@ -476,29 +758,49 @@ HD void taps_of(const LrUnit &u, int *t) {
     for (int j = 0; j < 3; j++) t[p * 3 + j] = u.wiener[p][j];
 }
 
-// First pass: one CTA per unit (all planes; the unit's index in LRUNITS).
-__global__ void __launch_bounds__(THREADS) k_lr_fit(const FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
-                                                   const uint8_t *src, Fit *fits) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
-  const int gu = blockIdx.x;
-  int plane = 2;
-  while (plane > 0 && gu < fp->lr_unit_off[plane]) plane--;
-  const int u = gu - fp->lr_unit_off[plane];
-  if (threadIdx.x == 0) unit_geom(fp, plane, u / fp->lr_unit_cols[plane], u % fp->lr_unit_cols[plane], &sh.geom);
+// The unit `gu` of LRUNITS: its plane, place and area, staged (the whole CTA).
+__device__ void load_unit(const FrameParams *fp, int gu, const uint8_t *cdef, const uint8_t *dbk, const uint8_t *src,
+                          const Layout &l, uint8_t *smem, Shared &sh) {
+  if (threadIdx.x == 0) {
+    int plane = 2;
+    while (plane > 0 && gu < fp->lr_unit_off[plane]) plane--;
+    const int u = gu - fp->lr_unit_off[plane];
+    unit_geom(fp, plane, u / fp->lr_unit_cols[plane], u % fp->lr_unit_cols[plane], &sh.geom);
+    unit_area(fp, sh.geom, &sh.area);
+  }
   __syncthreads();
-  const Geom g = sh.geom;
-  stage_window(fp, g, cdef, dbk, src, sh.win);
+  stage_unit(fp, sh.area, cdef, dbk, src, l, smem);
+}
+
+// First pass, all planes at once: CTA (unit, part). Part 0 fits the Wiener
+// filter and takes its SSEs (latency: the fit's ordered sums), parts 1 and 2
+// take half of the self-guided sets each, so a small frame's units spread over
+// three times the SMs. With one CTA per unit, a 4x4 block a thread and every
+// block's taps clamped and box sums formed anew, the pass took 7.06 ms for a
+// 1280x720 frame's units and 42.8 ms at 3840x2160; this form takes 0.81 and
+// 3.97 ms.
+constexpr int FIT_PARTS = 3;
+__global__ void __launch_bounds__(THREADS, 2) k_lr_fit(const FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
+                                                      const uint8_t *src, Fit *fits, Dims dims) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ Shared sh;
+  const Layout l = layout_of(dims);
+  const int gu = blockIdx.x / FIT_PARTS, part = blockIdx.x % FIT_PARTS;
+  load_unit(fp, gu, cdef, dbk, src, l, smem, sh);
   Fit &F = fits[gu];
-  LrUnit none = {};
-  none.type = RESTORE_NONE;
-  long long sseNone = unit_sse(fp, g, none, sh);
+  if (part > 0) {
+    sgr_sets(l, smem, part == 1 ? 0 : 8, part == 1 ? 8 : 16, F, sh);
+    return;
+  }
+  const int plane = sh.area.plane;
+  long long sseNone = none_sse(l, smem, sh);
   int w[2][3];
-  wiener_fit(fp, g, sh, w);
+  wiener_fit(l, smem, sh, w);
   // the fitted filter and its single-tap neighbours, in the refinement's order
-  int n = 0;
+  int n = 0, tt[6];
   LrUnit base = wiener_unit(w);
-  long long sseW = unit_sse(fp, g, base, sh);
+  taps_of(base, tt);
+  long long sseW = wiener_unit_sse(l, smem, tt, sh);
   if (threadIdx.x == 0) {
     taps_of(base, F.taps[n]);
     F.sse[n] = sseW;
@@ -510,28 +812,14 @@ __global__ void __launch_bounds__(THREADS) k_lr_fit(const FrameParams *fp, const
         LrUnit t = base;
         t.wiener[pass][j] += d;
         if (t.wiener[pass][j] < T(Wiener_Taps_Min)[j] || t.wiener[pass][j] > T(Wiener_Taps_Max)[j]) continue;
-        long long sse = unit_sse(fp, g, t, sh);
+        taps_of(t, tt);
+        long long sse = wiener_unit_sse(l, smem, tt, sh);
         if (threadIdx.x == 0) {
           taps_of(t, F.taps[n]);
           F.sse[n] = sse;
         }
         n++;
       }
-  for (int set = 0; set < 16; set++) {
-    int xqd[2];
-    sgr_fit(fp, g, set, sh, xqd);
-    LrUnit s = {};
-    s.type = RESTORE_SGRPROJ;
-    s.set = set;
-    s.xqd[0] = xqd[0];
-    s.xqd[1] = xqd[1];
-    long long sse = unit_sse(fp, g, s, sh);
-    if (threadIdx.x == 0) {
-      F.xqd[set][0] = xqd[0];
-      F.xqd[set][1] = xqd[1];
-      F.sgr_sse[set] = sse;
-    }
-  }
   if (threadIdx.x == 0) {
     F.sse_none = sseNone;
     F.n = n;
@@ -540,9 +828,6 @@ __global__ void __launch_bounds__(THREADS) k_lr_fit(const FrameParams *fp, const
   }
 }
 
-// SSE of Wiener candidate t: the first pass's value when it has one, else
-// computed by the whole CTA from the unit's window, staged at the first such
-// candidate of the unit (every thread calls this with the same t).
 // Index of the cache entry holding taps tt (entries are distinct), or -1:
 // thread i compares entry i (the whole CTA).
 __device__ int cache_find(const int (*taps)[6], int n, const int *tt, Shared &sh) {
@@ -560,22 +845,6 @@ __device__ int cache_find(const int (*taps)[6], int n, const int *tt, Shared &sh
   return f;
 }
 
-__device__ long long wiener_sse(const FrameParams *fp, const Fit &F, const Geom &g, const uint8_t *cdef,
-                                const uint8_t *dbk, const uint8_t *src, const LrUnit &t, Shared &sh, bool &staged) {
-  int tt[6];
-  taps_of(t, tt);
-  int f = cache_find(F.taps, F.n, tt, sh);
-  if (f >= 0) return F.sse[f];
-  if (!staged) {
-    stage_window(fp, g, cdef, dbk, src, sh.win);
-    staged = true;
-  }
-  return unit_sse(fp, g, t, sh);
-}
-
-// Second pass: one CTA per plane, the units in order (lr_select's loop,
-// lr_search.c:276-355). Every thread runs the same scalar decisions; the SSE
-// of a candidate the first pass did not compute is evaluated by all of them.
 // Speculative refinement, one CTA per unit, after k_lr_fit: the Wiener
 // refinement of lr_select (lr_search.c:296-318) replayed for the unit under
 // guessed running references, computing and caching the SSE of every
@@ -587,8 +856,8 @@ __device__ long long wiener_sse(const FrameParams *fp, const Fit &F, const Geom 
 // of the two previous units (the true reference is usually the refined
 // filter of a recent unit). k_lr_select then finds most of its candidates
 // here and computes only the rest on the spot.
-__device__ void spec_path(const FrameParams *fp, int plane, const Geom &g, const uint8_t *cdef, const uint8_t *dbk,
-                          const uint8_t *src, const int fitted[2][3], const int ref[2][3], Shared &sh, bool &staged) {
+__device__ void spec_path(const FrameParams *fp, int plane, const Layout &l, const uint8_t *smem, const int fitted[2][3],
+                          const int ref[2][3], Shared &sh) {
   LrUnit w = wiener_unit(fitted);
   int tw[2][3], tx[2] = {0, 0};
   memcpy(tw, ref, sizeof tw);
@@ -606,11 +875,7 @@ __device__ void spec_path(const FrameParams *fp, int plane, const Geom &g, const
         long long sse = f >= 0 ? sh.csse[f] : -1;
         if (sse < 0) {
           if (n >= CACHE) return;  // full: the serial choice computes the rest
-          if (!staged) {
-            stage_window(fp, g, cdef, dbk, src, sh.win);
-            staged = true;
-          }
-          sse = unit_sse(fp, g, t, sh);  // the whole CTA; every thread gets the sum
+          sse = wiener_unit_sse(l, smem, tt, sh);  // the whole CTA; every thread gets the sum
           if (threadIdx.x == 0) {
             for (int k = 0; k < 6; k++) sh.ctaps[n][k] = tt[k];
             sh.csse[n] = sse;
@@ -628,31 +893,25 @@ __device__ void spec_path(const FrameParams *fp, int plane, const Geom &g, const
 }
 
 __global__ void __launch_bounds__(THREADS) k_lr_spec(const FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
-                                                    const uint8_t *src, Fit *fits) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
+                                                    const uint8_t *src, Fit *fits, Dims dims) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ Shared sh;
+  const Layout l = layout_of(dims);
   const int gu = blockIdx.x;
-  int plane = 2;
-  while (plane > 0 && gu < fp->lr_unit_off[plane]) plane--;
-  const int u = gu - fp->lr_unit_off[plane];
   Fit &F = fits[gu];
-  if (threadIdx.x == 0) {
-    unit_geom(fp, plane, u / fp->lr_unit_cols[plane], u % fp->lr_unit_cols[plane], &sh.geom);
-    sh.cn = F.n;
-  }
+  if (threadIdx.x == 0) sh.cn = F.n;
   for (int i = threadIdx.x; i < F.n * 6; i += THREADS) sh.ctaps[i / 6][i % 6] = F.taps[i / 6][i % 6];
   for (int i = threadIdx.x; i < F.n; i += THREADS) sh.csse[i] = F.sse[i];
-  __syncthreads();
-  const Geom g = sh.geom;
+  load_unit(fp, gu, cdef, dbk, src, l, smem, sh);
+  const int plane = sh.area.plane, u = gu - fp->lr_unit_off[plane];
   const int n0 = sh.cn;
   int fitted[2][3], ref[2][3];
   for (int pass = 0; pass < 2; pass++)
     for (int j = 0; j < 3; j++) fitted[pass][j] = F.w[pass][j];
-  bool staged = false;
   for (int q = 0; q < 3 && q <= u; q++) {
     for (int pass = 0; pass < 2; pass++)
       for (int j = 0; j < 3; j++) ref[pass][j] = q == 0 ? T(Wiener_Taps_Mid)[j] : fits[gu - q].w[pass][j];
-    spec_path(fp, plane, g, cdef, dbk, src, fitted, ref, sh, staged);
+    spec_path(fp, plane, l, smem, fitted, ref, sh);
   }
   __syncthreads();
   const int n1 = sh.cn;
@@ -661,97 +920,179 @@ __global__ void __launch_bounds__(THREADS) k_lr_spec(const FrameParams *fp, cons
   if (threadIdx.x == 0) F.n = n1;
 }
 
+// ---- the serial choice -------------------------------------------------------------------
+// One CTA per plane: warp 0 scans the units in order (lr_select's loop,
+// lr_search.c:276-355), the other warps wait for a candidate that neither
+// pass cached and filter the unit with it together. What depends on the
+// previous unit, the rates, is spread over the lanes: a filter's rate is the
+// sum of its taps' (unit_bits), the refinement moves one tap at a time and a
+// tap by at most one, so 18 lanes code each tap's three values once and a
+// candidate's rate is its predecessor's with one term exchanged; 16 lanes code
+// the self-guided sets. A candidate is 6 two-bit steps from the fitted filter:
+// lanes compare the cached candidates' codes at once. The next unit's record
+// is in flight meanwhile. (One thread's scan of all of it, the CTA looking the
+// cache up between barriers, took 33 us per luma unit; this scan takes 3.9 us:
+7.9 instead of 68.8 ms at 3840x2160.)
+constexpr int FIT_WORDS = (int)(sizeof(Fit) / 4), FIT_LANE = (FIT_WORDS + 31) / 32;
+static_assert(sizeof(Fit) % 4 == 0 && CACHE <= 64, "two cached candidates a lane");
+
+__device__ __forceinline__ void cta_bar() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+
+// The SSE of the missing candidate (every warp; wiener_unit_sse's barriers are
+// the CTA's).
+__device__ __noinline__ long long missing_sse(const FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
+                                              const uint8_t *src, const Layout &l, uint8_t *smem, Shared &sh) {
+  load_unit(fp, sh.miss_unit, cdef, dbk, src, l, smem, sh);
+  int tt[6];
+  for (int k = 0; k < 6; k++) tt[k] = sh.miss_taps[k];
+  return wiener_unit_sse(l, smem, tt, sh);
+}
+
 __global__ void __launch_bounds__(THREADS) k_lr_select(FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
                                                       const uint8_t *src, const Fit *fits, LrUnit *units,
-                                                      int lrTest, int *lrTypes) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
-  const int plane = blockIdx.x;
+                                                      int lrTest, int *lrTypes, Dims dims) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ Shared sh;
+  const Layout l = layout_of(dims);
+  const int plane = blockIdx.x, lane = threadIdx.x & 31;
   const int nUnits = fp->lr_unit_rows[plane] * fp->lr_unit_cols[plane], off = fp->lr_unit_off[plane];
-  int refW[2][3], refX[2];
-  for (int pass = 0; pass < 2; pass++) {
-    refX[pass] = T(Sgrproj_Xqd_Mid)[pass];
-    for (int j = 0; j < 3; j++) refW[pass][j] = T(Wiener_Taps_Mid)[j];
-  }
-  int used = 0;
-  for (int u = 0; u < nUnits; u++) {
-    __syncthreads();  // every thread is done with the previous unit's copy
-    {  // the unit's first-pass results into shared memory (the rate scan reads them many times)
-      const int *fs = reinterpret_cast<const int *>(fits + off + u);
-      int *fd = reinterpret_cast<int *>(&sh.fit);
-      for (int k = threadIdx.x; k < (int)(sizeof(Fit) / 4); k += THREADS) fd[k] = fs[k];
+  if (threadIdx.x >= 32) {
+    for (;;) {
+      cta_bar();
+      if (sh.miss_unit < 0) return;
+      missing_sse(fp, cdef, dbk, src, l, smem, sh);
+      cta_bar();
     }
+  }
+  const int first = plane ? 1 : 0;
+  const long long lambda = fp->lambda;
+  // lane 3 c + d + 1, c = 3 pass + j: tap c moved by d
+  const int myC = imin(lane / 3, 5), myJ = myC % 3, myD = lane % 3 - 1, myTap = lane < 18 && myJ >= first;
+  const int tapMin = T(Wiener_Taps_Min)[myJ], tapMax = T(Wiener_Taps_Max)[myJ], tapK = T(Wiener_Taps_K)[myJ];
+  int refW = T(Wiener_Taps_Mid)[lane % 3];                    // lane c < 6: running reference of tap c
+  int refX0 = T(Sgrproj_Xqd_Mid)[0], refX1 = T(Sgrproj_Xqd_Mid)[1];  // every lane
+  const int set = lane & 15, setR0 = T(Sgr_Params)[set][0], setR1 = T(Sgr_Params)[set][2];
+  int used = 0;
+  int nxt[FIT_LANE];
+  auto fetch = [&](int u) {
+#pragma unroll
+    for (int k = 0; k < FIT_LANE; k++)
+      if (k * 32 + lane < FIT_WORDS) nxt[k] = ((const int *)(fits + off + u))[k * 32 + lane];
+  };
+  if (nUnits > 0) fetch(0);
+  for (int u = 0; u < nUnits; u++) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < FIT_LANE; k++)
+      if (k * 32 + lane < FIT_WORDS) ((int *)&sh.fit)[k * 32 + lane] = nxt[k];
+    __syncwarp();
+    if (u + 1 < nUnits) fetch(u + 1);
     const Fit &F = sh.fit;
-    Geom g;
-    if (threadIdx.x == 0) unit_geom(fp, plane, u / fp->lr_unit_cols[plane], u % fp->lr_unit_cols[plane], &sh.geom);
-    __syncthreads();
-    g = sh.geom;
-    __syncthreads();
-    LrUnit best = {};
-    best.type = RESTORE_NONE;
-    long long bestCost = rd(fp, F.sse_none, 1);
-    int tw[2][3], tx[2];
-    LrUnit w = wiener_unit(F.w);
-    bool staged = false;
-    memcpy(tw, refW, sizeof tw);
-    memcpy(tx, refX, sizeof tx);
-    long long wc = rd(fp, F.sse[0], 2 + unit_bits(plane, w, tw, tx));
-    for (int pass = 0; pass < 2; pass++)
-      for (int j = plane ? 1 : 0; j < 3; j++)
-        for (int d = -1; d <= 1; d += 2) {
-          LrUnit t = w;
-          t.wiener[pass][j] += d;
-          if (t.wiener[pass][j] < T(Wiener_Taps_Min)[j] || t.wiener[pass][j] > T(Wiener_Taps_Max)[j]) continue;
-          memcpy(tw, refW, sizeof tw);
-          memcpy(tx, refX, sizeof tx);
-          long long tc = rd(fp, wiener_sse(fp, F, g, cdef, dbk, src, t, sh, staged), 2 + unit_bits(plane, t, tw, tx));
-          if (tc < wc) {
-            wc = tc;
-            w = t;
+    const int *fw = &F.w[0][0];
+    // rates of the taps' values (a value out of range is never a candidate)
+    int ref = __shfl_sync(0xffffffffu, refW, myC), v = fw[myC] + myD, tb = 0;
+    bool ok = myTap && v >= tapMin && v <= tapMax;
+    if (ok) tb = subexp_bits(tapMin, tapMax + 1, tapK, ref, v);
+    const unsigned okMask = __ballot_sync(0xffffffffu, ok);
+    // rate of this lane's self-guided set
+    int sb = 2 + 4;
+    if (setR0) sb += subexp_bits(T(Sgrproj_Xqd_Min)[0], T(Sgrproj_Xqd_Max)[0] + 1, 4, refX0, F.xqd[set][0]);
+    if (setR1) sb += subexp_bits(T(Sgrproj_Xqd_Min)[1], T(Sgrproj_Xqd_Max)[1] + 1, 4, refX1, F.xqd[set][1]);
+    // this lane's cached candidates as steps from the fitted filter: (d + 1) << 2 c
+    unsigned code[2];
+    long long csse[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      int i = lane + 32 * q;
+      code[q] = ~0u;
+      csse[q] = 0;
+      if (i < F.n) {
+        unsigned cd = 0;
+        for (int c = 0; c < 6; c++) cd |= (unsigned)((F.taps[i][c] - fw[c] + 1) & 3) << (2 * c);
+        code[q] = cd;
+        csse[q] = F.sse[i];
+      }
+    }
+    // the refinement (lr_search.c:296-318)
+    int bits = 2;
+    for (int c = 0; c < 6; c++)
+      if (c % 3 >= first) bits += __shfl_sync(0xffffffffu, tb, 3 * c + 1);
+    unsigned cur = 0x555;
+    long long wc = F.sse[0] * 16 + lambda * bits;
+    for (int c = 0; c < 6; c++) {
+      if (c % 3 < first) continue;
+      for (int d = -1; d <= 1; d += 2) {
+        int at = (int)(cur >> (2 * c)) & 3, to = at + d;  // d + 1 of the tap now and moved
+        if (!((okMask >> (3 * c + to)) & 1)) continue;
+        unsigned want = (cur & ~(3u << (2 * c))) | (unsigned)to << (2 * c);
+        int tbits = bits - __shfl_sync(0xffffffffu, tb, 3 * c + at) + __shfl_sync(0xffffffffu, tb, 3 * c + to);
+        unsigned m0 = __ballot_sync(0xffffffffu, code[0] == want), m1 = __ballot_sync(0xffffffffu, code[1] == want);
+        long long sse;
+        if (m0) sse = __shfl_sync(0xffffffffu, csse[0], __ffs(m0) - 1);
+        else if (m1) sse = __shfl_sync(0xffffffffu, csse[1], __ffs(m1) - 1);
+        else {
+          if (lane == 0) {
+            sh.miss_unit = off + u;
+            for (int k = 0; k < 6; k++) sh.miss_taps[k] = fw[k] + ((int)(want >> (2 * k)) & 3) - 1;
           }
+          __syncwarp();
+          cta_bar();
+          sse = missing_sse(fp, cdef, dbk, src, l, smem, sh);
+          cta_bar();
         }
+        long long tc = sse * 16 + lambda * tbits;
+        if (tc < wc) {
+          wc = tc;
+          cur = want;
+          bits = tbits;
+        }
+      }
+    }
+    int type = RESTORE_NONE, bestSet = 0;
+    long long bestCost = rd(fp, F.sse_none, 1);
     if (wc < bestCost) {
       bestCost = wc;
-      best = w;
+      type = RESTORE_WIENER;
     }
-    for (int set = 0; set < 16; set++) {
-      LrUnit s = {};
-      s.type = RESTORE_SGRPROJ;
-      s.set = set;
-      s.xqd[0] = F.xqd[set][0];
-      s.xqd[1] = F.xqd[set][1];
-      memcpy(tw, refW, sizeof tw);
-      memcpy(tx, refX, sizeof tx);
-      long long sc = rd(fp, F.sgr_sse[set], 2 + unit_bits(plane, s, tw, tx));
-      if (sc < bestCost) {
-        bestCost = sc;
-        best = s;
+    // first least of the sets' costs (with lrTest: of their SSEs)
+    const bool testSgr = lrTest && (u & 1);
+    long long sc = testSgr ? F.sgr_sse[set] : F.sgr_sse[set] * 16 + lambda * sb;
+    int si = set;
+    for (int o = 8; o; o >>= 1) {
+      long long oc = __shfl_xor_sync(0xffffffffu, sc, o);
+      int oi = __shfl_xor_sync(0xffffffffu, si, o);
+      if (oc < sc || (oc == sc && oi < si)) {
+        sc = oc;
+        si = oi;
       }
     }
-    if (lrTest) {
-      // Wiener on even units, the self-guided set of least SSE on odd ones
-      if (!(u & 1)) {
-        best = w;
-      } else {
-        long long bs = -1;
-        for (int set = 0; set < 16; set++) {
-          long long v = F.sgr_sse[set];
-          if (bs < 0 || v < bs) {
-            bs = v;
-            best = LrUnit{};
-            best.type = RESTORE_SGRPROJ;
-            best.set = set;
-            best.xqd[0] = F.xqd[set][0];
-            best.xqd[1] = F.xqd[set][1];
-          }
-        }
-      }
+    if (testSgr || sc < bestCost) {
+      type = RESTORE_SGRPROJ;
+      bestSet = si;
     }
-    unit_bits(plane, best, refW, refX);
-    if (threadIdx.x == 0) units[off + u] = best;
-    used |= best.type != RESTORE_NONE;
+    if (lrTest && !(u & 1)) type = RESTORE_WIENER;  // Wiener on even units, the least SSE's set on odd ones
+    // the unit's record (type, set, xqd[2], wiener[2][3], pad[2]), and the references it leaves
+    const int tapv = lane < 6 ? fw[lane] + ((int)(cur >> (2 * lane)) & 3) - 1 : 0;  // tap `lane` of the refined filter
+    const int wv = __shfl_sync(0xffffffffu, tapv, lane >= 4 && lane < 10 ? lane - 4 : 0);
+    int o = 0;
+    if (lane == 0) o = type;
+    else if (type == RESTORE_SGRPROJ) o = lane == 1 ? bestSet : lane == 2 ? F.xqd[bestSet][0] : lane == 3 ? F.xqd[bestSet][1] : 0;
+    else if (type == RESTORE_WIENER && lane >= 4 && lane < 10) o = wv;
+    if (lane < (int)(sizeof(LrUnit) / 4)) ((int *)(units + off + u))[lane] = o;
+    if (type == RESTORE_WIENER) {
+      if (lane < 6 && lane % 3 >= first) refW = tapv;
+    } else if (type == RESTORE_SGRPROJ) {
+      refX0 = F.xqd[bestSet][0];
+      refX1 = F.xqd[bestSet][1];
+    }
+    used |= type != RESTORE_NONE;
   }
-  if (threadIdx.x == 0) fp->lr_type[plane] = lrTypes[plane] = used ? RESTORE_SWITCHABLE : RESTORE_NONE;
+  if (lane == 0) {
+    sh.miss_unit = -1;
+    fp->lr_type[plane] = lrTypes[plane] = used ? RESTORE_SWITCHABLE : RESTORE_NONE;
+  }
+  __syncwarp();
+  cta_bar();
 }
 
 }  // namespace lrs

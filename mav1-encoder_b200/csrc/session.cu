@@ -429,9 +429,10 @@ extern "C" int mav1cu_session_create(int width, int height, int max_cdef_presets
     s->resident_recon = imax(1, sms * imin(1, imax(1, per)));
   }
   cudaFuncSetAttribute(ana::k_analyze_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANA_SMEM(16));
-  cudaFuncSetAttribute(lrs::k_lr_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(lrs::Shared));
-  cudaFuncSetAttribute(lrs::k_lr_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(lrs::Shared));
-  cudaFuncSetAttribute(lrs::k_lr_spec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(lrs::Shared));
+  {
+    lrs::Layout l = lrs::layout_of(lrs::MAX_DIMS);
+    cudaFuncSetAttribute(lrs::k_lr_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, lrs::smem_fit(l));
+  }
   *out = s;
   return MAV1CU_OK;
 }
@@ -782,21 +783,23 @@ extern "C" int mav1cu_lr_search(mav1cu_session *s, int lr_test) {
   if (need_params(s)) return s->err;
   int n = lr_units_of(s->fp);
   if (n <= 0 || n > s->max_lr_units) return set_error(s, MAV1CU_ERR_ARG, "loop-restoration search: %d units", n);
+  lrs::Dims d = lrs::unit_dims(s->fp);
+  lrs::Layout l = lrs::layout_of(d);
+  if (d.w > lrs::MAX_UNIT_W || d.h > lrs::MAX_UNIT_H)
+    return set_error(s, MAV1CU_ERR_ARG, "loop-restoration search: units of %d x %d samples", d.w, d.h);
   export_fence(s);  // LRUNITS and the plane types are exported
   s->lr_searched = 1;
-  lrs::k_lr_fit<<<n, lrs::THREADS, sizeof(lrs::Shared), s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC),
-                                                                       U8(s, MAV1CU_BUF_DBK), U8(s, MAV1CU_BUF_SRC),
-                                                                       s->lrfit);
+  lrs::k_lr_fit<<<n * lrs::FIT_PARTS, lrs::THREADS, lrs::smem_fit(l), s->stream>>>(
+      DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK), U8(s, MAV1CU_BUF_SRC), s->lrfit, d);
   if (after_launch(s, "loop-restoration fit")) return s->err;
   // the refinement's candidates under guessed references, for all units at
   // once: the serial choice below finds most of its SSEs cached
-  lrs::k_lr_spec<<<n, lrs::THREADS, sizeof(lrs::Shared), s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC),
-                                                                        U8(s, MAV1CU_BUF_DBK), U8(s, MAV1CU_BUF_SRC),
-                                                                        s->lrfit);
+  lrs::k_lr_spec<<<n, lrs::THREADS, lrs::smem_sse(l), s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK),
+                                                                  U8(s, MAV1CU_BUF_SRC), s->lrfit, d);
   if (after_launch(s, "loop-restoration speculative refinement")) return s->err;
-  lrs::k_lr_select<<<3, lrs::THREADS, sizeof(lrs::Shared), s->stream>>>(
+  lrs::k_lr_select<<<3, lrs::THREADS, lrs::smem_sse(l), s->stream>>>(
       (FrameParams *)s->buf[MAV1CU_BUF_PARAMS], U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK), U8(s, MAV1CU_BUF_SRC),
-      s->lrfit, (LrUnit *)s->buf[MAV1CU_BUF_LRUNITS], lr_test, s->lr_types);
+      s->lrfit, (LrUnit *)s->buf[MAV1CU_BUF_LRUNITS], lr_test, s->lr_types, d);
   return after_launch(s, "loop-restoration selection");
 }
 

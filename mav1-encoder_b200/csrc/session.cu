@@ -81,12 +81,11 @@ struct mav1cu_session {
   int32_t *mats_t;         // MATS with every matrix transposed (row passes read it along the output index)
   int mats_dirty;          // MATS changed since mats_t was derived
   int mats_exposed;        // MATS's device address was handed out: derive mats_t before every recon
-  int *waves;              // superblocks in wave order
-  int *status;             // device status: [0] error, [1] abort, [2] queue head, [3] intra blocks, [4] queue tail
+  int *status;             // device status: [0] error, [1] abort
   int *blk_at;             // block index per 4x4 luma unit
-  int *blk_list;           // recon claim list
-  int *blk_done;           // per-block completion flags of the recon launch: luma, then chroma
-  int *dep_count, *succ_count, *succ, *queue, *corners;  // intra ready queue and corner bits (rec::Ctx)
+  int *flow;               // the intra dataflow's zeroed state: counters, successor counts, ready queues (rec::Ctx)
+  int *dep_count, *succ;   // its dependency counts and successor lists
+  rec::IntraTask *tasks;   // its block records
   int resident_recon;      // intra recon workers (CTAs, one per SM)
   int4 *xcounts;           // compact export: per-superblock counts, block and level bases, zero run / fit flag
   int *xblk_base, *xcoef_base, *xmeta;
@@ -104,8 +103,6 @@ struct mav1cu_session {
   int lr_searched;         // the current frame's LR units and types come from mav1cu_lr_search
   int64_t device_bytes;    // device memory this session allocated
   int fault_hold, fault_spins;  // failure-detection test: the next recon's held block and poll limit
-  std::vector<int> wave_start, wave_len;
-  int wave_tile_w;
   FrameParams fp;          // host copy of the current parameters
   int have_params;
   int64_t launches;
@@ -282,8 +279,8 @@ extern "C" void mav1cu_build_fwd_matrices(int32_t *mats) {
 static void free_all(mav1cu_session *s) {
   for (int i = 0; i < MAV1CU_BUF_COUNT; i++)
     if (s->buf[i]) cudaFree(s->buf[i]);
-  void *extra[] = {s->qp[0], s->qp[1], s->dsrc, s->dref[0], s->dref[1], s->ys, s->uvs, s->waves, s->status, s->blk_at, s->blk_list,
-                   s->blk_done, s->mats_t, s->dep_count, s->succ_count, s->succ, s->queue, s->corners,
+  void *extra[] = {s->qp[0], s->qp[1], s->dsrc, s->dref[0], s->dref[1], s->ys, s->uvs, s->status, s->blk_at, s->flow,
+                   s->mats_t, s->dep_count, s->succ, s->tasks,
                    s->xcounts, s->xblk_base, s->xcoef_base, s->xmeta, s->lrfit, s->lr_types};
   for (void *p : extra)
     if (p) cudaFree(p);
@@ -320,9 +317,8 @@ static int64_t session_bytes(const Geometry &g, int maxPresets) {
   b += sizeof(LrUnit) * lrUnits;                                       // LRUNITS
   b += (sizeof(int64_t) + sizeof(BlockInfo)) * A_ITEMS * nsb;          // ACOSTS AINFOS
   b += 2 * 16 * plane + 3 * dplane + 2 * mi;                           // quarter-pel, decimated, edge marks
-  b += sizeof(int) * (nsb + 8 + mi) + sizeof(int32_t) * 4096 * 15;     // waves, status, block map, mats_t
-  b += sizeof(int) * nblk * (4 + MAX_SUCC);                            // ready queue state
-  b += sizeof(int) * MAX_BLOCKS_PER_SB * nsb * 3;                      // claim list, completion flags
+  b += sizeof(int) * (8 + mi) + sizeof(int32_t) * 4096 * 15;           // status, block map, mats_t
+  b += sizeof(int) * (rec::CNT_WORDS + nblk * (5 + MAX_SUCC)) + sizeof(rec::IntraTask) * nblk;  // intra dataflow
   b += sizeof(int4) * nsb + 2 * sizeof(int) * nsb + sizeof(int) * 4;   // export scratch
   b += sizeof(lrs::Fit) * lrUnits + sizeof(int) * 4;                   // LR search
   return (int64_t)b;
@@ -369,19 +365,15 @@ extern "C" int mav1cu_session_create(int width, int height, int max_cdef_presets
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->dref[1], dplane);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->ys, (size_t)g.mi_rows * g.mi_cols);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->uvs, (size_t)g.mi_rows * g.mi_cols);
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->waves, sizeof(int) * nsb);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->status, sizeof(int) * 8);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->blk_at, sizeof(int) * g.mi_rows * g.mi_cols);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->mats_t, sizeof(int32_t) * 4096 * 15);
   size_t nblk = MAX_BLOCKS_PER_SB * nsb;
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->dep_count, sizeof(int) * nblk);
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->succ_count, sizeof(int) * nblk);
+  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->flow, sizeof(int) * (rec::CNT_WORDS + 3 * nblk));
+  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->dep_count, sizeof(int) * 2 * nblk);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->succ, sizeof(int) * nblk * MAX_SUCC);
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->queue, sizeof(int) * nblk);
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->corners, sizeof(int) * nblk);
+  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->tasks, sizeof(rec::IntraTask) * nblk);
   s->mats_dirty = 1;
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->blk_list, sizeof(int) * MAX_BLOCKS_PER_SB * nsb);
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->blk_done, 2 * sizeof(int) * MAX_BLOCKS_PER_SB * nsb);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->xcounts, sizeof(int4) * nsb);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->xblk_base, sizeof(int) * nsb);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->xcoef_base, sizeof(int) * nsb);
@@ -416,17 +408,18 @@ extern "C" int mav1cu_session_create(int width, int height, int max_cdef_presets
     mav1cu_session_destroy(s);
     return code;
   }
-  cudaFuncSetAttribute(rec::k_recon_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec::SMEM_INTRA);
+  cudaFuncSetAttribute(rec::k_recon_blocks<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec::SMEM_SINGLE);
+  cudaFuncSetAttribute(rec::k_recon_blocks<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec::SMEM_SEARCH);
+  cudaFuncSetAttribute(rec::k_recon_lossless, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec::SMEM_INTRA);
   cudaFuncSetAttribute(rec::k_recon_inter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec::SMEM_INTER);
   {
-    int dev = 0, sms = 0, per = 0;
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rec::k_recon_blocks, rec::INTRA_THREADS, rec::SMEM_INTRA);
-    // at most one worker per SM (the kernel keeps max(8, intra blocks / 8) of
-    // them): the ready queue keeps them on ready blocks, and the rest of each
-    // SM stays free for the other engines' kernels
-    s->resident_recon = imax(1, sms * imin(1, imax(1, per)));
+    // at most one luma and one chroma worker per SM (the kernel keeps max(8,
+    // intra blocks / 8) of each): the rest of each SM stays free for the
+    // other engines' kernels
+    s->resident_recon = imax(1, sms);
   }
   cudaFuncSetAttribute(ana::k_analyze_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANA_SMEM(16));
   {
@@ -485,32 +478,6 @@ extern "C" int mav1cu_copy(mav1cu_session *s, int dst, int src, size_t bytes) {
   return check_cuda(s, cudaMemcpyAsync(s->buf[dst], s->buf[src], bytes, cudaMemcpyDeviceToDevice, s->stream), "copy");
 }
 
-// Superblocks in wave order: wave (c - tileStart) + 2r holds the superblocks
-// whose left, above-left, above and above-right neighbours (same tile
-// column) are in earlier waves. The recon claim list follows this order.
-static int build_waves(mav1cu_session *s, int tile_w_sb) {
-  const Geometry &g = s->g;
-  int nw = tile_w_sb + 2 * (g.sb_rows - 1);
-  std::vector<int> list;
-  s->wave_start.assign(nw, 0);
-  s->wave_len.assign(nw, 0);
-  for (int w = 0; w < nw; w++) {
-    s->wave_start[w] = (int)list.size();
-    for (int r = 0; r < g.sb_rows; r++)
-      for (int c = 0; c < g.sb_cols; c++)
-        if ((c % tile_w_sb) + 2 * r == w) list.push_back(r * g.sb_cols + c);
-    s->wave_len[w] = (int)list.size() - s->wave_start[w];
-  }
-  s->wave_tile_w = tile_w_sb;
-  // in the session's stream order: a plain cudaMemcpy from pageable memory
-  // may return before the data lands, and the stream's kernels (non-blocking
-  // stream) would not wait for it; the async copy stages the list before it
-  // returns
-  return check_cuda(s, cudaMemcpyAsync(s->waves, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice,
-                                       s->stream),
-                    "waves");
-}
-
 extern "C" int mav1cu_set_params(mav1cu_session *s, const mav1cu_frame_params *fp) {
   if (s->err) return s->err;
   const Geometry &g = s->g;
@@ -520,7 +487,6 @@ extern "C" int mav1cu_set_params(mav1cu_session *s, const mav1cu_frame_params *f
   s->fp = *fp;
   s->have_params = 1;
   s->lr_searched = 0;
-  if (s->wave_tile_w != fp->tile_w_sb && build_waves(s, fp->tile_w_sb)) return s->err;
   // by value through a launch: asynchronous for any caller memory (a copy
   // from pageable memory may wait for the stream's earlier work)
   drv::k_store_params<<<1, 128, 0, s->stream>>>(*fp, (FrameParams *)s->buf[MAV1CU_BUF_PARAMS]);
@@ -662,44 +628,38 @@ extern "C" int mav1cu_recon(mav1cu_session *s) {
   }
   c.status = s->status;
   c.blk_at = s->blk_at;
-  c.done = s->blk_done;
+  const int nsb = s->g.num_sbs, nblk = MAX_BLOCKS_PER_SB * nsb;
+  c.nblk = nblk;
+  c.counters = s->flow;
+  c.succ_count = s->flow + rec::CNT_WORDS;
+  c.queue = c.succ_count + nblk;
+  c.dep_count = s->dep_count;
+  c.succ = s->succ;
+  c.tasks = s->tasks;
   c.spin_limit = s->fault_spins > 0 ? s->fault_spins : SPIN_LIMIT;
   c.hold = s->fault_spins > 0 ? s->fault_hold : -1;
   s->fault_spins = 0;
-  int nsb = s->g.num_sbs;
-  if (check_cuda(s, cudaMemsetAsync(s->blk_done, 0, 2 * sizeof(int) * MAX_BLOCKS_PER_SB * nsb, s->stream),
-                 "recon flags"))
-    return s->err;
   if (!s->fp.frame_is_intra) {
     rec::k_recon_inter<<<nsb, rec::INTER_THREADS, rec::SMEM_INTER, s->stream>>>(c);
     if (after_launch(s, "recon inter blocks")) return s->err;
   }
   // leaf frames code inter blocks only (the analysis never keeps intra there)
   if (s->fp.leaf && !s->fp.frame_is_intra) return MAV1CU_OK;
-  rec::k_block_map<<<(nsb + 3) / 4, 128, 0, s->stream>>>(DP(s), c.blocks, c.sbs, s->blk_at);
-  if (after_launch(s, "recon unit map")) return s->err;
-  rec::k_block_order<<<1, 1024, 0, s->stream>>>(c.blocks, c.sbs, s->waves, nsb, s->blk_list, s->status + 3);
-  if (after_launch(s, "recon claim list")) return s->err;
-  size_t nblk = (size_t)MAX_BLOCKS_PER_SB * nsb;
-  if (check_cuda(s, cudaMemsetAsync(s->succ_count, 0, sizeof(int) * nblk, s->stream), "recon successors") ||
-      check_cuda(s, cudaMemsetAsync(s->queue, 0, sizeof(int) * nblk, s->stream), "recon queue") ||
-      check_cuda(s, cudaMemsetAsync(s->status + 2, 0, sizeof(int), s->stream), "recon queue head") ||
-      check_cuda(s, cudaMemsetAsync(s->status + 4, 0, sizeof(int), s->stream), "recon queue tail"))
+  if (check_cuda(s, cudaMemsetAsync(s->flow, 0, sizeof(int) * (rec::CNT_WORDS + 3 * (size_t)nblk), s->stream),
+                 "recon dataflow"))
     return s->err;
-  c.dep_count = s->dep_count;
-  c.succ_count = s->succ_count;
-  c.succ = s->succ;
-  c.queue = s->queue;
-  c.corners = s->corners;
-  c.qtail = s->status + 4;
-  rec::k_block_deps<<<(unsigned)imin((int)((nblk + 3) / 4), 4 * s->resident_recon), 128, 0, s->stream>>>(
-      c, s->blk_list, s->status + 3);
+  rec::k_block_map<<<nsb, rec::MAP_THREADS, 0, s->stream>>>(DP(s), c.blocks, c.sbs, s->blk_at, c.counters);
+  if (after_launch(s, "recon unit map")) return s->err;
+  if (s->fp.lossless) {
+    rec::k_recon_lossless<<<nblk, rec::INTRA_THREADS, rec::SMEM_INTRA, s->stream>>>(c);
+    return after_launch(s, "recon lossless blocks");
+  }
+  rec::k_block_deps<<<(nblk + 3) / 4, 128, 0, s->stream>>>(c);
   if (after_launch(s, "recon dependencies")) return s->err;
-  rec::Claim q;
-  q.list = s->blk_list;
-  q.total = s->status + 3;
-  q.next = s->status + 2;
-  rec::k_recon_blocks<<<s->resident_recon, rec::INTRA_THREADS, rec::SMEM_INTRA, s->stream>>>(c, q);
+  if (s->fp.tx_search || s->fp.tx_mode_select)
+    rec::k_recon_blocks<true><<<2 * s->resident_recon, rec::SEARCH_THREADS, rec::SMEM_SEARCH, s->stream>>>(c);
+  else
+    rec::k_recon_blocks<false><<<2 * s->resident_recon, rec::SINGLE_THREADS, rec::SMEM_SINGLE, s->stream>>>(c);
   return after_launch(s, "recon intra blocks");
 }
 
@@ -953,7 +913,6 @@ extern "C" int mav1cu_synchronize(mav1cu_session *s) {
   if (st[0])
     return set_error(s, MAV1CU_ERR_DEVICE, "device status %d: %s", st[0],
                      st[0] == 2   ? "a recon successor list overflowed"
-                     : st[0] == 3 ? "a recon chroma-edge dependency wait gave up"
                      : st[0] == 4 ? "a recon source bulk-copy wait gave up"
                                   : "a recon ready-queue wait gave up");
   return MAV1CU_OK;

@@ -112,7 +112,6 @@ struct Smem {
   int maxLumaW, maxLumaH;
   int flag;
   int me;      // index of the block being coded
-  int next;    // release()'s block
   int r0, c0;  // its superblock's first 4x4 row / column
   // views of the reconstruction and the source: plane origins (absolute
   // plane coordinates) and strides; the frames for an inter block, the
@@ -142,7 +141,6 @@ struct Smem {
       int32_t fmat[3][FMAT_SMALL];   // forward matrices of lengths 4, 8, 16 per kind
       int32_t fmatT[3][FMAT_SMALL];  // the same transposed
       int edge[3][EDGE_LEN];   // AboveRow, LeftCol, filter copy
-      uint8_t save[64 * 64];   // the block's luma before the tx_depth candidates
       // tiles: rows and columns -1 .. 2n - 1 around the block (its own
       // samples, the above row over the above-right units, the left column
       // over the below-left units), and its source
@@ -194,7 +192,8 @@ struct CtaSync {
 
 // One row of the inverse transform at a fixed width: dequantised levels ->
 // row transform -> clamp, into resid (stride RS).
-template <int LW, int RS>
+// RAW: q holds levels, dequantised here; otherwise dequantised levels.
+template <int LW, int RS, bool RAW>
 __device__ __forceinline__ void inv_row(int32_t *resid, const int32_t *q, int i, int th, int dcQ, int acQ, int denom, int rect, int rk,
                         int rowShift) {
   constexpr int W = 1 << LW, TW = W < 32 ? W : 32;
@@ -202,7 +201,8 @@ __device__ __forceinline__ void inv_row(int32_t *resid, const int32_t *q, int i,
   int nz = 0;
 #pragma unroll
   for (int j = 0; j < W; j++) {
-    t[j] = (j < TW && i < th) ? tx::dequant_level(q[i * TW + j], (i == 0 && j == 0) ? dcQ : acQ, denom) : 0;
+    int v = (j < TW && i < th) ? q[i * TW + j] : 0;
+    t[j] = RAW ? tx::dequant_level(v, (i == 0 && j == 0) ? dcQ : acQ, denom) : v;
     nz |= t[j];
   }
   if (!nz) {
@@ -246,7 +246,7 @@ __device__ __forceinline__ void inv_col(int32_t *resid, int j, int w, int ck, in
 // half 1 the odd half and the rest, tx::idct_odd), which halves the
 // sequential butterfly chain of the largest transforms. Each thread loads
 // its permuted inputs directly; the pre-join halves meet in resid.
-template <int LW, int RS>
+template <int LW, int RS, bool RAW>
 __device__ __forceinline__ void inv_row_split(int32_t *resid, const int32_t *q, int i, int half, int th, int dcQ, int acQ, int denom,
                               int rect, int rowShift) {
   constexpr int W = 1 << LW, HW = W / 2, TW = W < 32 ? W : 32;
@@ -256,7 +256,8 @@ __device__ __forceinline__ void inv_row_split(int32_t *resid, const int32_t *q, 
 #pragma unroll
   for (int k = 0; k < HW; k++) {
     int j = tx::brev(LW, k + half * HW);
-    t[k] = (j < TW && i < th) ? tx::dequant_level(q[i * TW + j], (i == 0 && j == 0) ? dcQ : acQ, denom) : 0;
+    int v = (j < TW && i < th) ? q[i * TW + j] : 0;
+    t[k] = RAW ? tx::dequant_level(v, (i == 0 && j == 0) ? dcQ : acQ, denom) : v;
     nz |= t[k];
   }
   nz |= __shfl_xor_sync(pair, nz, 1);
@@ -332,16 +333,16 @@ __device__ __forceinline__ void inverse_2d_upto(Smem &sm, const int32_t *q, int 
   int rk = tx::row_kind(txType), ck = tx::col_kind(txType);
   if (MAXL >= 5 && lw >= 5 && rk == tx::KIND_DCT) {
     for (int p = threadIdx.x; p < 2 * h; p += RT) {
-      if (lw == 5) inv_row_split<5, 64>(sm.resid, q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
-      else inv_row_split<6, 64>(sm.resid, q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
+      if (lw == 5) inv_row_split<5, 64, true>(sm.resid, q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
+      else inv_row_split<6, 64, true>(sm.resid, q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
     }
   } else for (int i = threadIdx.x; i < h; i += RT) {
     switch (lw) {
-      case 2: inv_row<2, 64>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
-      case 3: inv_row<3, 64>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
-      case 4: inv_row<4, 64>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
-      case 5: if (MAXL >= 5) inv_row<5, 64>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
-      default: if (MAXL >= 6) inv_row<6, 64>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      case 2: inv_row<2, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      case 3: inv_row<3, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      case 4: inv_row<4, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      case 5: if (MAXL >= 5) inv_row<5, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      default: if (MAXL >= 6) inv_row<6, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
     }
   }
   __syncthreads();
@@ -376,7 +377,7 @@ __device__ __forceinline__ void inverse_2d_fixed(Smem &sm, const int32_t *q, int
                                                  int rowShift, uint8_t *rec, int rs, int x, int y) {
   constexpr int W = 1 << LW, H = 1 << LH, rect = LW - LH == 1 || LH - LW == 1;
   int rk = tx::row_kind(txType), ck = tx::col_kind(txType);
-  for (int i = threadIdx.x; i < H; i += RT) inv_row<LW, 64>(sm.resid, q, i, H, dcQ, acQ, 1, rect, rk, rowShift);
+  for (int i = threadIdx.x; i < H; i += RT) inv_row<LW, 64, true>(sm.resid, q, i, H, dcQ, acQ, 1, rect, rk, rowShift);
   __syncthreads();
   int fud = tx::flip_ud(txType), flr = tx::flip_lr(txType);
   for (int j = threadIdx.x; j < W; j += RT) inv_col<LH, 64>(sm.resid, j, W, ck, fud, flr, rec, rs, x, y);
@@ -1308,7 +1309,8 @@ struct IntraTask {
   int bits;                  // BlockDecoded of the corner units: bit 0 / 1 luma above-right / below-left, bit 2 / 3 chroma
   int maxLumaW, maxLumaH;    // CfL's luma limits
   PlaneTask p[2];            // luma, chroma
-  int pad[11];
+  int angle_y, bsize;
+  int pad[9];
 };
 static_assert(sizeof(IntraTask) == 128, "one coalesced load of a warp");
 
@@ -1373,11 +1375,15 @@ __global__ void __launch_bounds__(MAP_THREADS) k_block_map(const FrameParams *fp
   if (lane == 0 && intra) atomicAdd(total, intra);
 }
 
+// Orders this thread's (and, after a barrier, its CTA's) accesses before it
+// with those after it, at device scope.
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // Appends a block to a ready queue (kind 0: luma, 1: chroma). What the caller
 // knows complete is visible to whoever takes the block.
 __device__ __forceinline__ void push_ready(const Ctx &c, int kind, int blk) {
   int t = atomicAdd(c.counters + CNT_TAIL + kind, 1);
-  __threadfence();
+  fence_gpu();
   atomicExch(c.queue + kind * c.nblk + t, blk + 1);
 }
 
@@ -1411,6 +1417,8 @@ __global__ void __launch_bounds__(128) k_block_deps(Ctx c) {
     for (int p = 0; p < 3; p++) task->coef[p] = b.coef_off[p];
     task->interp = b.interp_filter & 0x30;
     task->bits = cb;
+    task->angle_y = b.angle_y;
+    task->bsize = b.bsize;
     task->maxLumaW = b.mi_col * 4 + block_w(b.bsize);
     task->maxLumaH = b.mi_row * 4 + block_h(b.bsize);
   }
@@ -1485,12 +1493,135 @@ struct IntraShared {
   int32_t fmat[3][FMAT_SMALL], fmatT[3][FMAT_SMALL];
   int smw[124];      // smooth weights of lengths 4, 8, 16, 32, 64 from (1 << log2) - 4
   IntraTask task;
-  int next, popped, alphaU;  // release()'s and pop_ready()'s block; U's CfL alpha
+  int ahead[8][32];  // records of the first successors (feed)
+  int alphaU;        // U's CfL alpha
   union {
     PlaneMem<64> y;
     PlaneMem<32> uv[2];
   };
 };
+
+// What a prediction does to its edges, and a directional mode's slopes.
+struct EdgePrep {
+  int pAngle, dx, dy, upA, upL;  // pred::IntraState
+  int sa, sl, corner, za, zl;    // filter strengths (0: none), the corner filter, samples covered (the corner included)
+};
+
+// Edge filter (7.11.2.12) and upsampling (7.11.2.11) of a block's edges, both
+// sides at once.
+template <int NT>
+__device__ __forceinline__ void prepare_edges(const Group<NT> &g, const EdgePrep &e, int *above, int *left, int *ta, int *tl, int w,
+                                              int h) {
+  const int tid = g.tid;
+  if (e.corner | e.sa | e.sl) {
+    const int za = e.sa ? e.za : 0, zl = e.sl ? e.zl : 0;
+    if (e.corner) {
+      if (tid == 0) left[-1] = above[-1] = round2(left[0] * 5 + above[-1] * 6 + above[0] * 5, 4);
+      g.sync();
+    }
+    if (za | zl) {
+      for (int i = tid; i < za + zl; i += NT) {
+        if (i < za) ta[i] = above[i - 1];
+        else tl[i - za] = left[i - za - 1];
+      }
+      g.sync();
+      for (int i = tid; i < za + zl; i += NT) {
+        int a = i < za, k = a ? i : i - za, z = a ? za : zl, s = a ? e.sa : e.sl;
+        const int *src = a ? ta : tl;
+        if (k == 0) continue;
+        int acc = 0;
+        for (int j = 0; j < 5; j++) acc += T(Intra_Edge_Kernel)[s - 1][j] * src[clip3(0, z - 1, k - 2 + j)];
+        (a ? above : left)[k - 1] = (acc + 8) >> 4;
+      }
+      g.sync();
+    }
+  }
+  if (e.upA | e.upL) {
+    const int nA = e.upA ? w + (e.pAngle < 90 ? h : 0) : 0, nL = e.upL ? h + (e.pAngle > 180 ? w : 0) : 0;
+    const int cA = e.upA ? nA + 3 : 0, cL = e.upL ? nL + 3 : 0;
+    for (int i = tid; i < cA + cL; i += NT) {
+      int a = i < cA, k = a ? i : i - cA, n = a ? nA : nL;
+      (a ? ta : tl)[k] = (a ? above : left)[k == 0 ? -1 : imin(k - 2, n - 1)];
+    }
+    g.sync();
+    for (int i = tid; i < nA + nL; i += NT) {
+      int a = i < nA, k = a ? i : i - nA;
+      const int *d = (a ? ta : tl) + k;
+      int *buf = a ? above : left;
+      buf[2 * k - 1] = clip1(round2(-d[0] + 9 * d[1] + 9 * d[2] - d[3], 4));
+      buf[2 * k] = d[2];
+      if (k == 0) buf[-2] = d[0];
+    }
+    g.sync();
+  }
+}
+
+// DC_PRED's value (pred::intra_dc), by every warp for itself.
+__device__ __forceinline__ int dc_value(const int *above, const int *left, int lw, int lh, int haveAbove, int haveLeft) {
+  const int w = 1 << lw, h = 1 << lh, lane = threadIdx.x & 31;
+  int sA = 0, sL = 0;
+  for (int i = lane; i < w; i += 32) sA += above[i];
+  for (int i = lane; i < h; i += 32) sL += left[i];
+  sA = __reduce_add_sync(0xffffffffu, sA);
+  sL = __reduce_add_sync(0xffffffffu, sL);
+  if (haveLeft && haveAbove) return (sA + sL + ((w + h) >> 1)) / (w + h);
+  if (haveLeft) return (sL + (h >> 1)) >> lh;
+  if (haveAbove) return (sA + (w >> 1)) >> lw;
+  return 128;
+}
+
+// Samples (i, j0 .. j0 + 3) of a w x h prediction from prepared edges
+// (pred::intra_pixel; wX, wY: smooth weights of w and h).
+__device__ __forceinline__ void predict4(int mode, const EdgePrep &e, const int *above, const int *left, const int *wX, const int *wY,
+                                         int w, int h, int i, int j0, int dcv, int (&p)[4]) {
+  const int upA = e.upA, upL = e.upL, dx = e.dx, dy = e.dy;
+  if (mode == DC_PRED) {
+    for (int k = 0; k < 4; k++) p[k] = dcv;
+  } else if (intra_is_directional(mode)) {
+    if (e.pAngle < 90) {
+      int idx = (i + 1) * dx, shift = ((idx << upA) >> 1) & 0x1F, b0 = (idx >> (6 - upA)) + (j0 << upA), mx = (w + h - 1) << upA;
+      for (int k = 0; k < 4; k++) {
+        int b = b0 + (k << upA);
+        p[k] = b < mx ? round2(above[b] * (32 - shift) + above[b + 1] * shift, 5) : above[mx];
+      }
+    } else if (e.pAngle > 90 && e.pAngle < 180) {
+      for (int k = 0; k < 4; k++) {
+        int j = j0 + k, idx = (j << 6) - (i + 1) * dx, b = idx >> (6 - upA), up = upA;
+        const int *ed = above;
+        if (b < -(1 << upA)) {
+          idx = (i << 6) - (j + 1) * dy;
+          b = idx >> (6 - upL);
+          ed = left;
+          up = upL;
+        }
+        int shift = ((idx * (1 << up)) >> 1) & 0x1F;
+        p[k] = round2(ed[b] * (32 - shift) + ed[b + 1] * shift, 5);
+      }
+    } else if (e.pAngle > 180) {
+      for (int k = 0; k < 4; k++) {
+        int idx = (j0 + k + 1) * dy, b = (idx >> (6 - upL)) + (i << upL), shift = ((idx << upL) >> 1) & 0x1F;
+        p[k] = round2(left[b] * (32 - shift) + left[b + 1] * shift, 5);
+      }
+    } else if (e.pAngle == 90) {
+      for (int k = 0; k < 4; k++) p[k] = above[j0 + k];
+    } else {
+      for (int k = 0; k < 4; k++) p[k] = left[i];
+    }
+  } else if (mode == PAETH_PRED) {
+    int L = left[i], C = above[-1];
+    for (int k = 0; k < 4; k++) {
+      int A = above[j0 + k], base = A + L - C, pl = iabs(base - L), pt = iabs(base - A), pc = iabs(base - C);
+      p[k] = pl <= pt && pl <= pc ? L : pt <= pc ? A : C;
+    }
+  } else {  // SMOOTH, SMOOTH_V, SMOOTH_H
+    int L = left[i], LB = left[h - 1], AR = above[w - 1], wy = wY[i];
+    for (int k = 0; k < 4; k++) {
+      int A = above[j0 + k], wx = wX[j0 + k];
+      int v = wy * A + (256 - wy) * LB, hh = wx * L + (256 - wx) * AR;
+      p[k] = mode == SMOOTH_PRED ? round2(v + hh, 9) : mode == SMOOTH_V_PRED ? round2(v, 8) : round2(hh, 8);
+    }
+  }
+}
 
 template <int LW, int RS, int NT>
 __device__ __forceinline__ void fwd_rows_g(const int32_t *resid, int32_t *tmp, const int32_t *MhT, int h, int tid) {
@@ -1514,7 +1645,7 @@ __device__ __forceinline__ int64_t fwd_col_g(const int32_t *tmp, const int32_t *
   return s;
 }
 
-// Inverse transform of the levels in m.q, added into m.px.
+// Inverse transform of the dequantised levels in m.q, added into m.px.
 template <int MAXD, int NT, int LOW, int HIGH>
 __device__ __forceinline__ void inverse_g(PlaneMem<MAXD> &m, const Group<NT> &g, int lw, int lh, int type, int txSz, int dcQ, int acQ) {
   constexpr int RS = MAXD + 1;
@@ -1522,14 +1653,14 @@ __device__ __forceinline__ void inverse_g(PlaneMem<MAXD> &m, const Group<NT> &g,
   const int rect = iabs(lw - lh) == 1, rk = tx::row_kind(type), ck = tx::col_kind(type);
   if (HIGH >= 5 && lw >= 5) {
     for (int p = g.tid; p < 2 * h; p += NT) {
-      if (lw == 5) inv_row_split<5, RS>(m.resid, m.q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
-      else if (HIGH >= 6) inv_row_split<6, RS>(m.resid, m.q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
+      if (lw == 5) inv_row_split<5, RS, false>(m.resid, m.q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
+      else if (HIGH >= 6) inv_row_split<6, RS, false>(m.resid, m.q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
     }
   } else {
     for (int i = g.tid; i < h; i += NT) {
-      if (lw == 2) inv_row<2, RS>(m.resid, m.q, i, th, dcQ, acQ, denom, rect, rk, rowShift);
-      else if (lw == 3) inv_row<3, RS>(m.resid, m.q, i, th, dcQ, acQ, denom, rect, rk, rowShift);
-      else if (lw == 4) inv_row<4, RS>(m.resid, m.q, i, th, dcQ, acQ, denom, rect, rk, rowShift);
+      if (lw == 2) inv_row<2, RS, false>(m.resid, m.q, i, th, dcQ, acQ, denom, rect, rk, rowShift);
+      else if (lw == 3) inv_row<3, RS, false>(m.resid, m.q, i, th, dcQ, acQ, denom, rect, rk, rowShift);
+      else if (lw == 4) inv_row<4, RS, false>(m.resid, m.q, i, th, dcQ, acQ, denom, rect, rk, rowShift);
     }
   }
   g.sync();
@@ -1702,61 +1833,10 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
     }
   }
   g.sync();
-  const int pAngle = t.ang & 511, dx = (t.ang >> 9) & 2047, dy = t.ang >> 20;
-  const int upA = (geo >> 12) & 1, upL = (geo >> 13) & 1;
-  if (geo & (0x1fu << 14)) {  // edge filter (7.11.2.12)
-    const int sa = (geo >> 14) & 3, sl = (geo >> 16) & 3, za = sa ? (int)(t.flt & 0xffff) : 0, zl = sl ? (int)(t.flt >> 16) : 0;
-    if ((geo >> 18) & 1) {
-      if (tid == 0) left[-1] = above[-1] = round2(left[0] * 5 + above[-1] * 6 + above[0] * 5, 4);
-      g.sync();
-    }
-    if (za | zl) {
-      for (int i = tid; i < za + zl; i += NT) {
-        if (i < za) ta[i] = above[i - 1];
-        else tl[i - za] = left[i - za - 1];
-      }
-      g.sync();
-      for (int i = tid; i < za + zl; i += NT) {
-        int a = i < za, k = a ? i : i - za, z = a ? za : zl, s = a ? sa : sl;
-        const int *src = a ? ta : tl;
-        if (k == 0) continue;
-        int acc = 0;
-        for (int j = 0; j < 5; j++) acc += T(Intra_Edge_Kernel)[s - 1][j] * src[clip3(0, z - 1, k - 2 + j)];
-        (a ? above : left)[k - 1] = (acc + 8) >> 4;
-      }
-      g.sync();
-    }
-  }
-  if (upA | upL) {  // upsampling (7.11.2.11)
-    const int nA = upA ? w + (pAngle < 90 ? h : 0) : 0, nL = upL ? h + (pAngle > 180 ? w : 0) : 0;
-    const int cA = upA ? nA + 3 : 0, cL = upL ? nL + 3 : 0;
-    for (int i = tid; i < cA + cL; i += NT) {
-      int a = i < cA, k = a ? i : i - cA, n = a ? nA : nL;
-      (a ? ta : tl)[k] = (a ? above : left)[k == 0 ? -1 : imin(k - 2, n - 1)];
-    }
-    g.sync();
-    for (int i = tid; i < nA + nL; i += NT) {
-      int a = i < nA, k = a ? i : i - nA;
-      const int *d = (a ? ta : tl) + k;
-      int *buf = a ? above : left;
-      buf[2 * k - 1] = clip1(round2(-d[0] + 9 * d[1] + 9 * d[2] - d[3], 4));
-      buf[2 * k] = d[2];
-      if (k == 0) buf[-2] = d[0];
-    }
-    g.sync();
-  }
-  int dcv = 0;
-  if (mode == DC_PRED) {
-    int sA = 0, sL = 0;
-    for (int i = lane; i < w; i += 32) sA += above[i];
-    for (int i = lane; i < h; i += 32) sL += left[i];
-    sA = __reduce_add_sync(0xffffffffu, sA);
-    sL = __reduce_add_sync(0xffffffffu, sL);
-    if (haveLeft && haveAbove) dcv = (sA + sL + ((w + h) >> 1)) / (w + h);
-    else if (haveLeft) dcv = (sL + (h >> 1)) >> lh;
-    else if (haveAbove) dcv = (sA + (w >> 1)) >> lw;
-    else dcv = 128;
-  }
+  const EdgePrep e = {(int)(t.ang & 511), (int)((t.ang >> 9) & 2047), (int)(t.ang >> 20), (int)((geo >> 12) & 1), (int)((geo >> 13) & 1),
+                      (int)((geo >> 14) & 3), (int)((geo >> 16) & 3), (int)((geo >> 18) & 1), (int)(t.flt & 0xffff), (int)(t.flt >> 16)};
+  prepare_edges(g, e, above, left, ta, tl, w, h);
+  const int dcv = mode == DC_PRED ? dc_value(above, left, lw, lh, haveAbove, haveLeft) : 0;
   const int cfl = plane && ((geo >> 19) & 1);
   if (cfl) {
     if constexpr (MAXD == 32) cfl_g(c, sh, m, g, t, plane, dcv, sv);
@@ -1773,60 +1853,16 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
     int p[4];
     if (cfl) {
       uint32_t v = *(const uint32_t *)(m.px + 4 * k);
-      for (int e = 0; e < 4; e++) p[e] = (v >> (8 * e)) & 255;
-    } else if (mode == DC_PRED) {
-      for (int e = 0; e < 4; e++) p[e] = dcv;
-    } else if (intra_is_directional(mode)) {
-      if (pAngle < 90) {
-        int idx = (i + 1) * dx, shift = ((idx << upA) >> 1) & 0x1F, b0 = (idx >> (6 - upA)) + (j0 << upA), mx = (w + h - 1) << upA;
-        for (int e = 0; e < 4; e++) {
-          int b = b0 + (e << upA);
-          p[e] = b < mx ? round2(above[b] * (32 - shift) + above[b + 1] * shift, 5) : above[mx];
-        }
-      } else if (pAngle > 90 && pAngle < 180) {
-        for (int e = 0; e < 4; e++) {
-          int j = j0 + e, idx = (j << 6) - (i + 1) * dx, b = idx >> (6 - upA);
-          const int *ed = above;
-          int up = upA;
-          if (b < -(1 << upA)) {
-            idx = (i << 6) - (j + 1) * dy;
-            b = idx >> (6 - upL);
-            ed = left;
-            up = upL;
-          }
-          int shift = ((idx * (1 << up)) >> 1) & 0x1F;
-          p[e] = round2(ed[b] * (32 - shift) + ed[b + 1] * shift, 5);
-        }
-      } else if (pAngle > 180) {
-        for (int e = 0; e < 4; e++) {
-          int idx = (j0 + e + 1) * dy, b = (idx >> (6 - upL)) + (i << upL), shift = ((idx << upL) >> 1) & 0x1F;
-          p[e] = round2(left[b] * (32 - shift) + left[b + 1] * shift, 5);
-        }
-      } else if (pAngle == 90) {
-        for (int e = 0; e < 4; e++) p[e] = above[j0 + e];
-      } else {
-        for (int e = 0; e < 4; e++) p[e] = left[i];
-      }
-    } else if (mode == PAETH_PRED) {
-      int L = left[i], C = above[-1];
-      for (int e = 0; e < 4; e++) {
-        int A = above[j0 + e], base = A + L - C, pl = iabs(base - L), pt = iabs(base - A), pc = iabs(base - C);
-        p[e] = pl <= pt && pl <= pc ? L : pt <= pc ? A : C;
-      }
-    } else {  // SMOOTH, SMOOTH_V, SMOOTH_H
-      int L = left[i], LB = left[h - 1], AR = above[w - 1], wy = wY[i];
-      for (int e = 0; e < 4; e++) {
-        int A = above[j0 + e], wx = wX[j0 + e];
-        int v = wy * A + (256 - wy) * LB, hh = wx * L + (256 - wx) * AR;
-        p[e] = mode == SMOOTH_PRED ? round2(v + hh, 9) : mode == SMOOTH_V_PRED ? round2(v, 8) : round2(hh, 8);
-      }
+      for (int k4 = 0; k4 < 4; k4++) p[k4] = (v >> (8 * k4)) & 255;
+    } else {
+      predict4(mode, e, above, left, wX, wY, w, h, i, j0, dcv, p);
     }
     uint32_t pk = 0;
     int32_t *rr = m.resid + i * RS + j0;
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      pk |= (uint32_t)(p[e] & 255) << (8 * e);
-      rr[e] = (int)((sv[q] >> (8 * e)) & 255) - p[e];
+    for (int k4 = 0; k4 < 4; k4++) {
+      pk |= (uint32_t)(p[k4] & 255) << (8 * k4);
+      rr[k4] = (int)((sv[q] >> (8 * k4)) & 255) - p[k4];
     }
     *(uint32_t *)(m.px + 4 * k) = pk;
   }
@@ -1868,7 +1904,7 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
     int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
     int first = k == 0;
     int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
-    m.q[k] = lv;
+    m.q[k] = tx::dequant_level(lv, first ? dcQ : acQ, denom);
     coefOut[k] = lv;
     nz |= lv;
   }
@@ -1887,7 +1923,8 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
 }
 
 // The workers' shared constants.
-__device__ void load_intra_shared(const Ctx &c, IntraShared &sh) {
+template <class Shared>
+__device__ void load_intra_shared(const Ctx &c, Shared &sh) {
   const int nt = blockDim.x;
   for (int k = threadIdx.x; k < (int)(sizeof(FrameParams) / 4); k += nt) ((int *)&sh.fpc)[k] = ((const int *)c.fp)[k];
   if (threadIdx.x < 6) {
@@ -1920,7 +1957,7 @@ __device__ int pop_ready(const Ctx &c, int kind, int total) {
   for (int spins = 0;; spins++) {
     int v = *vslot, d = *done;
     if (v) {
-      __threadfence();
+      fence_gpu();
       return v - 1;
     }
     if (d >= total || *abort) return -1;
@@ -1933,36 +1970,89 @@ __device__ int pop_ready(const Ctx &c, int kind, int total) {
   }
 }
 
-// After the block's samples of one kind are written by the whole CTA: one
-// dependency fewer for each successor (and, after luma, for its own chroma).
-// A successor this was the last for goes on in this CTA (the first of them)
-// or to its queue. succ: this thread's entry of the successor list.
-// Returns the block to go on with, or -1. The whole CTA calls it.
-__device__ __forceinline__ int release(const Ctx &c, int *next, int me, int kind, int succ) {
-  if (threadIdx.x == 0) *next = -1;
-  __syncthreads();  // every thread's writes precede the releasing threads' fence
-  const bool own = kind == 0 && threadIdx.x == MAX_SUCC;
-  if (succ >= 0 || own) {
-    __threadfence();
-    int s = own ? me : succ, dk = own ? 1 : kind;
-    if (atomicSub(c.dep_count + dk * c.nblk + s, 1) == 1) {
-      __threadfence();
-      if (own || atomicCAS(next, -1, s) != -1) push_ready(c, dk, s);
+// A worker CTA's last warp: it takes blocks, loads their records for the
+// coding warps and releases successors, so that queue traffic runs beside the
+// coding. Barrier 4: the record is in place (me -1: no more); barrier 5: the
+// block is coded and written. While the block is coded the warp fetches the
+// records of its first successors; when one of them becomes ready by this
+// block, it goes to the coding warps at once and the other ready ones are
+// queued after that.
+constexpr int CODERS = 128, WORKER_THREADS = CODERS + 32, AHEAD = 8;
+template <int N>
+__device__ __forceinline__ void record_bar() { asm volatile("bar.sync 4, %0;" ::"n"(N) : "memory"); }
+template <int N>
+__device__ __forceinline__ void coded_bar() { asm volatile("bar.sync 5, %0;" ::"n"(N) : "memory"); }
+
+// ahead: records do not change during the launch (with a luma search they
+// carry the luma limits that chroma reads).
+template <bool AHEAD_OK, int N, class Shared>
+__device__ void feed(const Ctx &c, Shared &sh, int kind, int total) {
+  const int lane = threadIdx.x & 31;
+  auto record_word = [&](int b) {
+    return __ldcg(lane == 1 ? c.succ_count + b : (const int *)(c.tasks + b) + lane);
+  };
+  int push[3] = {-1, -1, -1}, pushOwn = -1;  // ready blocks still to be queued
+  for (int me = -1, at = -1;;) {
+    if (me < 0) {
+      if (lane == 0) me = pop_ready(c, kind, total);
+      me = __shfl_sync(0xffffffffu, me, 0);
+      if (me < 0) {
+        if (lane == 0) sh.task.me = -1;
+        __syncwarp();
+        record_bar<N>();
+        return;
+      }
+    }
+    ((int *)&sh.task)[lane] = at >= 0 ? sh.ahead[at][lane] : record_word(me);
+    __syncwarp();
+    const int n = imin(sh.task.nsucc, MAX_SUCC);
+    record_bar<N>();
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      if (push[q] >= 0) push_ready(c, kind, push[q]);
+    if (pushOwn >= 0) push_ready(c, 1, pushOwn);
+    int s[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) s[q] = lane + 32 * q < n ? __ldcg(c.succ + (size_t)me * MAX_SUCC + lane + 32 * q) : -1;
+    if (AHEAD_OK) {
+#pragma unroll
+      for (int k = 0; k < AHEAD; k++) {
+        int b = __shfl_sync(0xffffffffu, s[0], k);
+        if (k < n) sh.ahead[k][lane] = record_word(b);
+      }
+    }
+    coded_bar<N>();
+    fence_gpu();
+    int ready[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      ready[q] = s[q] >= 0 && atomicSub(c.dep_count + kind * c.nblk + s[q], 1) == 1;
+    pushOwn = kind == 0 && lane == 31 && atomicSub(c.dep_count + c.nblk + me, 1) == 1 ? me : -1;
+    if (lane == 0) atomicAdd(c.counters + CNT_DONE + kind, 1);
+    fence_gpu();
+    int next = -1;
+    at = -1;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      unsigned r = __ballot_sync(0xffffffffu, ready[q]);
+      if (next < 0 && r) {
+        int f = __ffs(r) - 1;
+        next = __shfl_sync(0xffffffffu, s[q], f);
+        if (lane == f) ready[q] = 0;
+        if (AHEAD_OK && q == 0 && f < AHEAD) at = f;
+      }
+      push[q] = ready[q] ? s[q] : -1;
+    }
+    me = next;
+    if (me < 0) {  // nothing to go on with: queue what is ready (own chroma) before waiting
+#pragma unroll
+      for (int q = 0; q < 3; q++) push[q] = -1;
+      if (pushOwn >= 0) push_ready(c, 1, pushOwn);
+      pushOwn = -1;
     }
   }
-  if (threadIdx.x == MAX_SUCC + 1) atomicAdd(c.counters + CNT_DONE + kind, 1);
-  __syncthreads();
-  return *next;
 }
 
-// This thread's entry of the block's successor list, or -1.
-__device__ __forceinline__ int successor(const Ctx &c, int me, int nsucc, int mine) {
-  return (int)threadIdx.x < imin(nsucc, MAX_SUCC) ? mine : -1;
-}
-
-constexpr int SINGLE_THREADS = 128, SEARCH_THREADS = 256;
-constexpr size_t SMEM_SINGLE = sizeof(IntraShared);
-constexpr size_t SMEM_SEARCH = sizeof(Smem) > sizeof(IntraShared) ? sizeof(Smem) : sizeof(IntraShared);
 // Workers per kind: as many as the frame's blocks can use, so that on frames
 // of few intra blocks the other SMs stay free for the other engine's kernels.
 #ifndef MAV1CU_BLOCKS_PER_WORKER
@@ -1975,21 +2065,14 @@ constexpr int BLOCKS_PER_WORKER = MAV1CU_BLOCKS_PER_WORKER, MIN_WORKERS = MAV1CU
 
 // ---- workers of frames whose luma blocks are one transform block of one type (no
 // transform type or depth search, not lossless)
-__device__ void luma_worker(const Ctx &c, IntraShared &sh, int total) {
-  const Group<SINGLE_THREADS> g{(int)threadIdx.x, 1};
-  const int tid = threadIdx.x;
-  for (int me = -1;;) {
-    if (me < 0) {
-      if (tid == 0) sh.popped = pop_ready(c, 0, total);
-      __syncthreads();
-      me = sh.popped;
-      if (me < 0) return;
-    }
-    if (tid < 32) ((int *)&sh.task)[tid] = __ldcg(tid == 1 ? c.succ_count + me : (const int *)(c.tasks + me) + tid);
-    const int mine = tid < MAX_SUCC ? __ldcg(c.succ + (size_t)me * MAX_SUCC + tid) : -1;
-    __syncthreads();
-    const int nz = code_single<64, SINGLE_THREADS>(c, sh, sh.y, g, sh.task.p[0], 0);
-    if (tid == SINGLE_THREADS - 1) {
+__device__ void luma_worker(const Ctx &c, IntraShared &sh) {
+  const Group<CODERS> g{(int)threadIdx.x, 1};
+  for (;;) {
+    record_bar<WORKER_THREADS>();
+    const int me = sh.task.me;
+    if (me < 0) return;
+    const int nz = code_single<64, CODERS>(c, sh, sh.y, g, sh.task.p[0], 0);
+    if (g.tid == CODERS - 1) {
       BlockInfo *gb = c.blocks + me;
       gb->tx_depth = 0;
       gb->interp_filter = sh.task.interp;
@@ -1997,130 +2080,504 @@ __device__ void luma_worker(const Ctx &c, IntraShared &sh, int total) {
       gb->tx_types_lo &= ~15;
       gb->eob[0] = nz;
     }
-    me = release(c, &sh.next, me, 0, successor(c, me, sh.task.nsucc, mine));
+    coded_bar<WORKER_THREADS>();
   }
 }
 
-// Chroma: U and V at once, half of the CTA each.
-template <int NT>
-__device__ void chroma_worker(const Ctx &c, IntraShared &sh, int total) {
-  const int tid = threadIdx.x, plane = 1 + tid / NT;
-  const Group<NT> g{tid % NT, plane};
+// Chroma: U and V at once, half of the coding warps each.
+__device__ void chroma_worker(const Ctx &c, IntraShared &sh) {
+  constexpr int NT = CODERS / 2;
+  const int plane = 1 + (int)threadIdx.x / NT;
+  const Group<NT> g{(int)threadIdx.x % NT, plane};
   PlaneMem<32> &m = sh.uv[plane - 1];
-  for (int me = -1;;) {
-    if (me < 0) {
-      if (tid == 0) sh.popped = pop_ready(c, 1, total);
-      __syncthreads();
-      me = sh.popped;
-      if (me < 0) return;
-    }
-    if (tid < 32) ((int *)&sh.task)[tid] = __ldcg(tid == 1 ? c.succ_count + me : (const int *)(c.tasks + me) + tid);
-    const int mine = tid < MAX_SUCC ? __ldcg(c.succ + (size_t)me * MAX_SUCC + tid) : -1;
-    __syncthreads();
+  for (;;) {
+    record_bar<WORKER_THREADS>();
+    const int me = sh.task.me;
+    if (me < 0) return;
     const int nz = code_single<32, NT>(c, sh, m, g, sh.task.p[1], plane);
     if (g.tid == NT - 1) {
       BlockInfo *gb = c.blocks + me;
       gb->eob[plane] = nz;
       if ((sh.task.p[1].geo >> 19) & 1) (plane == 1 ? gb->cfl_alpha_u : gb->cfl_alpha_v) = m.alpha;
     }
-    me = release(c, &sh.next, me, 1, successor(c, me, sh.task.nsucc, mine));
+    coded_bar<WORKER_THREADS>();
   }
 }
 
-// Luma of one block with the transform type and depth searches: every depth
-// from the same pixels (BlockDecoded inside the block follows the depth's own
-// transform order), the winner re-coded last unless it already was.
-__device__ void search_luma(const Ctx &c, Smem &sm) {
-  const FrameParams *fp = c.fp;
-  BlockInfo &b = sm.blk;
-  const int bs = b.bsize, tid = threadIdx.x;
-  if (tid == 0) b.tx_depth = 0;
-  const int maxDepth = fp->tx_mode_select ? imin(MAX_TX_DEPTH, T(Max_Tx_Depth)[bs]) : 0;
-  if (maxDepth == 0) {
-    code_plane<false>(c, sm, 0, T(Max_Tx_Size_Rect)[bs]);
-    return;
+// ---- luma with the transform type and depth searches ---------------------------------------
+//
+// The candidates of a transform block do not depend on one another: a warp
+// takes each (at most 7 types up to 16 x 16, DCT alone above), with its own
+// scratch, and the least cost is chosen after one barrier. The depths follow
+// one another, every one from the same pixels; the best one's pixels, types
+// and levels are kept when a later depth overwrites them, instead of coding it
+// again. A transform block's candidates used to run one after another on the
+// whole CTA, 11,000 cycles each with ten barriers, for every depth and once
+// more for the winner.
+constexpr int SEARCH_CODERS = 256, SEARCH_WORKERS = SEARCH_CODERS + 32, CAND_RS = 17;
+struct Cand {
+  int32_t r[16 * CAND_RS], t[16 * CAND_RS], q[256];
+};
+struct SearchShared {
+  FrameParams fpc;
+  uint64_t qinv[3][2];
+  int32_t fmat[3][FMAT_SMALL], fmatT[3][FMAT_SMALL];
+  int smw[124];
+  IntraTask task;
+  int ahead[8][32];
+  long long cost[8];
+  int eob[8];
+  long long red[8];
+  int lo, hi, type0, anyNz, maxW, maxH;  // the block's tx_types, tx_type, eob[0], CfL limits as coded so far
+  int bestTypes[16], types[16], bestN, bestNz, bestW, bestH;
+  int above[132], left[132];             // the block's edges from the corner at [0]
+  __align__(4) uint8_t px[64 * 64], best[64 * 64], src[64 * 64];  // stride 64
+  int32_t bestCoef[64 * 64];
+  union {
+    PlaneMem<64> m;
+    Cand cand[SEARCH_CODERS / 32];
+  };
+};
+
+template <int LW>
+__device__ __forceinline__ void cand_rows(Cand &cd, const int32_t *MhT, int h, int lane) {
+  constexpr int W = 1 << LW;
+  for (int k = lane; k < h << LW; k += 32) {
+    int i = k >> LW, kk = k & (W - 1);
+    const int32_t *r = cd.r + i * CAND_RS, *m = MhT + kk;
+    int64_t s = 0;
+#pragma unroll
+    for (int j = 0; j < W; j++) s += (int64_t)r[j] * m[j * W];
+    cd.t[i * CAND_RS + kk] = (int32_t)round2l(s, 16);
   }
-  int w = block_w(bs), h = block_h(bs);
-  int rs = sm.rstride[0];
-  uint8_t *px = sm.recp[0] + b.mi_row * 4 * rs + b.mi_col * 4;
-  for (int k = tid; k < w * h; k += RT) sm.save[k] = px[(k / w) * rs + (k % w)];
-  __syncthreads();
-  long long best = -1;
-  int bestD = 0;
-  for (int d = 0; d <= maxDepth + 1; d++) {
-    int depth = d <= maxDepth ? d : bestD;
-    if (d == maxDepth + 1 && bestD == maxDepth) break;
-    if (d > 0) {
-      for (int k = tid; k < w * h; k += RT) px[(k / w) * rs + (k % w)] = sm.save[k];
-      __syncthreads();
-    }
-    long long cst = code_plane<false>(c, sm, 0, depth_tx_size(bs, depth)) + (long long)fp->lambda * 8 * depth;
-    if (d <= maxDepth && (best < 0 || cst < best)) {
-      best = cst;
-      bestD = depth;
-    }
-    if (d == maxDepth + 1) break;
+}
+template <int LH>
+__device__ __forceinline__ int64_t cand_col(const Cand &cd, const int32_t *Mv, int k2, int kk) {
+  constexpr int H = 1 << LH;
+  const int32_t *m = Mv + k2 * H;
+  int64_t s = 0;
+#pragma unroll
+  for (int i = 0; i < H; i++) s += (int64_t)m[i] * cd.t[i * CAND_RS + kk];
+  return s;
+}
+__device__ __forceinline__ int level_bits(int l) { return l == 0 ? 6 : 8 * (2 + 2 * (31 - __clz(iabs(l)))); }
+
+// One candidate type of a transform block up to 16 x 16 (prediction in sh.px
+// at (x, y) of the block): its levels (cd.q), its residual (cd.r), eob and
+// cost, by one warp (code_tx_block's candidate loop, k_recon.h:101-153).
+__device__ __noinline__ void eval_candidate(SearchShared &sh, Cand &cd, int ci, int type, int txSz, int x, int y, int lane) {
+  const FrameParams *fp = &sh.fpc;
+  const int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh, n = 1 << (lw + lh);
+  const uint8_t *sp = sh.src + y * 64 + x, *pp = sh.px + y * 64 + x;
+  for (int k = lane; k < n; k += 32) {
+    int i = k >> lw, j = k & (w - 1);
+    cd.r[i * CAND_RS + j] = (int)sp[i * 64 + j] - (int)pp[i * 64 + j];
   }
-  if (tid == 0) b.tx_depth = bestD;
-  __syncthreads();
+  __syncwarp();
+  const int rk = tx::row_kind(type), ck = tx::col_kind(type);
+  const int32_t *Mh = sh.fmatT[rk] + (lw == 2 ? 0 : lw == 3 ? 16 : 80), *Mv = sh.fmat[ck] + (lh == 2 ? 0 : lh == 3 ? 16 : 80);
+  if (lane == 0) {
+    WORK(W_REC_FWD_MAC, n * w + n * h);
+    WORK(W_REC_QUANT, n);
+  }
+  if (lw == 2) cand_rows<2>(cd, Mh, h, lane);
+  else if (lw == 3) cand_rows<3>(cd, Mh, h, lane);
+  else cand_rows<4>(cd, Mh, h, lane);
+  __syncwarp();
+  const int dcQ = fp->dc_q[0], acQ = fp->ac_q[0], shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
+  const uint64_t invDc = sh.qinv[0][0], invAc = sh.qinv[0][1];
+  const int16_t *inv = d_inv_scan + d_inv_scan_off[scan_class(type)][txSz];
+  int eob = 0;
+  for (int k = lane; k < n; k += 32) {
+    int k2 = k >> lw, kk = k & (w - 1);
+    int64_t s = lh == 2 ? cand_col<2>(cd, Mv, k2, kk) : lh == 3 ? cand_col<3>(cd, Mv, k2, kk) : cand_col<4>(cd, Mv, k2, kk);
+    s = s * ((int64_t)1 << shifts);
+    if (rect) s = round2l(s, 12) * 5793;
+    int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
+    int first = k == 0;
+    int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, 1, first ? invDc : invAc);  // dq_denom 1 up to 16 x 16
+    cd.q[k] = lv;
+    if (lv) eob = imax(eob, inv[k] + 1);
+  }
+  eob = __reduce_max_sync(0xffffffffu, eob);
+  __syncwarp();
+  int bits = 0, sse = 0;
+  if (eob == 0) {
+    bits = 8;
+    for (int k = lane; k < n; k += 32) {
+      int d = cd.r[(k >> lw) * CAND_RS + (k & (w - 1))];
+      sse += d * d;
+    }
+  } else {
+    for (int k = lane; k < n; k += 32)
+      if (inv[k] < eob) bits += level_bits(cd.q[k]);
+    bits = __reduce_add_sync(0xffffffffu, bits) + 8 * 6 + 8 * 2 * (31 - __clz(eob + 1));
+    const int rowShift = T(Transform_Row_Shift)[txSz];
+    if (lane == 0) WORK(W_REC_INV_OPS, 3 * n * (lw + lh));
+    if (lane < h) {
+      if (lw == 2) inv_row<2, CAND_RS, true>(cd.r, cd.q, lane, h, dcQ, acQ, 1, rect, rk, rowShift);
+      else if (lw == 3) inv_row<3, CAND_RS, true>(cd.r, cd.q, lane, h, dcQ, acQ, 1, rect, rk, rowShift);
+      else inv_row<4, CAND_RS, true>(cd.r, cd.q, lane, h, dcQ, acQ, 1, rect, rk, rowShift);
+    }
+    __syncwarp();
+    if (lane < w) {
+      if (lh == 2) inv_col<2, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
+      else if (lh == 3) inv_col<3, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
+      else inv_col<4, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
+    }
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) {
+      int i = k >> lw, j = k & (w - 1);
+      int d = (int)sp[i * 64 + j] - clip1((int)pp[i * 64 + j] + cd.r[i * CAND_RS + j]);
+      sse += d * d;
+    }
+  }
+  sse = __reduce_add_sync(0xffffffffu, sse);  // at most 256 * 255^2
+  if (lane == 0) {
+    sh.cost[ci] = (long long)sse * 16 + (long long)fp->lambda * bits / 8;
+    sh.eob[ci] = eob;
+  }
 }
 
-__device__ void luma_search_worker(const Ctx &cg, Smem &sm, int total) {
-  const Ctx c = load_shared<false>(cg, sm);
-  const int tid = threadIdx.x;
-  for (int me = -1;;) {
-    if (me < 0) {
-      if (tid == 0) sm.flag = pop_ready(c, 0, total);
-      __syncthreads();
-      me = sm.flag;
-      __syncthreads();
-      if (me < 0) return;
+__device__ __forceinline__ long long group_sum(SearchShared &sh, const Group<SEARCH_CODERS> &g, long long v) {
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  g.sync();
+  if ((g.tid & 31) == 0) sh.red[g.tid >> 5] = v;
+  g.sync();
+  v = 0;
+  for (int k = 0; k < SEARCH_CODERS / 32; k++) v += sh.red[k];
+  return v;
+}
+
+// A transform block with a length above 16 (DCT alone): the group's threads
+// together; its reconstruction goes to sh.px, its levels to coefOut. Returns
+// the cost; *eobOut the eob.
+__device__ __noinline__ long long code_large(const Ctx &c, SearchShared &sh, const Group<SEARCH_CODERS> g, int txSz, int x, int y,
+                                             int32_t *coefOut, int *eobOut) {
+  const FrameParams *fp = &sh.fpc;
+  PlaneMem<64> &m = sh.m;
+  constexpr int NT = SEARCH_CODERS, RS = 65;
+  const int tid = g.tid, lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh;
+  const int tw = imin(32, w), th = imin(32, h), ltw = imin(5, lw);
+  for (int k = tid; k < w * h; k += NT) {
+    int i = k >> lw, j = k & (w - 1), p = sh.px[(y + i) * 64 + x + j];
+    m.px[k] = (uint8_t)p;
+    m.resid[i * RS + j] = (int)sh.src[(y + i) * 64 + x + j] - p;
+  }
+  g.sync();
+  const int32_t *Mh = lw <= 4 ? sh.fmatT[0] + (lw == 2 ? 0 : lw == 3 ? 16 : 80) : c.mats_t + fwd_slot(0, lw);
+  const int32_t *Mv = lh <= 4 ? sh.fmat[0] + (lh == 2 ? 0 : lh == 3 ? 16 : 80) : c.mats + fwd_slot(0, lh);
+  if (tid == 0) {
+    WORK(W_REC_FWD_MAC, h * tw * w + th * tw * h);
+    WORK(W_REC_QUANT, th * tw);
+  }
+  switch (lw) {
+    case 3: fwd_rows_g<3, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
+    case 4: fwd_rows_g<4, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
+    case 5: fwd_rows_g<5, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
+    default: fwd_rows_g<6, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
+  }
+  g.sync();
+  const int dcQ = fp->dc_q[0], acQ = fp->ac_q[0], shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
+  const int denom = tx::dq_denom(txSz);
+  const uint64_t invDc = sh.qinv[0][0], invAc = sh.qinv[0][1];
+  const int16_t *inv = d_inv_scan + d_inv_scan_off[0][txSz];
+  int eob = 0;
+  for (int k = tid; k < th * tw; k += NT) {
+    int k2 = k >> ltw, kk = k & (tw - 1);
+    int64_t s;
+    switch (lh) {
+      case 3: s = fwd_col_g<3>(m.tmp, Mv, k2, kk); break;
+      case 4: s = fwd_col_g<4>(m.tmp, Mv, k2, kk); break;
+      case 5: s = fwd_col_g<5>(m.tmp, Mv, k2, kk); break;
+      default: s = fwd_col_g<6>(m.tmp, Mv, k2, kk); break;
     }
-    IntraTask *task = c.tasks + me;
-    if (tid < (int)(sizeof(BlockInfo) / 4)) ((int *)&sm.blk)[tid] = __ldcg((const int *)(c.blocks + me) + tid);
-    if (tid == 32) {
-      int sb = me / MAX_BLOCKS_PER_SB;
-      sm.me = me;
-      sm.r0 = (sb / c.fp->sb_cols) * 16;
-      sm.c0 = (sb % c.fp->sb_cols) * 16;
-      sm.maxLumaW = sm.maxLumaH = 0;
+    s = s * ((int64_t)1 << shifts);
+    if (rect) s = round2l(s, 12) * 5793;
+    int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
+    int first = k == 0;
+    int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
+    m.q[k] = tx::dequant_level(lv, first ? dcQ : acQ, denom);
+    coefOut[k] = lv;
+    if (lv) eob = imax(eob, inv[k] + 1);
+  }
+  eob = __reduce_max_sync(0xffffffffu, eob);
+  if ((tid & 31) == 0) sh.eob[tid >> 5] = eob;
+  g.sync();
+  for (int k = 0; k < NT / 32; k++) eob = imax(eob, sh.eob[k]);
+  long long bits = 0, sse = 0;
+  if (eob == 0) {
+    bits = tid == 0 ? 8 : 0;
+  } else {
+    for (int k = tid; k < th * tw; k += NT)
+      if (inv[k] < eob) bits += level_bits(coefOut[k]);  // this thread's own stores
+    if (tid == 0) bits += 8 * 6 + 8 * 2 * (31 - __clz(eob + 1));
+    if (tid == 0) WORK(W_REC_INV_OPS, 3 * (1 << (lw + lh)) * (lw + lh));
+    inverse_large<64, NT>(m, g, lw, lh, DCT_DCT, txSz, dcQ, acQ);
+  }
+  for (int k = tid; k < w * h; k += NT) {
+    int i = k >> lw, j = k & (w - 1), v = m.px[k];
+    int d = (int)sh.src[(y + i) * 64 + x + j] - v;
+    sse += d * d;
+    sh.px[(y + i) * 64 + x + j] = (uint8_t)v;
+  }
+  sse = group_sum(sh, g, sse);
+  bits = group_sum(sh, g, bits);
+  *eobOut = eob;
+  return sse * 16 + (long long)fp->lambda * bits / 8;
+}
+
+// The block's luma at one transform size (code_plane, k_recon.h:190-291):
+// returns the cost. sh.types lists the transform blocks' types, *nTx their number.
+__device__ long long code_depth(const Ctx &c, SearchShared &sh, const Group<SEARCH_CODERS> &g, int txSz, int *nTx) {
+  const FrameParams *fp = &sh.fpc;
+  const PlaneTask &t = sh.task.p[0];
+  const int tid = g.tid, lane = tid & 31, warp = tid >> 5;
+  const unsigned geo = t.geo;
+  const int bw = 1 << (geo & 7), bh = 1 << ((geo >> 3) & 7), mode = (geo >> 6) & 15;
+  const int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh;
+  const int maxX = fp->mi_cols * 4 - 1, maxY = fp->mi_rows * 4 - 1;
+  const int set = get_tx_set(txSz, 0, fp->reduced_tx_set);
+  unsigned cands = 0;  // types, a nibble each, in the set's order
+  int numCands = 0;
+  if (!fp->tx_search || set == TX_SET_DCTONLY) {
+    numCands = 1;
+  } else {
+    for (int k = 0; k < 16; k++)
+      if (tx_type_in_set(set, k, 0)) cands |= (unsigned)k << (4 * numCands++);
+  }
+  pred::IntraArgs ia;
+  ia.mode = mode;
+  ia.angleDelta = sh.task.angle_y;
+  ia.log2W = lw;
+  ia.log2H = lh;
+  ia.edgeFilter = fp->enable_intra_edge_filter;
+  ia.filterType = (sh.task.interp >> 4) & 1;
+  pred::IntraState st;
+  pred::intra_state(ia, &st);
+  EdgePrep e = {st.pAngle, st.dx, st.dy, st.upAbove, st.upLeft, 0, 0, 0, 0, 0};
+  const bool filtered = intra_is_directional(mode) && ia.edgeFilter && st.pAngle != 90 && st.pAngle != 180;
+  PlaneMem<64> &m = sh.m;
+  // the edge arrays lie behind the candidates' scratch
+  static_assert(offsetof(PlaneMem<64>, edge) >= sizeof(Cand) * (SEARCH_CODERS / 32), "edges and candidates overlap");
+  int *above = m.edge[0] + EDGE_OFF, *left = m.edge[1] + EDGE_OFF;
+  long long total = 0;
+  int idx = 0;
+  for (int y = 0; y < bh; y += h)
+    for (int x = 0; x < bw; x += w) {
+      const int X = t.x + x, Y = t.y + y;
+      if (X > maxX || Y > maxY) continue;
+      const int haveLeft = ((geo >> 10) & 1) || x > 0, haveAbove = ((geo >> 11) & 1) || y > 0;
+      const int ar = y == 0 ? (x + w == bw ? sh.task.bits & 1 : 1) : x + w < bw;
+      const int bl = x == 0 ? (y + h == bh ? (sh.task.bits >> 1) & 1 : 1) : 0;
+      {
+        const int n = w + h, nA = imin(maxX, X + (ar ? 2 * w : w) - 1) - X + 1, nL = imin(maxY, Y + (bl ? 2 * h : h) - 1) - Y + 1;
+        // sample (x + dx, y - 1) / (x - 1, y + dy) of the block: its own pixels or its edges
+        auto up = [&](int d) { return y > 0 && (x > 0 || d >= 0) ? (int)sh.px[(y - 1) * 64 + x + d] : y > 0 ? sh.left[y] : sh.above[x + d + 1]; };
+        auto lf = [&](int d) { return x > 0 ? (int)sh.px[(y + d) * 64 + x - 1] : sh.left[y + d + 1]; };
+        for (int i = tid; i < 2 * n + 1; i += SEARCH_CODERS) {
+          if (i < n) above[i] = haveAbove ? up(imin(i, nA - 1)) : haveLeft ? lf(0) : 127;
+          else if (i < 2 * n) left[i - n] = haveLeft ? lf(imin(i - n, nL - 1)) : haveAbove ? up(0) : 129;
+          else above[-1] = left[-1] = haveAbove && haveLeft ? up(-1) : haveAbove ? up(0) : haveLeft ? lf(0) : 128;
+        }
+      }
+      g.sync();
+      if (filtered) {
+        e.corner = st.pAngle > 90 && st.pAngle < 180 && w + h >= 24;
+        e.sa = haveAbove ? pred::edge_strength(w, h, ia.filterType, st.pAngle - 90) : 0;
+        e.sl = haveLeft ? pred::edge_strength(w, h, ia.filterType, st.pAngle - 180) : 0;
+        e.za = imin(w, maxX - X + 1) + (st.pAngle < 90 ? h : 0) + 1;
+        e.zl = imin(h, maxY - Y + 1) + (st.pAngle > 180 ? w : 0) + 1;
+      }
+      prepare_edges(g, e, above, left, m.edge[2], m.edge[3], w, h);
+      const int dcv = mode == DC_PRED ? dc_value(above, left, lw, lh, haveAbove, haveLeft) : 0;
+      if (tid == 0) WORK(W_REC_INTRA_PX, w * h);
+      const int *wX = sh.smw + w - 4, *wY = sh.smw + h - 4;
+      for (int k = tid; k < (w * h) >> 2; k += SEARCH_CODERS) {
+        int i = k >> (lw - 2), j0 = (k & ((w >> 2) - 1)) * 4, p[4];
+        predict4(mode, e, above, left, wX, wY, w, h, i, j0, dcv, p);
+        *(uint32_t *)(sh.px + (y + i) * 64 + x + j0) =
+            (uint32_t)(p[0] & 255) | (uint32_t)(p[1] & 255) << 8 | (uint32_t)(p[2] & 255) << 16 | (uint32_t)(p[3] & 255) << 24;
+      }
+      g.sync();
+      int32_t *coefOut = c.coefs + sh.task.coef[0] + (idx << (lw + lh));
+      int type = DCT_DCT, eob = 0;
+      if (lw > 4 || lh > 4) {
+        total += code_large(c, sh, g, txSz, x, y, coefOut, &eob);
+      } else {
+        if (warp < numCands) eval_candidate(sh, sh.cand[warp], warp, (cands >> (4 * warp)) & 15, txSz, x, y, lane);
+        g.sync();
+        int bi = 0;
+        long long bc = sh.cost[0];
+        for (int k = 1; k < numCands; k++)
+          if (sh.cost[k] < bc) {
+            bc = sh.cost[k];
+            bi = k;
+          }
+        total += bc;
+        eob = sh.eob[bi];
+        const Cand &cd = sh.cand[bi];
+        if (eob) type = (cands >> (4 * bi)) & 15;
+        for (int k = tid; k < w * h; k += SEARCH_CODERS) {
+          coefOut[k] = cd.q[k];
+          if (eob) {
+            int i = k >> lw, j = k & (w - 1);
+            uint8_t *o = sh.px + (y + i) * 64 + x + j;
+            *o = (uint8_t)clip1((int)*o + cd.r[i * CAND_RS + j]);
+          }
+        }
+      }
+      if (tid == 0) {
+        if (idx < 16) sh.types[idx] = type;
+        if (idx == 0) sh.anyNz = 0;
+        sh.anyNz |= eob > 0;
+        sh.maxW = X + w;
+        sh.maxH = Y + h;
+      }
+      idx++;
+      g.sync();
     }
-    const int mine = tid < MAX_SUCC ? __ldcg(c.succ + (size_t)me * MAX_SUCC + tid) : -1;
-    const int nsucc = __ldcg(c.succ_count + me), cb = __ldcg(&task->bits);
-    __syncthreads();
-    stage_block<1>(c, sm, c.rec, cb);
-    search_luma(c, sm);
-    unstage_intra(c, sm, 1);
+  *nTx = idx;
+  return total;
+}
+
+__device__ __forceinline__ void set_types(SearchShared &sh, const int *types, int n) {
+  for (int k = 0; k < imin(n, 16); k++) {
+    int s = 4 * (k & 7);
+    int &v = k < 8 ? sh.lo : sh.hi;
+    v = (int32_t)(((uint32_t)v & ~(15u << s)) | (uint32_t)types[k] << s);
+  }
+  if (n > 0) sh.type0 = types[0];
+}
+
+__device__ void search_worker(const Ctx &c, SearchShared &sh) {
+  const Group<SEARCH_CODERS> g{(int)threadIdx.x, 1};
+  const FrameParams *fp = &sh.fpc;
+  const int tid = g.tid, fs = fp->stride[0];
+  for (;;) {
+    record_bar<SEARCH_WORKERS>();
+    const int me = sh.task.me;
+    if (me < 0) return;
+    const PlaneTask &t = sh.task.p[0];
+    const int lw = t.geo & 7, w = 1 << lw, h = 1 << ((t.geo >> 3) & 7), wl = lw - 2;
+    const uint8_t *sp = c.src + fp->offset[0] + (size_t)t.y * fs + t.x;
+    uint8_t *rp = c.rec + fp->offset[0] + (size_t)t.y * fs + t.x;
+    BlockInfo *gb = c.blocks + me;
+    const bool crosses = t.x + w > fp->mi_cols * 4 || t.y + h > fp->mi_rows * 4;  // transform blocks outside the frame stay as they are
+    {  // the block's edges (the corner at [0]), source and record
+      const int haveLeft = (t.geo >> 10) & 1, haveAbove = (t.geo >> 11) & 1, ext = imin(w, h);
+      const int nA = imin(t.lim & 0xffff, w + ext), nL = imin(t.lim >> 16, h + ext);
+      for (int i = tid; i < nA + nL + 2; i += SEARCH_CODERS) {
+        if (i <= nA) {
+          if (haveAbove && (i > 0 || haveLeft)) sh.above[i] = ldpx(rp - fs + i - 1);
+        } else if (haveLeft) {
+          int r = i - nA - 1;
+          if (r > 0 || haveAbove) sh.left[r] = ldpx(rp + (r - 1) * fs - 1);
+        }
+      }
+      for (int k = tid; k < (w * h) >> 2; k += SEARCH_CODERS) {
+        int i = k >> wl, j = 4 * (k & ((1 << wl) - 1));
+        *(uint32_t *)(sh.src + i * 64 + j) = __ldg((const uint32_t *)(sp + i * fs + j));
+      }
+      if (tid == 0) {
+        sh.lo = gb->tx_types_lo;
+        sh.hi = gb->tx_types_hi;
+        sh.type0 = gb->tx_type;
+        sh.anyNz = sh.maxW = sh.maxH = 0;
+      }
+    }
+    g.sync();
+    const int bs = sh.task.bsize;
+    const int maxDepth = fp->tx_mode_select ? imin(MAX_TX_DEPTH, T(Max_Tx_Depth)[bs]) : 0;
+    long long best = -1;
+    int bestD = 0;
+    for (int d = 0; d <= maxDepth; d++) {
+      if (crosses) {
+        for (int k = tid; k < (w * h) >> 2; k += SEARCH_CODERS) {
+          int i = k >> wl, j = 4 * (k & ((1 << wl) - 1));
+          *(uint32_t *)(sh.px + i * 64 + j) = __ldcg((const uint32_t *)(rp + i * fs + j));
+        }
+        g.sync();
+      }
+      const int txSz = depth_tx_size(bs, d);
+      int n = 0;
+      long long cst = code_depth(c, sh, g, txSz, &n) + (long long)fp->lambda * 8 * d;
+      if (tid == 0) set_types(sh, sh.types, n);
+      if (best < 0 || cst < best) {
+        best = cst;
+        bestD = d;
+        if (d < maxDepth) {  // kept for when a later depth has overwritten it
+          for (int k = tid; k < (w * h) >> 2; k += SEARCH_CODERS) {
+            int i = k >> wl, j = 4 * (k & ((1 << wl) - 1));
+            *(uint32_t *)(sh.best + i * 64 + j) = *(const uint32_t *)(sh.px + i * 64 + j);
+          }
+          const int32_t *cf = c.coefs + sh.task.coef[0];
+          for (int k = tid; k < w * h; k += SEARCH_CODERS) sh.bestCoef[k] = __ldcg(cf + k);
+          if (tid == 0) {
+            for (int k = 0; k < imin(n, 16); k++) sh.bestTypes[k] = sh.types[k];
+            sh.bestN = n;
+            sh.bestNz = sh.anyNz;
+            sh.bestW = sh.maxW;
+            sh.bestH = sh.maxH;
+          }
+        }
+      }
+      g.sync();
+    }
+    const uint8_t *px = sh.px;
+    if (bestD < maxDepth) {
+      // the winner's transform blocks over what the later depths left
+      px = sh.best;
+      const int txSz = depth_tx_size(bs, bestD), ltx = T(Tx_Width_Log2)[txSz] + T(Tx_Height_Log2)[txSz];
+      const int per = imin(32, 1 << T(Tx_Width_Log2)[txSz]) * imin(32, 1 << T(Tx_Height_Log2)[txSz]);
+      int32_t *cf = c.coefs + sh.task.coef[0];
+      for (int k = tid; k < sh.bestN << ltx; k += SEARCH_CODERS)
+        if ((k & ((1 << ltx) - 1)) < per) cf[k] = sh.bestCoef[k];
+      if (tid == 0) {
+        set_types(sh, sh.bestTypes, sh.bestN);
+        sh.anyNz = sh.bestNz;
+        sh.maxW = sh.bestW;
+        sh.maxH = sh.bestH;
+      }
+    }
+    for (int k = tid; k < (w * h) >> 2; k += SEARCH_CODERS) {
+      int i = k >> wl, j = 4 * (k & ((1 << wl) - 1));
+      *(uint32_t *)(rp + i * fs + j) = *(const uint32_t *)(px + i * 64 + j);
+    }
     if (tid == 0) {
-      BlockInfo *gb = c.blocks + me;
-      gb->tx_depth = sm.blk.tx_depth;
-      gb->interp_filter = sm.blk.interp_filter & 0x30;
-      gb->tx_type = sm.blk.tx_type;
-      gb->tx_types_lo = sm.blk.tx_types_lo;
-      gb->tx_types_hi = sm.blk.tx_types_hi;
-      gb->eob[0] = sm.blk.eob[0];
-      task->maxLumaW = sm.maxLumaW;  // the last transform block coded: CfL's limits
-      task->maxLumaH = sm.maxLumaH;
+      gb->tx_depth = bestD;
+      gb->interp_filter = sh.task.interp;
+      gb->tx_type = sh.type0;
+      gb->tx_types_lo = sh.lo;
+      gb->tx_types_hi = sh.hi;
+      gb->eob[0] = sh.anyNz;
+      c.tasks[me].maxLumaW = sh.maxW;  // the last transform block coded: CfL's limits
+      c.tasks[me].maxLumaH = sh.maxH;
     }
-    me = release(c, &sm.next, me, 0, successor(c, me, nsucc, mine));
+    coded_bar<SEARCH_WORKERS>();
   }
 }
 
 // Every intra block of the frame, one persistent launch: even CTAs code luma,
 // odd ones chroma.
 template <bool SEARCH>
-__global__ void __launch_bounds__(SEARCH ? SEARCH_THREADS : SINGLE_THREADS, SEARCH ? 1 : 3) k_recon_blocks(Ctx c) {
+__global__ void __launch_bounds__(SEARCH ? SEARCH_WORKERS : WORKER_THREADS, SEARCH ? 2 : 3) k_recon_blocks(Ctx c) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int total = c.counters[CNT_TOTAL], kind = blockIdx.x & 1;
+  const int total = c.counters[CNT_TOTAL], kind = blockIdx.x & 1, tid = threadIdx.x;
   if ((int)(blockIdx.x >> 1) >= imax(MIN_WORKERS, total / BLOCKS_PER_WORKER)) return;
   if (SEARCH && kind == 0) {
-    luma_search_worker(c, *(Smem *)smem_raw, total);
+    SearchShared &sh = *(SearchShared *)smem_raw;
+    load_intra_shared(c, sh);
+    if (tid >= SEARCH_CODERS) feed<true, SEARCH_WORKERS>(c, sh, 0, total);
+    else search_worker(c, sh);
     return;
   }
   IntraShared &sh = *(IntraShared *)smem_raw;
   load_intra_shared(c, sh);
-  if (kind == 0) luma_worker(c, sh, total);
-  else chroma_worker<(SEARCH ? SEARCH_THREADS : SINGLE_THREADS) / 2>(c, sh, total);
+  if (tid >= WORKER_THREADS) return;
+  if (tid >= CODERS) feed<!SEARCH, WORKER_THREADS>(c, sh, kind, total);  // a luma search updates the records chroma reads
+  else if (kind == 0) luma_worker(c, sh);
+  else chroma_worker(c, sh);
 }
 
 // Lossless frames: the reconstruction is the source (the Walsh-Hadamard
@@ -2156,5 +2613,9 @@ __global__ void __launch_bounds__(INTRA_THREADS) k_recon_lossless(Ctx cg) {
     c.blocks[me] = sm.blk;
   }
 }
+
+constexpr size_t SMEM_SINGLE = sizeof(IntraShared);
+constexpr size_t SMEM_SEARCH = sizeof(SearchShared) > sizeof(IntraShared) ? sizeof(SearchShared) : sizeof(IntraShared);
+constexpr int SINGLE_THREADS = WORKER_THREADS, SEARCH_THREADS = SEARCH_WORKERS;
 
 }  // namespace rec

@@ -83,6 +83,7 @@ struct Ctx {
   struct IntraTask *tasks;
   int *dep_count, *succ_count, *succ;
   int *queue, *counters;
+  int *inter;           // the inter blocks: large ones from the front, smaller ones from the back
   // polls a dependency wait makes before it gives up (sets the error and
   // abort words); SPIN_LIMIT unless a test shortens it
   int spin_limit;
@@ -93,8 +94,9 @@ struct Ctx {
 };
 
 #define MAX_SUCC 96  // successors per block: at most 25 along each edge, with margin
-// Ctx::counters: intra blocks, then per kind (luma, chroma) slots claimed, blocks queued, blocks done
-enum { CNT_TOTAL, CNT_HEAD, CNT_TAIL = CNT_HEAD + 2, CNT_DONE = CNT_TAIL + 2, CNT_WORDS = 8 };
+// Ctx::counters: intra blocks, then per kind (luma, chroma) slots claimed, blocks queued, blocks done; the inter blocks of
+// at least 32x32 samples, the smaller ones, those taken
+enum { CNT_TOTAL, CNT_HEAD, CNT_TAIL = CNT_HEAD + 2, CNT_DONE = CNT_TAIL + 2, CNT_BIG = CNT_DONE + 2, CNT_SMALL, CNT_TAKEN, CNT_WORDS = 16 };
 
 #define TILE_OFF 4     // tile column of the block's first sample (word aligned; the left column at 3)
 #define TILE_Y 132     // luma tile stride: TILE_OFF + 2 * 64; rows -1 .. 127
@@ -102,7 +104,7 @@ enum { CNT_TOTAL, CNT_HEAD, CNT_TAIL = CNT_HEAD + 2, CNT_DONE = CNT_TAIL + 2, CN
 #define FMAT_SMALL 336 // 4 * 4 + 8 * 8 + 16 * 16
 
 struct Smem {
-  int32_t resid[64 * 64];  // residual, then the inverse transform's plane
+  __align__(16) int32_t resid[64 * 64];  // residual, then the inverse transform's plane
   int32_t tmp[64 * 32];    // forward row pass output
   int32_t q[32 * 32];      // levels of the current candidate
   int32_t qbest[32 * 32];  // levels kept by the tx type search
@@ -436,31 +438,281 @@ __global__ void k_transpose_mats(const int32_t *mats, int32_t *matsT) {
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) t[(e % n) * n + e / n] = m[e];
 }
 
-// Forward row pass at a fixed width: row i of the residual (sm.resid,
-// stride 64) times the kept TW rows of the Q20 matrix (read from its
-// transpose MhT), 64-bit sums rounded by 16 bits into sm.tmp (stride 32).
-template <int LW>
-__device__ void fwd_rows(Smem &sm, const int32_t *MhT, int h) {
-  constexpr int W = 1 << LW, LTW = LW < 5 ? LW : 5, TW = 1 << LTW;
-  for (int k = threadIdx.x; k < h * TW; k += RT) {
-    int i = k >> LTW, kk = k & (TW - 1);
-    const int32_t *r = sm.resid + i * 64, *m = MhT + kk;
-    int64_t s = 0;
+// Forward row pass: rows of the residual (RS apart) times the kept 32 (or w)
+// rows of the Q20 matrix (read from its transpose MhT), 64-bit sums rounded by
+// 16 bits into tmp (32 apart), by nt threads. Lengths up to 16: a thread an
+// output. Lengths 32 and 64: a warp takes 4 rows, a lane an output column, so
+// 4 matrix words and 4 16-byte residual words (the same for the whole warp)
+// serve 16 products; an output a thread, two loads a product, left the
+// multipliers waiting for shared memory.
+template <int LW, int RS>
+__device__ __forceinline__ void fwd_rows(const int32_t *resid, int32_t *tmp, const int32_t *MhT, int h, int tid, int nt) {
+  constexpr int W = 1 << LW;
+  if constexpr (LW <= 4) {
+    for (int k = tid; k < h << LW; k += nt) {
+      int i = k >> LW, kk = k & (W - 1);
+      const int32_t *r = resid + i * RS, *m = MhT + kk;
+      int64_t s = 0;
 #pragma unroll
-    for (int j = 0; j < W; j++) s += (int64_t)r[j] * m[j * W];
-    sm.tmp[i * 32 + kk] = (int32_t)round2l(s, 16);
+      for (int j = 0; j < W; j++) s += (int64_t)r[j] * m[j * W];
+      tmp[i * 32 + kk] = (int32_t)round2l(s, 16);
+    }
+  } else {
+    static_assert(RS % 4 == 0, "16-byte residual words");
+    const int kk = tid & 31;
+    for (int i = (tid >> 5) * 4; i < h; i += nt >> 3) {
+      int64_t s[4] = {0, 0, 0, 0};
+#pragma unroll 4
+      for (int j = 0; j < W; j += 4) {
+        int32_t m[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) m[q] = MhT[(j + q) * W + kk];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          int4 v = *(const int4 *)(resid + (i + r) * RS + j);
+          s[r] += (int64_t)v.x * m[0];
+          s[r] += (int64_t)v.y * m[1];
+          s[r] += (int64_t)v.z * m[2];
+          s[r] += (int64_t)v.w * m[3];
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++) tmp[(i + r) * 32 + kk] = (int32_t)round2l(s[r], 16);
+    }
+  }
+}
+template <int RS>
+__device__ __forceinline__ void fwd_rows_any(int lw, const int32_t *resid, int32_t *tmp, const int32_t *MhT, int h, int tid, int nt) {
+  switch (lw) {
+    case 2: fwd_rows<2, RS>(resid, tmp, MhT, h, tid, nt); break;
+    case 3: fwd_rows<3, RS>(resid, tmp, MhT, h, tid, nt); break;
+    case 4: fwd_rows<4, RS>(resid, tmp, MhT, h, tid, nt); break;
+    case 5: fwd_rows<5, RS>(resid, tmp, MhT, h, tid, nt); break;
+    default: if (RS > 64 || RS == 64) fwd_rows<6, RS>(resid, tmp, MhT, h, tid, nt); break;
   }
 }
 
-// Forward column sum at a fixed height for output (k2, kk).
+// Forward column pass: emit(k, sum) for output k = k2 * tw + kk of the th x tw
+// kept ones. The same split: lengths 32 and 64 give a thread 4 outputs of a
+// column.
+template <int LH, class Emit>
+__device__ __forceinline__ void fwd_cols(const int32_t *tmp, const int32_t *Mv, int ltw, int tid, int nt, Emit emit) {
+  constexpr int H = 1 << LH, TH = H < 32 ? H : 32;
+  const int tw = 1 << ltw, kk = tid & (tw - 1);  // nt is a multiple of tw
+  if constexpr (LH <= 4) {
+    for (int k = tid; k < TH << ltw; k += nt) {
+      const int32_t *m = Mv + (k >> ltw) * H;
+      int64_t s = 0;
+#pragma unroll
+      for (int i = 0; i < H; i++) s += (int64_t)m[i] * tmp[i * 32 + kk];
+      emit(k, s);
+    }
+  } else {
+    for (int k2 = (tid >> ltw) * 4; k2 < TH; k2 += (nt >> ltw) * 4) {
+      int64_t s[4] = {0, 0, 0, 0};
+#pragma unroll 4
+      for (int i = 0; i < H; i += 4) {
+        int32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = tmp[(i + q) * 32 + kk];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          int4 m = *(const int4 *)(Mv + (k2 + r) * H + i);
+          s[r] += (int64_t)m.x * v[0];
+          s[r] += (int64_t)m.y * v[1];
+          s[r] += (int64_t)m.z * v[2];
+          s[r] += (int64_t)m.w * v[3];
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++) emit((k2 + r) << ltw | kk, s[r]);
+    }
+  }
+}
+template <class Emit>
+__device__ __forceinline__ void fwd_cols_any(int lh, const int32_t *tmp, const int32_t *Mv, int ltw, int tid, int nt, Emit emit) {
+  switch (lh) {
+    case 2: fwd_cols<2>(tmp, Mv, ltw, tid, nt, emit); break;
+    case 3: fwd_cols<3>(tmp, Mv, ltw, tid, nt, emit); break;
+    case 4: fwd_cols<4>(tmp, Mv, ltw, tid, nt, emit); break;
+    case 5: fwd_cols<5>(tmp, Mv, ltw, tid, nt, emit); break;
+    default: fwd_cols<6>(tmp, Mv, ltw, tid, nt, emit); break;
+  }
+}
+// A column sum as the quantiser takes it (k_fwd.h:92-110).
+__device__ __forceinline__ int fwd_scale(int64_t s, int shifts, int rect) {
+  s = s * ((int64_t)1 << shifts);
+  if (rect) s = round2l(s, 12) * 5793;
+  return (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
+}
+
+// ---- one transform type candidate in a warp -------------------------------------------
+// Scratch: residual, then the inverse transform (rows CAND_RS apart), the
+// forward row pass, the levels.
+constexpr int CAND_RS = 17;
+struct Cand {
+  int32_t r[16 * CAND_RS], t[16 * CAND_RS], q[256];
+};
+// Source and prediction at the transform block, the forward matrices (rows
+// transposed), the quantiser's steps and reciprocals, lambda.
+struct CandIn {
+  const uint8_t *sp, *pp;
+  int ss, ps;
+  const int32_t *Mh, *Mv;
+  int dcQ, acQ;
+  uint64_t invDc, invAc;
+  int lambda;
+};
+template <int LW>
+__device__ __forceinline__ void cand_rows(Cand &cd, const int32_t *MhT, int h, int lane) {
+  constexpr int W = 1 << LW;
+  for (int k = lane; k < h << LW; k += 32) {
+    int i = k >> LW, kk = k & (W - 1);
+    const int32_t *r = cd.r + i * CAND_RS, *m = MhT + kk;
+    int64_t s = 0;
+#pragma unroll
+    for (int j = 0; j < W; j++) s += (int64_t)r[j] * m[j * W];
+    cd.t[i * CAND_RS + kk] = (int32_t)round2l(s, 16);
+  }
+}
 template <int LH>
-__device__ __forceinline__ int64_t fwd_col(const Smem &sm, const int32_t *Mv, int k2, int kk) {
+__device__ __forceinline__ int64_t cand_col(const Cand &cd, const int32_t *Mv, int k2, int kk) {
   constexpr int H = 1 << LH;
   const int32_t *m = Mv + k2 * H;
   int64_t s = 0;
 #pragma unroll
-  for (int i = 0; i < H; i++) s += (int64_t)m[i] * sm.tmp[i * 32 + kk];
+  for (int i = 0; i < H; i++) s += (int64_t)m[i] * cd.t[i * CAND_RS + kk];
   return s;
+}
+__device__ __forceinline__ int level_bits(int l) { return l == 0 ? 6 : 8 * (2 + 2 * (31 - __clz(iabs(l)))); }
+
+// One candidate type of a transform block up to 16 x 16 by one warp (the
+// candidate loop of code_tx_block, k_recon.h:101-153): its levels in cd.q, its
+// residual in cd.r (flipped types: in transform order), its eob; returns its
+// cost.
+__device__ __noinline__ long long cand_cost(const CandIn &in, Cand &cd, int type, int txSz, int lane, int *eobOut) {
+  const int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh, n = 1 << (lw + lh);
+  const int fx = tx::flip_lr(type) ? w - 1 : 0, fy = tx::flip_ud(type) ? h - 1 : 0;  // j ^ fx mirrors j
+  for (int k = lane; k < n; k += 32) {
+    int i = k >> lw, j = k & (w - 1), y = i ^ fy, x = j ^ fx;
+    cd.r[i * CAND_RS + j] = (int)in.sp[y * in.ss + x] - (int)in.pp[y * in.ps + x];
+  }
+  __syncwarp();
+  const int rk = tx::row_kind(type), ck = tx::col_kind(type);
+  if (lane == 0) {
+    WORK(W_REC_FWD_MAC, n * w + n * h);
+    WORK(W_REC_QUANT, n);
+  }
+  if (lw == 2) cand_rows<2>(cd, in.Mh, h, lane);
+  else if (lw == 3) cand_rows<3>(cd, in.Mh, h, lane);
+  else cand_rows<4>(cd, in.Mh, h, lane);
+  __syncwarp();
+  const int shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
+  const int16_t *inv = d_inv_scan + d_inv_scan_off[scan_class(type)][txSz];
+  int eob = 0;
+  for (int k = lane; k < n; k += 32) {
+    int k2 = k >> lw, kk = k & (w - 1);
+    int64_t s = lh == 2 ? cand_col<2>(cd, in.Mv, k2, kk) : lh == 3 ? cand_col<3>(cd, in.Mv, k2, kk) : cand_col<4>(cd, in.Mv, k2, kk);
+    int first = k == 0;
+    int lv = tx::quant_level(fwd_scale(s, shifts, rect), first ? in.dcQ : in.acQ, first ? 26 : 22, 1, first ? in.invDc : in.invAc);  // dq_denom 1 up to 16 x 16
+    cd.q[k] = lv;
+    if (lv) eob = imax(eob, inv[k] + 1);
+  }
+  eob = __reduce_max_sync(0xffffffffu, eob);
+  __syncwarp();
+  int bits = 0, sse = 0;
+  if (eob == 0) {
+    bits = 8;
+    for (int k = lane; k < n; k += 32) {
+      int d = cd.r[(k >> lw) * CAND_RS + (k & (w - 1))];
+      sse += d * d;
+    }
+  } else {
+    for (int k = lane; k < n; k += 32)
+      if (inv[k] < eob) bits += level_bits(cd.q[k]);
+    bits = __reduce_add_sync(0xffffffffu, bits) + 8 * 6 + 8 * 2 * (31 - __clz(eob + 1));
+    const int rowShift = T(Transform_Row_Shift)[txSz];
+    if (lane == 0) WORK(W_REC_INV_OPS, 3 * n * (lw + lh));
+    if (lane < h) {
+      if (lw == 2) inv_row<2, CAND_RS, true>(cd.r, cd.q, lane, h, in.dcQ, in.acQ, 1, rect, rk, rowShift);
+      else if (lw == 3) inv_row<3, CAND_RS, true>(cd.r, cd.q, lane, h, in.dcQ, in.acQ, 1, rect, rk, rowShift);
+      else inv_row<4, CAND_RS, true>(cd.r, cd.q, lane, h, in.dcQ, in.acQ, 1, rect, rk, rowShift);
+    }
+    __syncwarp();
+    if (lane < w) {
+      if (lh == 2) inv_col<2, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
+      else if (lh == 3) inv_col<3, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
+      else inv_col<4, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
+    }
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) {
+      int i = k >> lw, j = k & (w - 1), y = i ^ fy, x = j ^ fx;
+      int d = (int)in.sp[y * in.ss + x] - clip1((int)in.pp[y * in.ps + x] + cd.r[i * CAND_RS + j]);
+      sse += d * d;
+    }
+  }
+  sse = __reduce_add_sync(0xffffffffu, sse);  // at most 256 * 255^2
+  *eobOut = eob;
+  return (long long)sse * 16 + (long long)in.lambda * bits / 8;
+}
+
+// The type search of an inter transform block up to 16 x 16 (up to 16
+// candidates): the CTA's warps take them in turn, each keeping its best one's
+// scratch, and the first least cost is written out. Returns the eob.
+__device__ __noinline__ int search_types(const Ctx &c, Smem &sm, const uint8_t *sp, int ss, uint8_t *pp, int ps, int txSz, int plane,
+                                         const int *cands, int numCands, int32_t *coefOut, int *outType, long long *outCost) {
+  const FrameParams *fp = c.fp;
+  constexpr int WARPS = INTER_THREADS / 32;
+  static_assert(2 * WARPS * sizeof(Cand) <= offsetof(Smem, sse33), "two candidates a warp in the transform scratch");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh;
+  Cand *own = (Cand *)sm.resid + 2 * warp;
+  long long best = -1;
+  int bestI = 16, bestEob = 0, bestBuf = 0, cur = 0;
+  __syncthreads();
+  for (int ci = warp; ci < numCands; ci += WARPS) {
+    const int t = cands[ci];
+    const CandIn in = {sp, pp, ss, ps, c.mats_t + fwd_slot(tx::row_kind(t), lw), c.mats + fwd_slot(tx::col_kind(t), lh),
+                       fp->dc_q[plane], fp->ac_q[plane], sm.qinv[plane][0], sm.qinv[plane][1], fp->lambda};
+    int eob;
+    long long cost = cand_cost(in, own[cur], t, txSz, lane, &eob);
+    if (best < 0 || cost < best) {
+      best = cost;
+      bestI = ci;
+      bestEob = eob;
+      bestBuf = cur;
+      cur ^= 1;
+    }
+  }
+  if (lane == 0) {
+    sm.red[warp] = best;
+    sm.sse33[warp] = bestI;
+    sm.sse33[8 + warp] = bestEob;
+    sm.sse33[16 + warp] = bestBuf;
+  }
+  __syncthreads();
+  int bw = 0;
+  best = sm.red[0];
+  for (int k = 1; k < WARPS; k++)
+    if (sm.red[k] >= 0 && (sm.red[k] < best || (sm.red[k] == best && sm.sse33[k] < sm.sse33[bw]))) {
+      best = sm.red[k];
+      bw = k;
+    }
+  const int type = cands[sm.sse33[bw]], eob = sm.sse33[8 + bw];
+  const Cand &cd = ((Cand *)sm.resid)[2 * bw + sm.sse33[16 + bw]];
+  const int fx = tx::flip_lr(type) ? w - 1 : 0, fy = tx::flip_ud(type) ? h - 1 : 0;
+  for (int k = threadIdx.x; k < w * h; k += RT) {
+    coefOut[k] = cd.q[k];
+    if (eob) {
+      int i = k >> lw, j = k & (w - 1);
+      uint8_t *o = pp + (i ^ fy) * ps + (j ^ fx);
+      *o = (uint8_t)clip1((int)*o + cd.r[i * CAND_RS + j]);
+    }
+  }
+  __syncthreads();
+  *outType = eob ? type : DCT_DCT;
+  *outCost = best;
+  return eob;
 }
 
 // Transform, quantise and reconstruct one transform block whose prediction
@@ -537,7 +789,11 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
     return eob;
   }
 
-  int single = numCands == 1 && !fp->tx_mode_select;
+  if (INTER && numCands > 1 && lw <= 4 && lh <= 4)
+    return search_types(c, sm, src + y * stride + x, stride, rec + y * rs + x, rs, txSz, plane, cands, numCands, coefOut, outType,
+                        outCost);
+  // an inter block has no depth search: a single candidate's cost is not used
+  int single = numCands == 1;
   int shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
   int denom = tx::dq_denom(txSz);
   uint64_t invDc = sm.qinv[plane][0], invAc = sm.qinv[plane][1];  // derived once per CTA (load_shared)
@@ -558,36 +814,18 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
       WORK(W_REC_FWD_MAC, h * tw * w + th * tw * h);
       WORK(W_REC_QUANT, th * tw);
     }
-    switch (lw) {
-      case 2: fwd_rows<2>(sm, Mh, h); break;
-      case 3: fwd_rows<3>(sm, Mh, h); break;
-      case 4: fwd_rows<4>(sm, Mh, h); break;
-      case 5: fwd_rows<5>(sm, Mh, h); break;
-      default: fwd_rows<6>(sm, Mh, h); break;
-    }
+    fwd_rows_any<64>(lw, sm.resid, sm.tmp, Mh, h, tid, RT);
     __syncthreads();
     const int16_t *inv = d_inv_scan + d_inv_scan_off[scan_class(t)][txSz];
     int myEob = 0, myNz = 0;
     int ltw = imin(5, lw);
-    for (int k = tid; k < th * tw; k += RT) {
-      int k2 = k >> ltw, kk = k & (tw - 1);
-      int64_t s;
-      switch (lh) {
-        case 2: s = fwd_col<2>(sm, Mv, k2, kk); break;
-        case 3: s = fwd_col<3>(sm, Mv, k2, kk); break;
-        case 4: s = fwd_col<4>(sm, Mv, k2, kk); break;
-        case 5: s = fwd_col<5>(sm, Mv, k2, kk); break;
-        default: s = fwd_col<6>(sm, Mv, k2, kk); break;
-      }
-      s = s * ((int64_t)1 << shifts);
-      if (rect) s = round2l(s, 12) * 5793;
-      int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
+    fwd_cols_any(lh, sm.tmp, Mv, ltw, tid, RT, [&](int k, int64_t s) {
       int first = k == 0;
-      int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
+      int lv = tx::quant_level(fwd_scale(s, shifts, rect), first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
       sm.q[k] = lv;
       myNz |= lv != 0;
       if (!single && lv != 0) myEob = imax(myEob, inv[k] + 1);
-    }
+    });
     if (single) {
       // only "has coefficients" matters here (the writer derives the eob)
       int nz = __syncthreads_or(myNz);
@@ -1018,42 +1256,112 @@ __device__ long long code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
   return total;
 }
 
-// Inter prediction of a w x h block (spec 7.11.3.4), staged: the clamped
-// reference window (h + 7 rows of w + 7 samples) in shared memory, the
-// horizontal 8-tap pass of every window row (Round2 by InterRound0 = 3), then
-// the vertical pass per output sample - the values inter_sum forms sample
-// by sample (k_inter.h:451-504). mode 0: final samples (Round2 by 11,
-// clipped) into d (stride ds); 1: compound intermediates (Round2 by 7) into
-// sm.pred0; 2: Round2(pred0 + this block's intermediates, 5), clipped, into
-// d. Scratch: sm.tmp (window), sm.resid (horizontal pass).
-__device__ void predict_block(Smem &sm, const pred::Inter &ip, int lw, int h, int mode, uint8_t *d, int ds) {
-  int w = 1 << lw, W = w + 7, H = h + 7;
+// Inter prediction of a w x h block (spec 7.11.3.4) in three steps, staged in
+// shared memory: the clamped reference window (h + 7 rows of w + 7 samples),
+// the horizontal 8-tap pass of every window row (Round2 by InterRound0 = 3),
+// the vertical pass - the values inter_sum forms sample by sample
+// (k_inter.h:451-504). Every tap is even, so half taps (in 8 bits) give the
+// same rounded sum: (2 S + 4) >> 3 = (S + 2) >> 2, and a row's 4 sums take 8
+// byte dot products on 3 words instead of 32 loads and multiplies; the
+// vertical pass slides over 4 rows, 11 loads for 4 samples. Scratch: sm.tmp
+// (window), sm.resid (horizontal pass).
+constexpr int WIN_P = 80;  // window row pitch: up to 3 samples of alignment, 64 + 7 samples, a word for the last reads
+// The window's rows start at win + the returned offset. Inside the picture a
+// row is its aligned words; at its borders every sample is clamped.
+__device__ __noinline__ int load_window(Smem &sm, const uint8_t *ref, int stride, int lastX, int lastY, int ix0, int iy0, int w, int h) {
+  static_assert(sizeof(sm.tmp) >= (64 + 7) * WIN_P, "the window fits its scratch");
   uint8_t *win = (uint8_t *)sm.tmp;
-  if (threadIdx.x == 0) WORK(W_REC_INTER_PX, w * h);
+  const int W = w + 7, H = h + 7, lane = threadIdx.x & 31;
+  const int off = (int)((uintptr_t)(ref + ix0) & 3);  // rows are multiples of 32 samples apart
+  if (ix0 >= 0 && iy0 >= 0 && ix0 + W - 1 <= lastX && iy0 + H - 1 <= lastY) {
+    const uint8_t *q = ref + (size_t)iy0 * stride + ix0 - off;
+    const int nw = (off + W + 3) >> 2, n = H * nw;
+    const unsigned inv = 65535u / nw + 1;  // k / nw for k < 71 * 19
+    for (int base = threadIdx.x; base < n; base += 4 * RT) {
+      uint32_t v[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        int k = base + e * RT, R = (int)(k * inv >> 16);
+        if (k < n) v[e] = __ldg((const uint32_t *)(q + (size_t)R * stride) + (k - R * nw));
+      }
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        int k = base + e * RT, R = (int)(k * inv >> 16);
+        if (k < n) *(uint32_t *)(win + R * WIN_P + 4 * (k - R * nw)) = v[e];
+      }
+    }
+  } else {
+    for (int R = threadIdx.x >> 5; R < H; R += RT / 32) {
+      const uint8_t *row = ref + (size_t)clip3(0, lastY, iy0 + R) * stride;
+      for (int C = lane; C < W; C += 32) win[R * WIN_P + off + C] = __ldg(row + clip3(0, lastX, ix0 + C));
+    }
+  }
+  __syncthreads();
+  return off;
+}
+__device__ __forceinline__ int dp4(uint32_t px, int taps, int acc) {
+  int r;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(px), "r"(taps), "r"(acc));
+  return r;
+}
+__device__ __noinline__ void horizontal_pass(Smem &sm, int off, const int16_t *fh, int lw, int h) {
+  const uint8_t *win = (const uint8_t *)sm.tmp;
   int16_t *hs = (int16_t *)sm.resid;
-  for (int k = threadIdx.x; k < W * H; k += RT) {
-    int R = k / W, C = k - R * W;
-    win[k] = ip.ref[(size_t)clip3(0, ip.lastY, ip.iy0 + R) * ip.stride + clip3(0, ip.lastX, ip.ix0 + C)];
+  int t0 = 0, t1 = 0;
+  for (int t = 0; t < 4; t++) {
+    t0 |= ((fh[t] >> 1) & 255) << (8 * t);
+    t1 |= ((fh[t + 4] >> 1) & 255) << (8 * t);
+  }
+  const int lq = lw - 2, n = (h + 7) << lq;
+  for (int k = threadIdx.x; k < n; k += RT) {
+    int R = k >> lq, c = (k & ((1 << lq) - 1)) * 4;
+    const uint32_t *q = (const uint32_t *)(win + R * WIN_P + c);
+    // samples c .. c + 11 of the row, aligned
+    uint32_t a = __funnelshift_r(q[0], q[1], 8 * off), b = __funnelshift_r(q[1], q[2], 8 * off), d = __funnelshift_r(q[2], q[3], 8 * off);
+    int s0 = (dp4(b, t1, dp4(a, t0, 2))) >> 2;
+    int s1 = (dp4(__funnelshift_r(b, d, 8), t1, dp4(__funnelshift_r(a, b, 8), t0, 2))) >> 2;
+    int s2 = (dp4(__funnelshift_r(b, d, 16), t1, dp4(__funnelshift_r(a, b, 16), t0, 2))) >> 2;
+    int s3 = (dp4(__funnelshift_r(b, d, 24), t1, dp4(__funnelshift_r(a, b, 24), t0, 2))) >> 2;
+    *(uint2 *)(hs + (R << lw) + c) = make_uint2((s0 & 0xffff) | (uint32_t)s1 << 16, (s2 & 0xffff) | (uint32_t)s3 << 16);
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < H * w; k += RT) {
-    int R = k >> lw, cc = k & (w - 1);
-    const uint8_t *row = win + R * W + cc;
-    int s = 0;
+}
+// The vertical pass; out(row, column, sum before its rounding).
+template <class Out>
+__device__ __forceinline__ void vertical_pass(Smem &sm, const int16_t *fv, int lw, int h, Out out) {
+  const int16_t *hs = (const int16_t *)sm.resid;
+  const int w = 1 << lw, n = (h >> 2) << lw;
+  int f[8];
+  for (int t = 0; t < 8; t++) f[t] = fv[t];
+  for (int k = threadIdx.x; k < n; k += RT) {
+    int r = (k >> lw) * 4, c = k & (w - 1);
+    int v[11];
 #pragma unroll
-    for (int t = 0; t < 8; t++) s += ip.fh[t] * (int)row[t];
-    hs[k] = (int16_t)round2(s, 3);
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < h * w; k += RT) {
-    int r = k >> lw, cc = k & (w - 1);
-    int acc = 0;
+    for (int t = 0; t < 11; t++) v[t] = hs[((r + t) << lw) + c];
 #pragma unroll
-    for (int tv = 0; tv < 8; tv++) acc += ip.fv[tv] * (int)hs[(r + tv) * w + cc];
-    if (mode == 0) d[r * ds + cc] = (uint8_t)clip1(round2(acc, 11));
-    else if (mode == 1) sm.pred0[k] = (int16_t)round2(acc, 7);
-    else d[r * ds + cc] = (uint8_t)clip1(round2((int)sm.pred0[k] + round2(acc, 7), 5));
+    for (int q = 0; q < 4; q++) {
+      int acc = 0;
+#pragma unroll
+      for (int t = 0; t < 8; t++) acc += f[t] * v[q + t];
+      out(r + q, c, acc);
+    }
   }
+}
+// mode 0: final samples (Round2 by 11, clipped) into d (stride ds); 1:
+// compound intermediates (Round2 by 7) into sm.pred0; 2: Round2(pred0 + this
+// block's intermediates, 5), clipped, into d.
+__device__ __noinline__ void predict_block(Smem &sm, const pred::Inter &ip, int lw, int h, int mode, uint8_t *d, int ds) {
+  if (threadIdx.x == 0) WORK(W_REC_INTER_PX, h << lw);
+  const int off = load_window(sm, ip.ref, ip.stride, ip.lastX, ip.lastY, ip.ix0, ip.iy0, 1 << lw, h);
+  horizontal_pass(sm, off, ip.fh, lw, h);
+  if (mode == 0)
+    vertical_pass(sm, ip.fv, lw, h, [&](int r, int c, int acc) { d[r * ds + c] = (uint8_t)clip1(round2(acc, 11)); });
+  else if (mode == 1)
+    vertical_pass(sm, ip.fv, lw, h, [&](int r, int c, int acc) { sm.pred0[(r << lw) + c] = (int16_t)round2(acc, 7); });
+  else
+    vertical_pass(sm, ip.fv, lw, h, [&](int r, int c, int acc) {
+      d[r * ds + c] = (uint8_t)clip1(round2((int)sm.pred0[(r << lw) + c] + round2(acc, 7), 5));
+    });
   __syncthreads();
 }
 
@@ -1087,18 +1395,19 @@ __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parit
 
 // The superblock's source (luma 64 rows of 64 bytes, two chroma planes of
 // 32 rows of 32 bytes) into sm.srcSB: one bulk copy per row, a thread each,
-// all completing on sm.bar. Rows are 16-byte aligned in the padded frame
+// all completing on sm.bar's phase. Rows are 16-byte aligned in the padded frame
 // layout (luma stride sb_cols * 64, chroma sb_cols * 32, superblock columns
 // at multiples of 64 / 32 bytes, plane offsets multiples of 64). On a wait
 // past the limit the error and abort words are set (status 4) and the copies
 // are waited for again before the CTA goes on, so none lands after it.
-__device__ void stage_sb_source(const Ctx &c, Smem &sm, int sb) {
+__device__ void stage_sb_source(const Ctx &c, Smem &sm, int sb, unsigned phase) {
   static_assert(INTER_THREADS == 128, "one thread per source row");
   const FrameParams *fp = c.fp;
   int sbr = sb / fp->sb_cols, sbc = sb % fp->sb_cols, t = threadIdx.x;
   if (t == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // the previous block's reads of the tile come before the copies into it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&sm.bar)),
                  "r"(64 * 64 + 2 * 32 * 32)
                  : "memory");
@@ -1111,12 +1420,12 @@ __device__ void stage_sb_source(const Ctx &c, Smem &sm, int sb) {
     bulk_row(sm.srcSB + 64 * 64 + (p - 1) * 32 * 32 + r * 32,
              c.src + fp->offset[p] + (size_t)(sbr * 32 + r) * fp->stride[p] + sbc * 32, 32, &sm.bar);
   }
-  if (!bar_wait(&sm.bar, 0, c.spin_limit)) {
+  if (!bar_wait(&sm.bar, phase, c.spin_limit)) {
     if (t == 0) {
       atomicExch(c.status, 4);
       atomicExch(c.status + 1, 1);
     }
-    bar_wait(&sm.bar, 0, c.spin_limit);
+    bar_wait(&sm.bar, phase, c.spin_limit);
   }
 }
 
@@ -1149,6 +1458,46 @@ __device__ void unstage_inter(const Ctx &c, Smem &sm, int p) {
   __syncthreads();
 }
 
+// The dual interpolation filter search of a single-reference block
+// (k_recon.h:304-328): sm.blk's interp_filter.
+__device__ __noinline__ void filter_search(const Ctx &c, Smem &sm, const uint8_t *ref) {
+  const FrameParams *fp = c.fp;
+  BlockInfo &b = sm.blk;
+  const int bs = b.bsize, MiRow = b.mi_row, MiCol = b.mi_col, tid = threadIdx.x;
+  int w = block_w(bs), h = block_h(bs);
+  int x0 = MiCol * 4, y0 = MiRow * 4, stride = fp->stride[0], ss = sm.sstride[0];
+  const uint8_t *sp = sm.srcp[0] + y0 * ss + x0;
+  int vw = imin(w, fp->frame_w - x0), vh = imin(h, fp->frame_h - y0);
+  long long best = -1;
+  int bestPacked = 0, off = 0;
+  // the window once, a horizontal pass per horizontal filter, a vertical
+  // pass with its SSE per pair
+  for (int fh = 0; fh < 3; fh++)
+    for (int fv = 0; fv < 3; fv++) {
+      int packed = fv | (fh << 2);
+      pred::Inter ip;
+      pred::inter_setup(&ip, ref + fp->offset[0], stride, fp->frame_w, fp->frame_h, x0, y0, w, h, b.mv_row, b.mv_col,
+                        0, 0, packed);
+      if (fh == 0 && fv == 0) off = load_window(sm, ip.ref, ip.stride, ip.lastX, ip.lastY, ip.ix0, ip.iy0, w, h);
+      if (fv == 0) horizontal_pass(sm, off, ip.fh, floor_log2(w), h);
+      if (tid == 0) WORK(W_REC_INTER_PX, w * h);
+      int sse = 0;  // at most 32 samples of 255^2 a thread
+      vertical_pass(sm, ip.fv, floor_log2(w), h, [&](int r, int c, int acc) {
+        if (r < vh && c < vw) {
+          int d = clip1(round2(acc, 11)) - (int)sp[r * ss + c];
+          sse += d * d;
+        }
+      });
+      long long cst = cta_sum64(sse, sm) * 16 + (long long)fp->lambda * ((fv != 0) + (fh != 0));
+      if (best < 0 || cst < best) {
+        best = cst;
+        bestPacked = packed;
+      }
+    }
+  if (tid == 0) b.interp_filter = bestPacked;
+  __syncthreads();
+}
+
 // One inter block (recon_block, k_recon.h:293-394); sm.blk holds it. Its
 // planes are coded in sm.recT one after another, each written back after it.
 __device__ void recon_inter_block(const Ctx &c, Smem &sm, BlockInfo *gb) {
@@ -1158,7 +1507,7 @@ __device__ void recon_inter_block(const Ctx &c, Smem &sm, BlockInfo *gb) {
   int comp = b.ref_frame1 > INTRA_FRAME;
   const uint8_t *ref = b.ref_frame != LAST_FRAME ? c.gold : c.ref;
   const uint8_t *ref1 = c.gold;
-  int MiRow = b.mi_row, MiCol = b.mi_col;
+  const int MiRow = b.mi_row, MiCol = b.mi_col;
   if (threadIdx.x == 0) {
     sm.maxLumaW = sm.maxLumaH = 0;
     b.tx_depth = 0;
@@ -1167,38 +1516,7 @@ __device__ void recon_inter_block(const Ctx &c, Smem &sm, BlockInfo *gb) {
   if (threadIdx.x < 3) inter_views(c, sm, threadIdx.x);
   __syncthreads();
   int tid = threadIdx.x;
-  if (fp->switchable_interp && !comp) {
-    int w = block_w(bs), h = block_h(bs);
-    int x0 = MiCol * 4, y0 = MiRow * 4, stride = fp->stride[0], ss = sm.sstride[0], rs = sm.rstride[0];
-    uint8_t *px = sm.recp[0] + y0 * rs + x0;
-    const uint8_t *sp = sm.srcp[0] + y0 * ss + x0;
-    int vw = imin(w, fp->frame_w - x0), vh = imin(h, fp->frame_h - y0);
-    long long best = -1;
-    int bestPacked = 0;
-    for (int f = 0; f < 9; f++) {
-      int packed = (f % 3) | ((f / 3) << 2);
-      pred::Inter ip;
-      pred::inter_setup(&ip, ref + fp->offset[0], stride, fp->frame_w, fp->frame_h, x0, y0, w, h, b.mv_row, b.mv_col,
-                        0, 0, packed);
-      long long sse = 0;
-      predict_block(sm, ip, floor_log2(w), h, 0, px, rs);
-      for (int k = tid; k < w * h; k += RT) {
-        int i = k / w, j = k % w;
-        if (i < vh && j < vw) {
-          int d = (int)px[i * rs + j] - (int)sp[i * ss + j];
-          sse += d * d;
-        }
-      }
-      sse = cta_sum64(sse, sm);
-      long long cst = sse * 16 + (long long)fp->lambda * ((f % 3 != 0) + (f / 3 != 0));
-      if (best < 0 || cst < best) {
-        best = cst;
-        bestPacked = packed;
-      }
-    }
-    if (tid == 0) b.interp_filter = bestPacked;
-    __syncthreads();
-  }
+  if (fp->switchable_interp && !comp) filter_search(c, sm, ref);
   for (int plane = 0; plane < 3; plane++) {
     int sub = plane > 0, stride = fp->stride[plane];
     int baseX = (MiCol >> sub) * 4, baseY = (MiRow >> sub) * 4;
@@ -1254,25 +1572,32 @@ __device__ Ctx load_shared(const Ctx &c, Smem &sm) {
 
 
 
-// The inter blocks of the frame, one CTA per superblock (all at once: they
-// read reference pictures only).
+// The inter blocks of the frame (they read reference pictures only, so none
+// waits): persistent CTAs take them from the list, large ones first. With one
+// CTA per superblock the frame took as long as its most divided superblock
+// (2.4 ms for a 640x360 full-tool frame's 60, half of it now); CTAs assigned
+// by slot cost a 3840x2160 leaf frame 80 us in CTAs without a block.
 __global__ void __launch_bounds__(INTER_THREADS, 512 / INTER_THREADS) k_recon_inter(Ctx cg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *(Smem *)smem_raw;
+  const int big = cg.counters[CNT_BIG], total = big + cg.counters[CNT_SMALL], tid = threadIdx.x;
+  if ((int)blockIdx.x >= total) return;
   const Ctx c = load_shared<true>(cg, sm);
-  int sb = blockIdx.x, n = imax(0, imin(c.sbs[sb].num_blocks, MAX_BLOCKS_PER_SB));
-  if (threadIdx.x == 0) {
-    sm.r0 = (sb / c.fp->sb_cols) * 16;
-    sm.c0 = (sb % c.fp->sb_cols) * 16;
-  }
-  stage_sb_source(c, sm, sb);
-  for (int k = 0; k < n; k++) {
-    int me = sb * MAX_BLOCKS_PER_SB + k;
-    if (threadIdx.x == 0) sm.blk = c.blocks[me];
+  if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar)) : "memory");
+  for (unsigned phase = 0;; phase ^= 1) {
+    if (tid == 0) sm.flag = atomicAdd(c.counters + CNT_TAKEN, 1);
     __syncthreads();
-    if (sm.blk.is_inter) {
-      recon_inter_block(c, sm, c.blocks + me);
+    const int k = sm.flag;
+    if (k >= total) return;
+    const int me = c.inter[k < big ? k : c.nblk - 1 - (k - big)], sb = me / MAX_BLOCKS_PER_SB;
+    if (tid == 32) {
+      sm.r0 = (sb / c.fp->sb_cols) * 16;
+      sm.c0 = (sb % c.fp->sb_cols) * 16;
     }
+    if (tid < (int)(sizeof(BlockInfo) / 4)) ((int *)&sm.blk)[tid] = ((const int *)(c.blocks + me))[tid];
+    stage_sb_source(c, sm, sb, phase);
+    __syncthreads();
+    recon_inter_block(c, sm, c.blocks + me);
     __syncthreads();
   }
 }
@@ -1352,18 +1677,23 @@ __device__ PlaneTask plane_task(const FrameParams *fp, const BlockInfo &b, int s
   return t;
 }
 
-// Per frame, before the recon launch: the block index of every 4x4 luma unit
-// of the frame and the number of intra blocks (a CTA per superblock, a warp
-// per block, its lanes over the block's units).
+// Per frame, before the recon launches: the block index of every 4x4 luma
+// unit of the frame, the list of inter blocks and the number of intra blocks
+// (a CTA per superblock, a warp per block, its lanes over the block's units).
 constexpr int MAP_THREADS = 256;
 __global__ void __launch_bounds__(MAP_THREADS) k_block_map(const FrameParams *fp, const BlockInfo *blocks, const SbInfo *sbs, int *blkAt,
-                                                  int *total) {
+                                                  int *counters, int *inter, int nblk) {
   int sb = blockIdx.x, lane = threadIdx.x & 31, intra = 0;
   int cols = fp->mi_cols, rows = fp->mi_rows, n = imin(sbs[sb].num_blocks, MAX_BLOCKS_PER_SB);
   for (int k = threadIdx.x >> 5; k < n; k += MAP_THREADS / 32) {
     int idx = sb * MAX_BLOCKS_PER_SB + k;
     const BlockInfo &b = blocks[idx];
-    intra += !b.is_inter;
+    if (!b.is_inter) {
+      intra++;
+    } else if (lane == 0) {
+      if (block_w(b.bsize) * block_h(b.bsize) >= 32 * 32) inter[atomicAdd(counters + CNT_BIG, 1)] = idx;
+      else inter[nblk - 1 - atomicAdd(counters + CNT_SMALL, 1)] = idx;
+    }
     if (b.mi_row < 0 || b.mi_col < 0) continue;
     int h = imax(0, imin(T(Num_4x4_Blocks_High)[b.bsize], rows - b.mi_row));
     int lw = floor_log2(T(Num_4x4_Blocks_Wide)[b.bsize]), w = imax(0, imin(1 << lw, cols - b.mi_col));
@@ -1372,7 +1702,7 @@ __global__ void __launch_bounds__(MAP_THREADS) k_block_map(const FrameParams *fp
       if (c < w) blkAt[(b.mi_row + r) * cols + b.mi_col + c] = idx;
     }
   }
-  if (lane == 0 && intra) atomicAdd(total, intra);
+  if (lane == 0 && intra) atomicAdd(counters + CNT_TOTAL, intra);
 }
 
 // Orders this thread's (and, after a barrier, its CTA's) accesses before it
@@ -1479,9 +1809,11 @@ struct Group {
 // Working memory of a plane of at most MAXD x MAXD samples.
 template <int MAXD>
 struct PlaneMem {
-  int32_t resid[MAXD * (MAXD + 1)];  // residual, then the inverse transform's rows (stride MAXD + 1: rows in distinct banks)
+  // residual, then the inverse transform's rows: 16-byte aligned and 4 banks apart (8 rows a lane each meet no bank twice)
+  __align__(16) int32_t resid[MAXD * (MAXD + 4)];
   int32_t tmp[MAXD * 32];            // forward row pass; before it CfL's luma values
   int32_t q[32 * 32];
+  int32_t lv[MAXD == 64 ? 32 * 32 : 1];  // levels, where they are read again (code_large)
   int edge[4][EDGE_LEN];             // AboveRow, LeftCol, filter copies of both
   __align__(4) uint8_t px[MAXD * MAXD];  // prediction, then reconstruction (stride w)
   int sse[8][33];
@@ -1623,32 +1955,10 @@ __device__ __forceinline__ void predict4(int mode, const EdgePrep &e, const int 
   }
 }
 
-template <int LW, int RS, int NT>
-__device__ __forceinline__ void fwd_rows_g(const int32_t *resid, int32_t *tmp, const int32_t *MhT, int h, int tid) {
-  constexpr int W = 1 << LW, LTW = LW < 5 ? LW : 5, TW = 1 << LTW;
-  for (int k = tid; k < h * TW; k += NT) {
-    int i = k >> LTW, kk = k & (TW - 1);
-    const int32_t *r = resid + i * RS, *m = MhT + kk;
-    int64_t s = 0;
-#pragma unroll
-    for (int j = 0; j < W; j++) s += (int64_t)r[j] * m[j * W];
-    tmp[i * 32 + kk] = (int32_t)round2l(s, 16);
-  }
-}
-template <int LH>
-__device__ __forceinline__ int64_t fwd_col_g(const int32_t *tmp, const int32_t *Mv, int k2, int kk) {
-  constexpr int H = 1 << LH;
-  const int32_t *m = Mv + k2 * H;
-  int64_t s = 0;
-#pragma unroll
-  for (int i = 0; i < H; i++) s += (int64_t)m[i] * tmp[i * 32 + kk];
-  return s;
-}
-
 // Inverse transform of the dequantised levels in m.q, added into m.px.
 template <int MAXD, int NT, int LOW, int HIGH>
 __device__ __forceinline__ void inverse_g(PlaneMem<MAXD> &m, const Group<NT> &g, int lw, int lh, int type, int txSz, int dcQ, int acQ) {
-  constexpr int RS = MAXD + 1;
+  constexpr int RS = MAXD + 4;
   const int w = 1 << lw, h = 1 << lh, th = imin(32, h), rowShift = T(Transform_Row_Shift)[txSz], denom = tx::dq_denom(txSz);
   const int rect = iabs(lw - lh) == 1, rk = tx::row_kind(type), ck = tx::col_kind(type);
   if (HIGH >= 5 && lw >= 5) {
@@ -1797,7 +2107,7 @@ __device__ __forceinline__ void cfl_g(const Ctx &c, IntraShared &sh, PlaneMem<MA
 template <int MAXD, int NT>
 __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneMem<MAXD> &m, const Group<NT> g, const PlaneTask &t,
                                            int plane) {
-  constexpr int RS = MAXD + 1, MAXW = MAXD * MAXD / 4 / NT;
+  constexpr int RS = MAXD + 4, MAXW = MAXD * MAXD / 4 / NT;
   const FrameParams *fp = &sh.fpc;
   const int tid = g.tid, lane = tid & 31;
   const unsigned geo = t.geo;
@@ -1877,37 +2187,19 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
     WORK(W_REC_FWD_MAC, h * tw * w + th * tw * h);
     WORK(W_REC_QUANT, th * tw);
   }
-  switch (lw) {
-    case 2: if (MAXD == 32) fwd_rows_g<2, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    case 3: fwd_rows_g<3, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    case 4: fwd_rows_g<4, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    case 5: fwd_rows_g<5, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    default: if (MAXD == 64) fwd_rows_g<6, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-  }
+  fwd_rows_any<RS>(lw, m.resid, m.tmp, Mh, h, tid, NT);
   g.sync();
   const int shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1, denom = tx::dq_denom(txSz);
   const uint64_t invDc = sh.qinv[plane][0], invAc = sh.qinv[plane][1];
   int32_t *coefOut = c.coefs + sh.task.coef[plane];
   int nz = 0;
-  for (int k = tid; k < th * tw; k += NT) {
-    int k2 = k >> ltw, kk = k & (tw - 1);
-    int64_t s;
-    switch (lh) {
-      case 2: s = MAXD == 32 ? fwd_col_g<2>(m.tmp, Mv, k2, kk) : 0; break;
-      case 3: s = fwd_col_g<3>(m.tmp, Mv, k2, kk); break;
-      case 4: s = fwd_col_g<4>(m.tmp, Mv, k2, kk); break;
-      case 5: s = fwd_col_g<5>(m.tmp, Mv, k2, kk); break;
-      default: s = MAXD == 64 ? fwd_col_g<6>(m.tmp, Mv, k2, kk) : 0; break;
-    }
-    s = s * ((int64_t)1 << shifts);
-    if (rect) s = round2l(s, 12) * 5793;
-    int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
+  fwd_cols_any(lh, m.tmp, Mv, ltw, tid, NT, [&](int k, int64_t s) {
     int first = k == 0;
-    int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
+    int lv = tx::quant_level(fwd_scale(s, shifts, rect), first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
     m.q[k] = tx::dequant_level(lv, first ? dcQ : acQ, denom);
     coefOut[k] = lv;
     nz |= lv;
-  }
+  });
   nz = g.any(nz);
   if (nz) {
     if (tid == 0) WORK(W_REC_INV_OPS, 3 * (1 << (lw + lh)) * (lw + lh));
@@ -2114,10 +2406,7 @@ __device__ void chroma_worker(const Ctx &c, IntraShared &sh) {
 // again. A transform block's candidates used to run one after another on the
 // whole CTA, 11,000 cycles each with ten barriers, for every depth and once
 // more for the winner.
-constexpr int SEARCH_CODERS = 256, SEARCH_WORKERS = SEARCH_CODERS + 32, CAND_RS = 17;
-struct Cand {
-  int32_t r[16 * CAND_RS], t[16 * CAND_RS], q[256];
-};
+constexpr int SEARCH_CODERS = 256, SEARCH_WORKERS = SEARCH_CODERS + 32;
 struct SearchShared {
   FrameParams fpc;
   uint64_t qinv[3][2];
@@ -2139,102 +2428,17 @@ struct SearchShared {
   };
 };
 
-template <int LW>
-__device__ __forceinline__ void cand_rows(Cand &cd, const int32_t *MhT, int h, int lane) {
-  constexpr int W = 1 << LW;
-  for (int k = lane; k < h << LW; k += 32) {
-    int i = k >> LW, kk = k & (W - 1);
-    const int32_t *r = cd.r + i * CAND_RS, *m = MhT + kk;
-    int64_t s = 0;
-#pragma unroll
-    for (int j = 0; j < W; j++) s += (int64_t)r[j] * m[j * W];
-    cd.t[i * CAND_RS + kk] = (int32_t)round2l(s, 16);
-  }
-}
-template <int LH>
-__device__ __forceinline__ int64_t cand_col(const Cand &cd, const int32_t *Mv, int k2, int kk) {
-  constexpr int H = 1 << LH;
-  const int32_t *m = Mv + k2 * H;
-  int64_t s = 0;
-#pragma unroll
-  for (int i = 0; i < H; i++) s += (int64_t)m[i] * cd.t[i * CAND_RS + kk];
-  return s;
-}
-__device__ __forceinline__ int level_bits(int l) { return l == 0 ? 6 : 8 * (2 + 2 * (31 - __clz(iabs(l)))); }
-
-// One candidate type of a transform block up to 16 x 16 (prediction in sh.px
-// at (x, y) of the block): its levels (cd.q), its residual (cd.r), eob and
-// cost, by one warp (code_tx_block's candidate loop, k_recon.h:101-153).
-__device__ __noinline__ void eval_candidate(SearchShared &sh, Cand &cd, int ci, int type, int txSz, int x, int y, int lane) {
+// One candidate type in a warp: eval's result for candidate ci.
+__device__ __forceinline__ void eval_candidate(SearchShared &sh, Cand &cd, int ci, int type, int txSz, int x, int y, int lane) {
   const FrameParams *fp = &sh.fpc;
-  const int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh, n = 1 << (lw + lh);
-  const uint8_t *sp = sh.src + y * 64 + x, *pp = sh.px + y * 64 + x;
-  for (int k = lane; k < n; k += 32) {
-    int i = k >> lw, j = k & (w - 1);
-    cd.r[i * CAND_RS + j] = (int)sp[i * 64 + j] - (int)pp[i * 64 + j];
-  }
-  __syncwarp();
-  const int rk = tx::row_kind(type), ck = tx::col_kind(type);
-  const int32_t *Mh = sh.fmatT[rk] + (lw == 2 ? 0 : lw == 3 ? 16 : 80), *Mv = sh.fmat[ck] + (lh == 2 ? 0 : lh == 3 ? 16 : 80);
+  const int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], rk = tx::row_kind(type), ck = tx::col_kind(type);
+  const CandIn in = {sh.src + y * 64 + x, sh.px + y * 64 + x, 64, 64,
+                     sh.fmatT[rk] + (lw == 2 ? 0 : lw == 3 ? 16 : 80), sh.fmat[ck] + (lh == 2 ? 0 : lh == 3 ? 16 : 80),
+                     fp->dc_q[0], fp->ac_q[0], sh.qinv[0][0], sh.qinv[0][1], fp->lambda};
+  int eob;
+  long long cost = cand_cost(in, cd, type, txSz, lane, &eob);
   if (lane == 0) {
-    WORK(W_REC_FWD_MAC, n * w + n * h);
-    WORK(W_REC_QUANT, n);
-  }
-  if (lw == 2) cand_rows<2>(cd, Mh, h, lane);
-  else if (lw == 3) cand_rows<3>(cd, Mh, h, lane);
-  else cand_rows<4>(cd, Mh, h, lane);
-  __syncwarp();
-  const int dcQ = fp->dc_q[0], acQ = fp->ac_q[0], shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
-  const uint64_t invDc = sh.qinv[0][0], invAc = sh.qinv[0][1];
-  const int16_t *inv = d_inv_scan + d_inv_scan_off[scan_class(type)][txSz];
-  int eob = 0;
-  for (int k = lane; k < n; k += 32) {
-    int k2 = k >> lw, kk = k & (w - 1);
-    int64_t s = lh == 2 ? cand_col<2>(cd, Mv, k2, kk) : lh == 3 ? cand_col<3>(cd, Mv, k2, kk) : cand_col<4>(cd, Mv, k2, kk);
-    s = s * ((int64_t)1 << shifts);
-    if (rect) s = round2l(s, 12) * 5793;
-    int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
-    int first = k == 0;
-    int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, 1, first ? invDc : invAc);  // dq_denom 1 up to 16 x 16
-    cd.q[k] = lv;
-    if (lv) eob = imax(eob, inv[k] + 1);
-  }
-  eob = __reduce_max_sync(0xffffffffu, eob);
-  __syncwarp();
-  int bits = 0, sse = 0;
-  if (eob == 0) {
-    bits = 8;
-    for (int k = lane; k < n; k += 32) {
-      int d = cd.r[(k >> lw) * CAND_RS + (k & (w - 1))];
-      sse += d * d;
-    }
-  } else {
-    for (int k = lane; k < n; k += 32)
-      if (inv[k] < eob) bits += level_bits(cd.q[k]);
-    bits = __reduce_add_sync(0xffffffffu, bits) + 8 * 6 + 8 * 2 * (31 - __clz(eob + 1));
-    const int rowShift = T(Transform_Row_Shift)[txSz];
-    if (lane == 0) WORK(W_REC_INV_OPS, 3 * n * (lw + lh));
-    if (lane < h) {
-      if (lw == 2) inv_row<2, CAND_RS, true>(cd.r, cd.q, lane, h, dcQ, acQ, 1, rect, rk, rowShift);
-      else if (lw == 3) inv_row<3, CAND_RS, true>(cd.r, cd.q, lane, h, dcQ, acQ, 1, rect, rk, rowShift);
-      else inv_row<4, CAND_RS, true>(cd.r, cd.q, lane, h, dcQ, acQ, 1, rect, rk, rowShift);
-    }
-    __syncwarp();
-    if (lane < w) {
-      if (lh == 2) inv_col<2, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
-      else if (lh == 3) inv_col<3, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
-      else inv_col<4, CAND_RS>(cd.r, lane, w, ck, 0, 0, nullptr, 0, 0, 0);
-    }
-    __syncwarp();
-    for (int k = lane; k < n; k += 32) {
-      int i = k >> lw, j = k & (w - 1);
-      int d = (int)sp[i * 64 + j] - clip1((int)pp[i * 64 + j] + cd.r[i * CAND_RS + j]);
-      sse += d * d;
-    }
-  }
-  sse = __reduce_add_sync(0xffffffffu, sse);  // at most 256 * 255^2
-  if (lane == 0) {
-    sh.cost[ci] = (long long)sse * 16 + (long long)fp->lambda * bits / 8;
+    sh.cost[ci] = cost;
     sh.eob[ci] = eob;
   }
 }
@@ -2256,7 +2460,7 @@ __device__ __noinline__ long long code_large(const Ctx &c, SearchShared &sh, con
                                              int32_t *coefOut, int *eobOut) {
   const FrameParams *fp = &sh.fpc;
   PlaneMem<64> &m = sh.m;
-  constexpr int NT = SEARCH_CODERS, RS = 65;
+  constexpr int NT = SEARCH_CODERS, RS = 68;
   const int tid = g.tid, lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz], w = 1 << lw, h = 1 << lh;
   const int tw = imin(32, w), th = imin(32, h), ltw = imin(5, lw);
   for (int k = tid; k < w * h; k += NT) {
@@ -2271,36 +2475,21 @@ __device__ __noinline__ long long code_large(const Ctx &c, SearchShared &sh, con
     WORK(W_REC_FWD_MAC, h * tw * w + th * tw * h);
     WORK(W_REC_QUANT, th * tw);
   }
-  switch (lw) {
-    case 3: fwd_rows_g<3, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    case 4: fwd_rows_g<4, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    case 5: fwd_rows_g<5, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-    default: fwd_rows_g<6, RS, NT>(m.resid, m.tmp, Mh, h, tid); break;
-  }
+  fwd_rows_any<RS>(lw, m.resid, m.tmp, Mh, h, tid, NT);
   g.sync();
   const int dcQ = fp->dc_q[0], acQ = fp->ac_q[0], shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
   const int denom = tx::dq_denom(txSz);
   const uint64_t invDc = sh.qinv[0][0], invAc = sh.qinv[0][1];
   const int16_t *inv = d_inv_scan + d_inv_scan_off[0][txSz];
   int eob = 0;
-  for (int k = tid; k < th * tw; k += NT) {
-    int k2 = k >> ltw, kk = k & (tw - 1);
-    int64_t s;
-    switch (lh) {
-      case 3: s = fwd_col_g<3>(m.tmp, Mv, k2, kk); break;
-      case 4: s = fwd_col_g<4>(m.tmp, Mv, k2, kk); break;
-      case 5: s = fwd_col_g<5>(m.tmp, Mv, k2, kk); break;
-      default: s = fwd_col_g<6>(m.tmp, Mv, k2, kk); break;
-    }
-    s = s * ((int64_t)1 << shifts);
-    if (rect) s = round2l(s, 12) * 5793;
-    int v = (int)(s >= 0 ? round2l(s, 20) : -round2l(-s, 20));
+  fwd_cols_any(lh, m.tmp, Mv, ltw, tid, NT, [&](int k, int64_t s) {
     int first = k == 0;
-    int lv = tx::quant_level(v, first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
+    int lv = tx::quant_level(fwd_scale(s, shifts, rect), first ? dcQ : acQ, first ? 26 : 22, denom, first ? invDc : invAc);
     m.q[k] = tx::dequant_level(lv, first ? dcQ : acQ, denom);
+    m.lv[k] = lv;
     coefOut[k] = lv;
     if (lv) eob = imax(eob, inv[k] + 1);
-  }
+  });
   eob = __reduce_max_sync(0xffffffffu, eob);
   if ((tid & 31) == 0) sh.eob[tid >> 5] = eob;
   g.sync();
@@ -2310,7 +2499,7 @@ __device__ __noinline__ long long code_large(const Ctx &c, SearchShared &sh, con
     bits = tid == 0 ? 8 : 0;
   } else {
     for (int k = tid; k < th * tw; k += NT)
-      if (inv[k] < eob) bits += level_bits(coefOut[k]);  // this thread's own stores
+      if (inv[k] < eob) bits += level_bits(m.lv[k]);
     if (tid == 0) bits += 8 * 6 + 8 * 2 * (31 - __clz(eob + 1));
     if (tid == 0) WORK(W_REC_INV_OPS, 3 * (1 << (lw + lh)) * (lw + lh));
     inverse_large<64, NT>(m, g, lw, lh, DCT_DCT, txSz, dcQ, acQ);

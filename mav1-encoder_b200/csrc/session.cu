@@ -84,9 +84,10 @@ struct mav1cu_session {
   int *status;             // device status: [0] error, [1] abort
   int *blk_at;             // block index per 4x4 luma unit
   int *flow;               // the intra dataflow's zeroed state: counters, successor counts, ready queues (rec::Ctx)
-  int *dep_count, *succ;   // its dependency counts and successor lists
+  int *dep_count, *succ;   // its dependency counts (and the inter block list) and successor lists
   rec::IntraTask *tasks;   // its block records
-  int resident_recon;      // intra recon workers (CTAs, one per SM)
+  int resident_recon;      // intra recon workers of a kind (one per SM)
+  int resident_inter;      // inter recon CTAs resident at once
   int4 *xcounts;           // compact export: per-superblock counts, block and level bases, zero run / fit flag
   int *xblk_base, *xcoef_base, *xmeta;
   void *ximage;            // session-owned export image (page-locked, mapped), allocated on first request
@@ -318,7 +319,7 @@ static int64_t session_bytes(const Geometry &g, int maxPresets) {
   b += (sizeof(int64_t) + sizeof(BlockInfo)) * A_ITEMS * nsb;          // ACOSTS AINFOS
   b += 2 * 16 * plane + 3 * dplane + 2 * mi;                           // quarter-pel, decimated, edge marks
   b += sizeof(int) * (8 + mi) + sizeof(int32_t) * 4096 * 15;           // status, block map, mats_t
-  b += sizeof(int) * (rec::CNT_WORDS + nblk * (5 + MAX_SUCC)) + sizeof(rec::IntraTask) * nblk;  // intra dataflow
+  b += sizeof(int) * (rec::CNT_WORDS + nblk * (6 + MAX_SUCC)) + sizeof(rec::IntraTask) * nblk;  // intra dataflow
   b += sizeof(int4) * nsb + 2 * sizeof(int) * nsb + sizeof(int) * 4;   // export scratch
   b += sizeof(lrs::Fit) * lrUnits + sizeof(int) * 4;                   // LR search
   return (int64_t)b;
@@ -370,7 +371,7 @@ extern "C" int mav1cu_session_create(int width, int height, int max_cdef_presets
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->mats_t, sizeof(int32_t) * 4096 * 15);
   size_t nblk = MAX_BLOCKS_PER_SB * nsb;
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->flow, sizeof(int) * (rec::CNT_WORDS + 3 * nblk));
-  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->dep_count, sizeof(int) * 2 * nblk);
+  if (e == cudaSuccess) e = dmalloc(s, (void **)&s->dep_count, sizeof(int) * 3 * nblk);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->succ, sizeof(int) * nblk * MAX_SUCC);
   if (e == cudaSuccess) e = dmalloc(s, (void **)&s->tasks, sizeof(rec::IntraTask) * nblk);
   s->mats_dirty = 1;
@@ -420,6 +421,9 @@ extern "C" int mav1cu_session_create(int width, int height, int max_cdef_presets
     // intra blocks / 8) of each): the rest of each SM stays free for the
     // other engines' kernels
     s->resident_recon = imax(1, sms);
+    int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rec::k_recon_inter, rec::INTER_THREADS, rec::SMEM_INTER);
+    s->resident_inter = imax(1, sms * per);
   }
   cudaFuncSetAttribute(ana::k_analyze_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ANA_SMEM(16));
   {
@@ -634,22 +638,24 @@ extern "C" int mav1cu_recon(mav1cu_session *s) {
   c.succ_count = s->flow + rec::CNT_WORDS;
   c.queue = c.succ_count + nblk;
   c.dep_count = s->dep_count;
+  c.inter = s->dep_count + 2 * (size_t)nblk;
   c.succ = s->succ;
   c.tasks = s->tasks;
   c.spin_limit = s->fault_spins > 0 ? s->fault_spins : SPIN_LIMIT;
   c.hold = s->fault_spins > 0 ? s->fault_hold : -1;
   s->fault_spins = 0;
-  if (!s->fp.frame_is_intra) {
-    rec::k_recon_inter<<<nsb, rec::INTER_THREADS, rec::SMEM_INTER, s->stream>>>(c);
-    if (after_launch(s, "recon inter blocks")) return s->err;
-  }
   // leaf frames code inter blocks only (the analysis never keeps intra there)
-  if (s->fp.leaf && !s->fp.frame_is_intra) return MAV1CU_OK;
-  if (check_cuda(s, cudaMemsetAsync(s->flow, 0, sizeof(int) * (rec::CNT_WORDS + 3 * (size_t)nblk), s->stream),
+  const bool intra = !s->fp.leaf || s->fp.frame_is_intra;
+  if (check_cuda(s, cudaMemsetAsync(s->flow, 0, sizeof(int) * (rec::CNT_WORDS + (intra ? 3 * (size_t)nblk : 0)), s->stream),
                  "recon dataflow"))
     return s->err;
-  rec::k_block_map<<<nsb, rec::MAP_THREADS, 0, s->stream>>>(DP(s), c.blocks, c.sbs, s->blk_at, c.counters);
+  rec::k_block_map<<<nsb, rec::MAP_THREADS, 0, s->stream>>>(DP(s), c.blocks, c.sbs, s->blk_at, c.counters, c.inter, nblk);
   if (after_launch(s, "recon unit map")) return s->err;
+  if (!s->fp.frame_is_intra) {
+    rec::k_recon_inter<<<imin(nblk, s->resident_inter), rec::INTER_THREADS, rec::SMEM_INTER, s->stream>>>(c);
+    if (after_launch(s, "recon inter blocks")) return s->err;
+  }
+  if (!intra) return MAV1CU_OK;
   if (s->fp.lossless) {
     rec::k_recon_lossless<<<nblk, rec::INTRA_THREADS, rec::SMEM_INTRA, s->stream>>>(c);
     return after_launch(s, "recon lossless blocks");

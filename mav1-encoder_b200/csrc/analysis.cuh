@@ -50,8 +50,9 @@ __device__ __forceinline__ long long warp_sum64(long long v) {
 
 // The threads evaluating one candidate: a warp (rank = lane), half a warp
 // (the 8x8 level: a few 4x4 units per candidate; mask holds its lanes), or
-// for the 64x64 level a whole CTA (red: one shared word per warp). Sums are
+// for the 64x64 level a whole CTA (red: RED_WORDS shared words per warp). Sums are
 // the group's lanes' sums, then across the CTA's warps.
+constexpr int RED_WORDS = 14;  // 32-bit words of a warp's partial sums
 struct Grp {
   int rank, size;
   long long *red;
@@ -75,7 +76,30 @@ __device__ __forceinline__ long long gsum64(long long v, const Grp &g) {
   for (int k = 0; k < (g.size >> 5); k++) t += g.red[k];
   return t;
 }
-__device__ __forceinline__ int gsum(int v, const Grp &g) { return (int)gsum64(v, g); }
+// Sums of N 32-bit values over the group, every thread getting them (the
+// totals fit 32 bits): one barrier pair for all of them in a CTA group.
+template <int N>
+__device__ __forceinline__ void gsum_all(int (&v)[N], const Grp &g) {
+#pragma unroll
+  for (int k = 0; k < N; k++) v[k] = __reduce_add_sync(g.mask, v[k]);
+  if (g.size <= 32) return;
+  static_assert(N <= RED_WORDS, "a word per value and warp");
+  __syncthreads();
+  if ((g.rank & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < N; k++) ((int *)g.red)[(g.rank >> 5) * RED_WORDS + k] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    v[k] = 0;
+    for (int w = 0; w < (g.size >> 5); w++) v[k] += ((const int *)g.red)[w * RED_WORDS + k];
+  }
+}
+__device__ __forceinline__ int gsum(int v, const Grp &g) {
+  int a[1] = {v};
+  gsum_all(a, g);
+  return a[0];
+}
 
 HD int mode_bits8(int mode) {
   if (mode == DC_PRED) return 12;
@@ -111,8 +135,10 @@ __device__ int inter_plane_satd(const FrameParams *fp, const uint8_t *src, const
     if (usub > 1 && (((uy >> 2) + (ux >> 2)) & 1)) continue;
     int d[16];
     pred::inter_unit4(&ip, uy, ux, d);
-    for (int r = 0; r < 4; r++)
-      for (int c = 0; c < 4; c++) d[r * 4 + c] = (int)sp[(uy + r) * stride + ux + c] - d[r * 4 + c];
+    for (int r = 0; r < 4; r++) {
+      uint32_t sv = __ldg((const uint32_t *)(sp + (uy + r) * stride + ux));  // units start on words
+      for (int c = 0; c < 4; c++) d[r * 4 + c] = (int)((sv >> (8 * c)) & 255) - d[r * 4 + c];
+    }
     s += pred::satd4x4(d);
     WORK(W_ANA_SATD, 1);
     WORK(W_ANA_INTER_PX, 16);
@@ -143,14 +169,16 @@ __device__ void inter3(const FrameParams *fp, const uint8_t *src, const uint8_t 
       int d0[16], d1[16], d2[16];
       pred::inter_unit4(&pa, uy, ux, d0);
       pred::inter_unit4(&pb, uy, ux, d1);
-      for (int r = 0; r < 4; r++)
+      for (int r = 0; r < 4; r++) {
+        uint32_t sw = __ldg((const uint32_t *)(sp + (uy + r) * stride + ux));
         for (int c = 0; c < 4; c++) {
-          int sv = sp[(uy + r) * stride + ux + c];
+          int sv = (sw >> (8 * c)) & 255;
           int va = d0[r * 4 + c], vb = d1[r * 4 + c];
           d0[r * 4 + c] = sv - va;
           d1[r * 4 + c] = sv - vb;
           d2[r * 4 + c] = sv - ((va + vb + 1) >> 1);
         }
+      }
       l0 += pred::satd4x4(d0);
       l1 += pred::satd4x4(d1);
       l2 += pred::satd4x4(d2);
@@ -202,28 +230,237 @@ __device__ void build_edges(const FrameParams *fp, const uint8_t *plane, int str
   gsync(g);
 }
 
-// block_satd_s of the intra prediction `mode` (+delta) against the source.
-__device__ int intra_mode_satd(const FrameParams *fp, const uint8_t *plane, int stride, int planeIdx, int x, int y,
-                               int lw, int lh, int mode, int delta, const int *above, const int *left, const Grp &g) {
-  pred::IntraArgs a = ana_args(fp, planeIdx, x, y, lw, lh, mode, delta);
-  pred::IntraState st;
-  pred::intra_state(a, &st);
-  int dc = mode == DC_PRED ? pred::intra_dc(a, above, left) : 0;
-  int w = 1 << lw, h = 1 << lh, nux = w >> 2, nu = nux * (h >> 2), s = 0;
+// A directional prediction of the 4x4 unit at (ux, uy) from unfiltered edges
+// (pred::intra_pixel without upsampling): rows share a position and a phase
+// along the row above, columns along the column left, so a unit takes 5 edge
+// samples a row or column. With constant angle and slopes the branches fold.
+__device__ __forceinline__ int lerp5(int a, int b, int shift) { return round2(a * (32 - shift) + b * shift, 5); }
+__device__ __forceinline__ void dir_unit(int pAngle, int dx, int dy, const int *above, const int *left, int ux, int uy, int w, int h,
+                                         int (&p)[16]) {
+  if (pAngle < 90) {
+    const int mx = w + h - 1;  // at and beyond it every sample is the last one
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      int idx = (uy + r + 1) * dx, b = (idx >> 6) + ux, sh = (idx >> 1) & 31, e[5];
+#pragma unroll
+      for (int k = 0; k < 5; k++) e[k] = above[imin(b + k, mx)];
+#pragma unroll
+      for (int c = 0; c < 4; c++) p[r * 4 + c] = lerp5(e[c], e[c + 1], sh);
+    }
+  } else if (pAngle > 180) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      int idx = (ux + c + 1) * dy, b = (idx >> 6) + uy, sh = (idx >> 1) & 31, e[5];
+#pragma unroll
+      for (int k = 0; k < 5; k++) e[k] = left[b + k];
+#pragma unroll
+      for (int r = 0; r < 4; r++) p[r * 4 + c] = lerp5(e[r], e[r + 1], sh);
+    }
+  } else {
+    // from the row above where its position is at least -1, else from the
+    // column left: most units lie on one side
+    const int bl = ((ux << 6) - (uy + 4) * dx) >> 6, tr = (((ux + 3) << 6) - (uy + 1) * dx) >> 6;
+    if (tr >= -1) {
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        int idx = (ux << 6) - (uy + r + 1) * dx, b = idx >> 6, sh = (idx >> 1) & 31, e[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) e[k] = above[imax(b + k, -1)];
+#pragma unroll
+        for (int c = 0; c < 4; c++) p[r * 4 + c] = lerp5(e[c], e[c + 1], sh);
+      }
+    }
+    if (bl < -1) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        int idx = (uy << 6) - (ux + c + 1) * dy, b = idx >> 6, sh = (idx >> 1) & 31, e[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) e[k] = left[imax(b + k, -1)];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          if (((((ux + c) << 6) - (uy + r + 1) * dx) >> 6) < -1) p[r * 4 + c] = lerp5(e[r], e[r + 1], sh);
+      }
+    }
+  }
+}
+
+constexpr int32_t ANGLE_SLOPE[] = MAV1T_Dr_Intra_Derivative;
+template <int ANGLE>
+__device__ __forceinline__ void dir_unit_at(const int *above, const int *left, int ux, int uy, int w, int h, int (&p)[16]) {
+  constexpr int dx = ANGLE < 90 ? ANGLE_SLOPE[ANGLE] : ANGLE < 180 ? ANGLE_SLOPE[180 - ANGLE] : 0;
+  constexpr int dy = ANGLE > 180 ? ANGLE_SLOPE[270 - ANGLE] : ANGLE > 90 ? ANGLE_SLOPE[ANGLE - 90] : 0;
+  dir_unit(ANGLE, dx, dy, above, left, ux, uy, w, h, p);
+}
+
+// SATDs of one plane block's intra modes in `modes` (a bit each) against the
+// source, added to acc per mode (this thread's units; block_satd_s of
+// intra_satd, k_analysis.h:126-144). A unit's source and edges are read once
+// for all its modes. The transform of the difference is the difference of the
+// transforms, and a DC, vertical or horizontal prediction's transform is zero
+// but for its first coefficient, row or column: those three modes cost their
+// few changed coefficients. pAngle: a directional mode `dirMode` with a delta
+// (its own angle and slopes), evaluated besides the plain ones.
+__device__ __forceinline__ void intra_modes(const FrameParams *fp, const uint8_t *plane, int stride, int planeIdx, int x, int y, int lw,
+                                            int lh, unsigned modes, int dirMode, const pred::IntraState &ds, const int *above,
+                                            const int *left, const Grp &g, int (&acc)[13]) {
+  const int w = 1 << lw, h = 1 << lh, lnx = lw - 2, nu = 1 << (lw + lh - 4);
+  const uint8_t *sp = plane + y * stride + x;
+  int dc = 0;
+  if (modes >> DC_PRED & 1) {
+    pred::IntraArgs a = ana_args(fp, planeIdx, x, y, lw, lh, DC_PRED, 0);
+    dc = pred::intra_dc(a, above, left);
+  }
+  const int32_t *wX = pred::sm_weights(lw), *wY = pred::sm_weights(lh);
+  for (int u = g.rank; u < nu; u += g.size) {
+    const int ux = (u & ((1 << lnx) - 1)) * 4, uy = (u >> lnx) * 4;
+    int s[16], A[4], L[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      uint32_t v = __ldg((const uint32_t *)(sp + (uy + r) * stride + ux));
+#pragma unroll
+      for (int c = 0; c < 4; c++) s[r * 4 + c] = (v >> (8 * c)) & 255;
+      A[r] = above[ux + r];
+      L[r] = left[uy + r];
+    }
+    WORK(W_ANA_SATD, __popc(modes) + (dirMode >= 0));
+    WORK(W_ANA_INTRA_PX, 16 * (__popc(modes) + (dirMode >= 0)));
+    if (modes & (1u << DC_PRED | 1u << V_PRED | 1u << H_PRED)) {
+      // the source's transform, and its absolute sum without the first row / column
+      int t[16], f[16];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        int a0 = s[i * 4] + s[i * 4 + 1], a1 = s[i * 4] - s[i * 4 + 1], a2 = s[i * 4 + 2] + s[i * 4 + 3], a3 = s[i * 4 + 2] - s[i * 4 + 3];
+        t[i * 4] = a0 + a2;
+        t[i * 4 + 1] = a1 + a3;
+        t[i * 4 + 2] = a0 - a2;
+        t[i * 4 + 3] = a1 - a3;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        int a0 = t[j] + t[4 + j], a1 = t[j] - t[4 + j], a2 = t[8 + j] + t[12 + j], a3 = t[8 + j] - t[12 + j];
+        f[j] = a0 + a2;
+        f[4 + j] = a1 + a3;
+        f[8 + j] = a0 - a2;
+        f[12 + j] = a1 - a3;
+      }
+      int inner = 0;
+#pragma unroll
+      for (int i = 1; i < 4; i++)
+#pragma unroll
+        for (int j = 1; j < 4; j++) inner += iabs(f[i * 4 + j]);
+      const int row = iabs(f[1]) + iabs(f[2]) + iabs(f[3]), col = iabs(f[4]) + iabs(f[8]) + iabs(f[12]);
+      if (modes >> DC_PRED & 1) acc[DC_PRED] += inner + row + col + iabs(f[0] - 16 * dc);
+      auto edge4 = [](const int *v, int q0, int q1, int q2, int q3) {
+        int a0 = v[0] + v[1], a1 = v[0] - v[1], a2 = v[2] + v[3], a3 = v[2] - v[3];
+        return iabs(q0 - 4 * (a0 + a2)) + iabs(q1 - 4 * (a1 + a3)) + iabs(q2 - 4 * (a0 - a2)) + iabs(q3 - 4 * (a1 - a3));
+      };
+      if (modes >> V_PRED & 1) acc[V_PRED] += inner + col + edge4(A, f[0], f[1], f[2], f[3]);
+      if (modes >> H_PRED & 1) acc[H_PRED] += inner + row + edge4(L, f[0], f[4], f[8], f[12]);
+    }
+    auto add = [&](int m, const int (&p)[16]) {
+      int d[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) d[k] = s[k] - p[k];
+      acc[m] += pred::satd4x4(d);
+    };
+    int p[16];
+#define DIR_MODE(M, ANGLE)                                          \
+  if (modes >> M & 1) {                                             \
+    dir_unit_at<ANGLE>(above, left, ux, uy, w, h, p);               \
+    add(M, p);                                                      \
+  }
+    DIR_MODE(D45_PRED, 45)
+    DIR_MODE(D135_PRED, 135)
+    DIR_MODE(D113_PRED, 113)
+    DIR_MODE(D157_PRED, 157)
+    DIR_MODE(D203_PRED, 203)
+    DIR_MODE(D67_PRED, 67)
+#undef DIR_MODE
+    if (modes & (1u << SMOOTH_PRED | 1u << SMOOTH_V_PRED | 1u << SMOOTH_H_PRED)) {
+      const int LB = left[h - 1], AR = above[w - 1];
+      int v[16], hh[16];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        int wy = wY[uy + r];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          int wx = wX[ux + c];
+          v[r * 4 + c] = wy * A[c] + (256 - wy) * LB;
+          hh[r * 4 + c] = wx * L[r] + (256 - wx) * AR;
+        }
+      }
+      if (modes >> SMOOTH_PRED & 1) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) p[k] = round2(v[k] + hh[k], 9);
+        add(SMOOTH_PRED, p);
+      }
+      if (modes >> SMOOTH_V_PRED & 1) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) p[k] = round2(v[k], 8);
+        add(SMOOTH_V_PRED, p);
+      }
+      if (modes >> SMOOTH_H_PRED & 1) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) p[k] = round2(hh[k], 8);
+        add(SMOOTH_H_PRED, p);
+      }
+    }
+    if (modes >> PAETH_PRED & 1) {
+      const int C = above[-1];
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          int base = A[c] + L[r] - C, pl = iabs(base - L[r]), pt = iabs(base - A[c]), pc = iabs(base - C);
+          p[r * 4 + c] = pl <= pt && pl <= pc ? L[r] : pt <= pc ? A[c] : C;
+        }
+      add(PAETH_PRED, p);
+    }
+    if (dirMode >= 0) {
+      dir_unit(ds.pAngle, ds.dx, ds.dy, above, left, ux, uy, w, h, p);
+      int d[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) d[k] = s[k] - p[k];
+      int v = pred::satd4x4(d);
+#pragma unroll
+      for (int m = V_PRED; m <= D67_PRED; m++)
+        if (m == dirMode) acc[m] += v;
+    }
+  }
+}
+
+// This thread's SATDs of the six deltas of directional mode `mode` (-3 .. -1,
+// 1 .. 3), like intra_modes.
+__device__ __forceinline__ void intra_deltas(const FrameParams *fp, const uint8_t *plane, int stride, int x, int y, int lw, int lh,
+                                             int mode, const int *above, const int *left, const Grp &g, int (&acc)[6]) {
+  const int w = 1 << lw, h = 1 << lh, lnx = lw - 2, nu = 1 << (lw + lh - 4);
   const uint8_t *sp = plane + y * stride + x;
   for (int u = g.rank; u < nu; u += g.size) {
-    int ux = (u % nux) * 4, uy = (u / nux) * 4;
-    int d[16];
-    for (int r = 0; r < 4; r++)
-      for (int c = 0; c < 4; c++) {
-        int pv = mode == DC_PRED ? dc : pred::intra_pixel(a, st, above, left, uy + r, ux + c);
-        d[r * 4 + c] = (int)sp[(uy + r) * stride + ux + c] - pv;
-      }
-    s += pred::satd4x4(d);
-    WORK(W_ANA_SATD, 1);
-    WORK(W_ANA_INTRA_PX, 16);
+    const int ux = (u & ((1 << lnx) - 1)) * 4, uy = (u >> lnx) * 4;
+    int s[16];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      uint32_t v = __ldg((const uint32_t *)(sp + (uy + r) * stride + ux));
+#pragma unroll
+      for (int c = 0; c < 4; c++) s[r * 4 + c] = (v >> (8 * c)) & 255;
+    }
+    WORK(W_ANA_SATD, 6);
+    WORK(W_ANA_INTRA_PX, 96);
+#pragma unroll 1
+    for (int k = 0; k < 6; k++) {
+      pred::IntraArgs a = ana_args(fp, 0, x, y, lw, lh, mode, k < 3 ? k - 3 : k - 2);
+      pred::IntraState st;
+      pred::intra_state(a, &st);
+      int p[16], d[16];
+      dir_unit(st.pAngle, st.dx, st.dy, above, left, ux, uy, w, h, p);
+#pragma unroll
+      for (int e = 0; e < 16; e++) d[e] = s[e] - p[e];
+      int v = pred::satd4x4(d);
+#pragma unroll
+      for (int e = 0; e < 6; e++)
+        if (e == k) acc[e] += v;
+    }
   }
-  return gsum(s, g);
 }
 
 // CfL SATD of one chroma plane from source luma: DC prediction, the first
@@ -240,26 +477,37 @@ __device__ int cfl_plane_satd(const FrameParams *fp, const uint8_t *src, int p, 
   int sum = 0;
   for (int k = g.rank; k < n; k += g.size) sum += pred::cfl_luma(luma, ls, cx, cy, maxLumaW, maxLumaH, k / cw, k % cw);
   int avg = round2(gsum(sum, g), clw + clh);
+  // sse[16 +- a]: alpha +- a; the scaled luma of -a is that of a negated
   int sse[33];
+#pragma unroll
   for (int al = 0; al < 33; al++) sse[al] = 0;
   if (g.rank == 0) WORK(W_ANA_CFL, n * 33);
   for (int k = g.rank; k < n; k += g.size) {
-    int i = k / cw, j = k % cw;
-    int v = pred::cfl_luma(luma, ls, cx, cy, maxLumaW, maxLumaH, i, j) - avg;
-    int s0 = sp[i * stride + j];
-    for (int al = 0; al < 33; al++) {
-      int d = clip3(0, 255, dc + round2signed((al - 16) * v, 6)) - s0;
-      sse[al] += d * d;
+    int i = k >> clw, j = k & (cw - 1);
+    int v = pred::cfl_luma(luma, ls, cx, cy, maxLumaW, maxLumaH, i, j) - avg, av = iabs(v);
+    int s0 = sp[i * stride + j], d0 = clip3(0, 255, dc) - s0;
+    sse[16] += d0 * d0;
+#pragma unroll
+    for (int al = 1; al <= 16; al++) {
+      int t = (al * av + 32) >> 6;
+      if (v < 0) t = -t;
+      int dp = clip3(0, 255, dc + t) - s0, dm = clip3(0, 255, dc - t) - s0;
+      sse[16 + al] += dp * dp;
+      sse[16 - al] += dm * dm;
     }
   }
-  int bestA = 0;
-  long long best = -1;
-  for (int al = 0; al < 33; al++) {
-    long long t = gsum64(sse[al], g);
-    if (best < 0 || t < best) {
-      best = t;
-      bestA = al - 16;
-    }
+  int bestA = 0, best = -1;
+  for (int part = 0; part < 3; part++) {  // 11 sums at a time; at most 1024 samples of 255^2
+    int v[11];
+#pragma unroll
+    for (int k = 0; k < 11; k++) v[k] = part == 0 ? sse[k] : part == 1 ? sse[11 + k] : sse[22 + k];
+    gsum_all(v, g);
+#pragma unroll
+    for (int k = 0; k < 11; k++)
+      if (best < 0 || v[k] < best) {
+        best = v[k];
+        bestA = part * 11 + k - 16;
+      }
   }
   int nux = cw >> 2, nu = nux * (ch >> 2), s = 0;
   for (int u = g.rank; u < nu; u += g.size) {
@@ -345,11 +593,18 @@ __device__ long long eval_block(const Ctx &c, int mvNode, int miRow, int miCol, 
   int *ya = wm.edge[0][0] + EDGE_OFF, *yl = wm.edge[0][1] + EDGE_OFF;
   if (!skipIntra) {
     build_edges(fp, c.src + fp->offset[0], fp->stride[0], 0, x, y, lw, lh, ya, yl, g);
-    for (int mode = DC_PRED; mode <= PAETH_PRED; mode++) {
-      if (turbo_mode_off(fp, mode)) continue;
-      long long cst = intra_mode_satd(fp, c.src + fp->offset[0], fp->stride[0], 0, x, y, lw, lh, mode, 0, ya, yl, g) +
-                      (long long)lam * mode_bits8(mode) / 8;
-      if (best < 0 || cst < best) {
+    unsigned modes = 0;
+    for (int mode = DC_PRED; mode <= PAETH_PRED; mode++)
+      if (!turbo_mode_off(fp, mode)) modes |= 1u << mode;
+    int acc[13];
+#pragma unroll
+    for (int m = 0; m < 13; m++) acc[m] = 0;
+    intra_modes(fp, c.src + fp->offset[0], fp->stride[0], 0, x, y, lw, lh, modes, -1, pred::IntraState{}, ya, yl, g, acc);
+    gsum_all(acc, g);
+#pragma unroll
+    for (int mode = 0; mode < 13; mode++) {
+      long long cst = acc[mode] + (long long)lam * mode_bits8(mode) / 8;
+      if ((modes >> mode & 1) && (best < 0 || cst < best)) {
         best = cst;
         bestMode = mode;
       }
@@ -357,16 +612,16 @@ __device__ long long eval_block(const Ctx &c, int mvNode, int miRow, int miCol, 
   }
   if (skipIntra) best = 1LL << 40;
   if (intra_is_directional(bestMode) && !fp->fast) {
-    int base = bestMode;
-    for (int d = -MAX_ANGLE_DELTA; d <= MAX_ANGLE_DELTA; d++) {
-      if (d == 0) continue;
-      long long cst = intra_mode_satd(fp, c.src + fp->offset[0], fp->stride[0], 0, x, y, lw, lh, base, d, ya, yl, g) +
-                      (long long)lam * (mode_bits8(base) + 16) / 8;
-      if (cst < best) {
-        best = cst;
-        bestDelta = d;
+    int acc[6] = {0, 0, 0, 0, 0, 0};
+    intra_deltas(fp, c.src + fp->offset[0], fp->stride[0], x, y, lw, lh, bestMode, ya, yl, g, acc);
+    gsum_all(acc, g);
+    const long long rate = (long long)lam * (mode_bits8(bestMode) + 16) / 8;
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+      if (acc[k] + rate < best) {
+        best = acc[k] + rate;
+        bestDelta = k < 3 ? k - 3 : k - 2;
       }
-    }
   }
   int skipUv = fp->fast && interCost >= 0 && best + (long long)lam * 16 / 8 >= interCost;
   long long bestUv = skipUv ? 0 : -1;
@@ -375,16 +630,30 @@ __device__ long long eval_block(const Ctx &c, int mvNode, int miRow, int miCol, 
     for (int p = 1; p < 3; p++)
       build_edges(fp, c.src + fp->offset[p], fp->stride[p], p, cx, cy, clw, clh, wm.edge[p][0] + EDGE_OFF,
                   wm.edge[p][1] + EDGE_OFF, g);
-    for (int m = DC_PRED; m <= PAETH_PRED; m++) {
-      if (intra_is_directional(m) && m != V_PRED && m != H_PRED && m != bestMode) continue;
-      if (turbo_mode_off(fp, m)) continue;
-      int delta = (m == bestMode) ? bestDelta : 0;
-      long long cst = 0;
-      for (int p = 1; p < 3; p++)
-        cst += intra_mode_satd(fp, c.src + fp->offset[p], fp->stride[p], p, cx, cy, clw, clh, m, delta,
-                               wm.edge[p][0] + EDGE_OFF, wm.edge[p][1] + EDGE_OFF, g);
-      cst += (long long)lam * (m == DC_PRED ? 8 : 24) / 8;
-      if (bestUv < 0 || cst < bestUv) {
+    unsigned modes = 0;
+    for (int m = DC_PRED; m <= PAETH_PRED; m++)
+      if (!(intra_is_directional(m) && m != V_PRED && m != H_PRED && m != bestMode) && !turbo_mode_off(fp, m)) modes |= 1u << m;
+    // the luma mode's direction, with its delta, goes its own way
+    int dirMode = -1;
+    pred::IntraState ds = {};
+    if (intra_is_directional(bestMode) && (modes >> bestMode & 1) && !(bestDelta == 0 && (bestMode == V_PRED || bestMode == H_PRED))) {
+      pred::IntraArgs a = ana_args(fp, 1, cx, cy, clw, clh, bestMode, bestDelta);
+      pred::intra_state(a, &ds);
+      dirMode = bestMode;
+    }
+    const unsigned allowed = modes;
+    if (dirMode >= 0) modes &= ~(1u << dirMode);
+    int acc[13];
+#pragma unroll
+    for (int m = 0; m < 13; m++) acc[m] = 0;
+    for (int p = 1; p < 3; p++)
+      intra_modes(fp, c.src + fp->offset[p], fp->stride[p], p, cx, cy, clw, clh, modes, dirMode, ds, wm.edge[p][0] + EDGE_OFF,
+                  wm.edge[p][1] + EDGE_OFF, g, acc);
+    gsum_all(acc, g);
+#pragma unroll
+    for (int m = 0; m < 13; m++) {
+      long long cst = acc[m] + (long long)lam * (m == DC_PRED ? 8 : 24) / 8;
+      if ((allowed >> m & 1) && (bestUv < 0 || cst < bestUv)) {
         bestUv = cst;
         bestUvMode = m;
       }

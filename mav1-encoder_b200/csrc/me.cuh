@@ -335,8 +335,11 @@ __device__ int unit_satd_pred(const Frame &f, const Node &m, int mvr, int mvc, i
                     0, 0, EIGHTTAP);
   const uint8_t *sp = f.src + fp->offset[0] + (m.y + by) * fp->stride[0] + m.x + bx;
   int d[16];
-  for (int r = 0; r < 4; r++)
-    for (int c = 0; c < 4; c++) d[r * 4 + c] = (int)sp[r * fp->stride[0] + c] - pred::inter_pixel(&p, by + r, bx + c);
+  pred::inter_unit4(&p, by, bx, d);
+  for (int r = 0; r < 4; r++) {
+    uint32_t sv = __ldg((const uint32_t *)(sp + r * fp->stride[0]));  // units start on words
+    for (int c = 0; c < 4; c++) d[r * 4 + c] = (int)((sv >> (8 * c)) & 255) - d[r * 4 + c];
+  }
   return pred::satd4x4(d);
 }
 

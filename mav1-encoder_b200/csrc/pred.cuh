@@ -85,9 +85,40 @@ HD void inter_unit4(const Inter *p, int r0, int c0, int *o) {
     }
     return;
   }
+  int hs[11][4];
+#if defined(__CUDA_ARCH__)
+  // Inside the picture (the four aligned words of a row stay in it): a row's
+  // 4 sums are 8 byte dot products. Every tap is even, so half taps, which
+  // fit 8 bits, give the same rounded sum: (2 S + 4) >> 3 = (S + 2) >> 2.
+  if (p->ix0 + c0 >= 0 && p->iy0 + r0 >= 0 && p->ix0 + c0 + 15 <= p->lastX && p->iy0 + r0 + 10 <= p->lastY) {
+    const uint8_t *a = p->ref + (size_t)(p->iy0 + r0) * p->stride + p->ix0 + c0;
+    const int off = (int)((uintptr_t)a & 3);
+    const uint32_t *q = (const uint32_t *)(a - off);
+    int t0 = 0, t1 = 0;
+    for (int t = 0; t < 4; t++) {
+      t0 |= ((p->fh[t] >> 1) & 255) << (8 * t);
+      t1 |= ((p->fh[t + 4] >> 1) & 255) << (8 * t);
+    }
+    auto dp4 = [](uint32_t px, int taps, int acc) {
+      int r;
+      asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(px), "r"(taps), "r"(acc));
+      return r;
+    };
+#pragma unroll
+    for (int tv = 0; tv < 11; tv++) {
+      const uint32_t *w = q + (size_t)tv * (p->stride >> 2);  // strides are multiples of 32 samples
+      uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+      uint32_t x = __funnelshift_r(w0, w1, 8 * off), y = __funnelshift_r(w1, w2, 8 * off), z = __funnelshift_r(w2, w3, 8 * off);
+      hs[tv][0] = dp4(y, t1, dp4(x, t0, 2)) >> 2;
+#pragma unroll
+      for (int c = 1; c < 4; c++)
+        hs[tv][c] = dp4(__funnelshift_r(y, z, 8 * c), t1, dp4(__funnelshift_r(x, y, 8 * c), t0, 2)) >> 2;
+    }
+  } else
+#endif
+  {
   int xs[11];
   for (int t = 0; t < 11; t++) xs[t] = clip3(0, p->lastX, p->ix0 + c0 + t);
-  int hs[11][4];
   for (int tv = 0; tv < 11; tv++) {
     const uint8_t *row = p->ref + (size_t)clip3(0, p->lastY, p->iy0 + r0 + tv) * p->stride;
     int px[11];
@@ -97,6 +128,7 @@ HD void inter_unit4(const Inter *p, int r0, int c0, int *o) {
       for (int t = 0; t < 8; t++) s += p->fh[t] * px[c + t];
       hs[tv][c] = round2(s, 3);
     }
+  }
   }
   for (int r = 0; r < 4; r++)
     for (int c = 0; c < 4; c++) {
@@ -123,9 +155,10 @@ HD int satd4x4(const int *d) {
   for (int j = 0; j < 4; j++) {
     int a0 = t[0 * 4 + j] + t[1 * 4 + j], a1 = t[0 * 4 + j] - t[1 * 4 + j];
     int a2 = t[2 * 4 + j] + t[3 * 4 + j], a3 = t[2 * 4 + j] - t[3 * 4 + j];
-    s += iabs(a0 + a2) + iabs(a1 + a3) + iabs(a0 - a2) + iabs(a1 - a3);
+    // |a + b| + |a - b| = 2 max(|a|, |b|)
+    s += imax(iabs(a0), iabs(a2)) + imax(iabs(a1), iabs(a3));
   }
-  return s;
+  return 2 * s;
 }
 
 // ---- intra -------------------------------------------------------------------

@@ -28,8 +28,8 @@
 
 // dynamic shared memory of the analysis pass-1 kernel for candidate groups of
 // `group` threads: a WarpMem (edge scratch) per group (per warp for CTA groups)
-// and one reduction word per warp
-#define ANA_SMEM(group) (ana::ana_groups(group) * sizeof(ana::WarpMem) + ANA_THREADS / 32 * sizeof(long long))
+// and RED_WORDS reduction words per warp
+#define ANA_SMEM(group) (ana::ana_groups(group) * sizeof(ana::WarpMem) + ANA_THREADS / 32 * ana::RED_WORDS * sizeof(int))
 
 namespace {
 

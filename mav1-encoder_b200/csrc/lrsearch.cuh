@@ -19,10 +19,12 @@
 //   k_lr_spec    one CTA per unit: the Wiener refinement replayed under
 //                guessed running references, caching the SSE of every
 //                candidate it visits (SSEs do not depend on the references);
-//   k_lr_select  one CTA per plane, units in order: the rate comparisons of
-//                lr_select with the running references; a refinement
-//                candidate whose SSE neither pass cached is evaluated on the
-//                spot by the whole CTA.
+//   k_lr_choose  a warp per unit: lr_select's rate comparisons under guessed
+//                running references, twice;
+//   k_lr_select  one CTA per plane: the units whose references turned out
+//                different are chosen again, until every unit stands; a
+//                refinement candidate whose SSE no pass cached is evaluated on
+//                the spot by the whole CTA.
 //
 // Bit-exactness. SSEs, the self-guided sums and the first Wiener iteration
 // are integer-valued (every partial sum is an integer below 2^53, so double
@@ -46,11 +48,12 @@ constexpr int CACHE = 40;       // candidate SSEs a unit keeps from the first pa
 struct Fit {
   long long sse_none;
   int w[2][3];                  // fitted Wiener taps
-  int n;                        // cached Wiener candidates
+  int n, n0;                    // cached Wiener candidates; those of the first pass
   int taps[CACHE][6];           // their taps: pass 0 j 0..2, pass 1 j 0..2
   long long sse[CACHE];
   int xqd[16][2];               // fitted projection weights per self-guided set
   long long sgr_sse[16];
+  int used[8];                  // the choice: running references it was made with (taps, projection weights)
 };
 
 // The unit's 4x4 luma block range: rows [r0, r1), columns [c0, c1) of the
@@ -352,10 +355,6 @@ struct Shared {
   int ctaps[CACHE][6];
   long long csse[CACHE];
   int cn, found;
-  // k_lr_select: the unit's first-pass results; a candidate neither pass cached
-  Fit fit;
-  int miss_unit;                // its unit, or -1: the scan is done
-  int miss_taps[6];
 };
 
 // Sum of a 32-bit value over the warp, in 64 bits.
@@ -548,13 +547,26 @@ __device__ void wiener_fit(const Layout &l, uint8_t *smem, Shared &sh, int out[2
       } else if (warp == 0 && step > 0 && lane < nacc) {
         const int h = imin(bwf, a.h - ((step - 1) << lb)), n = h * a.w;
         double(*ph)[4] = phi + ((step - 1) & 1) * rowbuf;
+        // a batch of products is formed while the one before it is added up
         int k = 0;
-        for (; k + 8 <= n; k += 8) {
-          double m[8];
+        double m[8], nx[8];
+        if (n >= 8) {
 #pragma unroll
-          for (int q = 0; q < 8; q++) m[q] = dmul(ph[k + q][ia], ph[k + q][ib]);
+          for (int q = 0; q < 8; q++) m[q] = dmul(ph[q][ia], ph[q][ib]);
+        }
+        for (; k + 16 <= n; k += 8) {
+#pragma unroll
+          for (int q = 0; q < 8; q++) nx[q] = dmul(ph[k + 8 + q][ia], ph[k + 8 + q][ib]);
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            acc = dadd(acc, m[q]);
+            m[q] = nx[q];
+          }
+        }
+        if (n >= 8) {
 #pragma unroll
           for (int q = 0; q < 8; q++) acc = dadd(acc, m[q]);
+          k += 8;
         }
         for (; k < n; k++) acc = dadd(acc, dmul(ph[k][ia], ph[k][ib]));
       }
@@ -822,7 +834,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_lr_fit(const FrameParams *fp, co
       }
   if (threadIdx.x == 0) {
     F.sse_none = sseNone;
-    F.n = n;
+    F.n = F.n0 = n;
     for (int p = 0; p < 2; p++)
       for (int j = 0; j < 3; j++) F.w[p][j] = w[p][j];
   }
@@ -920,179 +932,283 @@ __global__ void __launch_bounds__(THREADS) k_lr_spec(const FrameParams *fp, cons
   if (threadIdx.x == 0) F.n = n1;
 }
 
-// ---- the serial choice -------------------------------------------------------------------
-// One CTA per plane: warp 0 scans the units in order (lr_select's loop,
-// lr_search.c:276-355), the other warps wait for a candidate that neither
-// pass cached and filter the unit with it together. What depends on the
-// previous unit, the rates, is spread over the lanes: a filter's rate is the
-// sum of its taps' (unit_bits), the refinement moves one tap at a time and a
-// tap by at most one, so 18 lanes code each tap's three values once and a
-// candidate's rate is its predecessor's with one term exchanged; 16 lanes code
-// the self-guided sets. A candidate is 6 two-bit steps from the fitted filter:
-// lanes compare the cached candidates' codes at once. The next unit's record
-// is in flight meanwhile. (One thread's scan of all of it, the CTA looking the
-// cache up between barriers, took 33 us per luma unit; this scan takes 3.9 us:
-// 7.9 instead of 68.8 ms at 3840x2160.)
-constexpr int FIT_WORDS = (int)(sizeof(Fit) / 4), FIT_LANE = (FIT_WORDS + 31) / 32;
+// ---- the choice ----------------------------------------------------------------------------
+// A unit's choice depends on the units before it only through the running
+// references: the taps of the last Wiener unit and the weights of the last
+// self-guided one. lr_select's serial scan (lr_search.c:276-355) is therefore
+// the one assignment in which every unit is chosen with the references its
+// predecessors leave, and it is found by guessing: k_lr_choose chooses every
+// unit at once, a warp each, first with its predecessor's fitted filter for
+// reference, then with the references the first choices leave; k_lr_select
+// (one CTA per plane) chooses again the units whose references differ from
+// those they were chosen with, until there are none. Unit by unit from the
+// first, such an assignment equals the scan's; nearly every unit stands after
+// the second guess. (A warp's scan of the units in order took 3.9 us a unit:
+// 7.9 ms for a 3840x2160 frame.)
+//
+// Within a unit: a filter's rate is the sum of its taps' (unit_bits), the
+// refinement moves one tap at a time and a tap by at most one, so 18 lanes
+// code each tap's three values once and a candidate's rate is its
+// predecessor's with one term exchanged; 16 lanes code the self-guided sets. A
+// candidate is 6 two-bit steps from the fitted filter: lanes compare the
+// cached candidates' codes at once.
+constexpr int FIT_WORDS = (int)(sizeof(Fit) / 4);
 static_assert(sizeof(Fit) % 4 == 0 && CACHE <= 64, "two cached candidates a lane");
+constexpr int UNUSED_REF = 0x7fffffff;  // Fit::used[0]: choose again
 
-__device__ __forceinline__ void cta_bar() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+// Chooses unit u of the plane (LRUNITS record `unit`) under the references
+// ref[0..5] (taps) and ref[6], ref[7] (weights), by one warp; F: the unit's
+// record in shared memory. False if a candidate's SSE is not cached: its taps
+// are then in miss (lane c: tap c), and the unit is not written.
+__device__ bool choose_unit(const FrameParams *fp, int plane, int u, const Fit &F, const int *ref, int lrTest, LrUnit *unit, int *miss) {
+  const int lane = threadIdx.x & 31, first = plane ? 1 : 0;
+  const long long lambda = fp->lambda;
+  const int *fw = &F.w[0][0];
+  // lane 3 c + d + 1, c = 3 pass + j: tap c moved by d (a value out of range is never a candidate)
+  const int myC = imin(lane / 3, 5), myJ = myC % 3;
+  const int tapMin = T(Wiener_Taps_Min)[myJ], tapMax = T(Wiener_Taps_Max)[myJ];
+  const int v = fw[myC] + lane % 3 - 1;
+  const bool ok = lane < 18 && myJ >= first && v >= tapMin && v <= tapMax;
+  const int tb = ok ? subexp_bits(tapMin, tapMax + 1, T(Wiener_Taps_K)[myJ], ref[myC], v) : 0;
+  const unsigned okMask = __ballot_sync(0xffffffffu, ok);
+  // rate of this lane's self-guided set
+  const int set = lane & 15;
+  int sb = 2 + 4;
+  if (T(Sgr_Params)[set][0]) sb += subexp_bits(T(Sgrproj_Xqd_Min)[0], T(Sgrproj_Xqd_Max)[0] + 1, 4, ref[6], F.xqd[set][0]);
+  if (T(Sgr_Params)[set][2]) sb += subexp_bits(T(Sgrproj_Xqd_Min)[1], T(Sgrproj_Xqd_Max)[1] + 1, 4, ref[7], F.xqd[set][1]);
+  // this lane's cached candidates as steps from the fitted filter: (d + 1) << 2 c
+  unsigned code[2];
+  long long csse[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    int i = lane + 32 * q;
+    code[q] = ~0u;
+    csse[q] = 0;
+    if (i < F.n) {
+      unsigned cd = 0;
+      for (int c = 0; c < 6; c++) cd |= (unsigned)((F.taps[i][c] - fw[c] + 1) & 3) << (2 * c);
+      code[q] = cd;
+      csse[q] = F.sse[i];
+    }
+  }
+  // the refinement (lr_search.c:296-318)
+  int bits = 2;
+  for (int c = 0; c < 6; c++)
+    if (c % 3 >= first) bits += __shfl_sync(0xffffffffu, tb, 3 * c + 1);
+  unsigned cur = 0x555;
+  long long wc = F.sse[0] * 16 + lambda * bits;
+  for (int c = 0; c < 6; c++) {
+    if (c % 3 < first) continue;
+    for (int d = -1; d <= 1; d += 2) {
+      int at = (int)(cur >> (2 * c)) & 3, to = at + d;  // d + 1 of the tap now and moved
+      if (!((okMask >> (3 * c + to)) & 1)) continue;
+      unsigned want = (cur & ~(3u << (2 * c))) | (unsigned)to << (2 * c);
+      int tbits = bits - __shfl_sync(0xffffffffu, tb, 3 * c + at) + __shfl_sync(0xffffffffu, tb, 3 * c + to);
+      unsigned m0 = __ballot_sync(0xffffffffu, code[0] == want), m1 = __ballot_sync(0xffffffffu, code[1] == want);
+      if (!(m0 | m1)) {
+        if (lane < 6) miss[lane] = fw[lane] + ((int)(want >> (2 * lane)) & 3) - 1;
+        __syncwarp();
+        return false;
+      }
+      long long sse = __shfl_sync(0xffffffffu, m0 ? csse[0] : csse[1], __ffs(m0 ? m0 : m1) - 1);
+      long long tc = sse * 16 + lambda * tbits;
+      if (tc < wc) {
+        wc = tc;
+        cur = want;
+        bits = tbits;
+      }
+    }
+  }
+  int type = RESTORE_NONE;
+  long long bestCost = rd(fp, F.sse_none, 1);
+  if (wc < bestCost) {
+    bestCost = wc;
+    type = RESTORE_WIENER;
+  }
+  // first least of the sets' costs (with lrTest on odd units: of their SSEs)
+  const bool testSgr = lrTest && (u & 1);
+  long long sc = testSgr ? F.sgr_sse[set] : F.sgr_sse[set] * 16 + lambda * sb;
+  int si = set;
+  for (int o = 8; o; o >>= 1) {
+    long long oc = __shfl_xor_sync(0xffffffffu, sc, o);
+    int oi = __shfl_xor_sync(0xffffffffu, si, o);
+    if (oc < sc || (oc == sc && oi < si)) {
+      sc = oc;
+      si = oi;
+    }
+  }
+  if (testSgr || sc < bestCost) type = RESTORE_SGRPROJ;
+  if (lrTest && !(u & 1)) type = RESTORE_WIENER;  // Wiener on even units, the least SSE's set on odd ones
+  // the record: type, set, xqd[2], wiener[2][3], pad[2]
+  const int tapv = lane < 6 ? fw[lane] + ((int)(cur >> (2 * lane)) & 3) - 1 : 0;
+  const int wv = __shfl_sync(0xffffffffu, tapv, lane >= 4 && lane < 10 ? lane - 4 : 0);
+  int o = 0;
+  if (lane == 0) o = type;
+  else if (type == RESTORE_SGRPROJ) o = lane == 1 ? si : lane == 2 ? F.xqd[si][0] : lane == 3 ? F.xqd[si][1] : 0;
+  else if (type == RESTORE_WIENER && lane >= 4 && lane < 10) o = wv;
+  if (lane < (int)(sizeof(LrUnit) / 4)) ((int *)unit)[lane] = o;
+  return true;
+}
 
-// The SSE of the missing candidate (every warp; wiener_unit_sse's barriers are
-// the CTA's).
-__device__ __noinline__ long long missing_sse(const FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
-                                              const uint8_t *src, const Layout &l, uint8_t *smem, Shared &sh) {
-  load_unit(fp, sh.miss_unit, cdef, dbk, src, l, smem, sh);
-  int tt[6];
-  for (int k = 0; k < 6; k++) tt[k] = sh.miss_taps[k];
-  return wiener_unit_sse(l, smem, tt, sh);
+struct ChooseMem {
+  Fit fit;
+  int ref[8], miss[6];
+};
+__device__ __forceinline__ void load_fit(const Fit *F, Fit &to) {
+  for (int k = threadIdx.x & 31; k < FIT_WORDS; k += 32) ((int *)&to)[k] = __ldcg((const int *)F + k);
+}
+__device__ __forceinline__ int default_ref(int k) { return k < 6 ? T(Wiener_Taps_Mid)[k % 3] : T(Sgrproj_Xqd_Mid)[k - 6]; }
+
+// A guess for every unit at once, a warp each. pass 0: the references are the
+// previous unit's fitted filter and the default weights; pass 1: what the
+// units before it chose in pass 0 (or, for one being chosen again meanwhile,
+// in this pass: a guess all the same, recorded as used).
+__global__ void __launch_bounds__(THREADS) k_lr_choose(const FrameParams *fp, Fit *fits, LrUnit *units, int lrTest, int n, int pass) {
+  __shared__ ChooseMem mem[WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gu = blockIdx.x * WARPS + warp;
+  if (gu >= n) return;
+  ChooseMem &m = mem[warp];
+  int plane = 2;
+  while (plane > 0 && gu < fp->lr_unit_off[plane]) plane--;
+  const int off = fp->lr_unit_off[plane], u = gu - off;
+  load_fit(fits + gu, m.fit);
+  int r = lane < 8 ? default_ref(lane) : 0;
+  if (pass == 0) {
+    if (u > 0 && lane < 6 && lane % 3 >= (plane ? 1 : 0)) r = __ldcg(&fits[gu - 1].w[0][0] + lane);
+  } else {
+    // the last Wiener and self-guided units before this one
+    int wi = -1, si = -1;
+    for (int e = u; e > 0 && (wi < 0 || si < 0); e -= 32) {
+      int k = e - 1 - lane, t = k >= 0 ? __ldcg(&units[off + k].type) : RESTORE_NONE;
+      unsigned mw = __ballot_sync(0xffffffffu, t == RESTORE_WIENER), ms = __ballot_sync(0xffffffffu, t == RESTORE_SGRPROJ);
+      if (wi < 0 && mw) wi = e - __ffs(mw);
+      if (si < 0 && ms) si = e - __ffs(ms);
+    }
+    if (wi >= 0 && lane < 6 && lane % 3 >= (plane ? 1 : 0)) r = __ldcg(&units[off + wi].wiener[0][0] + lane);
+    if (si >= 0 && lane >= 6 && lane < 8) r = __ldcg(&units[off + si].xqd[0] + lane - 6);
+  }
+  if (lane < 8) m.ref[lane] = r;
+  __syncwarp();
+  if (pass == 1) {  // chosen with these references already
+    int same = lane < 8 ? m.fit.used[lane] == r : 1;
+    if (__all_sync(0xffffffffu, same)) return;
+  }
+  bool done = choose_unit(fp, plane, u, m.fit, m.ref, lrTest, units + gu, m.miss);
+  if (!done && lane < (int)(sizeof(LrUnit) / 4) && pass == 0) ((int *)(units + gu))[lane] = 0;
+  if (lane < 8) fits[gu].used[lane] = done ? r : UNUSED_REF;
 }
 
 __global__ void __launch_bounds__(THREADS) k_lr_select(FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
-                                                      const uint8_t *src, const Fit *fits, LrUnit *units,
+                                                      const uint8_t *src, Fit *fits, LrUnit *units,
                                                       int lrTest, int *lrTypes, Dims dims) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ Shared sh;
+  __shared__ ChooseMem mem[WARPS];
+  __shared__ int lastW[THREADS], lastS[THREADS], todo, any, lowest, missUnit[WARPS];
+  constexpr int LIST = 256;
+  __shared__ int list[LIST];
   const Layout l = layout_of(dims);
-  const int plane = blockIdx.x, lane = threadIdx.x & 31;
+  const int plane = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, first = plane ? 1 : 0;
   const int nUnits = fp->lr_unit_rows[plane] * fp->lr_unit_cols[plane], off = fp->lr_unit_off[plane];
-  if (threadIdx.x >= 32) {
-    for (;;) {
-      cta_bar();
-      if (sh.miss_unit < 0) return;
-      missing_sse(fp, cdef, dbk, src, l, smem, sh);
-      cta_bar();
+  const int per = (nUnits + THREADS - 1) / THREADS, u0 = imin(nUnits, tid * per), u1 = imin(nUnits, u0 + per);
+  for (;;) {
+    // each thread's run of units: the last Wiener and self-guided unit before
+    // it, then every unit's references against those it was chosen with
+    if (tid == 0) {
+      todo = any = 0;
+      lowest = nUnits;
     }
-  }
-  const int first = plane ? 1 : 0;
-  const long long lambda = fp->lambda;
-  // lane 3 c + d + 1, c = 3 pass + j: tap c moved by d
-  const int myC = imin(lane / 3, 5), myJ = myC % 3, myD = lane % 3 - 1, myTap = lane < 18 && myJ >= first;
-  const int tapMin = T(Wiener_Taps_Min)[myJ], tapMax = T(Wiener_Taps_Max)[myJ], tapK = T(Wiener_Taps_K)[myJ];
-  int refW = T(Wiener_Taps_Mid)[lane % 3];                    // lane c < 6: running reference of tap c
-  int refX0 = T(Sgrproj_Xqd_Mid)[0], refX1 = T(Sgrproj_Xqd_Mid)[1];  // every lane
-  const int set = lane & 15, setR0 = T(Sgr_Params)[set][0], setR1 = T(Sgr_Params)[set][2];
-  int used = 0;
-  int nxt[FIT_LANE];
-  auto fetch = [&](int u) {
-#pragma unroll
-    for (int k = 0; k < FIT_LANE; k++)
-      if (k * 32 + lane < FIT_WORDS) nxt[k] = ((const int *)(fits + off + u))[k * 32 + lane];
-  };
-  if (nUnits > 0) fetch(0);
-  for (int u = 0; u < nUnits; u++) {
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < FIT_LANE; k++)
-      if (k * 32 + lane < FIT_WORDS) ((int *)&sh.fit)[k * 32 + lane] = nxt[k];
-    __syncwarp();
-    if (u + 1 < nUnits) fetch(u + 1);
-    const Fit &F = sh.fit;
-    const int *fw = &F.w[0][0];
-    // rates of the taps' values (a value out of range is never a candidate)
-    int ref = __shfl_sync(0xffffffffu, refW, myC), v = fw[myC] + myD, tb = 0;
-    bool ok = myTap && v >= tapMin && v <= tapMax;
-    if (ok) tb = subexp_bits(tapMin, tapMax + 1, tapK, ref, v);
-    const unsigned okMask = __ballot_sync(0xffffffffu, ok);
-    // rate of this lane's self-guided set
-    int sb = 2 + 4;
-    if (setR0) sb += subexp_bits(T(Sgrproj_Xqd_Min)[0], T(Sgrproj_Xqd_Max)[0] + 1, 4, refX0, F.xqd[set][0]);
-    if (setR1) sb += subexp_bits(T(Sgrproj_Xqd_Min)[1], T(Sgrproj_Xqd_Max)[1] + 1, 4, refX1, F.xqd[set][1]);
-    // this lane's cached candidates as steps from the fitted filter: (d + 1) << 2 c
-    unsigned code[2];
-    long long csse[2];
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      int i = lane + 32 * q;
-      code[q] = ~0u;
-      csse[q] = 0;
-      if (i < F.n) {
-        unsigned cd = 0;
-        for (int c = 0; c < 6; c++) cd |= (unsigned)((F.taps[i][c] - fw[c] + 1) & 3) << (2 * c);
-        code[q] = cd;
-        csse[q] = F.sse[i];
+    int w = -1, g = -1;
+    for (int u = u0; u < u1; u++) {
+      int t = __ldcg(&units[off + u].type);
+      if (t == RESTORE_WIENER) w = u;
+      else if (t == RESTORE_SGRPROJ) g = u;
+    }
+    lastW[tid] = w;
+    lastS[tid] = g;
+    __syncthreads();
+    for (int o = 1; o < THREADS; o <<= 1) {
+      int a = tid >= o ? lastW[tid - o] : -1, b = tid >= o ? lastS[tid - o] : -1;
+      __syncthreads();
+      lastW[tid] = imax(lastW[tid], a);
+      lastS[tid] = imax(lastS[tid], b);
+      __syncthreads();
+    }
+    if (w >= 0 || g >= 0) any = 1;
+    w = tid ? lastW[tid - 1] : -1;
+    g = tid ? lastS[tid - 1] : -1;
+    for (int u = u0; u < u1; u++) {
+      const Fit &F = fits[off + u];
+      bool same = true;
+      for (int k = 0; k < 8; k++) {
+        int r = default_ref(k);
+        if (k < 6 && w >= 0 && k % 3 >= first) r = __ldcg(&units[off + w].wiener[0][0] + k);
+        if (k >= 6 && g >= 0) r = __ldcg(&units[off + g].xqd[0] + k - 6);
+        same = same && r == __ldcg(F.used + k);
       }
+      if (!same) {  // what the list has no room for is found again in the next round
+        atomicMin(&lowest, u);
+        int slot = atomicAdd(&todo, 1);
+        if (slot < LIST) list[slot] = u;
+      }
+      int t = __ldcg(&units[off + u].type);
+      if (t == RESTORE_WIENER) w = u;
+      else if (t == RESTORE_SGRPROJ) g = u;
     }
-    // the refinement (lr_search.c:296-318)
-    int bits = 2;
-    for (int c = 0; c < 6; c++)
-      if (c % 3 >= first) bits += __shfl_sync(0xffffffffu, tb, 3 * c + 1);
-    unsigned cur = 0x555;
-    long long wc = F.sse[0] * 16 + lambda * bits;
-    for (int c = 0; c < 6; c++) {
-      if (c % 3 < first) continue;
-      for (int d = -1; d <= 1; d += 2) {
-        int at = (int)(cur >> (2 * c)) & 3, to = at + d;  // d + 1 of the tap now and moved
-        if (!((okMask >> (3 * c + to)) & 1)) continue;
-        unsigned want = (cur & ~(3u << (2 * c))) | (unsigned)to << (2 * c);
-        int tbits = bits - __shfl_sync(0xffffffffu, tb, 3 * c + at) + __shfl_sync(0xffffffffu, tb, 3 * c + to);
-        unsigned m0 = __ballot_sync(0xffffffffu, code[0] == want), m1 = __ballot_sync(0xffffffffu, code[1] == want);
-        long long sse;
-        if (m0) sse = __shfl_sync(0xffffffffu, csse[0], __ffs(m0) - 1);
-        else if (m1) sse = __shfl_sync(0xffffffffu, csse[1], __ffs(m1) - 1);
-        else {
-          if (lane == 0) {
-            sh.miss_unit = off + u;
-            for (int k = 0; k < 6; k++) sh.miss_taps[k] = fw[k] + ((int)(want >> (2 * k)) & 3) - 1;
-          }
-          __syncwarp();
-          cta_bar();
-          sse = missing_sse(fp, cdef, dbk, src, l, smem, sh);
-          cta_bar();
+    __syncthreads();
+    const int n = imin(todo, LIST);
+    if (n == 0) break;
+    // the first of them is always among them: it is chosen for good, so the rounds end
+    if (tid == 0 && todo > LIST) list[0] = lowest;
+    __syncthreads();
+    // again, a warp each; a candidate neither pass cached is filtered by the
+    // whole CTA, cached, and its unit chosen in a later round
+    for (int base = 0; base < n; base += WARPS) {
+      if (lane == 0) missUnit[warp] = -1;
+      if (base + warp < n) {
+        const int u = list[base + warp];
+        ChooseMem &m = mem[warp];
+        load_fit(fits + off + u, m.fit);
+        int wi = -1, si = -1;
+        for (int e = u; e > 0 && (wi < 0 || si < 0); e -= 32) {
+          int k = e - 1 - lane, t = k >= 0 ? __ldcg(&units[off + k].type) : RESTORE_NONE;
+          unsigned mw = __ballot_sync(0xffffffffu, t == RESTORE_WIENER), ms = __ballot_sync(0xffffffffu, t == RESTORE_SGRPROJ);
+          if (wi < 0 && mw) wi = e - __ffs(mw);
+          if (si < 0 && ms) si = e - __ffs(ms);
         }
-        long long tc = sse * 16 + lambda * tbits;
-        if (tc < wc) {
-          wc = tc;
-          cur = want;
-          bits = tbits;
+        int r = lane < 8 ? default_ref(lane) : 0;
+        if (wi >= 0 && lane < 6 && lane % 3 >= first) r = __ldcg(&units[off + wi].wiener[0][0] + lane);
+        if (si >= 0 && lane >= 6 && lane < 8) r = __ldcg(&units[off + si].xqd[0] + lane - 6);
+        if (lane < 8) m.ref[lane] = r;
+        __syncwarp();
+        bool done = choose_unit(fp, plane, u, m.fit, m.ref, lrTest, units + off + u, m.miss);
+        if (lane < 8) fits[off + u].used[lane] = done ? r : UNUSED_REF;
+        if (!done && lane == 0) missUnit[warp] = u;
+      }
+      __syncthreads();
+      for (int k = 0; k < WARPS; k++) {
+        const int u = missUnit[k];
+        if (u < 0) continue;  // the same for every thread
+        load_unit(fp, off + u, cdef, dbk, src, l, smem, sh);
+        int tt[6];
+        for (int c = 0; c < 6; c++) tt[c] = mem[k].miss[c];
+        long long sse = wiener_unit_sse(l, smem, tt, sh);
+        if (tid == 0) {
+          Fit &F = fits[off + u];
+          // a full cache keeps the first pass's candidates: a path under
+          // settled references needs at most 12 more
+          int at = F.n < CACHE ? F.n : F.n0;
+          for (int c = 0; c < 6; c++) F.taps[at][c] = tt[c];
+          F.sse[at] = sse;
+          F.n = at + 1;
+          __threadfence_block();
         }
+        __syncthreads();
       }
+      __syncthreads();
     }
-    int type = RESTORE_NONE, bestSet = 0;
-    long long bestCost = rd(fp, F.sse_none, 1);
-    if (wc < bestCost) {
-      bestCost = wc;
-      type = RESTORE_WIENER;
-    }
-    // first least of the sets' costs (with lrTest: of their SSEs)
-    const bool testSgr = lrTest && (u & 1);
-    long long sc = testSgr ? F.sgr_sse[set] : F.sgr_sse[set] * 16 + lambda * sb;
-    int si = set;
-    for (int o = 8; o; o >>= 1) {
-      long long oc = __shfl_xor_sync(0xffffffffu, sc, o);
-      int oi = __shfl_xor_sync(0xffffffffu, si, o);
-      if (oc < sc || (oc == sc && oi < si)) {
-        sc = oc;
-        si = oi;
-      }
-    }
-    if (testSgr || sc < bestCost) {
-      type = RESTORE_SGRPROJ;
-      bestSet = si;
-    }
-    if (lrTest && !(u & 1)) type = RESTORE_WIENER;  // Wiener on even units, the least SSE's set on odd ones
-    // the unit's record (type, set, xqd[2], wiener[2][3], pad[2]), and the references it leaves
-    const int tapv = lane < 6 ? fw[lane] + ((int)(cur >> (2 * lane)) & 3) - 1 : 0;  // tap `lane` of the refined filter
-    const int wv = __shfl_sync(0xffffffffu, tapv, lane >= 4 && lane < 10 ? lane - 4 : 0);
-    int o = 0;
-    if (lane == 0) o = type;
-    else if (type == RESTORE_SGRPROJ) o = lane == 1 ? bestSet : lane == 2 ? F.xqd[bestSet][0] : lane == 3 ? F.xqd[bestSet][1] : 0;
-    else if (type == RESTORE_WIENER && lane >= 4 && lane < 10) o = wv;
-    if (lane < (int)(sizeof(LrUnit) / 4)) ((int *)(units + off + u))[lane] = o;
-    if (type == RESTORE_WIENER) {
-      if (lane < 6 && lane % 3 >= first) refW = tapv;
-    } else if (type == RESTORE_SGRPROJ) {
-      refX0 = F.xqd[bestSet][0];
-      refX1 = F.xqd[bestSet][1];
-    }
-    used |= type != RESTORE_NONE;
   }
-  if (lane == 0) {
-    sh.miss_unit = -1;
-    fp->lr_type[plane] = lrTypes[plane] = used ? RESTORE_SWITCHABLE : RESTORE_NONE;
-  }
-  __syncwarp();
-  cta_bar();
+  if (tid == 0) fp->lr_type[plane] = lrTypes[plane] = any ? RESTORE_SWITCHABLE : RESTORE_NONE;
 }
 
 }  // namespace lrs

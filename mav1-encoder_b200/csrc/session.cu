@@ -763,6 +763,11 @@ extern "C" int mav1cu_lr_search(mav1cu_session *s, int lr_test) {
   lrs::k_lr_spec<<<n, lrs::THREADS, lrs::smem_sse(l), s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK),
                                                                   U8(s, MAV1CU_BUF_SRC), s->lrfit, d);
   if (after_launch(s, "loop-restoration speculative refinement")) return s->err;
+  for (int pass = 0; pass < 2; pass++) {
+    lrs::k_lr_choose<<<(n + lrs::WARPS - 1) / lrs::WARPS, lrs::THREADS, 0, s->stream>>>(
+        DP(s), s->lrfit, (LrUnit *)s->buf[MAV1CU_BUF_LRUNITS], lr_test, n, pass);
+    if (after_launch(s, "loop-restoration choice")) return s->err;
+  }
   lrs::k_lr_select<<<3, lrs::THREADS, lrs::smem_sse(l), s->stream>>>(
       (FrameParams *)s->buf[MAV1CU_BUF_PARAMS], U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK), U8(s, MAV1CU_BUF_SRC),
       s->lrfit, (LrUnit *)s->buf[MAV1CU_BUF_LRUNITS], lr_test, s->lr_types, d);

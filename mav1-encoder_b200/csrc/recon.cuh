@@ -1710,10 +1710,9 @@ __global__ void __launch_bounds__(MAP_THREADS) k_block_map(const FrameParams *fp
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 // Appends a block to a ready queue (kind 0: luma, 1: chroma). What the caller
-// knows complete is visible to whoever takes the block.
+// knows complete, it has ordered before by a fence (or an earlier launch).
 __device__ __forceinline__ void push_ready(const Ctx &c, int kind, int blk) {
   int t = atomicAdd(c.counters + CNT_TAIL + kind, 1);
-  fence_gpu();
   atomicExch(c.queue + kind * c.nblk + t, blk + 1);
 }
 
@@ -1825,7 +1824,7 @@ struct IntraShared {
   int32_t fmat[3][FMAT_SMALL], fmatT[3][FMAT_SMALL];
   int smw[124];      // smooth weights of lengths 4, 8, 16, 32, 64 from (1 << log2) - 4
   IntraTask task;
-  int ahead[8][32];  // records of the first successors (feed)
+  int coded;         // the coders are past the block's last stores (feed)
   int alphaU;        // U's CfL alpha
   union {
     PlaneMem<64> y;
@@ -2265,82 +2264,117 @@ __device__ int pop_ready(const Ctx &c, int kind, int total) {
 // A worker CTA's last warp: it takes blocks, loads their records for the
 // coding warps and releases successors, so that queue traffic runs beside the
 // coding. Barrier 4: the record is in place (me -1: no more); barrier 5: the
-// block is coded and written. While the block is coded the warp fetches the
-// records of its first successors; when one of them becomes ready by this
-// block, it goes to the coding warps at once and the other ready ones are
-// queued after that.
-constexpr int CODERS = 128, WORKER_THREADS = CODERS + 32, AHEAD = 8;
+// block is coded and written.
+//
+// While a block is coded the warp watches its successors' dependency counts: a
+// successor with one dependency left waits for this block alone, so it is the
+// next block whatever else happens, and its record is fetched at once. When
+// the block is coded the coding warps go on with it after two barriers, and
+// only then are the other successors released, with the fence and the atomics
+// that takes (about 3,000 cycles that used to lie between two blocks of a
+// chain, of 10,000). Otherwise the first successor that this block's release
+// makes ready follows.
+constexpr int CODERS = 128, WORKER_THREADS = CODERS + 32;
 template <int N>
 __device__ __forceinline__ void record_bar() { asm volatile("bar.sync 4, %0;" ::"n"(N) : "memory"); }
 template <int N>
 __device__ __forceinline__ void coded_bar() { asm volatile("bar.sync 5, %0;" ::"n"(N) : "memory"); }
 
-// ahead: records do not change during the launch (with a luma search they
-// carry the luma limits that chroma reads).
-template <bool AHEAD_OK, int N, class Shared>
+template <int N, class Shared>
 __device__ void feed(const Ctx &c, Shared &sh, int kind, int total) {
   const int lane = threadIdx.x & 31;
+  volatile int *coded = &sh.coded;
+  int *dep = c.dep_count + kind * c.nblk;
   auto record_word = [&](int b) {
     return __ldcg(lane == 1 ? c.succ_count + b : (const int *)(c.tasks + b) + lane);
   };
-  int push[3] = {-1, -1, -1}, pushOwn = -1;  // ready blocks still to be queued
-  for (int me = -1, at = -1;;) {
+  int s[3] = {-1, -1, -1};  // this lane's successors of the block being coded, or of `prev`
+  int push[3] = {-1, -1, -1}, own = -1;  // ready blocks still to be queued: successors, the block's own chroma (lane 0)
+  int prev = -1;                         // a block coded but not yet released, all but its successor `me`
+  for (int me = -1, word = 0;;) {
     if (me < 0) {
       if (lane == 0) me = pop_ready(c, kind, total);
       me = __shfl_sync(0xffffffffu, me, 0);
-      if (me < 0) {
-        if (lane == 0) sh.task.me = -1;
-        __syncwarp();
-        record_bar<N>();
-        return;
-      }
+      if (me >= 0) word = record_word(me);
     }
-    ((int *)&sh.task)[lane] = at >= 0 ? sh.ahead[at][lane] : record_word(me);
+    ((int *)&sh.task)[lane] = me < 0 ? -1 : word;
+    if (lane == 0) *coded = 0;
     __syncwarp();
-    const int n = imin(sh.task.nsucc, MAX_SUCC);
     record_bar<N>();
+    if (me < 0) return;
+    const int n = imin(__shfl_sync(0xffffffffu, word, 1), MAX_SUCC);
+    if (prev >= 0) {
+      fence_gpu();
+      int left[3], mine = 0;
 #pragma unroll
-    for (int q = 0; q < 3; q++)
-      if (push[q] >= 0) push_ready(c, kind, push[q]);
-    if (pushOwn >= 0) push_ready(c, 1, pushOwn);
-    int s[3];
+      for (int q = 0; q < 3; q++) left[q] = s[q] >= 0 && s[q] != me ? atomicSub(dep + s[q], 1) : 0;
+      if (kind == 0 && lane == 0) mine = atomicSub(c.dep_count + c.nblk + prev, 1);
+#pragma unroll
+      for (int q = 0; q < 3; q++) push[q] = left[q] == 1 ? s[q] : -1;
+      own = mine == 1 ? prev : -1;
+      fence_gpu();
+      if (lane == 0) atomicAdd(c.counters + CNT_DONE + kind, 1);
+      prev = -1;
+    }
+    // the successors and the pending queue entries, in flight together
 #pragma unroll
     for (int q = 0; q < 3; q++) s[q] = lane + 32 * q < n ? __ldcg(c.succ + (size_t)me * MAX_SUCC + lane + 32 * q) : -1;
-    if (AHEAD_OK) {
+    {
+      int t[3] = {0, 0, 0}, town = 0;
+      if (own >= 0) town = atomicAdd(c.counters + CNT_TAIL + 1, 1);
 #pragma unroll
-      for (int k = 0; k < AHEAD; k++) {
-        int b = __shfl_sync(0xffffffffu, s[0], k);
-        if (k < n) sh.ahead[k][lane] = record_word(b);
-      }
+      for (int q = 0; q < 3; q++)
+        if (push[q] >= 0) t[q] = atomicAdd(c.counters + CNT_TAIL + kind, 1);
+      if (own >= 0) atomicExch(c.queue + c.nblk + town, own + 1);
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+        if (push[q] >= 0) atomicExch(c.queue + kind * c.nblk + t[q], push[q] + 1);
     }
-    coded_bar<N>();
-    fence_gpu();
-    int ready[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-      ready[q] = s[q] >= 0 && atomicSub(c.dep_count + kind * c.nblk + s[q], 1) == 1;
-    pushOwn = kind == 0 && lane == 31 && atomicSub(c.dep_count + c.nblk + me, 1) == 1 ? me : -1;
-    if (lane == 0) atomicAdd(c.counters + CNT_DONE + kind, 1);
-    fence_gpu();
     int next = -1;
-    at = -1;
+    while (!*coded) {
+      unsigned r = __ballot_sync(0xffffffffu, s[0] >= 0 && *(volatile int *)(dep + imax(s[0], 0)) == 1);
+      if (r) {
+        fence_gpu();  // what its other dependencies wrote is visible, its record among it
+        next = __shfl_sync(0xffffffffu, s[0], __ffs(r) - 1);
+        word = record_word(next);
+        break;
+      }
+      __nanosleep(100);
+    }
+    __syncwarp();
+    coded_bar<N>();
+    if (next >= 0) {
+      prev = me;
+      me = next;
+      push[0] = push[1] = push[2] = own = -1;
+      continue;
+    }
+    fence_gpu();
+    int left[3], mine = 0;
+#pragma unroll
+    for (int q = 0; q < 3; q++) left[q] = s[q] >= 0 ? atomicSub(dep + s[q], 1) : 0;
+    if (kind == 0 && lane == 0) mine = atomicSub(c.dep_count + c.nblk + me, 1);
+    own = mine == 1 ? me : -1;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      unsigned r = __ballot_sync(0xffffffffu, ready[q]);
+      int ready = left[q] == 1;
+      unsigned r = __ballot_sync(0xffffffffu, ready);
       if (next < 0 && r) {
         int f = __ffs(r) - 1;
         next = __shfl_sync(0xffffffffu, s[q], f);
-        if (lane == f) ready[q] = 0;
-        if (AHEAD_OK && q == 0 && f < AHEAD) at = f;
+        if (lane == f) ready = 0;
       }
-      push[q] = ready[q] ? s[q] : -1;
+      push[q] = ready ? s[q] : -1;
     }
+    // what the other dependencies wrote is visible to the coders (and to whoever takes a queued block)
+    fence_gpu();
+    if (lane == 0) atomicAdd(c.counters + CNT_DONE + kind, 1);
     me = next;
-    if (me < 0) {  // nothing to go on with: queue what is ready (own chroma) before waiting
-#pragma unroll
-      for (int q = 0; q < 3; q++) push[q] = -1;
-      if (pushOwn >= 0) push_ready(c, 1, pushOwn);
-      pushOwn = -1;
+    if (me >= 0) {
+      word = record_word(me);
+    } else {  // nothing to go on with: queue the chroma before waiting
+      if (own >= 0) push_ready(c, 1, own);
+      own = -1;
     }
   }
 }
@@ -2372,6 +2406,7 @@ __device__ void luma_worker(const Ctx &c, IntraShared &sh) {
       gb->tx_types_lo &= ~15;
       gb->eob[0] = nz;
     }
+    if (g.tid == 0) sh.coded = 1;
     coded_bar<WORKER_THREADS>();
   }
 }
@@ -2392,6 +2427,7 @@ __device__ void chroma_worker(const Ctx &c, IntraShared &sh) {
       gb->eob[plane] = nz;
       if ((sh.task.p[1].geo >> 19) & 1) (plane == 1 ? gb->cfl_alpha_u : gb->cfl_alpha_v) = m.alpha;
     }
+    if (threadIdx.x == 0) sh.coded = 1;
     coded_bar<WORKER_THREADS>();
   }
 }
@@ -2413,7 +2449,7 @@ struct SearchShared {
   int32_t fmat[3][FMAT_SMALL], fmatT[3][FMAT_SMALL];
   int smw[124];
   IntraTask task;
-  int ahead[8][32];
+  int coded;
   long long cost[8];
   int eob[8];
   long long red[8];
@@ -2742,6 +2778,7 @@ __device__ void search_worker(const Ctx &c, SearchShared &sh) {
       gb->eob[0] = sh.anyNz;
       c.tasks[me].maxLumaW = sh.maxW;  // the last transform block coded: CfL's limits
       c.tasks[me].maxLumaH = sh.maxH;
+      sh.coded = 1;
     }
     coded_bar<SEARCH_WORKERS>();
   }
@@ -2757,14 +2794,14 @@ __global__ void __launch_bounds__(SEARCH ? SEARCH_WORKERS : WORKER_THREADS, SEAR
   if (SEARCH && kind == 0) {
     SearchShared &sh = *(SearchShared *)smem_raw;
     load_intra_shared(c, sh);
-    if (tid >= SEARCH_CODERS) feed<true, SEARCH_WORKERS>(c, sh, 0, total);
+    if (tid >= SEARCH_CODERS) feed<SEARCH_WORKERS>(c, sh, 0, total);
     else search_worker(c, sh);
     return;
   }
   IntraShared &sh = *(IntraShared *)smem_raw;
   load_intra_shared(c, sh);
   if (tid >= WORKER_THREADS) return;
-  if (tid >= CODERS) feed<!SEARCH, WORKER_THREADS>(c, sh, kind, total);  // a luma search updates the records chroma reads
+  if (tid >= CODERS) feed<WORKER_THREADS>(c, sh, kind, total);
   else if (kind == 0) luma_worker(c, sh);
   else chroma_worker(c, sh);
 }

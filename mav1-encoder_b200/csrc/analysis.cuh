@@ -1035,18 +1035,22 @@ __global__ void __launch_bounds__(32 * TABLE_WARPS) k_analyze_table(Ctx c) {
 HD int smooth_mode(int m) { return m == SMOOTH_PRED || m == SMOOTH_V_PRED || m == SMOOTH_H_PRED; }
 
 // Step 1: every mi covered by a block gets its luma / chroma smooth flag.
-__global__ void k_edge_marks(const FrameParams *fp, const BlockInfo *blocks, const SbInfo *sbs, uint8_t *ys,
-                             uint8_t *uvs) {
-  int sb = blockIdx.x, k = threadIdx.x;
-  if (k >= sbs[sb].num_blocks) return;
-  const BlockInfo *b = &blocks[sbs[sb].first_block + k];
-  int cols = fp->mi_cols, rows = fp->mi_rows;
-  int ysm = smooth_mode(b->y_mode) && !b->is_inter, uvsm = !b->is_inter && smooth_mode(b->uv_mode);
-  for (int r = b->mi_row; r < b->mi_row + T(Num_4x4_Blocks_High)[b->bsize] && r < rows; r++)
-    for (int cc = b->mi_col; cc < b->mi_col + T(Num_4x4_Blocks_Wide)[b->bsize] && cc < cols; cc++) {
+// A CTA per superblock, a warp per block, its lanes over the block's units.
+constexpr int MARK_THREADS = 256;
+__global__ void __launch_bounds__(MARK_THREADS) k_edge_marks(const FrameParams *fp, const BlockInfo *blocks, const SbInfo *sbs,
+                                                             uint8_t *ys, uint8_t *uvs) {
+  const int sb = blockIdx.x, lane = threadIdx.x & 31, n = sbs[sb].num_blocks, cols = fp->mi_cols, rows = fp->mi_rows;
+  for (int k = threadIdx.x >> 5; k < n; k += MARK_THREADS / 32) {
+    const BlockInfo *b = &blocks[sbs[sb].first_block + k];
+    int ysm = smooth_mode(b->y_mode) && !b->is_inter, uvsm = !b->is_inter && smooth_mode(b->uv_mode);
+    int lw = 31 - __clz(T(Num_4x4_Blocks_Wide)[b->bsize]), bh4 = T(Num_4x4_Blocks_High)[b->bsize];
+    for (int i = lane; i < bh4 << lw; i += 32) {
+      int r = b->mi_row + (i >> lw), cc = b->mi_col + (i & ((1 << lw) - 1));
+      if (r >= rows || cc >= cols) continue;
       ys[r * cols + cc] = (uint8_t)ysm;
       uvs[r * cols + cc] = (uint8_t)uvsm;
     }
+  }
 }
 
 // Step 2: get_filter_type( ) of each block from its above / left neighbours.

@@ -240,13 +240,18 @@ __device__ int dec_sad(const Frame &f, const Node &m, int dy, int dx) {
   return sad * 16;
 }
 
+// Rate of a full-pel vector (k_me.h:211-220).
+__device__ __forceinline__ int mv_cost(const FrameParams *fp, int dy, int dx) {
+  int bits = 2 + 2 * (31 - __clz(iabs(dy) * 8 + 1)) + 2 * (31 - __clz(iabs(dx) * 8 + 1));
+  return fp->ac_q[0] * bits / 64;
+}
+
 // Full-pel cost (k_me.h:211-220).
 __device__ int full_cost(const Frame &f, const Node &m, int dy, int dx) {
   const FrameParams *fp = f.fp;
-  int bits = 2 + 2 * floor_log2(iabs(dy) * 8 + 1) + 2 * floor_log2(iabs(dx) * 8 + 1);
-  if ((fp->turbo & T_ME_DEC) && m.step >= ME_COARSE_STEP) return dec_sad(f, m, dy, dx) + fp->ac_q[0] * bits / 64;
+  if ((fp->turbo & T_ME_DEC) && m.step >= ME_COARSE_STEP) return dec_sad(f, m, dy, dx) + mv_cost(fp, dy, dx);
   int rs = (fp->turbo & T_ME_RSUB) && m.step == 1 ? 2 : 1;
-  return full_sad(f, m, dy, dx, rs) + fp->ac_q[0] * bits / 64;
+  return full_sad(f, m, dy, dx, rs) + mv_cost(fp, dy, dx);
 }
 
 // The same cost with the warp's 32 lanes splitting one candidate's byte pairs
@@ -259,13 +264,19 @@ __device__ int full_cost(const Frame &f, const Node &m, int dy, int dx) {
 __device__ __noinline__ int warp_full_cost(const FrameParams *fp, const uint8_t *fsrc, const uint8_t *fref,
                                            const uint8_t *dsrc, const uint8_t *dref, int x, int y, int w, int step,
                                            int dy, int dx, int lane) {
-  int bits = 2 + 2 * floor_log2(iabs(dy) * 8 + 1) + 2 * floor_log2(iabs(dx) * 8 + 1);
   unsigned sad = 0;
   int scale;
   if ((fp->turbo & T_ME_DEC) && step >= ME_COARSE_STEP) {
     // dec_sad: n x n pairs of the decimated planes, lanes along rows
     int W = dec_w(fp), H = dec_h(fp), lg = floor_log2(w >> 2), n = 1 << lg;
     int x0 = x >> 2, y0 = y >> 2, oy = dy >> 2, ox = dx >> 2;
+    if (x0 + n + 4 <= W && y0 + n <= H && x0 + ox >= 0 && x0 + ox + n + 4 <= W && y0 + oy >= 0 && y0 + oy + n <= H) {
+      // inside, with the words around a row's ends: four pairs a word
+      for (int p = lane; p < n * n >> 2; p += 32) {
+        int i = p >> (lg - 2), j = (p & ((n >> 2) - 1)) * 4;
+        sad = __vsadu4(load_u32_unaligned(dsrc + (y0 + i) * W + x0 + j), load_u32_unaligned(dref + (y0 + i + oy) * W + x0 + ox + j)) + sad;
+      }
+    } else
     for (int p = lane; p < n * n; p += 32) {
       int i = p >> lg, j = p & (n - 1);
       int sy = imin(y0 + i, H - 1), ry = clip3(0, H - 1, y0 + i + oy);
@@ -294,8 +305,52 @@ __device__ __noinline__ int warp_full_cost(const FrameParams *fp, const uint8_t 
     }
     scale = rs;
   }
-  for (int off = 16; off > 0; off >>= 1) sad += __shfl_xor_sync(0xffffffffu, sad, off);
-  return (int)sad * scale + fp->ac_q[0] * bits / 64;
+  sad = __reduce_add_sync(0xffffffffu, sad);
+  return (int)sad * scale + mv_cost(fp, dy, dx);
+}
+
+// The full-pel refinement of +-2 samples around (cy, cx) with every candidate
+// inside the frame: `part` of `parts` warps takes its share of the node's
+// words, one word position a lane at a time. A position's 25 candidates read
+// 5 rows of 3 words (a candidate a lane read 2 unaligned words each, from
+// scattered rows) and the 25 sums are reduced over the warp; lane k returns
+// candidate k's part (0: the centre, 1 + raster index: the grid).
+__device__ __forceinline__ bool grid_inside(const FrameParams *fp, const Node &m) {
+  return m.step == 1 && m.range == 2 && m.x + m.cx >= 2 && m.y + m.cy >= 2 && m.x + m.cx + 2 + m.w <= fp->frame_w &&
+         m.y + m.cy + 2 + m.w <= fp->frame_h;
+}
+__device__ __noinline__ unsigned grid_sads(const FrameParams *fp, const uint8_t *fsrc, const uint8_t *fref, int x, int y, int w, int cy,
+                                           int cx, int rs, int lane, int part, int parts) {
+  const int stride = fp->stride[0], lgw = 31 - __clz(w >> 2), n = (w / rs) << lgw;
+  const uint8_t *src = fsrc + fp->offset[0] + y * stride + x;
+  const uint8_t *ref = fref + fp->offset[0] + (y + cy - 2) * stride + x + cx - 2;
+  const int off = (int)((uintptr_t)ref & 3);
+  ref -= off;
+  unsigned sad[25];
+#pragma unroll
+  for (int k = 0; k < 25; k++) sad[k] = 0;
+  for (int q = lane + part * 32; q < n; q += 32 * parts) {
+    const int i = (q >> lgw) * rs, j = (q & ((1 << lgw) - 1)) * 4;
+    const uint32_t sv = __ldg((const uint32_t *)(src + i * stride + j));
+#pragma unroll
+    for (int dy = 0; dy < 5; dy++) {
+      const uint32_t *p = (const uint32_t *)(ref + (i + dy) * stride + j);
+      const uint32_t a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+      // bytes -2 .. 5 around the word
+      const uint32_t lo = __funnelshift_r(a, b, 8 * off), hi = __funnelshift_r(b, c, 8 * off);
+      sad[dy * 5] = __vsadu4(sv, lo) + sad[dy * 5];
+#pragma unroll
+      for (int dx = 1; dx < 4; dx++) sad[dy * 5 + dx] = __vsadu4(sv, __funnelshift_r(lo, hi, 8 * dx)) + sad[dy * 5 + dx];
+      sad[dy * 5 + 4] = __vsadu4(sv, hi) + sad[dy * 5 + 4];
+    }
+  }
+  unsigned mine = 0;
+#pragma unroll
+  for (int k = 0; k < 25; k++) {
+    unsigned v = __reduce_add_sync(0xffffffffu, sad[k]);
+    if (lane == 1 + k || (k == 12 && lane == 0)) mine = v;
+  }
+  return mine * rs;
 }
 
 // SATD of 4x4 unit u of the node against the quarter-pel plane prediction at
@@ -311,12 +366,30 @@ __device__ int unit_satd_hp(const Frame &f, const Node &m, int mvr, int mvc, int
   if (ix >= 0 && ix + 8 <= W && iy >= 0 && iy + 4 <= H) {
     // inside the plane, and the two aligned words each row load stay in the
     // row: no clamping; the source row is word aligned (ux % 4 == 0)
+    // two 16-bit values a word, as hi * 65536 + lo: sums and differences of
+    // such words are those of their parts
+    int P[4], M[4];
+#pragma unroll
     for (int r = 0; r < 4; r++) {
       uint32_t pv = load_u32_unaligned(pl + (size_t)(iy + r) * W + ix);
       uint32_t sv = __ldg((const uint32_t *)(sp + r * fp->stride[0]));
-      for (int c = 0; c < 4; c++) d[r * 4 + c] = (int)((sv >> (8 * c)) & 255) - (int)((pv >> (8 * c)) & 255);
+      int e = (int)(sv & 0x00ff00ffu) - (int)(pv & 0x00ff00ffu), o = (int)((sv >> 8) & 0x00ff00ffu) - (int)((pv >> 8) & 0x00ff00ffu);
+      P[r] = e + o;
+      M[r] = e - o;
     }
-    return pred::satd4x4(d);
+    int sum = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int *v = h ? M : P;
+      int a = v[0] + v[1], b = v[0] - v[1], c = v[2] + v[3], e = v[2] - v[3];
+      int t[4] = {a + c, a - c, b + e, b - e};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {  // |lo + hi| + |lo - hi| = 2 max(|lo|, |hi|)
+        int lo = (int)(short)(t[k] & 0xffff), hi = (t[k] + 0x8000) >> 16;
+        sum += imax(iabs(lo), iabs(hi));
+      }
+    }
+    return 2 * sum;
   }
   for (int r = 0; r < 4; r++) {
     const uint8_t *row = pl + (size_t)clip3(0, H - 1, iy + r) * W;
@@ -379,16 +452,33 @@ __device__ void subpel_costs(const Frame &f, const Node &m, const int *cr, const
   int nu = (m.w >> 2) * (m.w >> 2);
   int st = hp && (fp->turbo & T_ME_USUB) && m.w >= 32 ? 2 : 1;
   int nus = (nu + st - 1) / st;
-  if (g.rank < ncand) cost[g.rank] = 0;
   if (g.rank == 0) WORK(W_ME_SATD, ncand * nus);
-  g.sync();
-  for (int p = g.rank; p < ncand * nus; p += g.size) {
-    int c = p / nus, u = (p % nus) * st;
-    int s = hp ? unit_satd_hp(f, m, cr[c], cc[c], u) : unit_satd_pred(f, m, cr[c], cc[c], u);
-    atomicAdd(&cost[c], s);
+  auto satd = [&](int c, int u) { return hp ? unit_satd_hp(f, m, cr[c], cc[c], u * st) : unit_satd_pred(f, m, cr[c], cc[c], u * st); };
+  if (nus >= g.size) {
+    // a candidate at a time, its units over the group (both powers of two)
+    if (g.size > 32) {
+      if (g.rank < ncand) cost[g.rank] = 0;
+      g.sync();
+    }
+    for (int c = 0; c < ncand; c++) {
+      int v = 0;
+      for (int u = g.rank; u < nus; u += g.size) v += satd(c, u);
+      v = __reduce_add_sync(g.mask, v);
+      if (g.size > 32) {
+        if ((g.rank & 31) == 0) atomicAdd(&cost[c], v * st);
+      } else if (g.rank == 0) {
+        cost[c] = v * st;
+      }
+    }
+  } else {
+    // several candidates at a time, nus lanes each
+    const int lg = 31 - __clz(nus), u = g.rank & (nus - 1);
+    for (int c = g.rank >> lg; c < ((ncand << lg) + g.size - 1) / g.size * (g.size >> lg); c += g.size >> lg) {
+      int v = c < ncand ? satd(c, u) : 0;
+      for (int o = nus >> 1; o; o >>= 1) v += __shfl_xor_sync(g.mask, v, o);
+      if (c < ncand && u == 0) cost[c] = v * st;
+    }
   }
-  g.sync();
-  if (g.rank < ncand) cost[g.rank] *= st;
   g.sync();
 }
 
@@ -405,6 +495,7 @@ __global__ void __launch_bounds__(128, MAV1CU_ME_MIN_CTAS) k_me_level(Frame f0, 
   __shared__ int s_cost[8][16];
   __shared__ int s_r[8][16], s_c[8][16];
   __shared__ unsigned long long s_best[4];
+  __shared__ unsigned s_sad[4][26];
   const Frame &f = blockIdx.y ? f1 : f0;
   const FrameParams *fp = f.fp;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -439,7 +530,20 @@ __global__ void __launch_bounds__(128, MAV1CU_ME_MIN_CTAS) k_me_level(Frame f0, 
       WORK(dec ? W_ME_DSAD : W_ME_SAD, (long long)m.count * (dec ? (m.w >> 2) * (m.w >> 2) : (m.w / rs) * m.w));
     }
     unsigned long long best = ~0ull;
-    if (whole_cta) {
+    const int grs = (fp->turbo & T_ME_RSUB) ? 2 : 1;
+    if (grp.size >= 32 && grid_inside(fp, m)) {
+      unsigned sad = grid_sads(fp, f.src, f.ref, m.x, m.y, m.w, m.cy, m.cx, grs, lane, whole_cta ? warp : 0, whole_cta ? 4 : 1);
+      if (whole_cta) {
+        if (lane < 26) s_sad[warp][lane] = sad;
+        __syncthreads();
+        if (lane < 26) sad = s_sad[0][lane] + s_sad[1][lane] + s_sad[2][lane] + s_sad[3][lane];
+      }
+      if (lane < 26) {
+        int dy, dx;
+        candidate(m, lane, &dy, &dx);
+        best = ((unsigned long long)((int)sad + mv_cost(fp, dy, dx)) << 32) | (unsigned)lane;
+      }
+    } else if (whole_cta) {
       // a warp per candidate, every lane holding the warp's running minimum
       for (int k = warp; k < m.count; k += 4) {
         int dy, dx;

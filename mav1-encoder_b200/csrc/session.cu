@@ -605,7 +605,7 @@ extern "C" int mav1cu_edge_types(mav1cu_session *s) {
   export_fence(s);
   BlockInfo *blocks = (BlockInfo *)s->buf[MAV1CU_BUF_BLOCKS];
   const SbInfo *sbs = (const SbInfo *)s->buf[MAV1CU_BUF_SBS];
-  ana::k_edge_marks<<<s->g.num_sbs, 64, 0, s->stream>>>(DP(s), blocks, sbs, s->ys, s->uvs);
+  ana::k_edge_marks<<<s->g.num_sbs, ana::MARK_THREADS, 0, s->stream>>>(DP(s), blocks, sbs, s->ys, s->uvs);
   if (after_launch(s, "edge marks")) return s->err;
   ana::k_edge_types<<<s->g.num_sbs, 64, 0, s->stream>>>(DP(s), blocks, sbs, s->ys, s->uvs);
   return after_launch(s, "edge types");
@@ -692,7 +692,7 @@ extern "C" int mav1cu_frame_core(mav1cu_session *s) {
 
 extern "C" int mav1cu_filter_info(mav1cu_session *s) {
   if (need_params(s)) return s->err;
-  flt::k_filter_info<<<s->g.num_sbs, 64, 0, s->stream>>>(DP(s), (const BlockInfo *)s->buf[MAV1CU_BUF_BLOCKS],
+  flt::k_filter_info<<<s->g.num_sbs, flt::INFO_THREADS, 0, s->stream>>>(DP(s), (const BlockInfo *)s->buf[MAV1CU_BUF_BLOCKS],
                                                            (const SbInfo *)s->buf[MAV1CU_BUF_SBS],
                                                            U8(s, MAV1CU_BUF_LFMASK));
   return after_launch(s, "filter info");
@@ -706,17 +706,16 @@ extern "C" int mav1cu_filter(mav1cu_session *s, int num_cdef_presets) {
   const FrameParams &fp = s->fp;
   if (fp.lf_level[0] || fp.lf_level[1] || fp.lf_level[2] || fp.lf_level[3]) {
     for (int pass = 0; pass < 2; pass++) {
-      long long lines = pass == 0 ? fp.mi_rows : fp.mi_cols, n = pass == 0 ? fp.mi_cols : fp.mi_rows;
-      long long threads = 3 * lines * n * 4;
-      flt::k_deblock<<<(unsigned)((threads + 255) / 256), 256, 0, s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC),
-                                                                               U8(s, MAV1CU_BUF_LFMASK), pass);
+      int lines = pass == 0 ? fp.mi_rows : fp.mi_cols, n = pass == 0 ? fp.mi_cols : fp.mi_rows;
+      flt::k_deblock<<<dim3((n * 4 + flt::LF_THREADS - 1) / flt::LF_THREADS, lines, 3), flt::LF_THREADS, 0, s->stream>>>(
+          DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_LFMASK), pass);
       if (after_launch(s, "deblock")) return s->err;
     }
   }
   if (num_cdef_presets > 0) {
-    int blocks = ((fp.mi_cols + 1) >> 1) * ((fp.mi_rows + 1) >> 1);
-    flt::k_cdef<<<blocks, 64, 0, s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_CDEFBUF),
-                                               (long long)s->g.frame_bytes, U8(s, MAV1CU_BUF_LFMASK), num_cdef_presets);
+    dim3 grid((fp.mi_cols + 15) >> 4, (fp.mi_rows + 1) >> 1);
+    flt::k_cdef<<<grid, flt::CDEF_THREADS, 0, s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_CDEFBUF),
+                                                           (long long)s->g.frame_bytes, U8(s, MAV1CU_BUF_LFMASK), num_cdef_presets);
     if (after_launch(s, "cdef")) return s->err;
   }
   return MAV1CU_OK;

@@ -133,19 +133,20 @@ __device__ __forceinline__ int leaf_no8(const FrameParams *fp) {
 }
 
 // Node setup (k_me.h:141-178).
-__device__ Node make_node(const FrameParams *fp, int sb, int level, int i, const int32_t *mv) {
+__device__ __forceinline__ Node make_node(const FrameParams *fp, int sb, int level, int i, const int32_t *mv) {
   Node m;
   int sbRow = sb / fp->sb_cols, sbCol = sb % fp->sb_cols, n = 1 << level;
   m.w = 64 >> level;
-  m.x = sbCol * 64 + (i % n) * m.w;
-  m.y = sbRow * 64 + (i / n) * m.w;
+  const int iy = i >> level, ix = i & (n - 1);
+  m.x = sbCol * 64 + ix * m.w;
+  m.y = sbRow * 64 + iy * m.w;
   m.valid = m.x < fp->frame_w && m.y < fp->frame_h;
   m.cy = m.cx = 0;
   m.range = fp->me_range;
   m.pr = m.pc = 0;
   m.copy = 0;
   if (level > 0) {
-    int pi = ((i / n) >> 1) * (n >> 1) + ((i % n) >> 1);
+    int pi = (iy >> 1) * (n >> 1) + (ix >> 1);
     const int32_t *par = mv + (sb * NUM_NODES + node_base(level - 1) + pi) * 2;
     m.pr = par[0];
     m.pc = par[1];
@@ -247,7 +248,7 @@ __device__ __forceinline__ int mv_cost(const FrameParams *fp, int dy, int dx) {
 }
 
 // Full-pel cost (k_me.h:211-220).
-__device__ int full_cost(const Frame &f, const Node &m, int dy, int dx) {
+__device__ __noinline__ int full_cost(const Frame f, const Node m, int dy, int dx) {
   const FrameParams *fp = f.fp;
   if ((fp->turbo & T_ME_DEC) && m.step >= ME_COARSE_STEP) return dec_sad(f, m, dy, dx) + mv_cost(fp, dy, dx);
   int rs = (fp->turbo & T_ME_RSUB) && m.step == 1 ? 2 : 1;
@@ -353,56 +354,66 @@ __device__ __noinline__ unsigned grid_sads(const FrameParams *fp, const uint8_t 
   return mine * rs;
 }
 
-// SATD of 4x4 unit u of the node against the quarter-pel plane prediction at
-// (mvr, mvc) (even, 1/8 units) (k_me.h:317-340).
-__device__ int unit_satd_hp(const Frame &f, const Node &m, int mvr, int mvc, int u) {
-  const FrameParams *fp = f.fp;
-  int W = fp->frame_w, H = fp->frame_h, nu = m.w >> 2;
-  int ux = m.x + (u % nu) * 4, uy = m.y + (u / nu) * 4;
-  const uint8_t *pl = f.qp + (size_t)(((mvr >> 1) & 3) * 4 + ((mvc >> 1) & 3)) * W * H;
-  int iy = uy + (mvr >> 3), ix = ux + (mvc >> 3);
-  const uint8_t *sp = f.src + fp->offset[0] + uy * fp->stride[0] + ux;
-  int d[16];
+// A row's 4-point Hadamard transform is four dot products of its bytes with
+// +-1 words; `h` picks the word. dp4s adds one to acc.
+__device__ __forceinline__ int dp4s(uint32_t px, uint32_t w, int acc) {
+  int r;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(px), "r"(w), "r"(acc));
+  return r;
+}
+__host__ __device__ constexpr uint32_t hadamard_word(int h) {
+  return h == 0 ? 0x01010101u : h == 1 ? 0xffff0101u : h == 2 ? 0x01ffff01u : 0xff01ff01u;  // ++++, ++--, +--+, +-+-
+}
+__host__ __device__ constexpr uint32_t hadamard_minus(int h) {
+  return h == 0 ? 0xffffffffu : h == 1 ? 0x0101ffffu : h == 2 ? 0xff0101ffu : 0x01ff01ffu;
+}
+
+// SATD of the 4x4 unit at (ux, uy) against the quarter-pel plane prediction at
+// (mvr, mvc) (even, 1/8 units) (k_me.h:317-340). S: the source rows'
+// transforms, formed once for all of a unit's candidates; a candidate's rows
+// are then 16 dot products, without unpacking a sample.
+__device__ __forceinline__ int unit_satd_hp(const uint8_t *qp, size_t planeSize, int W, int H, int ux, int uy, const int (&S)[16],
+                                            int mvr, int mvc) {
+  const uint8_t *pl = qp + (size_t)(((mvr >> 1) & 3) * 4 + ((mvc >> 1) & 3)) * planeSize;
+  const int iy = uy + (mvr >> 3), ix = ux + (mvc >> 3);
+  uint32_t pv[4];
   if (ix >= 0 && ix + 8 <= W && iy >= 0 && iy + 4 <= H) {
-    // inside the plane, and the two aligned words each row load stay in the
-    // row: no clamping; the source row is word aligned (ux % 4 == 0)
-    // two 16-bit values a word, as hi * 65536 + lo: sums and differences of
-    // such words are those of their parts
-    int P[4], M[4];
+    // inside the plane, and the two aligned words each row load stay in the row: no clamping
+    const uint8_t *a = pl + (size_t)iy * W + ix;
+    if ((W & 3) == 0) {
+      const int off = (int)((uintptr_t)a & 3);
+      const uint32_t *q = (const uint32_t *)(a - off);
 #pragma unroll
+      for (int r = 0; r < 4; r++) pv[r] = __funnelshift_r(__ldg(q + r * (W >> 2)), __ldg(q + r * (W >> 2) + 1), 8 * off);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; r++) pv[r] = load_u32_unaligned(a + (size_t)r * W);
+    }
+  } else {
     for (int r = 0; r < 4; r++) {
-      uint32_t pv = load_u32_unaligned(pl + (size_t)(iy + r) * W + ix);
-      uint32_t sv = __ldg((const uint32_t *)(sp + r * fp->stride[0]));
-      int e = (int)(sv & 0x00ff00ffu) - (int)(pv & 0x00ff00ffu), o = (int)((sv >> 8) & 0x00ff00ffu) - (int)((pv >> 8) & 0x00ff00ffu);
-      P[r] = e + o;
-      M[r] = e - o;
+      const uint8_t *row = pl + (size_t)clip3(0, H - 1, iy + r) * W;
+      uint32_t v = 0;
+      for (int c = 0; c < 4; c++) v |= (uint32_t)row[clip3(0, W - 1, ix + c)] << (8 * c);
+      pv[r] = v;
     }
-    int sum = 0;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int *v = h ? M : P;
-      int a = v[0] + v[1], b = v[0] - v[1], c = v[2] + v[3], e = v[2] - v[3];
-      int t[4] = {a + c, a - c, b + e, b - e};
-#pragma unroll
-      for (int k = 0; k < 4; k++) {  // |lo + hi| + |lo - hi| = 2 max(|lo|, |hi|)
-        int lo = (int)(short)(t[k] & 0xffff), hi = (t[k] + 0x8000) >> 16;
-        sum += imax(iabs(lo), iabs(hi));
-      }
-    }
-    return 2 * sum;
   }
-  for (int r = 0; r < 4; r++) {
-    const uint8_t *row = pl + (size_t)clip3(0, H - 1, iy + r) * W;
-    for (int c = 0; c < 4; c++) d[r * 4 + c] = (int)sp[r * fp->stride[0] + c] - (int)row[clip3(0, W - 1, ix + c)];
+  int sum = 0;
+#pragma unroll
+  for (int h = 0; h < 4; h++) {
+    int t[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) t[r] = dp4s(pv[r], hadamard_minus(h), S[4 * h + r]);
+    // |a + c| + |a - c| = 2 max(|a|, |c|)
+    sum += imax(iabs(t[0] + t[1]), iabs(t[2] + t[3])) + imax(iabs(t[0] - t[1]), iabs(t[2] - t[3]));
   }
-  return pred::satd4x4(d);
+  return 2 * sum;
 }
 
 // SATD of 4x4 unit u against the normative EIGHTTAP prediction of the node
 // at (mvr, mvc) (the non-plane path, k_me.h:254-257).
-__device__ int unit_satd_pred(const Frame &f, const Node &m, int mvr, int mvc, int u) {
+__device__ __noinline__ int unit_satd_pred(const Frame f, const Node m, int mvr, int mvc, int u) {
   const FrameParams *fp = f.fp;
-  int nu = m.w >> 2, bx = (u % nu) * 4, by = (u / nu) * 4;
+  const int ln = 31 - __clz(m.w >> 2), bx = (u & ((1 << ln) - 1)) * 4, by = (u >> ln) * 4;
   pred::Inter p;
   pred::inter_setup(&p, f.ref + fp->offset[0], fp->stride[0], fp->frame_w, fp->frame_h, m.x, m.y, m.w, m.w, mvr, mvc,
                     0, 0, EIGHTTAP);
@@ -425,8 +436,10 @@ __device__ __forceinline__ void sub_neighbour(const FrameParams *fp, int j, int 
 // The threads searching one node: the CTA (the 64x64 level), a warp, or
 // half a warp (the 8x8 level, whose nodes have at most 16 sub-pel pairs at
 // a time); mask holds the group's lanes of its warp.
+template <int SIZE>
 struct MeGrp {
-  int rank, size;
+  static constexpr int size = SIZE;
+  int rank;
   unsigned mask;
   __device__ __forceinline__ void sync() const {
     if (size > 32) __syncthreads();
@@ -435,7 +448,8 @@ struct MeGrp {
 };
 
 // Minimum over the group's lanes of its warp (the whole warp for a CTA group).
-__device__ __forceinline__ unsigned long long group_min(unsigned long long v, const MeGrp &g) {
+template <class Grp>
+__device__ __forceinline__ unsigned long long group_min(unsigned long long v, const Grp &g) {
   for (int off = g.size >= 32 ? 16 : g.size >> 1; off > 0; off >>= 1) {
     unsigned long long o = __shfl_xor_sync(g.mask, v, off);
     v = o < v ? o : v;
@@ -445,24 +459,46 @@ __device__ __forceinline__ unsigned long long group_min(unsigned long long v, co
 
 // Sub-pel costs of ncand candidates (mvr[c], mvc[c]) into cost[c] (shared,
 // private to the group), every (candidate, unit) pair spread over the group.
-__device__ void subpel_costs(const Frame &f, const Node &m, const int *cr, const int *cc, int ncand, int *cost,
-                             const MeGrp &g) {
+// ST: every ST-th unit counts.
+template <int LEVEL, bool HP, int ST, class Grp>
+__device__ __forceinline__ void subpel_costs(const Frame &f, const Node &m, const int *cr, const int *cc, int ncand, int *cost,
+                                             const Grp &g) {
   const FrameParams *fp = f.fp;
-  int hp = (fp->turbo & T_ME_HPEL) != 0;
-  int nu = (m.w >> 2) * (m.w >> 2);
-  int st = hp && (fp->turbo & T_ME_USUB) && m.w >= 32 ? 2 : 1;
-  int nus = (nu + st - 1) / st;
+  constexpr int st = ST, ln = 4 - LEVEL, nus = (1 << (2 * ln)) / ST;
   if (g.rank == 0) WORK(W_ME_SATD, ncand * nus);
-  auto satd = [&](int c, int u) { return hp ? unit_satd_hp(f, m, cr[c], cc[c], u * st) : unit_satd_pred(f, m, cr[c], cc[c], u * st); };
-  if (nus >= g.size) {
+  const int W = fp->frame_w, H = fp->frame_h, ss = fp->stride[0];
+  const size_t planeSize = (size_t)W * H;
+  // unit u of the node (every st-th counts): its place and, with planes, its source rows' transforms
+  int ux = 0, uy = 0;
+  int S[16];
+  auto take = [&](int u) {
+    ux = m.x + ((u * st) & ((1 << ln) - 1)) * 4;
+    uy = m.y + ((u * st) >> ln) * 4;
+    if (HP)
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const uint32_t v = __ldg((const uint32_t *)(f.src + fp->offset[0] + (uy + r) * ss + ux));
+#pragma unroll
+        for (int h = 0; h < 4; h++) S[4 * h + r] = dp4s(v, hadamard_word(h), 0);
+      }
+  };
+  auto satd = [&](int c, int u) {
+    return HP ? unit_satd_hp(f.qp, planeSize, W, H, ux, uy, S, cr[c], cc[c]) : unit_satd_pred(f, m, cr[c], cc[c], u * st);
+  };
+  if constexpr (nus >= Grp::size) {
     // a candidate at a time, its units over the group (both powers of two)
     if (g.size > 32) {
       if (g.rank < ncand) cost[g.rank] = 0;
       g.sync();
     }
+    constexpr bool one = nus == Grp::size;  // a unit a thread, the same for every candidate
+    if (one) take(g.rank);
     for (int c = 0; c < ncand; c++) {
       int v = 0;
-      for (int u = g.rank; u < nus; u += g.size) v += satd(c, u);
+      for (int u = g.rank; u < nus; u += g.size) {
+        if (!one) take(u);
+        v += satd(c, u);
+      }
       v = __reduce_add_sync(g.mask, v);
       if (g.size > 32) {
         if ((g.rank & 31) == 0) atomicAdd(&cost[c], v * st);
@@ -472,7 +508,9 @@ __device__ void subpel_costs(const Frame &f, const Node &m, const int *cr, const
     }
   } else {
     // several candidates at a time, nus lanes each
-    const int lg = 31 - __clz(nus), u = g.rank & (nus - 1);
+    constexpr int lg = 2 * ln;
+    const int u = g.rank & (nus - 1);
+    take(u);
     for (int c = g.rank >> lg; c < ((ncand << lg) + g.size - 1) / g.size * (g.size >> lg); c += g.size >> lg) {
       int v = c < ncand ? satd(c, u) : 0;
       for (int o = nus >> 1; o; o >>= 1) v += __shfl_xor_sync(g.mask, v, o);
@@ -482,32 +520,34 @@ __device__ void subpel_costs(const Frame &f, const Node &m, const int *cr, const
   g.sync();
 }
 
-// One search level: with group 128 the CTA's four warps per node (the 64x64
-// level: few, large nodes), with 32 a warp per (node, reference), with 16
-// half a warp (the 8x8 level); blockIdx.y selects the reference.
-// At least 5 CTAs per SM (at most 102 registers a thread): more resident
-// warps hide the L2 latency of the candidates' SAD rows (measured on the
-// 1080p clip: an ALTREF frame's search 0.46 -> 0.36 ms; 8 CTAs spill).
-#ifndef MAV1CU_ME_MIN_CTAS
-#define MAV1CU_ME_MIN_CTAS 5
-#endif
-__global__ void __launch_bounds__(128, MAV1CU_ME_MIN_CTAS) k_me_level(Frame f0, Frame f1, int level, int group) {
+// One search level: the CTA's four warps per node (the 64x64 level: few, large
+// nodes), a warp per (node, reference), or half a warp (the 8x8 level);
+// blockIdx.y selects the reference. Level and sub-pel path (HP: quarter-pel
+// planes) are compile-time: with one kernel for all of them the 16x16 level
+// executed 3,800 instructions a node, a seventh of them spilled registers.
+// 6 CTAs per SM with planes (80 registers a thread; 1-2% on the 1080p clip over
+// 5), 5 without (the prediction spills below 96).
+__host__ __device__ constexpr int me_group(int level) { return level == 0 ? 128 : level == 3 ? 16 : 32; }
+template <int LEVEL, bool HP>
+__global__ void __launch_bounds__(128, HP ? 6 : 5) k_me_level(Frame f0, Frame f1) {
   __shared__ int s_cost[8][16];
   __shared__ int s_r[8][16], s_c[8][16];
   __shared__ unsigned long long s_best[4];
   __shared__ unsigned s_sad[4][26];
-  const Frame &f = blockIdx.y ? f1 : f0;
+  const Frame f = blockIdx.y ? f1 : f0;
   const FrameParams *fp = f.fp;
+  constexpr int level = LEVEL, group = me_group(LEVEL);
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int whole_cta = group == 128, half = lane >> 4;
-  MeGrp grp = whole_cta ? MeGrp{(int)threadIdx.x, 128, 0xffffffffu}
-              : group == 32 ? MeGrp{lane, 32, 0xffffffffu}
-                            : MeGrp{lane & 15, 16, 0xffffu << (16 * half)};
+  constexpr bool whole_cta = group == 128;
+  const int half = lane >> 4;
+  const MeGrp<group> grp = whole_cta ? MeGrp<group>{(int)threadIdx.x, 0xffffffffu}
+                           : group == 32 ? MeGrp<group>{lane, 0xffffffffu}
+                                         : MeGrp<group>{lane & 15, 0xffffu << (16 * half)};
   int slotw = whole_cta ? 0 : group == 32 ? warp : 2 * warp + half;
   int nn = 1 << (2 * level);
   int g = whole_cta ? (int)blockIdx.x : (int)blockIdx.x * (128 / group) + slotw;
   if (g >= fp->sb_cols * fp->sb_rows * nn) return;
-  int sb = g / nn, i = g % nn;
+  int sb = g >> (2 * level), i = g & (nn - 1);
   Node m = make_node(fp, sb, level, i, f.mv);
   if (f.isGold && level == 3 && (fp->turbo & T_ME_G3COPY) && fp->leaf && !fp->frame_is_intra) m.copy = 1;
   int32_t *out = f.mv + (sb * NUM_NODES + node_base(level) + i) * 2;
@@ -556,7 +596,26 @@ __global__ void __launch_bounds__(128, MAV1CU_ME_MIN_CTAS) k_me_level(Frame f0, 
       for (int k = grp.rank; k < m.count; k += grp.size) {
         int dy, dx;
         candidate(m, k, &dy, &dx);
-        unsigned long long key = ((unsigned long long)(unsigned)full_cost(f, m, dy, dx) << 32) | (unsigned)k;
+        int cost;
+        if (LEVEL == 3 && grs == 2 && m.x + dx >= 0 && m.x + dx + 8 <= fp->frame_w && m.y + dy >= 0 && m.y + dy + 8 <= fp->frame_h) {
+          // full_sad of every second row of an 8x8 node inside the frame
+          const int stride = fp->stride[0];
+          const uint8_t *sp = f.src + fp->offset[0] + m.y * stride + m.x, *rp = f.ref + fp->offset[0] + (m.y + dy) * stride + m.x + dx;
+          const int off = (int)((uintptr_t)rp & 3);
+          rp -= off;
+          unsigned sad = 0;
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) {
+            const uint32_t *sw = (const uint32_t *)(sp + i * stride), *rw = (const uint32_t *)(rp + i * stride);
+            const uint32_t a = __ldg(rw), b = __ldg(rw + 1), c = __ldg(rw + 2);
+            sad = __vsadu4(__ldg(sw), __funnelshift_r(a, b, 8 * off)) + sad;
+            sad = __vsadu4(__ldg(sw + 1), __funnelshift_r(b, c, 8 * off)) + sad;
+          }
+          cost = (int)sad * 2 + mv_cost(fp, dy, dx);
+        } else {
+          cost = full_cost(f, m, dy, dx);
+        }
+        unsigned long long key = ((unsigned long long)(unsigned)cost << 32) | (unsigned)k;
         best = key < best ? key : best;
       }
     }
@@ -584,7 +643,12 @@ __global__ void __launch_bounds__(128, MAV1CU_ME_MIN_CTAS) k_me_level(Frame f0, 
     cc[0] = mvc;
   }
   grp.sync();
-  subpel_costs(f, m, cr, cc, 1, cost, grp);
+  auto costs = [&](int ncand) {
+    // large nodes may count every second unit
+    if (HP && LEVEL < 2 && (fp->turbo & T_ME_USUB)) subpel_costs<LEVEL, HP, LEVEL < 2 ? 2 : 1>(f, m, cr, cc, ncand, cost, grp);
+    else subpel_costs<LEVEL, HP, 1>(f, m, cr, cc, ncand, cost, grp);
+  };
+  costs(1);
   int bestS = cost[0];
   int minStep = m.w >= 32 && (fp->turbo & T_ME_HALF01) ? 4 : 2;
   int nb = (fp->turbo & T_ME_CROSS) ? 4 : 8;
@@ -597,7 +661,7 @@ __global__ void __launch_bounds__(128, MAV1CU_ME_MIN_CTAS) k_me_level(Frame f0, 
       cc[grp.rank] = mvc + dc;
     }
     grp.sync();
-    subpel_costs(f, m, cr, cc, nb, cost, grp);
+    costs(nb);
     // running strict minimum over the neighbours in order == first minimum
     int bk = -1, bc = bestS;
     for (int k = 0; k < nb; k++)

@@ -555,13 +555,15 @@ extern "C" int mav1cu_motion_search(mav1cu_session *s) {
     f[r].mv = (int32_t *)s->buf[r ? MAV1CU_BUF_MVGOLD : MAV1CU_BUF_MVFIELD];
     f[r].isGold = r;
   }
+  const bool hp = fp.turbo & T_ME_HPEL;
   for (int level = 0; level < 4; level++) {
-    int nodes = s->g.num_sbs << (2 * level);
-    // threads per node: the CTA for the 64x64 nodes, half a warp for the 8x8
-    // nodes, a warp otherwise
-    int group = level == 0 ? 128 : level == 3 ? 16 : 32;
-    dim3 grid((nodes + 128 / group - 1) / (128 / group), nref);
-    me::k_me_level<<<grid, 128, 0, s->stream>>>(f[0], f[1], level, group);
+    int nodes = s->g.num_sbs << (2 * level), per = 128 / me::me_group(level);
+    dim3 grid((nodes + per - 1) / per, nref);
+    auto *kernel = level == 0   ? (hp ? me::k_me_level<0, true> : me::k_me_level<0, false>)
+                   : level == 1 ? (hp ? me::k_me_level<1, true> : me::k_me_level<1, false>)
+                   : level == 2 ? (hp ? me::k_me_level<2, true> : me::k_me_level<2, false>)
+                                : (hp ? me::k_me_level<3, true> : me::k_me_level<3, false>);
+    kernel<<<grid, 128, 0, s->stream>>>(f[0], f[1]);
     if (after_launch(s, "motion search")) return s->err;
   }
   return MAV1CU_OK;

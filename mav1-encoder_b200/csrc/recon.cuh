@@ -8,30 +8,23 @@
 // the normative inverse transform added back into `rec`; optional luma
 // transform-type search and intra tx_depth search by 16 * SSE + lambda * bits.
 //
-// B200 mapping, two launches per frame:
-//  - k_recon_inter: a 128-thread CTA per superblock codes its inter blocks
-//    (they read reference pictures only, so every superblock starts at once)
-//    and publishes each block's completion flags;
-//  - k_recon_blocks: the intra blocks as dataflow. A prepass (k_block_map,
-//    k_block_order, k_block_deps) maps every 4x4 unit to its block, lists the
-//    intra blocks, and gives each one its dependency count (the intra blocks
-//    under its luma edge samples, spec 7.11.2 aboveLimit / leftLimit), its
-//    place in those blocks' successor lists and the BlockDecoded bits of its
-//    corner units; blocks without dependencies seed a ready queue. Persistent
-//    128-thread workers (at most one per SM, max(8, intra blocks / 8) of
-//    them) pop ready blocks, stage each one in shared memory in one batch of
-//    copies, code its luma, write it back, publish its luma flag and release
-//    its successors (the last release pushes a successor to the queue), then
-//    wait (bounded) on the chroma flags under its chroma edges and code its
-//    chroma. Every wait is bounded (Ctx::spin_limit polls); past it the
-//    worker sets the error and abort words and every worker stops.
+// B200 mapping, per frame:
+//  - k_block_map: the unit map, the list of inter blocks, the intra count;
+//  - k_recon_inter: persistent 128-thread CTAs take the inter blocks from the
+//    list (they read reference pictures only, so none waits);
+//  - k_block_deps: each intra block's record and its dependency count (the
+//    intra blocks under its edge samples, spec 7.11.2 aboveLimit / leftLimit),
+//    its place in those blocks' successor lists; blocks without dependencies
+//    seed the ready queue;
+//  - k_recon_blocks: the intra blocks as dataflow, luma and chroma as separate
+//    tasks with their own persistent workers. Every wait is bounded
+//    (Ctx::spin_limit polls); past it the worker sets the error and abort words
+//    and every worker stops;
+//  - lossless frames: k_recon_lossless, whose blocks do not wait.
 // BlockDecoded availability is a function of the decode order (the unit map
 // and the corner bits) or of the clear-flags rule (k_recon.h:402-414)
 // outside the superblock. Samples of the frame being written are read
-// through L2 (ldpx), as other SMs write them during the launch. Within a
-// transform block the CTA splits the residual, both matrix passes (64-bit
-// accumulation), the quantiser, the eob search (a max over inverse-scan
-// positions), the row / column inverse kernels and the reconstruction.
+// through L2 (ldpx), as other SMs write them during the launch.
 #pragma once
 
 #include "common.cuh"
@@ -40,8 +33,8 @@
 
 namespace rec {
 
-// Threads of the CTA coding a block: INTER_THREADS for the inter blocks of a
-// superblock, INTRA_THREADS for an intra block worker.
+// Threads of the CTA coding a block: INTER_THREADS for an inter block,
+// INTRA_THREADS for a lossless intra block.
 #define RT ((int)blockDim.x)
 #ifndef MAV1CU_INTER_THREADS
 #define MAV1CU_INTER_THREADS 128
@@ -126,7 +119,7 @@ struct Smem {
   uint64_t qinv[3][2];       // per plane: the quantiser's reciprocals of dc_q and ac_q (tx::quant_inv)
   int cornerAR[3], cornerBL[3];  // BlockDecoded of those units
   // What only one of the two kernels uses. k_recon_inter launches with the
-  // shared memory up to the end of its part (SMEM_INTER), k_recon_blocks
+  // shared memory up to the end of its part (SMEM_INTER), k_recon_lossless
   // with the whole struct, so neither holds the other's part on its SMs.
   union {
     struct {  // inter blocks
@@ -139,9 +132,7 @@ struct Smem {
       __align__(16) uint8_t recT[64 * 64];
       __align__(8) unsigned long long bar;  // completion of the source copies
     };
-    struct {  // intra blocks
-      int32_t fmat[3][FMAT_SMALL];   // forward matrices of lengths 4, 8, 16 per kind
-      int32_t fmatT[3][FMAT_SMALL];  // the same transposed
+    struct {  // lossless intra blocks
       int edge[3][EDGE_LEN];   // AboveRow, LeftCol, filter copy
       // tiles: rows and columns -1 .. 2n - 1 around the block (its own
       // samples, the above row over the above-right units, the left column
@@ -371,63 +362,14 @@ __device__ __noinline__ void inverse_2d_large(Smem &sm, const int32_t *q, int tx
   inverse_2d_upto<6>(sm, q, txSz, txType, dcQ, acQ, rec, rs, x, y);
 }
 
-// A size up to 16 x 16 with both lengths (and the rectangular scaling)
-// known at compile time: the passes of inverse_2d_upto for that size
-// (dequantisation denominator 1), straight-line.
-template <int LW, int LH>
-__device__ __forceinline__ void inverse_2d_fixed(Smem &sm, const int32_t *q, int txType, int dcQ, int acQ,
-                                                 int rowShift, uint8_t *rec, int rs, int x, int y) {
-  constexpr int W = 1 << LW, H = 1 << LH, rect = LW - LH == 1 || LH - LW == 1;
-  int rk = tx::row_kind(txType), ck = tx::col_kind(txType);
-  for (int i = threadIdx.x; i < H; i += RT) inv_row<LW, 64, true>(sm.resid, q, i, H, dcQ, acQ, 1, rect, rk, rowShift);
-  __syncthreads();
-  int fud = tx::flip_ud(txType), flr = tx::flip_lr(txType);
-  for (int j = threadIdx.x; j < W; j += RT) inv_col<LH, 64>(sm.resid, j, W, ck, fud, flr, rec, rs, x, y);
-  __syncthreads();
-}
-
-// SMALL_INLINE: sizes up to 16 inlined, one fixed-size copy per size (the
-// intra workers, whose chains wait on these latencies: a fixed-size 8x8
-// inverse takes about 40% fewer cycles than the length-generic one);
-// otherwise every size through the out-of-line copy (the inter kernel, where
-// that keeps its register budget).
-template <bool SMALL_INLINE>
+// Out of line: the kernel keeps its register budget.
 __device__ __forceinline__ void inverse_2d(Smem &sm, const int32_t *q, int txSz, int txType, int dcQ, int acQ,
                                            uint8_t *rec = nullptr, int rs = 0, int x = 0, int y = 0) {
   if (threadIdx.x == 0) {  // h rows of w points, then w columns of h points: 3 log2 N operations per point
     int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz];
     WORK(W_REC_INV_OPS, 3 * (1 << (lw + lh)) * (lw + lh));
   }
-  if (SMALL_INLINE) {
-    int rsh = T(Transform_Row_Shift)[txSz];
-    switch (txSz) {
-      case TX_4X4: inverse_2d_fixed<2, 2>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_8X8: inverse_2d_fixed<3, 3>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_16X16: inverse_2d_fixed<4, 4>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_4X8: inverse_2d_fixed<2, 3>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_8X4: inverse_2d_fixed<3, 2>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_8X16: inverse_2d_fixed<3, 4>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_16X8: inverse_2d_fixed<4, 3>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_4X16: inverse_2d_fixed<2, 4>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      case TX_16X4: inverse_2d_fixed<4, 2>(sm, q, txType, dcQ, acQ, rsh, rec, rs, x, y); return;
-      default: break;
-    }
-  }
   inverse_2d_large(sm, q, txSz, txType, dcQ, acQ, rec, rs, x, y);
-}
-
-// Forward matrix of a kind and length: for the intra workers lengths 4..16
-// from the CTA's shared copy, otherwise (and for the inter kernel, whose
-// shared memory holds the superblock's source instead) from the table in
-// global memory; fwd_matrix_t gives the transpose (the row pass reads it
-// along the output index, so the lanes of a warp read consecutive words).
-template <bool INTER>
-__device__ __forceinline__ const int32_t *fwd_matrix(const Ctx &c, const Smem &sm, int kind, int lg) {
-  return !INTER && lg <= 4 ? sm.fmat[kind] + (lg == 2 ? 0 : lg == 3 ? 16 : 80) : c.mats + fwd_slot(kind, lg);
-}
-template <bool INTER>
-__device__ __forceinline__ const int32_t *fwd_matrix_t(const Ctx &c, const Smem &sm, int kind, int lg) {
-  return !INTER && lg <= 4 ? sm.fmatT[kind] + (lg == 2 ? 0 : lg == 3 ? 16 : 80) : c.mats_t + fwd_slot(kind, lg);
 }
 
 // The transpose of every forward matrix (slot k: kind k / 5, length 4 << k % 5).
@@ -715,9 +657,74 @@ __device__ __noinline__ int search_types(const Ctx &c, Smem &sm, const uint8_t *
   return eob;
 }
 
-// Transform, quantise and reconstruct one transform block whose prediction
+// A lossless 4x4 transform block whose prediction is in `rec`: transform,
+// levels and reconstruction by one thread. Returns the eob.
+__device__ int code_wht(const Ctx &c, Smem &sm, const uint8_t *src, int stride, uint8_t *rec, int rs, int x, int y, int plane,
+                        int32_t *coefOut) {
+  const int dcQ = c.fp->dc_q[plane], acQ = c.fp->ac_q[plane], tid = threadIdx.x;
+  // 4x4 Walsh-Hadamard, exact inverse of the spec's (k_fwd.h:112-136); one thread
+  if (tid == 0) {
+    int r[16], t[16];
+    for (int i = 0; i < 4; i++)
+      for (int j = 0; j < 4; j++) r[i * 4 + j] = (int)src[(y + i) * stride + x + j] - (int)rec[(y + i) * rs + x + j];
+    for (int j = 0; j < 4; j++) {
+      int a1 = r[0 * 4 + j], b1 = r[1 * 4 + j], c1 = r[2 * 4 + j], d1 = r[3 * 4 + j];
+      a1 += b1;
+      d1 = d1 - c1;
+      int e1 = (a1 - d1) >> 1;
+      b1 = e1 - b1;
+      c1 = e1 - c1;
+      a1 -= c1;
+      d1 += b1;
+      t[0 * 4 + j] = a1; t[1 * 4 + j] = c1; t[2 * 4 + j] = d1; t[3 * 4 + j] = b1;
+    }
+    for (int i = 0; i < 4; i++) {
+      int a1 = t[i * 4 + 0], b1 = t[i * 4 + 1], c1 = t[i * 4 + 2], d1 = t[i * 4 + 3];
+      a1 += b1;
+      d1 -= c1;
+      int e1 = (a1 - d1) >> 1;
+      b1 = e1 - b1;
+      c1 = e1 - c1;
+      a1 -= c1;
+      d1 += b1;
+      sm.q[i * 4 + 0] = a1; sm.q[i * 4 + 1] = c1; sm.q[i * 4 + 2] = d1; sm.q[i * 4 + 3] = b1;
+    }
+    int eob = 0;
+    const int16_t *inv = d_inv_scan + d_inv_scan_off[0][TX_4X4];
+    for (int k = 0; k < 16; k++) {
+      coefOut[k] = sm.q[k];
+      if (sm.q[k] != 0) eob = imax(eob, inv[k] + 1);
+    }
+    if (eob > 0) {
+      int32_t rr[4][4];
+      for (int i = 0; i < 4; i++) {
+        int32_t tt[4];
+        for (int j = 0; j < 4; j++) tt[j] = tx::dequant_level(sm.q[i * 4 + j], (i == 0 && j == 0) ? dcQ : acQ, 1);
+        tx::iwht(tt, 2);
+        for (int j = 0; j < 4; j++) rr[i][j] = tt[j];
+      }
+      for (int j = 0; j < 4; j++) {
+        int32_t tt[4];
+        for (int i = 0; i < 4; i++) tt[i] = clip3(-(1 << 15), (1 << 15) - 1, rr[i][j]);
+        tx::iwht(tt, 0);
+        for (int i = 0; i < 4; i++) rr[i][j] = tt[i];
+      }
+      for (int i = 0; i < 4; i++)
+        for (int j = 0; j < 4; j++) {
+          int o = (y + i) * rs + x + j;
+          rec[o] = (uint8_t)clip1((int)rec[o] + rr[i][j]);
+        }
+    }
+    sm.flag = eob;
+  }
+  __syncthreads();
+  int eob = sm.flag;
+  __syncthreads();
+  return eob;
+}
+
+// Transform, quantise and reconstruct one inter transform block whose prediction
 // is in `rec` (code_tx_block, k_recon.h:60-173). Returns the eob.
-template <bool INTER>
 __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *src, int stride, uint8_t *rec, int rs, int x, int y, int txSz,
                        int plane, const int *cands, int numCands, int32_t *coefOut, int *outType, long long *outCost) {
   const FrameParams *fp = c.fp;
@@ -725,71 +732,7 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
   int w = 1 << lw, h = 1 << lh, tw = imin(32, w), th = imin(32, h);
   int dcQ = fp->dc_q[plane], acQ = fp->ac_q[plane];
   int tid = threadIdx.x;
-  if (fp->lossless) {
-    // 4x4 Walsh-Hadamard, exact inverse of the spec's (k_fwd.h:112-136); one thread
-    if (tid == 0) {
-      int r[16], t[16];
-      for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) r[i * 4 + j] = (int)src[(y + i) * stride + x + j] - (int)rec[(y + i) * rs + x + j];
-      for (int j = 0; j < 4; j++) {
-        int a1 = r[0 * 4 + j], b1 = r[1 * 4 + j], c1 = r[2 * 4 + j], d1 = r[3 * 4 + j];
-        a1 += b1;
-        d1 = d1 - c1;
-        int e1 = (a1 - d1) >> 1;
-        b1 = e1 - b1;
-        c1 = e1 - c1;
-        a1 -= c1;
-        d1 += b1;
-        t[0 * 4 + j] = a1; t[1 * 4 + j] = c1; t[2 * 4 + j] = d1; t[3 * 4 + j] = b1;
-      }
-      for (int i = 0; i < 4; i++) {
-        int a1 = t[i * 4 + 0], b1 = t[i * 4 + 1], c1 = t[i * 4 + 2], d1 = t[i * 4 + 3];
-        a1 += b1;
-        d1 -= c1;
-        int e1 = (a1 - d1) >> 1;
-        b1 = e1 - b1;
-        c1 = e1 - c1;
-        a1 -= c1;
-        d1 += b1;
-        sm.q[i * 4 + 0] = a1; sm.q[i * 4 + 1] = c1; sm.q[i * 4 + 2] = d1; sm.q[i * 4 + 3] = b1;
-      }
-      int eob = 0;
-      const int16_t *inv = d_inv_scan + d_inv_scan_off[0][TX_4X4];
-      for (int k = 0; k < 16; k++) {
-        coefOut[k] = sm.q[k];
-        if (sm.q[k] != 0) eob = imax(eob, inv[k] + 1);
-      }
-      if (eob > 0) {
-        int32_t rr[4][4];
-        for (int i = 0; i < 4; i++) {
-          int32_t tt[4];
-          for (int j = 0; j < 4; j++) tt[j] = tx::dequant_level(sm.q[i * 4 + j], (i == 0 && j == 0) ? dcQ : acQ, 1);
-          tx::iwht(tt, 2);
-          for (int j = 0; j < 4; j++) rr[i][j] = tt[j];
-        }
-        for (int j = 0; j < 4; j++) {
-          int32_t tt[4];
-          for (int i = 0; i < 4; i++) tt[i] = clip3(-(1 << 15), (1 << 15) - 1, rr[i][j]);
-          tx::iwht(tt, 0);
-          for (int i = 0; i < 4; i++) rr[i][j] = tt[i];
-        }
-        for (int i = 0; i < 4; i++)
-          for (int j = 0; j < 4; j++) {
-            int o = (y + i) * rs + x + j;
-            rec[o] = (uint8_t)clip1((int)rec[o] + rr[i][j]);
-          }
-      }
-      sm.flag = eob;
-    }
-    __syncthreads();
-    int eob = sm.flag;
-    __syncthreads();
-    *outType = DCT_DCT;
-    *outCost = 0;
-    return eob;
-  }
-
-  if (INTER && numCands > 1 && lw <= 4 && lh <= 4)
+  if (numCands > 1 && lw <= 4 && lh <= 4)
     return search_types(c, sm, src + y * stride + x, stride, rec + y * rs + x, rs, txSz, plane, cands, numCands, coefOut, outType,
                         outCost);
   // an inter block has no depth search: a single candidate's cost is not used
@@ -809,7 +752,7 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
       sm.resid[i * 64 + j] = (int)src[(y + yy) * stride + x + xx] - (int)rec[(y + yy) * rs + x + xx];
     }
     __syncthreads();
-    const int32_t *Mh = fwd_matrix_t<INTER>(c, sm, tx::row_kind(t), lw), *Mv = fwd_matrix<INTER>(c, sm, tx::col_kind(t), lh);
+    const int32_t *Mh = c.mats_t + fwd_slot(tx::row_kind(t), lw), *Mv = c.mats + fwd_slot(tx::col_kind(t), lh);
     if (tid == 0) {  // row pass h x tw outputs of w terms, column pass th x tw outputs of h terms
       WORK(W_REC_FWD_MAC, h * tw * w + th * tw * h);
       WORK(W_REC_QUANT, th * tw);
@@ -830,7 +773,7 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
       // only "has coefficients" matters here (the writer derives the eob)
       int nz = __syncthreads_or(myNz);
       for (int k = tid; k < tw * th; k += RT) coefOut[k] = sm.q[k];
-      if (nz) inverse_2d<!INTER>(sm, sm.q, txSz, t, dcQ, acQ, rec, rs, x, y);
+      if (nz) inverse_2d(sm, sm.q, txSz, t, dcQ, acQ, rec, rs, x, y);
       *outType = nz ? t : DCT_DCT;
       *outCost = 0;
       return nz;
@@ -839,7 +782,7 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
     long long sse = 0;
     if (eob > 0) {
       // keep the residual-free path's SSE source intact: the inverse reuses resid
-      inverse_2d<!INTER>(sm, sm.q, txSz, t, dcQ, acQ);
+      inverse_2d(sm, sm.q, txSz, t, dcQ, acQ);
       for (int k = tid; k < h * w; k += RT) {
         int i = k >> lw, j = k & (w - 1);
         int yy = fud ? (h - 1 - i) : i, xx = flr ? (w - 1 - j) : j;
@@ -879,7 +822,7 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
   for (int k = tid; k < tw * th; k += RT) coefOut[k] = qsrc[k];
   if (bestEob > 0) {
     int fud = tx::flip_ud(bestType), flr = tx::flip_lr(bestType);
-    if (numCands > 1) inverse_2d<!INTER>(sm, qsrc, txSz, bestType, dcQ, acQ);
+    if (numCands > 1) inverse_2d(sm, qsrc, txSz, bestType, dcQ, acQ);
     for (int k = tid; k < h * w; k += RT) {
       int i = k >> lw, j = k & (w - 1);
       int yy = fud ? (h - 1 - i) : i, xx = flr ? (w - 1 - j) : j;
@@ -1237,10 +1180,12 @@ __device__ long long code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
         sm.maxLumaW = startX + stepX * 4;
         sm.maxLumaH = startY + stepY * 4;
       }
-      int t = DCT_DCT;
+      int t = DCT_DCT, eob = 0;
       long long cst = 0;
-      int eob = code_tx<INTER>(c, sm, spx, stride, px, rs, startX, startY, txSz, plane, cands, numCands,
-                        c.coefs + b.coef_off[plane] + txIdx * T(Tx_Width)[txSz] * T(Tx_Height)[txSz], &t, &cst);
+      int32_t *coefOut = c.coefs + b.coef_off[plane] + txIdx * T(Tx_Width)[txSz] * T(Tx_Height)[txSz];
+      if (fp->lossless) eob = code_wht(c, sm, spx, stride, px, rs, startX, startY, plane, coefOut);
+      else if constexpr (INTER)
+        eob = code_tx(c, sm, spx, stride, px, rs, startX, startY, txSz, plane, cands, numCands, coefOut, &t, &cst);
       total += cst;
       if (threadIdx.x == 0 && plane == 0) {
         tx_type_set(b, txIdx, t);
@@ -1542,10 +1487,8 @@ __device__ void recon_inter_block(const Ctx &c, Smem &sm, BlockInfo *gb) {
   if (tid == 0) *gb = b;
 }
 
-// The CTA's shared copies of the frame parameters, the quantiser's
-// reciprocals and (intra workers) the forward matrices of lengths 4..16;
-// returns the context reading them.
-template <bool INTER>
+// The CTA's shared copies of the frame parameters and the quantiser's
+// reciprocals; returns the context reading them.
 __device__ Ctx load_shared(const Ctx &c, Smem &sm) {
   const int *src = (const int *)c.fp;
   int *dst = (int *)&sm.fpc;
@@ -1557,20 +1500,9 @@ __device__ Ctx load_shared(const Ctx &c, Smem &sm) {
     int p = threadIdx.x >> 1, q = (threadIdx.x & 1) ? c.fp->ac_q[p] : c.fp->dc_q[p];
     sm.qinv[p][threadIdx.x & 1] = q > 0 ? tx::quant_inv(q) : 0;
   }
-  if (!INTER)  // the inter kernel's shared memory ends before the intra part
-    for (int kind = 0; kind < 3; kind++)
-      for (int lg = 2; lg <= 4; lg++) {
-        int n = 1 << (2 * lg), off = lg == 2 ? 0 : lg == 3 ? 16 : 80;
-        for (int k = threadIdx.x; k < n; k += RT) {
-          sm.fmat[kind][off + k] = c.mats[fwd_slot(kind, lg) + k];
-          sm.fmatT[kind][off + k] = c.mats_t[fwd_slot(kind, lg) + k];
-        }
-      }
   __syncthreads();
   return cs;
 }
-
-
 
 // The inter blocks of the frame (they read reference pictures only, so none
 // waits): persistent CTAs take them from the list, large ones first. With one
@@ -1582,7 +1514,7 @@ __global__ void __launch_bounds__(INTER_THREADS, 512 / INTER_THREADS) k_recon_in
   Smem &sm = *(Smem *)smem_raw;
   const int big = cg.counters[CNT_BIG], total = big + cg.counters[CNT_SMALL], tid = threadIdx.x;
   if ((int)blockIdx.x >= total) return;
-  const Ctx c = load_shared<true>(cg, sm);
+  const Ctx c = load_shared(cg, sm);
   if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar)) : "memory");
   for (unsigned phase = 0;; phase ^= 1) {
     if (tid == 0) sm.flag = atomicAdd(c.counters + CNT_TAKEN, 1);
@@ -2108,7 +2040,7 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
                                            int plane) {
   constexpr int RS = MAXD + 4, MAXW = MAXD * MAXD / 4 / NT;
   const FrameParams *fp = &sh.fpc;
-  const int tid = g.tid, lane = tid & 31;
+  const int tid = g.tid;
   const unsigned geo = t.geo;
   const int lw = geo & 7, lh = (geo >> 3) & 7, w = 1 << lw, h = 1 << lh, wl = lw - 2, nw = 1 << (lw + lh - 2);
   const int mode = (geo >> 6) & 15, haveLeft = (geo >> 10) & 1, haveAbove = (geo >> 11) & 1;
@@ -2382,7 +2314,7 @@ __device__ void feed(const Ctx &c, Shared &sh, int kind, int total) {
 // Workers per kind: as many as the frame's blocks can use, so that on frames
 // of few intra blocks the other SMs stay free for the other engine's kernels.
 #ifndef MAV1CU_BLOCKS_PER_WORKER
-#define MAV1CU_BLOCKS_PER_WORKER 8
+#define MAV1CU_BLOCKS_PER_WORKER 16
 #endif
 #ifndef MAV1CU_MIN_WORKERS
 #define MAV1CU_MIN_WORKERS 8
@@ -2787,7 +2719,7 @@ __device__ void search_worker(const Ctx &c, SearchShared &sh) {
 // Every intra block of the frame, one persistent launch: even CTAs code luma,
 // odd ones chroma.
 template <bool SEARCH>
-__global__ void __launch_bounds__(SEARCH ? SEARCH_WORKERS : WORKER_THREADS, SEARCH ? 2 : 3) k_recon_blocks(Ctx c) {
+__global__ void __launch_bounds__(SEARCH ? SEARCH_WORKERS : WORKER_THREADS, SEARCH ? 2 : 4) k_recon_blocks(Ctx c) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int total = c.counters[CNT_TOTAL], kind = blockIdx.x & 1, tid = threadIdx.x;
   if ((int)(blockIdx.x >> 1) >= imax(MIN_WORKERS, total / BLOCKS_PER_WORKER)) return;
@@ -2816,7 +2748,7 @@ __global__ void __launch_bounds__(INTRA_THREADS) k_recon_lossless(Ctx cg) {
   Smem &sm = *(Smem *)smem_raw;
   const int me = blockIdx.x, sb = me / MAX_BLOCKS_PER_SB, tid = threadIdx.x;
   if (me % MAX_BLOCKS_PER_SB >= cg.sbs[sb].num_blocks || cg.blocks[me].is_inter) return;
-  const Ctx c = load_shared<false>(cg, sm);
+  const Ctx c = load_shared(cg, sm);
   const FrameParams *fp = c.fp;
   const int r0 = (sb / fp->sb_cols) * 16, c0 = (sb % fp->sb_cols) * 16;
   if (tid < (int)(sizeof(BlockInfo) / 4)) ((int *)&sm.blk)[tid] = ((const int *)(c.blocks + me))[tid];

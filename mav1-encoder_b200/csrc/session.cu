@@ -86,7 +86,7 @@ struct mav1cu_session {
   int *flow;               // the intra dataflow's zeroed state: counters, successor counts, ready queues (rec::Ctx)
   int *dep_count, *succ;   // its dependency counts (and the inter block list) and successor lists
   rec::IntraTask *tasks;   // its block records
-  int resident_recon;      // intra recon workers of a kind (one per SM)
+  int resident_recon;      // intra recon workers of a kind
   int resident_inter;      // inter recon CTAs resident at once
   int4 *xcounts;           // compact export: per-superblock counts, block and level bases, zero run / fit flag
   int *xblk_base, *xcoef_base, *xmeta;
@@ -417,10 +417,11 @@ extern "C" int mav1cu_session_create(int width, int height, int max_cdef_presets
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // at most one luma and one chroma worker per SM (the kernel keeps max(8,
-    // intra blocks / 8) of each): the rest of each SM stays free for the
-    // other engines' kernels
-    s->resident_recon = imax(1, sms);
+    // as many luma and chroma workers together as there are SMs, so one CTA
+    // an SM and the rest of it for the other engines' kernels. With a worker of
+    // each kind on every SM one session's frame was no faster (1440p key frame
+    // 5.2 ms) and three sessions at once were slower: 4.3 against 2.7 ms a frame
+    s->resident_recon = imax(1, sms / 2);
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rec::k_recon_inter, rec::INTER_THREADS, rec::SMEM_INTER);
     s->resident_inter = imax(1, sms * per);

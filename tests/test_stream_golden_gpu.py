@@ -77,3 +77,23 @@ def test_lr_search_unit_sizes(w, h):
     finally:
         sess.close()
     assert not bad, bad
+
+
+# pictures of one superblock and of less, of partial superblocks on either side, of several tile columns, a wide
+# one of one superblock row: the edges of the dataflow's records, the filter tiles and the refinement windows
+SIZES = [(64, 64), (72, 72), (130, 66), (66, 194), (392, 40), (264, 136)]
+TOOLS = {
+    "turbo": dict(q=110, turbo=1, keyint=4, tiles=1),
+    "full": dict(q=90, altref=4, golden=1, tiles=1, me_range=64),
+    "lossless": dict(q=0, fast=1),
+}
+
+
+@pytest.mark.skipif(not oracle.available(), reason="oracle not built")
+@pytest.mark.parametrize("tools", sorted(TOOLS))
+@pytest.mark.parametrize("w,h", SIZES)
+def test_stream_sizes_match_oracle(w, h, tools):
+    spec = synthetic.ClipSpec(w, h, 4, seed=w + 3 * h, rects=3, rect_size=(8, 32))
+    tr, _, frames, _, _ = parity.trace_clip(spec, 4, **TOOLS[tools])
+    bad = [(k, o) for k, o in parity.stream_vs_oracle(tr, frames, TOOLS[tools], spec) if any(o.values())]
+    assert not bad, bad

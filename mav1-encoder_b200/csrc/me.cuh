@@ -39,70 +39,112 @@ struct Frame {
 HD int dec_w(const FrameParams *fp) { return (fp->frame_w + 3) >> 2; }
 HD int dec_h(const FrameParams *fp) { return (fp->frame_h + 3) >> 2; }
 
+// acc + the dot product of four unsigned samples and four signed factors
+__device__ __forceinline__ int dp4s(uint32_t px, uint32_t w, int acc) {
+  int r;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(px), "r"(w), "r"(acc));
+  return r;
+}
+
 // ---- quarter-pel and decimated planes -----------------------------------------
 
 // Plane fy * 4 + fx holds the EIGHTTAP prediction of (y + fy / 4, x + fx / 4)
 // (k_me.h:289-313): horizontal Round2( ., 3 ), vertical Round2( ., 11 ), Clip1.
-// A CTA of 32 x 8 threads makes a QP_TW x QP_TH tile of all 16 planes: the
-// clamped reference window (QP_TH + 7 rows, QP_TW + 7 columns) is staged in
-// shared memory once, the horizontal pass (4 phases) runs once per window
-// row and column, and each thread forms 4 consecutive samples of one row for
-// every plane, stored as one 32-bit word where the plane row allows. Every
-// sample is the same sums and roundings as the per-sample definition.
-constexpr int QP_TW = 128, QP_TH = 8, QP_THREADS = 256;
+// Integer work bounds it, not the 16 W H bytes written: 8 multiply-adds a
+// pass and sample, clip and pack took 115 us for a 3840x2160 picture. So
+// - the two outer taps of this filter are zero and every tap is even: half
+//   taps fit 8 bits, (2 S + 4) >> 3 = (S + 2) >> 2 and (2 S + 1024) >> 11 =
+//   (S + 512) >> 10 exactly, a horizontal sum is 2 byte dot products and a
+//   vertical one 3 dot products of a 16-bit row pair, and a full-sample phase
+//   is the same code with the tap 64;
+// - a thread walks down 4 columns of one horizontal phase with the last rows'
+//   sums as pairs in registers: no shared memory, 5 extra rows in QP_ROWS + 5.
+// 3840x2160: 115 -> 56 us a picture (2.4 TB/s of writes; a leaf frame 1.47 -> 1.38 ms).
+// The four phases of a strip are four warps of one CTA, so the reference rows
+// come from L1 for three of them.
+constexpr int QP_TW = 128, QP_ROWS = 16, QP_STRIPS = 2, QP_TH = QP_ROWS * QP_STRIPS, QP_THREADS = 128 * QP_STRIPS;
+constexpr int QP_FILTERS MAV1T_Subpel_Filters_DIMS = MAV1T_Subpel_Filters;
 
-__global__ void __launch_bounds__(QP_THREADS) k_qpel_planes(const FrameParams *fp, const uint8_t *ref, uint8_t *qp) {
-  __shared__ uint8_t win[QP_TH + 7][QP_TW + 8];
-  __shared__ __align__(16) int16_t hs[4][QP_TH + 7][QP_TW];
+// Half taps t0 .. t0 + 3 of a quarter-pel phase (those past tap 6 are zero) as bytes.
+__host__ __device__ constexpr int qp_half(int phase, int t0) {
+  uint32_t w = 0;
+  for (int t = 0; t < 4 && t0 + t < 8; t++) w |= (uint32_t)((QP_FILTERS[EIGHTTAP][4 * phase][t0 + t] / 2) & 255) << (8 * t);
+  return (int)w;
+}
+constexpr bool qp_taps_fit() {
+  for (int p = 0; p < 4; p++) {
+    const auto &f = QP_FILTERS[EIGHTTAP][4 * p];
+    if (f[0] || f[7]) return false;
+    for (int t = 0; t < 8; t++)
+      if (f[t] % 2 || f[t] < -256 || f[t] > 254) return false;
+  }
+  return true;
+}
+static_assert(qp_taps_fit(), "the quarter-pel filters have six even taps of at most 9 bits");
+
+__global__ void __launch_bounds__(QP_THREADS, 4) k_qpel_planes(const FrameParams *fp, const uint8_t *ref, uint8_t *qp) {
   const int W = fp->frame_w, H = fp->frame_h, stride = fp->stride[0];
-  const uint8_t *rp = ref + fp->offset[0];
-  const int x0 = blockIdx.x * QP_TW, y0 = blockIdx.y * QP_TH, tid = threadIdx.x;
-  for (int i = tid; i < (QP_TH + 7) * (QP_TW + 7); i += QP_THREADS) {
-    int r = i / (QP_TW + 7), c = i - r * (QP_TW + 7);
-    win[r][c] = rp[clip3(0, H - 1, y0 + r - 3) * stride + clip3(0, W - 1, x0 + c - 3)];
+  const int tid = threadIdx.x, fx = (tid >> 5) & 3;
+  const int x = blockIdx.x * QP_TW + (tid & 31) * 4, y0 = blockIdx.y * QP_TH + (tid >> 7) * QP_ROWS;
+  // taps: the horizontal pass over the strips' rows (4 phases), the vertical pass per output of 16 planes
+  if (tid == 0)
+    WORK(W_QPEL_TAPS, (QP_ROWS + 5) * QP_STRIPS * QP_TW * 4 * 6 +
+                          imin(QP_TH, H - (int)blockIdx.y * QP_TH) * imin(QP_TW, W - (int)blockIdx.x * QP_TW) * 16 * 6);
+  if (x >= W || y0 >= H) return;
+  constexpr int T0[4] = {qp_half(0, 1), qp_half(1, 1), qp_half(2, 1), qp_half(3, 1)};
+  constexpr int T1[4] = {qp_half(0, 5), qp_half(1, 5), qp_half(2, 5), qp_half(3, 5)};
+  const int t0 = fx < 2 ? (fx ? T0[1] : T0[0]) : (fx == 2 ? T0[2] : T0[3]);
+  const int t1 = fx < 2 ? (fx ? T1[1] : T1[0]) : (fx == 2 ? T1[2] : T1[3]);
+  // The columns x - 4 .. x + 7 as three aligned words (strides are multiples
+  // of 32 samples); columns outside the picture take its edge sample.
+  const uint8_t *col = ref + fp->offset[0] + x;
+  const int before = x ? -4 : 0, after = x + 4 < stride ? 4 : 0;
+  const uint32_t sel0 = x ? 0x3210 : 0;
+  uint32_t sel1 = 0, sel2 = 0;
+  for (int j = 0; j < 4; j++) {
+    sel1 |= (uint32_t)imin(j, W - 1 - x) << (4 * j);
+    sel2 |= (uint32_t)imin(4 + j, W - 1 - x) << (4 * j);
   }
-  __syncthreads();
-  for (int i = tid; i < (QP_TH + 7) * QP_TW; i += QP_THREADS) {
-    int r = i / QP_TW, x = i - r * QP_TW;
-    int px[8];
-    for (int u = 0; u < 8; u++) px[u] = win[r][x + u];
-    for (int fx = 0; fx < 4; fx++) {
-      const int32_t *f = d_Subpel_Filters[EIGHTTAP][4 * fx];
-      int sum = 0;
-      for (int u = 0; u < 8; u++) sum += f[u] * px[u];
-      hs[fx][r][x] = (int16_t)round2(sum, 3);
+  const size_t n = (size_t)W * H;
+  uint8_t *out = qp + fx * n + (size_t)y0 * W + x;
+  const bool word = (W & 3) == 0;  // every plane row 4-byte aligned
+  int prev[4], pair[5][4];  // the last row's sums; sums of rows r and r + 1 as halves, for the last five r
+#pragma unroll
+  for (int r = 0; r < QP_ROWS + 5; r++) {
+    const uint8_t *row = col + (size_t)clip3(0, H - 1, y0 + r - 2) * stride;
+    uint32_t l0 = __ldg((const uint32_t *)(row + before)), l1 = __ldg((const uint32_t *)row),
+             l2 = __ldg((const uint32_t *)(row + after));
+    uint32_t w0 = __byte_perm(l0, l0, sel0), w1 = __byte_perm(l1, l2, sel1), w2 = __byte_perm(l1, l2, sel2);
+    int h[4];
+    h[0] = dp4s(__funnelshift_r(w1, w2, 16), t1, dp4s(__funnelshift_r(w0, w1, 16), t0, 2)) >> 2;
+    h[1] = dp4s(__funnelshift_r(w1, w2, 24), t1, dp4s(__funnelshift_r(w0, w1, 24), t0, 2)) >> 2;
+    h[2] = dp4s(w2, t1, dp4s(w1, t0, 2)) >> 2;
+    h[3] = dp4s(w2 >> 8, t1, dp4s(__funnelshift_r(w1, w2, 8), t0, 2)) >> 2;
+    for (int k = 0; k < 4; k++) {
+      if (r) pair[(r - 1) % 5][k] = (int)__byte_perm((uint32_t)prev[k], (uint32_t)h[k], 0x5410);
+      prev[k] = h[k];
     }
-  }
-  __syncthreads();
-  // taps: the horizontal pass over the window (4 phases), the vertical pass per output of 16 planes
-  if (tid == 0) WORK(W_QPEL_TAPS, (QP_TH + 7) * QP_TW * 4 * 8 + imin(QP_TH, H - y0) * imin(QP_TW, W - x0) * 16 * 8);
-  const int ty = tid >> 5, xx = (tid & 31) * 4, y = y0 + ty, x = x0 + xx;
-  if (y >= H || x >= W) return;
-  const size_t n = (size_t)W * H, o = (size_t)y * W + x;
-  const bool word = (W & 3) == 0 && x + 3 < W;  // 4-byte aligned and inside the row
-  for (int fx = 0; fx < 4; fx++) {
-    // this thread's 8 rows x 4 columns of horizontal sums, one 8-byte load per row
-    int hv[8][4];
-    for (int t = 0; t < 8; t++) {
-      int2 w2 = *(const int2 *)&hs[fx][ty + t][xx];
-      hv[t][0] = (int16_t)(w2.x & 0xffff);
-      hv[t][1] = (int16_t)(w2.x >> 16);
-      hv[t][2] = (int16_t)(w2.y & 0xffff);
-      hv[t][3] = (int16_t)(w2.y >> 16);
-    }
+    if (r < 5) continue;
+    if (y0 + r - 5 >= H) return;
     for (int fy = 0; fy < 4; fy++) {
-      const int32_t *f = d_Subpel_Filters[EIGHTTAP][4 * fy];
-      uint8_t *plane = qp + (size_t)(fy * 4 + fx) * n;
-      uint32_t packed = 0;
+      int v[4];
       for (int k = 0; k < 4; k++) {
-        int sum = 0;
-        for (int t = 0; t < 8; t++) sum += f[t] * hv[t][k];
-        uint32_t v = (uint32_t)clip1(round2(sum, 11));
-        if (word) packed |= v << (8 * k);
-        else if (x + k < W) plane[o + k] = (uint8_t)v;
+        int s = __dp2a_hi(pair[(r - 3) % 5][k], T0[fy], 512);
+        if (fy) s = __dp2a_lo(pair[(r - 1) % 5][k], T1[fy], __dp2a_lo(pair[(r - 5) % 5][k], T0[fy], s));
+        v[k] = s >> 10;
       }
-      if (word) *(uint32_t *)(plane + o) = packed;
+      uint8_t *o = out + (size_t)fy * 4 * n;
+      if (word) {
+        uint32_t hi, packed;  // saturating to 0 .. 255
+        asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(v[3]), "r"(v[2]));
+        asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(packed) : "r"(v[1]), "r"(v[0]), "r"(hi));
+        *(uint32_t *)o = packed;
+      } else {
+        for (int k = 0; k < 4; k++)
+          if (x + k < W) o[k] = (uint8_t)clip1(v[k]);
+      }
     }
+    out += W;
   }
 }
 
@@ -355,12 +397,7 @@ __device__ __noinline__ unsigned grid_sads(const FrameParams *fp, const uint8_t 
 }
 
 // A row's 4-point Hadamard transform is four dot products of its bytes with
-// +-1 words; `h` picks the word. dp4s adds one to acc.
-__device__ __forceinline__ int dp4s(uint32_t px, uint32_t w, int acc) {
-  int r;
-  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(px), "r"(w), "r"(acc));
-  return r;
-}
+// +-1 words; `h` picks the word.
 __host__ __device__ constexpr uint32_t hadamard_word(int h) {
   return h == 0 ? 0x01010101u : h == 1 ? 0xffff0101u : h == 2 ? 0x01ffff01u : 0xff01ff01u;  // ++++, ++--, +--+, +-+-
 }

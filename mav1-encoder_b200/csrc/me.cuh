@@ -543,6 +543,16 @@ __device__ __forceinline__ void subpel_costs(const Frame &f, const Node &m, cons
         cost[c] = v * st;
       }
     }
+  } else if constexpr (nus >= 32) {
+    // several candidates at a time, nus / 32 warps of the CTA each
+    if (g.rank < ncand) cost[g.rank] = 0;
+    g.sync();
+    const int u = g.rank & (nus - 1);
+    take(u);
+    for (int c = g.rank / nus; c < ncand; c += Grp::size / nus) {
+      int v = __reduce_add_sync(g.mask, satd(c, u));
+      if ((g.rank & 31) == 0) atomicAdd(&cost[c], v * st);
+    }
   } else {
     // several candidates at a time, nus lanes each
     constexpr int lg = 2 * ln;
@@ -557,25 +567,35 @@ __device__ __forceinline__ void subpel_costs(const Frame &f, const Node &m, cons
   g.sync();
 }
 
-// One search level: the CTA's four warps per node (the 64x64 level: few, large
-// nodes), a warp per (node, reference), or half a warp (the 8x8 level);
+// One search level: a whole CTA per node (the 64x64 level: few, large nodes),
+// a warp per (node, reference), or half a warp (the 8x8 level);
 // blockIdx.y selects the reference. Level and sub-pel path (HP: quarter-pel
 // planes) are compile-time: with one kernel for all of them the 16x16 level
 // executed 3,800 instructions a node, a seventh of them spilled registers.
 // 6 CTAs per SM with planes (80 registers a thread; 1-2% on the 1080p clip over
 // 5), 5 without (the prediction spills below 96).
-__host__ __device__ constexpr int me_group(int level) { return level == 0 ? 128 : level == 3 ? 16 : 32; }
+// Without planes every full-range candidate is a full SAD and every sub-pel
+// unit its own prediction, and a picture has few large nodes (640x360: 60 and
+// 240): 16 warps take a 64x64 node and 4 a 32x32 one.
+// A clip alone, 4 warps and 1 before: 352x288 lossless 2.40 -> 1.95 ms, 363x241
+// low delay 11.5 -> 10.9, 640x360 with every tool 25.5 -> 24.4; 3840x2160, where
+// the nodes fill the chip anyway, 114.3 -> 114.8 (runs differ by 0.3).
+__host__ __device__ constexpr int me_group(int level, bool hp) {
+  return level == 0 ? (hp ? 128 : 512) : level == 1 && !hp ? 128 : level == 3 ? 16 : 32;
+}
+__host__ __device__ constexpr int me_threads(int level, bool hp) { return level == 0 && !hp ? 512 : 128; }
 template <int LEVEL, bool HP>
-__global__ void __launch_bounds__(128, HP ? 6 : 5) k_me_level(Frame f0, Frame f1) {
+__global__ void __launch_bounds__(me_threads(LEVEL, HP), HP ? 6 : LEVEL == 0 ? 1 : 5) k_me_level(Frame f0, Frame f1) {
   __shared__ int s_cost[8][16];
   __shared__ int s_r[8][16], s_c[8][16];
-  __shared__ unsigned long long s_best[4];
-  __shared__ unsigned s_sad[4][26];
+  constexpr int group = me_group(LEVEL, HP), warps = me_threads(LEVEL, HP) / 32;
+  constexpr bool whole_cta = group == 32 * warps;
+  __shared__ unsigned long long s_best[warps];
+  __shared__ unsigned s_sad[warps][26];
   const Frame f = blockIdx.y ? f1 : f0;
   const FrameParams *fp = f.fp;
-  constexpr int level = LEVEL, group = me_group(LEVEL);
+  constexpr int level = LEVEL;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr bool whole_cta = group == 128;
   const int half = lane >> 4;
   const MeGrp<group> grp = whole_cta ? MeGrp<group>{(int)threadIdx.x, 0xffffffffu}
                            : group == 32 ? MeGrp<group>{lane, 0xffffffffu}
@@ -609,11 +629,13 @@ __global__ void __launch_bounds__(128, HP ? 6 : 5) k_me_level(Frame f0, Frame f1
     unsigned long long best = ~0ull;
     const int grs = (fp->turbo & T_ME_RSUB) ? 2 : 1;
     if (grp.size >= 32 && grid_inside(fp, m)) {
-      unsigned sad = grid_sads(fp, f.src, f.ref, m.x, m.y, m.w, m.cy, m.cx, grs, lane, whole_cta ? warp : 0, whole_cta ? 4 : 1);
+      unsigned sad = grid_sads(fp, f.src, f.ref, m.x, m.y, m.w, m.cy, m.cx, grs, lane, whole_cta ? warp : 0, whole_cta ? warps : 1);
       if (whole_cta) {
         if (lane < 26) s_sad[warp][lane] = sad;
         __syncthreads();
-        if (lane < 26) sad = s_sad[0][lane] + s_sad[1][lane] + s_sad[2][lane] + s_sad[3][lane];
+        sad = 0;
+        if (lane < 26)
+          for (int w = 0; w < warps; w++) sad += s_sad[w][lane];
       }
       if (lane < 26) {
         int dy, dx;
@@ -622,7 +644,7 @@ __global__ void __launch_bounds__(128, HP ? 6 : 5) k_me_level(Frame f0, Frame f1
       }
     } else if (whole_cta) {
       // a warp per candidate, every lane holding the warp's running minimum
-      for (int k = warp; k < m.count; k += 4) {
+      for (int k = warp; k < m.count; k += warps) {
         int dy, dx;
         candidate(m, k, &dy, &dx);
         int cost = warp_full_cost(fp, f.src, f.ref, f.dsrc, f.dref, m.x, m.y, m.w, m.step, dy, dx, lane);
@@ -661,7 +683,7 @@ __global__ void __launch_bounds__(128, HP ? 6 : 5) k_me_level(Frame f0, Frame f1
       __syncthreads();
       if (lane == 0) s_best[warp] = best;
       __syncthreads();
-      for (int w = 0; w < 4; w++) best = s_best[w] < best ? s_best[w] : best;
+      for (int w = 0; w < warps; w++) best = s_best[w] < best ? s_best[w] : best;
     }
     candidate(m, (int)(best & 0xffffffffu), &by, &bx);
   }

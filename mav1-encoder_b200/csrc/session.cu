@@ -558,13 +558,13 @@ extern "C" int mav1cu_motion_search(mav1cu_session *s) {
   }
   const bool hp = fp.turbo & T_ME_HPEL;
   for (int level = 0; level < 4; level++) {
-    int nodes = s->g.num_sbs << (2 * level), per = 128 / me::me_group(level);
+    int nodes = s->g.num_sbs << (2 * level), threads = me::me_threads(level, hp), per = threads / me::me_group(level, hp);
     dim3 grid((nodes + per - 1) / per, nref);
     auto *kernel = level == 0   ? (hp ? me::k_me_level<0, true> : me::k_me_level<0, false>)
                    : level == 1 ? (hp ? me::k_me_level<1, true> : me::k_me_level<1, false>)
                    : level == 2 ? (hp ? me::k_me_level<2, true> : me::k_me_level<2, false>)
                                 : (hp ? me::k_me_level<3, true> : me::k_me_level<3, false>);
-    kernel<<<grid, 128, 0, s->stream>>>(f[0], f[1]);
+    kernel<<<grid, threads, 0, s->stream>>>(f[0], f[1]);
     if (after_launch(s, "motion search")) return s->err;
   }
   return MAV1CU_OK;

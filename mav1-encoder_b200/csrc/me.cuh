@@ -12,12 +12,12 @@
 // rows on packed bytes with __vsadu4; interior candidates read unaligned
 // words through funnel shifts), and the warp reduces the 64-bit key
 // (cost << 32 | index) with shuffles, which yields exactly the serial first
-// minimum. The 64x64 level has few nodes: a CTA per node, its four warps
+// minimum. The 64x64 level has few nodes: a CTA per node, its warps
 // taking candidates in turn and each warp's lanes splitting a candidate's
 // byte pairs. Sub-pel candidates x 4x4 units are spread over the lanes and
 // summed in shared memory. Quarter-pel planes (16 per reference, EIGHTTAP,
 // the T_ME_HPEL mode) are built once per reference picture by their own
-// kernel, one thread per sample.
+// kernel.
 #pragma once
 
 #include "common.cuh"
@@ -298,7 +298,7 @@ __device__ __noinline__ int full_cost(const Frame f, const Node m, int dy, int d
 }
 
 // The same cost with the warp's 32 lanes splitting one candidate's byte pairs
-// (the 64x64 level: few nodes, so each CTA's four warps take candidates in
+// (levels of few nodes, a CTA each: its warps take candidates in
 // turn instead of one thread a candidate). Every lane returns the total. The
 // sums are the ones full_sad / dec_sad form, in another order: unsigned
 // integer addition, so the cost is the same.

@@ -194,6 +194,32 @@ HD int ldpx(const uint8_t *p) {
 #endif
 }
 
+// The lanes whose ready() holds, as soon as a poll finds any; 0 once done()
+// holds for a lane, or after `limit` polls. done() reads a word that other
+// warps set, so the lanes of one poll may read different values: the warp goes
+// by the vote, never by a lane's own value, so that every lane takes part in
+// the same full-mask operations. Warp: any, ballot, pause.
+#if defined(__CUDACC__)
+#define WARP_FN __device__ __forceinline__
+struct FullWarp {
+  __device__ __forceinline__ bool any(bool p) const { return __any_sync(0xffffffffu, p); }
+  __device__ __forceinline__ unsigned ballot(bool p) const { return __ballot_sync(0xffffffffu, p); }
+  __device__ __forceinline__ void pause() const { __nanosleep(100); }
+};
+#else
+#define WARP_FN inline
+#endif
+template <class Warp, class Done, class Ready>
+WARP_FN unsigned watch_ready(const Warp &warp, int limit, Done done, Ready ready) {
+  for (int polls = 0; polls < limit; polls++) {
+    if (warp.any(done())) return 0;
+    unsigned r = warp.ballot(ready());
+    if (r) return r;
+    warp.pause();
+  }
+  return 0;
+}
+
 HD int block_w(int bs) { return 4 * T(Num_4x4_Blocks_Wide)[bs]; }
 HD int block_h(int bs) { return 4 * T(Num_4x4_Blocks_High)[bs]; }
 

@@ -2262,16 +2262,14 @@ __device__ void feed(const Ctx &c, Shared &sh, int kind, int total) {
       for (int q = 0; q < 3; q++)
         if (push[q] >= 0) atomicExch(c.queue + kind * c.nblk + t[q], push[q] + 1);
     }
+    // (what the watch misses, the release below finds: its limit only ends the look-ahead)
     int next = -1;
-    while (!*coded) {
-      unsigned r = __ballot_sync(0xffffffffu, s[0] >= 0 && *(volatile int *)(dep + imax(s[0], 0)) == 1);
-      if (r) {
-        fence_gpu();  // what its other dependencies wrote is visible, its record among it
-        next = __shfl_sync(0xffffffffu, s[0], __ffs(r) - 1);
-        word = record_word(next);
-        break;
-      }
-      __nanosleep(100);
+    const unsigned r = watch_ready(FullWarp(), c.spin_limit, [&] { return *coded != 0; },
+                                   [&] { return s[0] >= 0 && *(volatile int *)(dep + imax(s[0], 0)) == 1; });
+    if (r) {
+      fence_gpu();  // what its other dependencies wrote is visible, its record among it
+      next = __shfl_sync(0xffffffffu, s[0], __ffs(r) - 1);
+      word = record_word(next);
     }
     __syncwarp();
     coded_bar<N>();
@@ -2338,7 +2336,7 @@ __device__ void luma_worker(const Ctx &c, IntraShared &sh) {
       gb->tx_types_lo &= ~15;
       gb->eob[0] = nz;
     }
-    if (g.tid == 0) sh.coded = 1;
+    if (g.tid == 0) *(volatile int *)&sh.coded = 1;
     coded_bar<WORKER_THREADS>();
   }
 }
@@ -2359,7 +2357,7 @@ __device__ void chroma_worker(const Ctx &c, IntraShared &sh) {
       gb->eob[plane] = nz;
       if ((sh.task.p[1].geo >> 19) & 1) (plane == 1 ? gb->cfl_alpha_u : gb->cfl_alpha_v) = m.alpha;
     }
-    if (threadIdx.x == 0) sh.coded = 1;
+    if (threadIdx.x == 0) *(volatile int *)&sh.coded = 1;
     coded_bar<WORKER_THREADS>();
   }
 }
@@ -2710,7 +2708,7 @@ __device__ void search_worker(const Ctx &c, SearchShared &sh) {
       gb->eob[0] = sh.anyNz;
       c.tasks[me].maxLumaW = sh.maxW;  // the last transform block coded: CfL's limits
       c.tasks[me].maxLumaH = sh.maxH;
-      sh.coded = 1;
+      *(volatile int *)&sh.coded = 1;
     }
     coded_bar<SEARCH_WORKERS>();
   }

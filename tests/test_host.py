@@ -133,6 +133,27 @@ def test_butterfly_sums_fit_32_bits(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+def test_warp_watch_keeps_the_lanes_together(tmp_path):
+    """The feeder warp's bounded watch (watch_ready) takes every lane through
+    the same full-mask operations when the lanes read the flag differently
+    (tests/native/warp_watch_check.cpp)."""
+    import shutil
+    import subprocess
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no host C++ compiler")
+    exe = tmp_path / "warp_watch_check"
+    subprocess.run([cxx, "-O2", "-std=c++17", "-pthread", "-I", os.path.join(ROOT, "include"),
+                    "-I", os.path.join(ROOT, "mav1-encoder_b200", "csrc"), "-x", "c++",
+                    os.path.join(ROOT, "tests", "native", "warp_watch_check.cpp"), "-o", str(exe)],
+                   check=True, capture_output=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+    # the feeder has no loop of its own on the flag
+    text = open(os.path.join(ROOT, "mav1-encoder_b200", "csrc", "recon.cuh")).read()
+    assert "watch_ready(" in text and "while (!*coded)" not in text
+
+
 def test_forward_matrices_identical_from_concurrent_threads():
     """Sessions are created from several host threads at once (one encoder per
     thread); the forward-matrix table each one gets must be the same."""

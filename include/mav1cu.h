@@ -207,7 +207,9 @@ int mav1cu_lr_search(mav1cu_session *s, int lr_test);
  * give up after spin_limit polls instead of about 2^22. The waiting workers
  * then set the session's device status and stop; the launch returns, the
  * context stays usable, and mav1cu_synchronize reports MAV1CU_ERR_DEVICE.
- * The session stays in error afterwards. No counterpart in the reference. */
+ * The session stays in error afterwards. A lossless frame's intra blocks wait
+ * for no other; there hold_block itself waits, gives up the same way and is
+ * not coded. No counterpart in the reference. */
 int mav1cu_debug_recon_fault(mav1cu_session *s, int hold_block, int spin_limit);
 
 /* Waits for the session stream; returns the sticky error state. */

@@ -2746,6 +2746,18 @@ __global__ void __launch_bounds__(INTRA_THREADS) k_recon_lossless(Ctx cg) {
   Smem &sm = *(Smem *)smem_raw;
   const int me = blockIdx.x, sb = me / MAX_BLOCKS_PER_SB, tid = threadIdx.x;
   if (me % MAX_BLOCKS_PER_SB >= cg.sbs[sb].num_blocks || cg.blocks[me].is_inter) return;
+  if (me == cg.hold) {  // never released (Ctx::hold): its wait gives up, like a dependency wait of k_recon_blocks
+    if (tid == 0) {
+      volatile int *abort = cg.status + 1;
+      int spins = 0;
+      while (!*abort && spins++ <= cg.spin_limit) __nanosleep(32);
+      if (!*abort) {
+        atomicExch(cg.status, 1);
+        atomicExch(cg.status + 1, 1);
+      }
+    }
+    return;
+  }
   const Ctx c = load_shared(cg, sm);
   const FrameParams *fp = c.fp;
   const int r0 = (sb / fp->sb_cols) * 16, c0 = (sb % fp->sb_cols) * 16;

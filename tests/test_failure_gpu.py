@@ -22,8 +22,8 @@ def padded_source(frame, geom):
     return np.concatenate(out)
 
 
-def key_frame_session(w, h, seed):
-    cfg = mav1cu.cli_config(w, h, q=100, turbo=1)
+def key_frame_session(w, h, seed, flags=dict(q=100, turbo=1)):
+    cfg = mav1cu.cli_config(w, h, **flags)
     fp, _ = mav1cu.frame_params(cfg, mav1cu.plan(cfg, 1)[0])
     frame = next(synthetic.generate(synthetic.ClipSpec(w, h, 1, seed=seed)))
     s = mav1cu.Session(w, h)
@@ -62,6 +62,26 @@ def test_never_released_dependency_reports_device_error():
         finally:
             good.close()
     assert np.array_equal(outs[0], outs[1])
+
+
+# the kernels with a transform search and of lossless frames
+@pytest.mark.parametrize("flags", [dict(q=90), dict(q=0, fast=1)], ids=["search", "lossless"])
+def test_held_block_reports_device_error_in_every_recon_kernel(flags):
+    w, h = 160, 96
+    bad = key_frame_session(w, h, 83, flags)
+    try:
+        assert bad.lib.mav1cu_debug_recon_fault(bad.h, 0, 4096) == 0
+        bad.frame_core()
+        with pytest.raises(mav1cu.Mav1cuError, match="gave up"):
+            bad.synchronize()
+    finally:
+        bad.close()
+    good = key_frame_session(w, h, 83, flags)
+    try:
+        good.frame_core()
+        good.synchronize()
+    finally:
+        good.close()
 
 
 def test_fault_hook_rejects_bad_arguments():

@@ -329,12 +329,28 @@ def run_ours(args, rank, world):
         st.close()
     del frames_dev, flush
     torch.cuda.synchronize()
-    e2e = e2e_api(args, frames_host, world)
+    e2e = e2e_api(args, frames_host, world) if api_missing() is None else None
     if world > 1:
-        per_step, per_seq, e2e["ms"], e2e["ms_one"] = max_over_ranks(
-            [per_step, per_seq, e2e["ms"], e2e["ms_one"]], f"cuda:{dev}")
+        t = max_over_ranks([per_step, per_seq] + ([e2e["ms"], e2e["ms_one"]] if e2e else []), f"cuda:{dev}")
+        per_step, per_seq = t[:2]
+        if e2e:
+            e2e["ms"], e2e["ms_one"] = t[2:]
     return dict(ms=per_step, ms_seq=per_seq, launches=nlaunch, clocks=clk.summary(), kern=kern, gops=len(gops),
                 e2e=e2e)
+
+
+def api_missing():
+    """Why there is no libmav1.so, or None: its entropy coder is compiled from
+    the reference's sources, so it cannot be built where they are absent."""
+    import mav1api
+    return None if mav1api.available() else "libmav1.so not built (its entropy coder needs the reference's sources)"
+
+
+def oracle_missing():
+    """Why the reference's CPU path cannot run here, or None."""
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle
+    return None if oracle.available() else "oracle/_ref not built (needs the reference's sources)"
 
 
 def e2e_api(args, frames_host, world):
@@ -713,6 +729,9 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return
+        if oracle_missing():
+            print(json.dumps({"impl": "reference", "unavailable": oracle_missing()}))
+            return
         walls, fps_ideal = [], []
         for i in range(args.warmup + args.steps):
             fps, wall, ideal = cpu_reference(REF_SAMPLE)
@@ -749,12 +768,11 @@ def main():
         frames = SPEC.frames * world
         value = frames / (r["ms"] * 1e-3)
         x = r["e2e"]
-        e2e = frames / (x["ms"] * 1e-3)
         line = {"metric": METRIC, "value": round(value, 2), "unit": "fps", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": round(r["ms"], 3), "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "u8/int32", "data": "synthetic", "config": CONFIG,
                 "parallelism": "replicas" if world > 1 else "single",
-                "e2e": {"value": round(e2e, 2), "unit": "fps", "h2d_bytes_per_step": x["h2d"],
+                "e2e": x and {"value": round(frames / (x["ms"] * 1e-3), 2), "unit": "fps", "h2d_bytes_per_step": x["h2d"],
                         "d2h_bytes_per_step": x["d2h"], "ms_per_step": round(x["ms"], 2),
                         "path": "libmav1.so (mav1.h): host frames in, IVF temporal units and reconstructions out",
                         "bitexact_to_oracle": x["bitexact"], "encoders": x["encoders"],
@@ -764,12 +782,14 @@ def main():
                              "fps_one_stream": round(frames / (r["ms_seq"] * 1e-3), 2)},
                 "gpu_launches": int(r["launches"]), "clocks": r["clocks"],
                 "roofline": roofline(r["kern"], peaks, run_work_counts() if r["kern"] else None)}
-        if not args.no_batch:
+        if not x:
+            line["e2e_unavailable"] = api_missing()
+        if not args.no_batch and x:
             try:
                 line["batch"] = batch_bench(args)
             except Exception as ex:  # reported in the line; the clip's numbers stand on their own
                 line["batch"] = {"error": f"{type(ex).__name__}: {ex}"}
-        if not args.no_cpu_baseline:
+        if not args.no_cpu_baseline and not oracle_missing():
             fps, wall, ideal = cpu_reference(args.cpu_sample)
             line["cpu_baseline"] = {"value": round(fps, 3), "unit": "fps", "cores": cores, "kind": "reference",
                                     "sample": f"the clip's first {args.cpu_sample} frames through the reference's "

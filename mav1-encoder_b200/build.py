@@ -15,7 +15,7 @@ host/writer.c and the reference's own entropy coder and OBU writer
 (src/obu.c, tile_writer.c, mvpred.c, entenc.c, cdfs.c, bitwriter.c and the
 LR-unit rate coding of lr_search.c), compiled in place from the reference
 checkout named by MAV1_REFERENCE. Where that checkout is absent, an existing
-libmav1.so is kept as it is.
+libmav1.so is kept as it is, and build_all() builds the device libraries alone.
 """
 import glob
 import os
@@ -126,9 +126,19 @@ def build_cli(verbose=False):
     return out
 
 
+def api_buildable():
+    """Whether build_api() can give a libmav1.so here: the reference's sources or an earlier build."""
+    return os.path.isdir(os.path.join(REFERENCE, "src")) or os.path.exists(API_LIB)
+
+
 def build_all(force=False, verbose=False):
+    """The device library, its counting build and, where it can be built, libmav1.so (its path, else None)."""
     build(force=force, verbose=verbose)
     build_count(force=force, verbose=verbose)
+    if not api_buildable():
+        print(f"libmav1.so skipped: its entropy coder is compiled from the reference's sources (MAV1_REFERENCE={REFERENCE})",
+              flush=True)
+        return None
     return build_api(force=force, verbose=verbose)
 
 

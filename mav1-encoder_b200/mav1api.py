@@ -46,6 +46,11 @@ _lib = None
 _libc = ctypes.CDLL(None)
 
 
+def available():
+    """Whether libmav1.so is there (it is built where the reference's sources are)."""
+    return os.path.exists(LIB_PATH)
+
+
 def lib():
     global _lib
     if _lib is None:

@@ -2,6 +2,10 @@
 through the CUDA stages (via the C ABI) and compares every output with the
 oracle's, field by field. Each stage gets the oracle's own inputs, so a
 mismatch is attributed to exactly one stage."""
+import hashlib
+import json
+import os
+
 import numpy as np
 
 import mav1cu
@@ -273,7 +277,6 @@ def check_all(sess, tr, cfg, stages=STAGES):
 
 
 # ---- whole-stream comparisons -------------------------------------------------------
-import os
 import re
 
 _TABLES = None
@@ -461,3 +464,54 @@ def export_vs_packed(image, blocks, sbs, coefs, cdef, p):
               mav1cu.LRUNIT_DTYPE.itemsize * int(h["lr_units"]) + (0 if irec is None else len(irec)))
     out["bytes"] = int(h["bytes"] != nbytes)
     return out
+
+
+# ---- device streams against committed hashes ---------------------------------------
+# clip and flags of the small entries of golden/oracle_hashes.json (golden/make_golden.py)
+GOLDEN_CLIPS = {
+    "c0_turbo_q125": (dict(width=352, height=288, frames=30, seed=1), dict(q=125, turbo=1, keyint=30, tiles=0)),
+    "full_203x131": (dict(width=203, height=131, frames=9, seed=41, rects=3, rect_size=(16, 48)),
+                     dict(q=90, altref=4, golden=1, tiles=1, me_range=64)),
+    "lowdelay_lr_150x102": (dict(width=150, height=102, frames=6, seed=42, rects=2, rect_size=(16, 40)),
+                            dict(q=200, golden=1, keyint=4, lr_test=1)),
+    "lossless_96x64": (dict(width=96, height=64, frames=3, seed=43, rects=1, rect_size=(16, 32)), dict(q=0, fast=1)),
+}
+
+
+def stream_recon_sha16(spec, flags):
+    """The first 16 hex digits of the SHA-256 of every shown reconstruction, in
+    output order, of a clip coded through a device-resident stream."""
+    import torch
+
+    clip = [torch.from_numpy(np.frombuffer(synthetic.packed(f), np.uint8).copy()).cuda() for f in synthetic.generate(spec)]
+    torch.cuda.synchronize()
+    cfg = mav1cu.cli_config(spec.width, spec.height, **flags)
+    g = mav1cu.geometry(spec.width, spec.height)
+    st = mav1cu.Stream(cfg)
+    shown, slots = [], [None] * 8
+    try:
+        for job in mav1cu.plan(cfg, spec.frames):
+            sess = st.encode(job, clip[int(job["disp"])].data_ptr(), True)
+            st.synchronize()
+            rec = visible(sess.download("REC", count=g["frame_bytes"]), g)
+            sha = hashlib.sha256(rec.tobytes()).hexdigest()[:16]
+            for k in range(8):
+                if (0xFF if job["is_key"] else int(job["refresh"])) >> k & 1:
+                    slots[k] = sha
+            if not job["hidden"]:
+                shown.append(sha)
+            if job["show_existing"] >= 0:
+                shown.append(slots[int(job["show_existing"])])
+    finally:
+        st.close()
+    return shown
+
+
+def golden_stream(name):
+    """A golden clip's shown reconstructions through a stream, and the oracle's."""
+    want = json.load(open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "oracle_hashes.json")))[name]
+    kw, flags = GOLDEN_CLIPS[name]
+    spec = synthetic.ClipSpec(**kw)
+    if synthetic.clip_sha256(spec) != want["clip"]:
+        raise AssertionError(f"{name}: the generated clip differs from the hashed one")
+    return stream_recon_sha16(spec, flags), want["recon_sha16"]

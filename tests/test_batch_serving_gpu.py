@@ -14,7 +14,8 @@ import oracle
 import serve
 import synthetic
 
-pytestmark = pytest.mark.gpu
+# libmav1.so is built where the reference's sources are (its entropy coder is compiled from them)
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not mav1api.available(), reason="libmav1.so not built")]
 
 
 def _h(b):

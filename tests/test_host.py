@@ -133,6 +133,22 @@ def test_butterfly_sums_fit_32_bits(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+def test_builds_without_the_reference_sources(monkeypatch, tmp_path, capsys):
+    """Without the reference's sources the device libraries are built and
+    libmav1.so is skipped with a line that says why; asking for it alone is an
+    error."""
+    import build
+    made = []
+    monkeypatch.setattr(build, "build", lambda **k: made.append("device"))
+    monkeypatch.setattr(build, "build_count", lambda **k: made.append("count"))
+    monkeypatch.setattr(build, "REFERENCE", str(tmp_path / "absent"))
+    monkeypatch.setattr(build, "API_LIB", str(tmp_path / "libmav1.so"))
+    assert build.build_all() is None and made == ["device", "count"]
+    assert "libmav1.so skipped" in capsys.readouterr().out
+    with pytest.raises(RuntimeError, match="reference sources"):
+        build.build_api()
+
+
 def test_warp_watch_keeps_the_lanes_together(tmp_path):
     """The feeder warp's bounded watch (watch_ready) takes every lane through
     the same full-mask operations when the lanes read the flag differently

@@ -6,11 +6,6 @@ loop restoration), the low-delay path with forced loop-restoration units, and
 lossless coding; no oracle build is needed. Loop-restoration units at the
 sizes where the search's layout changes are checked against the oracle where
 it is built."""
-import hashlib
-import json
-import os
-
-import numpy as np
 import pytest
 
 import mav1cu
@@ -20,47 +15,11 @@ import synthetic
 
 pytestmark = pytest.mark.gpu
 
-HERE = os.path.dirname(os.path.abspath(__file__))
-GOLDEN = json.load(open(os.path.join(HERE, "golden", "oracle_hashes.json")))
-# clip and flags of each golden entry (tests/golden/make_golden.py)
-CASES = {
-    "c0_turbo_q125": (dict(width=352, height=288, frames=30, seed=1), dict(q=125, turbo=1, keyint=30, tiles=0)),
-    "full_203x131": (dict(width=203, height=131, frames=9, seed=41, rects=3, rect_size=(16, 48)),
-                     dict(q=90, altref=4, golden=1, tiles=1, me_range=64)),
-    "lowdelay_lr_150x102": (dict(width=150, height=102, frames=6, seed=42, rects=2, rect_size=(16, 40)),
-                            dict(q=200, golden=1, keyint=4, lr_test=1)),
-    "lossless_96x64": (dict(width=96, height=64, frames=3, seed=43, rects=1, rect_size=(16, 32)), dict(q=0, fast=1)),
-}
 
-
-@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("name", sorted(parity.GOLDEN_CLIPS))
 def test_stream_reconstructions_match_golden(name):
-    import torch
-    kw, flags = CASES[name]
-    spec = synthetic.ClipSpec(**kw)
-    assert synthetic.clip_sha256(spec) == GOLDEN[name]["clip"]
-    clip = [torch.from_numpy(np.frombuffer(synthetic.packed(f), np.uint8).copy()).cuda() for f in synthetic.generate(spec)]
-    torch.cuda.synchronize()
-    cfg = mav1cu.cli_config(spec.width, spec.height, **flags)
-    g = mav1cu.geometry(spec.width, spec.height)
-    st = mav1cu.Stream(cfg)
-    shown, slots = [], [None] * 8
-    try:
-        for job in mav1cu.plan(cfg, spec.frames):
-            sess = st.encode(job, clip[int(job["disp"])].data_ptr(), True)
-            st.synchronize()
-            rec = parity.visible(sess.download("REC", count=g["frame_bytes"]), g)
-            sha = hashlib.sha256(rec.tobytes()).hexdigest()[:16]
-            for k in range(8):
-                if (0xFF if job["is_key"] else int(job["refresh"])) >> k & 1:
-                    slots[k] = sha
-            if not job["hidden"]:
-                shown.append(sha)
-            if job["show_existing"] >= 0:
-                shown.append(slots[int(job["show_existing"])])
-    finally:
-        st.close()
-    assert shown == GOLDEN[name]["recon_sha16"]
+    shown, want = parity.golden_stream(name)
+    assert shown == want
 
 
 # one unit narrower and lower than 64 samples, the largest units (95 columns, 103 luma / 99 chroma rows), units

@@ -197,9 +197,18 @@ int mav1cu_restore(mav1cu_session *s);
  * deblocked frame). Writes LRUNITS and lr_type of the device PARAMS record
  * (and of the next export's parameters section). lr_test: Mav1Config.lr_test
  * (Wiener on even units, the self-guided set of least SSE on odd ones).
+ * Units of 64 samples (and the remainder the last row and column of units
+ * take): a unit above 95 x 103 samples is MAV1CU_ERR_ARG, which no unit size
+ * of 64 or less reaches.
  * Replaces lr_select (lr_search.c:244-359), a host step of the reference's
  * run_frame_core (encoder.c:636-638). */
 int mav1cu_lr_search(mav1cu_session *s, int lr_test);
+
+/* A test hook of the restoration search: how many units a round of the choice
+ * takes again (1..256) and how many candidate SSEs a unit keeps (25..40). The
+ * chosen units do not depend on them; small values make the rounds overflow
+ * and the caches refill on a small picture. No counterpart in the reference. */
+int mav1cu_debug_lr_room(mav1cu_session *s, int list, int cache);
 
 /* Failure detection without a device fault (a test hook): the session's next
  * mav1cu_recon counts one more luma dependency for intra block hold_block

@@ -24,7 +24,7 @@
 //   k_lr_select  one CTA per plane: the units whose references turned out
 //                different are chosen again, until every unit stands; a
 //                refinement candidate whose SSE no pass cached is evaluated on
-//                the spot by the whole CTA.
+//                the spot by the whole CTA, for units with settled references.
 //
 // Bit-exactness. SSEs, the self-guided sums and the first Wiener iteration
 // are integer-valued (every partial sum is an integer below 2^53, so double
@@ -43,6 +43,8 @@ namespace lrs {
 
 constexpr int THREADS = 256;
 constexpr int CACHE = 40;       // candidate SSEs a unit keeps from the first pass and the speculative pass
+constexpr int MIN_CACHE = 25;   // the first pass's 13 at most, and the 12 a path under settled references can add
+constexpr int LIST = 256;       // units k_lr_select chooses again in a round
 
 // What the first pass leaves for the serial choice, per unit.
 struct Fit {
@@ -869,7 +871,7 @@ __device__ int cache_find(const int (*taps)[6], int n, const int *tt, Shared &sh
 // filter of a recent unit). k_lr_select then finds most of its candidates
 // here and computes only the rest on the spot.
 __device__ void spec_path(const FrameParams *fp, int plane, const Layout &l, const uint8_t *smem, const int fitted[2][3],
-                          const int ref[2][3], Shared &sh) {
+                          const int ref[2][3], int room, Shared &sh) {
   LrUnit w = wiener_unit(fitted);
   int tw[2][3], tx[2] = {0, 0};
   memcpy(tw, ref, sizeof tw);
@@ -886,7 +888,7 @@ __device__ void spec_path(const FrameParams *fp, int plane, const Layout &l, con
         int f = cache_find(sh.ctaps, n, tt, sh);
         long long sse = f >= 0 ? sh.csse[f] : -1;
         if (sse < 0) {
-          if (n >= CACHE) return;  // full: the serial choice computes the rest
+          if (n >= room) return;  // full: the serial choice computes the rest
           sse = wiener_unit_sse(l, smem, tt, sh);  // the whole CTA; every thread gets the sum
           if (threadIdx.x == 0) {
             for (int k = 0; k < 6; k++) sh.ctaps[n][k] = tt[k];
@@ -904,8 +906,9 @@ __device__ void spec_path(const FrameParams *fp, int plane, const Layout &l, con
       }
 }
 
+// room: cached candidates a unit keeps (CACHE unless a test lowers it)
 __global__ void __launch_bounds__(THREADS) k_lr_spec(const FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
-                                                    const uint8_t *src, Fit *fits, Dims dims) {
+                                                    const uint8_t *src, Fit *fits, Dims dims, int room) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ Shared sh;
   const Layout l = layout_of(dims);
@@ -923,7 +926,7 @@ __global__ void __launch_bounds__(THREADS) k_lr_spec(const FrameParams *fp, cons
   for (int q = 0; q < 3 && q <= u; q++) {
     for (int pass = 0; pass < 2; pass++)
       for (int j = 0; j < 3; j++) ref[pass][j] = q == 0 ? T(Wiener_Taps_Mid)[j] : fits[gu - q].w[pass][j];
-    spec_path(fp, plane, l, smem, fitted, ref, sh);
+    spec_path(fp, plane, l, smem, fitted, ref, room, sh);
   }
   __syncthreads();
   const int n1 = sh.cn;
@@ -1059,6 +1062,23 @@ __device__ __forceinline__ void load_fit(const Fit *F, Fit &to) {
 }
 __device__ __forceinline__ int default_ref(int k) { return k < 6 ? T(Wiener_Taps_Mid)[k % 3] : T(Sgrproj_Xqd_Mid)[k - 6]; }
 
+// The references that the units before u leave, lane k < 8 the k-th (a warp):
+// the last Wiener unit's taps, the last self-guided unit's weights.
+__device__ int running_ref(const LrUnit *units, int u, int first) {
+  const int lane = threadIdx.x & 31;
+  int wi = -1, si = -1;
+  for (int e = u; e > 0 && (wi < 0 || si < 0); e -= 32) {
+    int k = e - 1 - lane, t = k >= 0 ? __ldcg(&units[k].type) : RESTORE_NONE;
+    unsigned mw = __ballot_sync(0xffffffffu, t == RESTORE_WIENER), ms = __ballot_sync(0xffffffffu, t == RESTORE_SGRPROJ);
+    if (wi < 0 && mw) wi = e - __ffs(mw);
+    if (si < 0 && ms) si = e - __ffs(ms);
+  }
+  int r = lane < 8 ? default_ref(lane) : 0;
+  if (wi >= 0 && lane < 6 && lane % 3 >= first) r = __ldcg(&units[wi].wiener[0][0] + lane);
+  if (si >= 0 && lane >= 6 && lane < 8) r = __ldcg(&units[si].xqd[0] + lane - 6);
+  return r;
+}
+
 // A guess for every unit at once, a warp each. pass 0: the references are the
 // previous unit's fitted filter and the default weights; pass 1: what the
 // units before it chose in pass 0 (or, for one being chosen again meanwhile,
@@ -1076,16 +1096,7 @@ __global__ void __launch_bounds__(THREADS) k_lr_choose(const FrameParams *fp, Fi
   if (pass == 0) {
     if (u > 0 && lane < 6 && lane % 3 >= (plane ? 1 : 0)) r = __ldcg(&fits[gu - 1].w[0][0] + lane);
   } else {
-    // the last Wiener and self-guided units before this one
-    int wi = -1, si = -1;
-    for (int e = u; e > 0 && (wi < 0 || si < 0); e -= 32) {
-      int k = e - 1 - lane, t = k >= 0 ? __ldcg(&units[off + k].type) : RESTORE_NONE;
-      unsigned mw = __ballot_sync(0xffffffffu, t == RESTORE_WIENER), ms = __ballot_sync(0xffffffffu, t == RESTORE_SGRPROJ);
-      if (wi < 0 && mw) wi = e - __ffs(mw);
-      if (si < 0 && ms) si = e - __ffs(ms);
-    }
-    if (wi >= 0 && lane < 6 && lane % 3 >= (plane ? 1 : 0)) r = __ldcg(&units[off + wi].wiener[0][0] + lane);
-    if (si >= 0 && lane >= 6 && lane < 8) r = __ldcg(&units[off + si].xqd[0] + lane - 6);
+    r = running_ref(units + off, u, plane ? 1 : 0);
   }
   if (lane < 8) m.ref[lane] = r;
   __syncwarp();
@@ -1098,20 +1109,34 @@ __global__ void __launch_bounds__(THREADS) k_lr_choose(const FrameParams *fp, Fi
   if (lane < 8) fits[gu].used[lane] = done ? r : UNUSED_REF;
 }
 
+// The units whose references differ from those they were chosen with, until
+// there are none: in rounds, all of them at once, a warp each, while no
+// candidate's SSE is missing. A missing one is filtered by the whole CTA, and
+// only for a unit whose references are settled (everything before it stands):
+// from the first miss on the first unit that differs and those after it are
+// taken in order, a warp alone between two misses, up to a run of units that
+// stand. Filtering misses for every unit of a round as well, under references
+// that the next round changed again, took 164 ms a 3840x2160 frame at
+// quantizer 255, where a scan of all units had left the whole search at 140;
+// now 55 ms (quantizer 150: 34 -> 23; 20, without misses: 5.3 as before).
+// listRoom, room: units a round chooses again, cached candidates a unit keeps
+// (LIST and CACHE unless a test lowers them; at least 1 and MIN_CACHE).
+constexpr int ROUNDS = 4;     // rounds before the units are taken in order in any case
+constexpr int STANDING = 16;  // standing units after which the whole plane is looked at again
 __global__ void __launch_bounds__(THREADS) k_lr_select(FrameParams *fp, const uint8_t *cdef, const uint8_t *dbk,
                                                       const uint8_t *src, Fit *fits, LrUnit *units,
-                                                      int lrTest, int *lrTypes, Dims dims) {
+                                                      int lrTest, int *lrTypes, Dims dims, int listRoom, int room) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ Shared sh;
   __shared__ ChooseMem mem[WARPS];
-  __shared__ int lastW[THREADS], lastS[THREADS], todo, any, lowest, missUnit[WARPS];
-  constexpr int LIST = 256;
+  __shared__ int lastW[THREADS], lastS[THREADS], todo, any, lowest, missed, job;
   __shared__ int list[LIST];
   const Layout l = layout_of(dims);
   const int plane = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, first = plane ? 1 : 0;
   const int nUnits = fp->lr_unit_rows[plane] * fp->lr_unit_cols[plane], off = fp->lr_unit_off[plane];
   const int per = (nUnits + THREADS - 1) / THREADS, u0 = imin(nUnits, tid * per), u1 = imin(nUnits, u0 + per);
-  for (;;) {
+  if (tid == 0) missed = 0;
+  for (int round = 0;; round++) {
     // each thread's run of units: the last Wiener and self-guided unit before
     // it, then every unit's references against those it was chosen with
     if (tid == 0) {
@@ -1149,64 +1174,90 @@ __global__ void __launch_bounds__(THREADS) k_lr_select(FrameParams *fp, const ui
       if (!same) {  // what the list has no room for is found again in the next round
         atomicMin(&lowest, u);
         int slot = atomicAdd(&todo, 1);
-        if (slot < LIST) list[slot] = u;
+        if (slot < listRoom) list[slot] = u;
       }
       int t = __ldcg(&units[off + u].type);
       if (t == RESTORE_WIENER) w = u;
       else if (t == RESTORE_SGRPROJ) g = u;
     }
     __syncthreads();
-    const int n = imin(todo, LIST);
+    const int n = imin(todo, listRoom), low = lowest;
     if (n == 0) break;
-    // the first of them is always among them: it is chosen for good, so the rounds end
-    if (tid == 0 && todo > LIST) list[0] = lowest;
-    __syncthreads();
-    // again, a warp each; a candidate neither pass cached is filtered by the
-    // whole CTA, cached, and its unit chosen in a later round
-    for (int base = 0; base < n; base += WARPS) {
-      if (lane == 0) missUnit[warp] = -1;
-      if (base + warp < n) {
-        const int u = list[base + warp];
-        ChooseMem &m = mem[warp];
-        load_fit(fits + off + u, m.fit);
-        int wi = -1, si = -1;
-        for (int e = u; e > 0 && (wi < 0 || si < 0); e -= 32) {
-          int k = e - 1 - lane, t = k >= 0 ? __ldcg(&units[off + k].type) : RESTORE_NONE;
-          unsigned mw = __ballot_sync(0xffffffffu, t == RESTORE_WIENER), ms = __ballot_sync(0xffffffffu, t == RESTORE_SGRPROJ);
-          if (wi < 0 && mw) wi = e - __ffs(mw);
-          if (si < 0 && ms) si = e - __ffs(ms);
+    if (missed || round >= ROUNDS) {
+      // in order from the first unit that differs
+      int u = low, r = 0, stood = 0, staged = -1;
+      bool again = false;  // unit u, its record loaded, after a miss
+      if (warp == 0) r = running_ref(units + off, u, first);
+      for (;;) {
+        if (warp == 0) {
+          ChooseMem &m = mem[0];
+          int miss = -1;
+          for (; u < nUnits && stood < STANDING; u++, again = false) {
+            if (!again) {
+              bool same = lane >= 8 || __ldcg(&fits[off + u].used[lane & 7]) == r;
+              stood = __all_sync(0xffffffffu, same) ? stood + 1 : 0;
+              if (stood == 0) {
+                load_fit(fits + off + u, m.fit);
+                if (lane < 8) m.ref[lane] = r;
+                __syncwarp();
+              }
+            }
+            if (stood == 0) {
+              if (!choose_unit(fp, plane, u, m.fit, m.ref, lrTest, units + off + u, m.miss)) {
+                miss = u;
+                again = true;
+                break;
+              }
+              if (lane < 8) fits[off + u].used[lane] = r;
+              __syncwarp();
+            }
+            const int t = __ldcg(&units[off + u].type);
+            if (t == RESTORE_WIENER && lane < 6 && lane % 3 >= first) r = __ldcg(&units[off + u].wiener[0][0] + lane);
+            if (t == RESTORE_SGRPROJ && lane >= 6 && lane < 8) r = __ldcg(&units[off + u].xqd[0] + lane - 6);
+          }
+          if (lane == 0) job = miss;
         }
-        int r = lane < 8 ? default_ref(lane) : 0;
-        if (wi >= 0 && lane < 6 && lane % 3 >= first) r = __ldcg(&units[off + wi].wiener[0][0] + lane);
-        if (si >= 0 && lane >= 6 && lane < 8) r = __ldcg(&units[off + si].xqd[0] + lane - 6);
-        if (lane < 8) m.ref[lane] = r;
-        __syncwarp();
-        bool done = choose_unit(fp, plane, u, m.fit, m.ref, lrTest, units + off + u, m.miss);
-        if (lane < 8) fits[off + u].used[lane] = done ? r : UNUSED_REF;
-        if (!done && lane == 0) missUnit[warp] = u;
-      }
-      __syncthreads();
-      for (int k = 0; k < WARPS; k++) {
-        const int u = missUnit[k];
-        if (u < 0) continue;  // the same for every thread
-        load_unit(fp, off + u, cdef, dbk, src, l, smem, sh);
+        __syncthreads();
+        const int ju = job;
+        if (ju < 0) break;
+        if (staged != ju) load_unit(fp, off + ju, cdef, dbk, src, l, smem, sh);
+        staged = ju;
         int tt[6];
-        for (int c = 0; c < 6; c++) tt[c] = mem[k].miss[c];
+        for (int c = 0; c < 6; c++) tt[c] = mem[0].miss[c];
         long long sse = wiener_unit_sse(l, smem, tt, sh);
         if (tid == 0) {
-          Fit &F = fits[off + u];
+          Fit &F = mem[0].fit;
           // a full cache keeps the first pass's candidates: a path under
           // settled references needs at most 12 more
-          int at = F.n < CACHE ? F.n : F.n0;
+          int at = F.n < room ? F.n : F.n0;
           for (int c = 0; c < 6; c++) F.taps[at][c] = tt[c];
           F.sse[at] = sse;
           F.n = at + 1;
-          __threadfence_block();
         }
         __syncthreads();
       }
-      __syncthreads();
+      continue;
     }
+    // the first of them is always among them, once: it is chosen for good, so the rounds end
+    if (tid == 0 && todo > listRoom) {
+      for (int k = 1; k < n; k++)
+        if (list[k] == low) list[k] = list[0];
+      list[0] = low;
+    }
+    __syncthreads();
+    for (int k = warp; k < n; k += WARPS) {
+      const int u = list[k];
+      ChooseMem &m = mem[warp];
+      load_fit(fits + off + u, m.fit);
+      const int r = running_ref(units + off, u, first);
+      if (lane < 8) m.ref[lane] = r;
+      __syncwarp();
+      bool done = choose_unit(fp, plane, u, m.fit, m.ref, lrTest, units + off + u, m.miss);
+      if (lane < 8) fits[off + u].used[lane] = done ? r : UNUSED_REF;
+      if (!done && lane == 0) missed = 1;
+      __syncwarp();
+    }
+    __syncthreads();
   }
   if (tid == 0) fp->lr_type[plane] = lrTypes[plane] = any ? RESTORE_SWITCHABLE : RESTORE_NONE;
 }

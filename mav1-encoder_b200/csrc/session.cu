@@ -104,6 +104,7 @@ struct mav1cu_session {
   int lr_searched;         // the current frame's LR units and types come from mav1cu_lr_search
   int64_t device_bytes;    // device memory this session allocated
   int fault_hold, fault_spins;  // failure-detection test: the next recon's held block and poll limit
+  int lr_list = lrs::LIST, lr_cache = lrs::CACHE;  // room of the LR choice's rounds and candidate caches
   FrameParams fp;          // host copy of the current parameters
   int have_params;
   int64_t launches;
@@ -763,7 +764,7 @@ extern "C" int mav1cu_lr_search(mav1cu_session *s, int lr_test) {
   // the refinement's candidates under guessed references, for all units at
   // once: the serial choice below finds most of its SSEs cached
   lrs::k_lr_spec<<<n, lrs::THREADS, lrs::smem_sse(l), s->stream>>>(DP(s), U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK),
-                                                                  U8(s, MAV1CU_BUF_SRC), s->lrfit, d);
+                                                                  U8(s, MAV1CU_BUF_SRC), s->lrfit, d, s->lr_cache);
   if (after_launch(s, "loop-restoration speculative refinement")) return s->err;
   for (int pass = 0; pass < 2; pass++) {
     lrs::k_lr_choose<<<(n + lrs::WARPS - 1) / lrs::WARPS, lrs::THREADS, 0, s->stream>>>(
@@ -772,8 +773,16 @@ extern "C" int mav1cu_lr_search(mav1cu_session *s, int lr_test) {
   }
   lrs::k_lr_select<<<3, lrs::THREADS, lrs::smem_sse(l), s->stream>>>(
       (FrameParams *)s->buf[MAV1CU_BUF_PARAMS], U8(s, MAV1CU_BUF_REC), U8(s, MAV1CU_BUF_DBK), U8(s, MAV1CU_BUF_SRC),
-      s->lrfit, (LrUnit *)s->buf[MAV1CU_BUF_LRUNITS], lr_test, s->lr_types, d);
+      s->lrfit, (LrUnit *)s->buf[MAV1CU_BUF_LRUNITS], lr_test, s->lr_types, d, s->lr_list, s->lr_cache);
   return after_launch(s, "loop-restoration selection");
+}
+
+extern "C" int mav1cu_debug_lr_room(mav1cu_session *s, int list, int cache) {
+  if (list < 1 || list > lrs::LIST || cache < lrs::MIN_CACHE || cache > lrs::CACHE)
+    return set_error(s, MAV1CU_ERR_ARG, "LR choice: room for %d units, %d candidates", list, cache);
+  s->lr_list = list;
+  s->lr_cache = cache;
+  return MAV1CU_OK;
 }
 
 // ---- compact export of the writer inputs ------------------------------------------

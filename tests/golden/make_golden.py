@@ -121,8 +121,25 @@ def run_batch():
     return out
 
 
+def run_stream():
+    """The export images of parity.stream_clips, and the restoration units of
+    parity.lr_frame, as the device library in the tree makes them on this
+    machine's GPU. The committed files are not this tree's own output: they
+    were written on a B200 by the library of revision 18ba9bf, whose every stage
+    had been compared with the oracle byte for byte, before the kernels were
+    rewritten (its choice of restoration units was the serial scan)."""
+    sys.path.insert(0, os.path.dirname(HERE))
+    import parity
+    return {name: {"clip": synthetic.clip_sha256(spec), "image_sha16": [parity.sha16(i) for i in parity.stream_images(spec, flags)]}
+            for name, (spec, flags) in parity.stream_clips().items()}, parity.lr_hashes()
+
+
 if __name__ == "__main__":
-    if "--batch" in sys.argv:
+    if "--stream" in sys.argv:
+        out = run_stream()
+        for path, v in zip(("stream_hashes.json", "lr_hashes.json"), out):
+            json.dump(v, open(os.path.join(HERE, path), "w"), indent=1, sort_keys=True)
+    elif "--batch" in sys.argv:
         out = run_batch()
         json.dump(out, open(os.path.join(HERE, "batch_hashes.json"), "w"), indent=1, sort_keys=True)
     elif "--large" in sys.argv:

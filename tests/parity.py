@@ -515,3 +515,131 @@ def golden_stream(name):
     if synthetic.clip_sha256(spec) != want["clip"]:
         raise AssertionError(f"{name}: the generated clip differs from the hashed one")
     return stream_recon_sha16(spec, flags), want["recon_sha16"]
+
+
+# Clips whose exported images have committed hashes (golden/stream_hashes.json): pictures of one superblock and of
+# less, of partial superblocks on either side, of several tile columns, a wide one of one superblock row, with three
+# tool sets; restoration units narrower and lower than 64 samples, the largest (95 columns, 103 luma / 99 chroma
+# rows), units cut mid-stripe, several a row with a remainder of one block, every unit forced to a filter (the
+# search keeps RESTORE_NONE in nearly all units of these clips).
+STREAM_SIZES = [(64, 64), (72, 72), (130, 66), (66, 194), (392, 40), (264, 136)]
+STREAM_TOOLS = {
+    "turbo": dict(q=110, turbo=1, keyint=4, tiles=1),
+    "full": dict(q=90, altref=4, golden=1, tiles=1, me_range=64),
+    "lossless": dict(q=0, fast=1),
+}
+LR_SIZES = [(48, 40), (95, 95), (159, 159), (191, 190), (130, 98), (67, 223)]
+
+
+def stream_clips():
+    """Name -> (clip, flags)."""
+    out = {f"{t}_{w}x{h}": (synthetic.ClipSpec(w, h, 4, seed=w + 3 * h, rects=3, rect_size=(8, 32)), STREAM_TOOLS[t])
+           for t in STREAM_TOOLS for w, h in STREAM_SIZES}
+    for w, h in LR_SIZES:
+        out[f"lr_{w}x{h}"] = (synthetic.ClipSpec(w, h, 2, seed=w * 7 + h, rects=2, rect_size=(12, 30)),
+                              dict(q=120, golden=1, tiles=0, lr_test=1))
+    return out
+
+
+def stream_images(spec, flags):
+    """Every frame's export image (writer inputs and reconstruction), in coding
+    order, of a clip coded through a device-resident stream."""
+    import torch
+
+    clip = [torch.from_numpy(np.frombuffer(synthetic.packed(f), np.uint8).copy()).cuda() for f in synthetic.generate(spec)]
+    cfg = mav1cu.cli_config(spec.width, spec.height, **flags)
+    st = mav1cu.Stream(cfg)
+    out = []
+    try:
+        for job in mav1cu.plan(cfg, spec.frames):
+            image = torch.zeros(st.session.export_capacity(), dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            sess = st.encode(job, clip[int(job["disp"])].data_ptr(), True)
+            sess.export(image.data_ptr(), image.numel(), rec=True)
+            st.synchronize()
+            out.append(image.cpu().numpy())
+    finally:
+        st.close()
+    return out
+
+
+def sha16(a):
+    return hashlib.sha256(a.tobytes()).hexdigest()[:16]
+
+
+# ---- restoration units of made-up frames ----------------------------------------------
+# sizes of the frames, all of LR_SIZES and one of 306 luma units: more than the choice has threads or list entries
+LR_FRAMES = LR_SIZES + [(640, 360), (1152, 1088)]
+
+
+def lr_frame(w, h, seed):
+    """(source, CDEF output, deblocked frame) in the session's padded layout:
+    a texture, and in every 80 x 80 tile of the other two the texture itself,
+    a blur, noise or an offset of their own, so that restoration filters pay in
+    some units and not in others, and with other taps."""
+    rng = np.random.default_rng(seed)
+    g = mav1cu.geometry(w, h)
+    out = [[], [], []]
+    for p in range(3):
+        ph, pw, tile = g["plane_h"][p], g["stride"][p], 40 if p else 80
+        x = rng.integers(0, 256, (ph, pw)).astype(np.int64)
+        blur = lambda v: (v + 2 * np.roll(v, 1, 1) + np.roll(v, 2, 1) + 2) >> 2
+        blur2 = lambda v: blur(blur(v).T).T
+        fine, x = np.clip(128 + (blur2(x) - 128) * 2, 0, 255), blur2(blur2(blur2(x)))
+        src = np.clip(128 + (x - 128) * 3, 0, 255)
+        noise = rng.integers(-9, 10, (ph, pw))
+        for ty in range(0, ph, tile):
+            for tx in range(0, pw, tile):
+                if rng.integers(0, 2):
+                    src[ty:ty + tile, tx:tx + tile] = fine[ty:ty + tile, tx:tx + tile]
+        bx = (src + np.roll(src, 1, 1) * 2 + np.roll(src, -1, 1) * 2 + 2) // 5
+        by = (src + np.roll(src, 1, 0) * 2 + np.roll(src, -1, 0) * 2 + 2) // 5
+        rec = src.copy()
+        for ty in range(0, ph, tile):
+            for tx in range(0, pw, tile):
+                t = (slice(ty, ty + tile), slice(tx, tx + tile))
+                kind, a = int(rng.integers(0, 8)), int(rng.integers(2, 9))
+                if kind == 1:
+                    rec[t] = (src[t] * (8 - a) + bx[t] * a) // 8
+                elif kind == 2:
+                    rec[t] = (src[t] * (8 - a) + by[t] * a) // 8
+                elif kind in (3, 4):
+                    rec[t] = src[t] + noise[t] * a // 5
+                elif kind == 5:
+                    rec[t] = src[t] + ((src[t] - bx[t]) * a) // 8
+        dbk = rec + rng.integers(-2, 3, (ph, pw))
+        for o, v in zip(out, (src, rec, dbk)):
+            o.append(np.clip(v, 0, 255).astype(np.uint8).ravel())
+    return [np.concatenate(o) for o in out]
+
+
+def lr_units(w, h, lr_test, room=None, q=150):
+    """(units, lr_type) that the restoration search chooses for lr_frame."""
+    cfg = mav1cu.cli_config(w, h, q=q)
+    fp, _ = mav1cu.frame_params(cfg, mav1cu.plan(cfg, 1)[0])
+    src, rec, dbk = lr_frame(w, h, 3 * w + h)
+    s = mav1cu.Session(w, h)
+    try:
+        if room:
+            assert s.lib.mav1cu_debug_lr_room(s.h, *room) == 0
+        s.set_params(fp)
+        for buf, v in (("SRC", src), ("REC", rec), ("DBK", dbk)):
+            s.upload(buf, v)
+        assert s.lib.mav1cu_lr_search(s.h, lr_test) == 0
+        s.synchronize()
+        p = s.download("PARAMS").view(PARAMS_DTYPE)[0]
+        n = int(p["lr_unit_off"][2]) + int(p["lr_unit_rows"][2]) * int(p["lr_unit_cols"][2])
+        return s.download("LRUNITS").view(LRUNIT_DTYPE)[:n].copy(), p["lr_type"].copy()
+    finally:
+        s.close()
+
+
+def lr_hashes():
+    """Per frame size: the hash of the made-up frame, and of the chosen units without and with lr_test."""
+    out = {}
+    for w, h in LR_FRAMES:
+        got = [lr_units(w, h, t) for t in (0, 1)]
+        out[f"{w}x{h}"] = {"frame": sha16(np.concatenate(lr_frame(w, h, 3 * w + h))),
+                           "units": [sha16(u) + sha16(t) for u, t in got],
+                           "types": [np.bincount(u["type"], minlength=3).tolist() for u, _ in got]}
+    return out

@@ -24,6 +24,7 @@ import synthetic
 pytestmark = pytest.mark.gpu
 
 HERE = os.path.dirname(os.path.abspath(__file__))
+HASHES = json.load(open(os.path.join(HERE, "golden", "stream_hashes.json")))
 LR_HASHES = json.load(open(os.path.join(HERE, "golden", "lr_hashes.json")))
 
 
@@ -31,6 +32,13 @@ LR_HASHES = json.load(open(os.path.join(HERE, "golden", "lr_hashes.json")))
 def test_stream_reconstructions_match_golden(name):
     shown, want = parity.golden_stream(name)
     assert shown == want
+
+
+@pytest.mark.parametrize("name", sorted(parity.stream_clips()))
+def test_stream_images_match_golden(name):
+    spec, flags = parity.stream_clips()[name]
+    assert synthetic.clip_sha256(spec) == HASHES[name]["clip"]
+    assert [parity.sha16(i) for i in parity.stream_images(spec, flags)] == HASHES[name]["image_sha16"]
 
 
 @pytest.mark.parametrize("w,h", parity.LR_FRAMES)

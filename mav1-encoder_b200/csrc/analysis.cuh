@@ -1035,16 +1035,18 @@ __global__ void __launch_bounds__(32 * TABLE_WARPS) k_analyze_table(Ctx c) {
 HD int smooth_mode(int m) { return m == SMOOTH_PRED || m == SMOOTH_V_PRED || m == SMOOTH_H_PRED; }
 
 // Step 1: every mi covered by a block gets its luma / chroma smooth flag.
-// A CTA per superblock, a warp per block, its lanes over the block's units.
-constexpr int MARK_THREADS = 256;
+// A CTA per superblock, 4 to 32 lanes per block over its units (k_filter_info's
+// split).
+constexpr int MARK_THREADS = 4 * MAX_BLOCKS_PER_SB;
 __global__ void __launch_bounds__(MARK_THREADS) k_edge_marks(const FrameParams *fp, const BlockInfo *blocks, const SbInfo *sbs,
                                                              uint8_t *ys, uint8_t *uvs) {
-  const int sb = blockIdx.x, lane = threadIdx.x & 31, n = sbs[sb].num_blocks, cols = fp->mi_cols, rows = fp->mi_rows;
-  for (int k = threadIdx.x >> 5; k < n; k += MARK_THREADS / 32) {
+  const int sb = blockIdx.x, n = sbs[sb].num_blocks, lg = lanes_per_block(n), lane = threadIdx.x & ((1 << lg) - 1);
+  const int cols = fp->mi_cols, rows = fp->mi_rows;
+  for (int k = threadIdx.x >> lg; k < n; k += MARK_THREADS >> lg) {
     const BlockInfo *b = &blocks[sbs[sb].first_block + k];
     int ysm = smooth_mode(b->y_mode) && !b->is_inter, uvsm = !b->is_inter && smooth_mode(b->uv_mode);
     int lw = 31 - __clz(T(Num_4x4_Blocks_Wide)[b->bsize]), bh4 = T(Num_4x4_Blocks_High)[b->bsize];
-    for (int i = lane; i < bh4 << lw; i += 32) {
+    for (int i = lane; i < bh4 << lw; i += 1 << lg) {
       int r = b->mi_row + (i >> lw), cc = b->mi_col + (i & ((1 << lw) - 1));
       if (r >= rows || cc >= cols) continue;
       ys[r * cols + cc] = (uint8_t)ysm;

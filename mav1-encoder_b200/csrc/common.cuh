@@ -223,6 +223,10 @@ WARP_FN unsigned watch_ready(const Warp &warp, int limit, Done done, Ready ready
 HD int block_w(int bs) { return 4 * T(Num_4x4_Blocks_Wide)[bs]; }
 HD int block_h(int bs) { return 4 * T(Num_4x4_Blocks_High)[bs]; }
 
+// log2 of the lanes per block with which a CTA of 4 * MAX_BLOCKS_PER_SB threads
+// takes all blocks of a superblock at once.
+HD int lanes_per_block(int blocks) { return blocks <= 8 ? 5 : blocks <= 16 ? 4 : blocks <= 32 ? 3 : 2; }
+
 // Tile column bounds (uniform spacing, one tile row; k_common.h:89-94).
 HD int tile_col_start(const FrameParams *fp, int miCol) { return ((miCol >> 4) / fp->tile_w_sb) * fp->tile_w_sb * 16; }
 HD int tile_col_end(const FrameParams *fp, int miCol) {

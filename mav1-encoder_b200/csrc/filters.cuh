@@ -19,18 +19,23 @@
 namespace flt {
 
 // ---- loop filter info (encoder.c:513-526) --------------------------------------------
-// A CTA per superblock, a warp per block, its lanes over the block's units (a
-// thread per block wrote a 64x64 block's 256 units one after another).
-constexpr int INFO_THREADS = 256;
+// A CTA per superblock whose blocks go at once, 4 to 32 lanes each over a
+// block's units, the more the fewer blocks there are. (A thread per block wrote
+// a 64x64 block's 256 units one after another, 24 us for any frame that has
+// one; a warp per block took the 64 blocks of a divided superblock in 8 turns,
+// 11.1 us on a 352x288 key frame of small blocks against a thread's 8.8, 14.9
+// on a 3840x2160 one. This takes 7.5 and 9.2, and 7 for large blocks.)
+constexpr int INFO_THREADS = 4 * MAX_BLOCKS_PER_SB;
 __global__ void __launch_bounds__(INFO_THREADS) k_filter_info(const FrameParams *fp, const BlockInfo *blocks, const SbInfo *sbs,
                                                               uint8_t *info) {
-  const int sb = blockIdx.x, lane = threadIdx.x & 31, n = sbs[sb].num_blocks, rows = fp->mi_rows, cols = fp->mi_cols;
-  for (int k = threadIdx.x >> 5; k < n; k += INFO_THREADS / 32) {
+  const int sb = blockIdx.x, n = sbs[sb].num_blocks, lg = lanes_per_block(n), lane = threadIdx.x & ((1 << lg) - 1);
+  const int rows = fp->mi_rows, cols = fp->mi_cols;
+  for (int k = threadIdx.x >> lg; k < n; k += INFO_THREADS >> lg) {
     const BlockInfo *b = &blocks[sbs[sb].first_block + k];
     int skip = b->eob[0] == 0 && b->eob[1] == 0 && b->eob[2] == 0;
     int lw = 31 - __clz(T(Num_4x4_Blocks_Wide)[b->bsize]), bh4 = T(Num_4x4_Blocks_High)[b->bsize];
     uint8_t v = (uint8_t)(b->bsize | (skip << 5) | (b->tx_depth << 6));
-    for (int i = lane; i < bh4 << lw; i += 32) {
+    for (int i = lane; i < bh4 << lw; i += 1 << lg) {
       int y = b->mi_row + (i >> lw), x = b->mi_col + (i & ((1 << lw) - 1));
       if (y < rows && x < cols) info[y * cols + x] = v;
     }

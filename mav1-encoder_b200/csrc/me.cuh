@@ -302,16 +302,20 @@ __device__ __noinline__ int full_cost(const Frame f, const Node m, int dy, int d
 // turn instead of one thread a candidate). Every lane returns the total. The
 // sums are the ones full_sad / dec_sad form, in another order: unsigned
 // integer addition, so the cost is the same.
-// Not inlined, with its arguments by value: the kernel's other levels keep
-// their registers (inlined, the kernel spills at its 96-register bound).
+// Not inlined, with its arguments by value: the kernel's other parts keep
+// their registers. The node width is a constant: as an argument it cost the
+// whole search of a 3840x2160 picture 5,938 us against 4,994, of a 640x360 one
+// 693 against 531 (full sums, +-64 samples).
+template <int w>
 __device__ __noinline__ int warp_full_cost(const FrameParams *fp, const uint8_t *fsrc, const uint8_t *fref,
-                                           const uint8_t *dsrc, const uint8_t *dref, int x, int y, int w, int step,
+                                           const uint8_t *dsrc, const uint8_t *dref, int x, int y, int step,
                                            int dy, int dx, int lane) {
+  constexpr int lg = w == 64 ? 4 : w == 32 ? 3 : 2, n = 1 << lg;  // words of a row, and pairs of a decimated one
   unsigned sad = 0;
   int scale;
   if ((fp->turbo & T_ME_DEC) && step >= ME_COARSE_STEP) {
     // dec_sad: n x n pairs of the decimated planes, lanes along rows
-    int W = dec_w(fp), H = dec_h(fp), lg = floor_log2(w >> 2), n = 1 << lg;
+    int W = dec_w(fp), H = dec_h(fp);
     int x0 = x >> 2, y0 = y >> 2, oy = dy >> 2, ox = dx >> 2;
     if (x0 + n + 4 <= W && y0 + n <= H && x0 + ox >= 0 && x0 + ox + n + 4 <= W && y0 + oy >= 0 && y0 + oy + n <= H) {
       // inside, with the words around a row's ends: four pairs a word
@@ -331,16 +335,16 @@ __device__ __noinline__ int warp_full_cost(const FrameParams *fp, const uint8_t 
     int rs = (fp->turbo & T_ME_RSUB) && step == 1 ? 2 : 1;
     int stride = fp->stride[0], W = fp->frame_w, Hh = fp->frame_h;
     const uint8_t *src = fsrc + fp->offset[0], *ref = fref + fp->offset[0];
-    int lgw = floor_log2(w >> 2), nw = (w / rs) << lgw;
+    const int nw = (w / rs) << lg;
     if (x + dx >= 0 && x + dx + w <= W && y + dy >= 0 && y + dy + w <= Hh) {
       for (int q = lane; q < nw; q += 32) {
-        int i = (q >> lgw) * rs, j = q & ((1 << lgw) - 1);
+        int i = (q >> lg) * rs, j = q & (n - 1);
         uint32_t s = __ldg((const uint32_t *)(src + (y + i) * stride + x) + j);
         sad = __vsadu4(s, load_u32_unaligned(ref + (y + i + dy) * stride + x + dx + 4 * j)) + sad;
       }
     } else {
       for (int q = lane; q < nw; q += 32) {
-        int i = (q >> lgw) * rs, j = q & ((1 << lgw) - 1);
+        int i = (q >> lg) * rs, j = q & (n - 1);
         const uint8_t *s = src + (y + i) * stride + x + 4 * j;
         const uint8_t *r = ref + clip3(0, Hh - 1, y + i + dy) * stride;
         for (int b = 0; b < 4; b++) sad = __sad((int)s[b], (int)r[clip3(0, W - 1, x + 4 * j + b + dx)], sad);
@@ -362,9 +366,11 @@ __device__ __forceinline__ bool grid_inside(const FrameParams *fp, const Node &m
   return m.step == 1 && m.range == 2 && m.x + m.cx >= 2 && m.y + m.cy >= 2 && m.x + m.cx + 2 + m.w <= fp->frame_w &&
          m.y + m.cy + 2 + m.w <= fp->frame_h;
 }
-__device__ __noinline__ unsigned grid_sads(const FrameParams *fp, const uint8_t *fsrc, const uint8_t *fref, int x, int y, int w, int cy,
-                                           int cx, int rs, int lane, int part, int parts) {
-  const int stride = fp->stride[0], lgw = 31 - __clz(w >> 2), n = (w / rs) << lgw;
+template <int w, int parts>
+__device__ __noinline__ unsigned grid_sads(const FrameParams *fp, const uint8_t *fsrc, const uint8_t *fref, int x, int y, int cy,
+                                           int cx, int rs, int lane, int part) {
+  constexpr int lgw = w == 64 ? 4 : w == 32 ? 3 : 2;
+  const int stride = fp->stride[0], n = (w / rs) << lgw;
   const uint8_t *src = fsrc + fp->offset[0] + y * stride + x;
   const uint8_t *ref = fref + fp->offset[0] + (y + cy - 2) * stride + x + cx - 2;
   const int off = (int)((uintptr_t)ref & 3);
@@ -573,13 +579,15 @@ __device__ __forceinline__ void subpel_costs(const Frame &f, const Node &m, cons
 // planes) are compile-time: with one kernel for all of them the 16x16 level
 // executed 3,800 instructions a node, a seventh of them spilled registers.
 // 6 CTAs per SM with planes (80 registers a thread; 1-2% on the 1080p clip over
-// 5), 5 without (the prediction spills below 96).
+// 5), 5 without (96 registers, of which the prediction spills up to 208 bytes a
+// thread at the 8x8 level).
 // Without planes every full-range candidate is a full SAD and every sub-pel
 // unit its own prediction, and a picture has few large nodes (640x360: 60 and
 // 240): 16 warps take a 64x64 node and 4 a 32x32 one.
-// A clip alone, 4 warps and 1 before: 352x288 lossless 2.40 -> 1.95 ms, 363x241
-// low delay 11.5 -> 10.9, 640x360 with every tool 25.5 -> 24.4; 3840x2160, where
-// the nodes fill the chip anyway, 114.3 -> 114.8 (runs differ by 0.3).
+// The whole search of a frame, 4 warps and 1 against this, +-64 samples and +-32:
+// 640x360 920 -> 531 us and 573 -> 338, 1920x1080 1,815 -> 1,543 and 1,125 -> 961,
+// 3840x2160, where the nodes nearly fill the chip anyway, 5,190 -> 4,994 and
+// 3,121 -> 3,078.
 __host__ __device__ constexpr int me_group(int level, bool hp) {
   return level == 0 ? (hp ? 128 : 512) : level == 1 && !hp ? 128 : level == 3 ? 16 : 32;
 }
@@ -629,7 +637,7 @@ __global__ void __launch_bounds__(me_threads(LEVEL, HP), HP ? 6 : LEVEL == 0 ? 1
     unsigned long long best = ~0ull;
     const int grs = (fp->turbo & T_ME_RSUB) ? 2 : 1;
     if (grp.size >= 32 && grid_inside(fp, m)) {
-      unsigned sad = grid_sads(fp, f.src, f.ref, m.x, m.y, m.w, m.cy, m.cx, grs, lane, whole_cta ? warp : 0, whole_cta ? warps : 1);
+      unsigned sad = grid_sads<(64 >> LEVEL), whole_cta ? warps : 1>(fp, f.src, f.ref, m.x, m.y, m.cy, m.cx, grs, lane, whole_cta ? warp : 0);
       if (whole_cta) {
         if (lane < 26) s_sad[warp][lane] = sad;
         __syncthreads();
@@ -647,7 +655,7 @@ __global__ void __launch_bounds__(me_threads(LEVEL, HP), HP ? 6 : LEVEL == 0 ? 1
       for (int k = warp; k < m.count; k += warps) {
         int dy, dx;
         candidate(m, k, &dy, &dx);
-        int cost = warp_full_cost(fp, f.src, f.ref, f.dsrc, f.dref, m.x, m.y, m.w, m.step, dy, dx, lane);
+        int cost = warp_full_cost<(64 >> LEVEL)>(fp, f.src, f.ref, f.dsrc, f.dref, m.x, m.y, m.step, dy, dx, lane);
         unsigned long long key = ((unsigned long long)(unsigned)cost << 32) | (unsigned)k;
         best = key < best ? key : best;
       }

@@ -323,7 +323,8 @@ __device__ __forceinline__ void intra_modes(const FrameParams *fp, const uint8_t
       L[r] = left[uy + r];
     }
     WORK(W_ANA_SATD, __popc(modes) + (dirMode >= 0));
-    WORK(W_ANA_INTRA_PX, 16 * (__popc(modes) + (dirMode >= 0)));
+    // DC, V and H are never predicted sample by sample
+    WORK(W_ANA_INTRA_PX, 16 * (__popc(modes & ~(1u << DC_PRED | 1u << V_PRED | 1u << H_PRED)) + (dirMode >= 0)));
     if (modes & (1u << DC_PRED | 1u << V_PRED | 1u << H_PRED)) {
       // the source's transform, and its absolute sum without the first row / column
       int t[16], f[16];
@@ -817,12 +818,13 @@ __device__ int depth_pruned(const FrameParams *fp, const int64_t *costs, int sbI
 __host__ __device__ constexpr int ana_groups(int group) { return group < 32 ? ANA_THREADS / group : ANA_THREADS / 32; }
 // At least 4 CTAs per SM (at most 128 registers a thread): the level's
 // candidates are latency-bound SATD and filter sums, and the extra resident
-// warps hide more of it (measured on the 1080p clip: key-frame analysis
-// 2.47 -> 1.74 ms at 168 -> 128 registers; 5 CTAs spill and lose again).
-#ifndef MAV1CU_ANA_MIN_CTAS
-#define MAV1CU_ANA_MIN_CTAS 4
-#endif
-__global__ void __launch_bounds__(ANA_THREADS, MAV1CU_ANA_MIN_CTAS) k_analyze_level(Ctx c, int level, int slots, int group) {
+// warps hide more of it, although one kernel for every level and kind of
+// candidate spills 676 bytes a thread at 128. The shared intra pass made an
+// inter frame whose blocks all skip it a little slower (3840x2160, a constant
+// picture: 147 -> 153 us). Sums of the allowed modes alone made a 3840x2160 key
+// frame with every tool 16.4 -> 17.2 ms; CfL and the angles out of line made
+// that inter frame 159 us.
+__global__ void __launch_bounds__(ANA_THREADS, 4) k_analyze_level(Ctx c, int level, int slots, int group) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpMem *wmem = (WarpMem *)smem_raw;
   long long *red = (long long *)(wmem + ana_groups(group));

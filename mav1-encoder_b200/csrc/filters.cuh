@@ -407,30 +407,22 @@ HD int lr_src(const FrameParams *fp, int plane, const LrBlock *lb, const uint8_t
   return cdef[fp->offset[plane] + y * stride + x];
 }
 
-// The samples the loop-restoration filters read: get_source_sample( ) for
-// the filter taps, and the CDEF output at the block's own positions. FrameSrc
-// reads the frame buffers; the parameter search reads shared-memory windows
-// (lrs::WinSrc) through the same filter code.
-struct FrameSrc {
+// The samples the loop-restoration filters read, get_source_sample( ) for the
+// filter taps and the CDEF output at the block's own positions, and the picture
+// they write. (The parameter search has its own filters, over a unit's samples
+// in shared memory.)
+struct LrFrame {
   const FrameParams *fp;
   int plane;
   const uint8_t *cdef, *dbk;
+  uint8_t *out;
   HD int tap(const LrBlock *lb, int x, int y) const { return lr_src(fp, plane, lb, cdef, dbk, x, y); }
   HD int own(int x, int y) const { return cdef[fp->offset[plane] + y * fp->stride[plane] + x]; }
-};
-
-// Output of the filters: sink(x, y, value) for plane sample (x, y). The apply
-// kernel stores it, the parameter search accumulates its squared error.
-struct StoreSink {
-  const FrameParams *fp;
-  int plane;
-  uint8_t *out;
-  HD void operator()(int x, int y, int v) { out[fp->offset[plane] + y * fp->stride[plane] + x] = (uint8_t)v; }
+  HD void store(int x, int y, int v) const { out[fp->offset[plane] + y * fp->stride[plane] + x] = (uint8_t)v; }
 };
 
 // Wiener filter (spec 7.17.4, 8-bit rounding).
-template <class Src, class Sink>
-HD void lr_wiener_to(const LrBlock *lb, const Src &in, const LrUnit *u, Sink &sink) {
+HD void lr_wiener(const LrBlock *lb, const LrFrame &in, const LrUnit *u) {
   int vf[7], hf[7];
   vf[3] = 128;
   hf[3] = 128;
@@ -454,20 +446,12 @@ HD void lr_wiener_to(const LrBlock *lb, const Src &in, const LrUnit *u, Sink &si
     for (int c = 0; c < lb->w; c++) {
       int s = 0;
       for (int t = 0; t < 7; t++) s += vf[t] * inter[r + t][c];
-      sink(lb->x + c, lb->y + r, clip3(0, 255, round2(s, round1)));
+      in.store(lb->x + c, lb->y + r, clip3(0, 255, round2(s, round1)));
     }
 }
 
-HD void lr_wiener(const FrameParams *fp, int plane, const LrBlock *lb, const uint8_t *cdef, const uint8_t *dbk,
-                  uint8_t *out, const LrUnit *u) {
-  FrameSrc in{fp, plane, cdef, dbk};
-  StoreSink sink{fp, plane, out};
-  lr_wiener_to(lb, in, u, sink);
-}
-
 // Box filter (spec 7.17.3); F gets w x h values (row stride 4).
-template <class Src>
-HD void lr_box(const LrBlock *lb, const Src &in, int set, int pass, int *F) {
+HD void lr_box(const LrBlock *lb, const LrFrame &in, int set, int pass, int *F) {
   int r = T(Sgr_Params)[set][pass * 2 + 0];
   if (r == 0) return;
   int eps = T(Sgr_Params)[set][pass * 2 + 1];
@@ -517,10 +501,11 @@ HD void lr_box(const LrBlock *lb, const Src &in, int set, int pass, int *F) {
   }
 }
 
-// Self-guided projection (spec 7.17.2) of a block whose box-filter outputs
-// are flt0 / flt1.
-template <class Src, class Sink>
-HD void lr_sgr_project(const LrBlock *lb, const Src &in, const LrUnit *u, const int *flt0, const int *flt1, Sink &sink) {
+// Self-guided filter (spec 7.17.2): the box filters' outputs projected.
+HD void lr_sgr(const LrBlock *lb, const LrFrame &in, const LrUnit *u) {
+  int flt0[16], flt1[16];
+  lr_box(lb, in, u->set, 0, flt0);
+  lr_box(lb, in, u->set, 1, flt1);
   int w0 = u->xqd[0], w1 = u->xqd[1];
   int w2 = (1 << SGRPROJ_PRJ_BITS) - w0 - w1;
   int r0 = T(Sgr_Params)[u->set][0], r1 = T(Sgr_Params)[u->set][2];
@@ -530,19 +515,8 @@ HD void lr_sgr_project(const LrBlock *lb, const Src &in, const LrUnit *u, const 
       int v = w1 * uu;
       v += r0 ? w0 * flt0[i * 4 + j] : w0 * uu;
       v += r1 ? w2 * flt1[i * 4 + j] : w2 * uu;
-      sink(lb->x + j, lb->y + i, clip3(0, 255, round2(v, SGRPROJ_RST_BITS + SGRPROJ_PRJ_BITS)));
+      in.store(lb->x + j, lb->y + i, clip3(0, 255, round2(v, SGRPROJ_RST_BITS + SGRPROJ_PRJ_BITS)));
     }
-}
-
-// Self-guided filter (spec 7.17.2).
-HD void lr_sgr(const FrameParams *fp, int plane, const LrBlock *lb, const uint8_t *cdef, const uint8_t *dbk, uint8_t *out,
-               const LrUnit *u) {
-  FrameSrc in{fp, plane, cdef, dbk};
-  int flt0[16], flt1[16];
-  lr_box(lb, in, u->set, 0, flt0);
-  lr_box(lb, in, u->set, 1, flt1);
-  StoreSink sink{fp, plane, out};
-  lr_sgr_project(lb, in, u, flt0, flt1, sink);
 }
 
 // Thread per (plane, 4x4 luma block): loop_restore_block( ) with the unit's
@@ -559,10 +533,11 @@ __global__ void k_lr_apply(const FrameParams *fp, const uint8_t *cdef, const uin
   if (fp->lr_type[plane] == RESTORE_NONE) u.type = RESTORE_NONE;
   else u = units[fp->lr_unit_off[plane] + lb.unitRow * fp->lr_unit_cols[plane] + lb.unitCol];
   WORK(W_LR_TAPS, lb.w * lb.h * (u.type == RESTORE_WIENER ? 14 : u.type == RESTORE_SGRPROJ ? 34 : 0));
+  const LrFrame in{fp, plane, cdef, dbk, out};
   if (u.type == RESTORE_WIENER) {
-    lr_wiener(fp, plane, &lb, cdef, dbk, out, &u);
+    lr_wiener(&lb, in, &u);
   } else if (u.type == RESTORE_SGRPROJ) {
-    lr_sgr(fp, plane, &lb, cdef, dbk, out, &u);
+    lr_sgr(&lb, in, &u);
   } else {
     int stride = fp->stride[plane];
     for (int y = 0; y < lb.h; y++)

@@ -12,10 +12,10 @@
 // serial scan over the units. Everything that does not depend on those
 // references is computed first, for all units at once:
 //
-//   k_lr_fit     one CTA per unit: the SSE of RESTORE_NONE, the Wiener fit,
+//   k_lr_fit     three CTAs per unit: the SSE of RESTORE_NONE, the Wiener fit,
 //                the SSE of the fitted filter and of its single-tap
-//                neighbours (the candidates the refinement tries first), and
-//                per self-guided set the fit and its SSE;
+//                neighbours (the candidates the refinement tries first); and
+//                for half of the self-guided sets each the fit and its SSE;
 //   k_lr_spec    one CTA per unit: the Wiener refinement replayed under
 //                guessed running references, caching the SSE of every
 //                candidate it visits (SSEs do not depend on the references);
@@ -389,7 +389,7 @@ __device__ long long none_sse(const Layout &l, const uint8_t *smem, Shared &sh) 
 }
 
 // SSE of the unit filtered with Wiener taps tt (pass 0 vertical j 0..2, pass 1
-// horizontal) against the source: flt::lr_wiener_to's sums and clips. A warp
+// horizontal) against the source: flt::lr_wiener's sums and clips. A warp
 // takes 16 rows of 32 columns, a lane a column: it keeps the last 7 rows'
 // horizontal sums in registers, so a row costs 7 samples read and 8 multiplies
 // instead of every 4x4 block filtering 10 rows for 4 (a 64 x 64 unit: 8 tasks,

@@ -8,16 +8,17 @@
 // minimum of the 4x4-SATD over the node. The levels depend on each other
 // (children search around the parent's vector) and run as separate launches.
 //
-// B200 mapping: one warp per (node, reference). Lanes take candidates (SAD
-// rows on packed bytes with __vsadu4; interior candidates read unaligned
-// words through funnel shifts), and the warp reduces the 64-bit key
-// (cost << 32 | index) with shuffles, which yields exactly the serial first
-// minimum. The 64x64 level has few nodes: a CTA per node, its warps
-// taking candidates in turn and each warp's lanes splitting a candidate's
-// byte pairs. Sub-pel candidates x 4x4 units are spread over the lanes and
-// summed in shared memory. Quarter-pel planes (16 per reference, EIGHTTAP,
-// the T_ME_HPEL mode) are built once per reference picture by their own
-// kernel.
+// B200 mapping: a kernel per level and sub-pel mode (k_me_level). A node and
+// reference is searched by half a warp (8x8), a warp, or a CTA (64x64, and 32x32
+// without quarter-pel planes). Half a warp's and a warp's lanes take
+// candidates (SAD rows on packed bytes with __vsadu4; interior candidates read
+// unaligned words through funnel shifts); a CTA's warps take candidates in
+// turn, a warp's lanes splitting one's byte pairs; the refinement of +-2
+// samples reads a window of 5 rows of 3 words for all its 25 candidates. The
+// 64-bit key (cost << 32 | index) is reduced to its minimum, which is exactly
+// the serial first minimum. Sub-pel candidates x 4x4 units are spread over the
+// group. Quarter-pel planes (16 per reference, EIGHTTAP, the T_ME_HPEL mode)
+// are built once per reference picture by their own kernel.
 #pragma once
 
 #include "common.cuh"
@@ -476,9 +477,9 @@ __device__ __forceinline__ void sub_neighbour(const FrameParams *fp, int j, int 
   *dc = (k == 0 || k == 3 || k == 5) ? -step : ((k == 1 || k == 6) ? 0 : step);
 }
 
-// The threads searching one node: the CTA (the 64x64 level), a warp, or
-// half a warp (the 8x8 level, whose nodes have at most 16 sub-pel pairs at
-// a time); mask holds the group's lanes of its warp.
+// The threads searching one node (me_group): a CTA, a warp, or half a warp (the
+// 8x8 level, whose nodes have at most 16 sub-pel pairs at a time); mask holds
+// the group's lanes of its warp.
 template <int SIZE>
 struct MeGrp {
   static constexpr int size = SIZE;
@@ -573,8 +574,8 @@ __device__ __forceinline__ void subpel_costs(const Frame &f, const Node &m, cons
   g.sync();
 }
 
-// One search level: a whole CTA per node (the 64x64 level: few, large nodes),
-// a warp per (node, reference), or half a warp (the 8x8 level);
+// One search level: a whole CTA per node (few, large nodes), a warp per (node,
+// reference), or half a warp (the 8x8 level);
 // blockIdx.y selects the reference. Level and sub-pel path (HP: quarter-pel
 // planes) are compile-time: with one kernel for all of them the 16x16 level
 // executed 3,800 instructions a node, a seventh of them spilled registers.

@@ -36,13 +36,7 @@ namespace rec {
 // Threads of the CTA coding a block: INTER_THREADS for an inter block,
 // INTRA_THREADS for a lossless intra block.
 #define RT ((int)blockDim.x)
-#ifndef MAV1CU_INTER_THREADS
-#define MAV1CU_INTER_THREADS 128
-#endif
-#ifndef MAV1CU_INTRA_THREADS
-#define MAV1CU_INTRA_THREADS 128
-#endif
-constexpr int INTER_THREADS = MAV1CU_INTER_THREADS, INTRA_THREADS = MAV1CU_INTRA_THREADS;
+constexpr int INTER_THREADS = 128, INTRA_THREADS = 128;
 #define FWD_SLOT_SIZE 4096
 HD int fwd_slot(int kind, int log2n) { return (kind * 5 + log2n - 2) * FWD_SLOT_SIZE; }
 
@@ -106,7 +100,6 @@ struct Smem {
   BlockInfo blk;
   int maxLumaW, maxLumaH;
   int flag;
-  int me;      // index of the block being coded
   int r0, c0;  // its superblock's first 4x4 row / column
   // views of the reconstruction and the source: plane origins (absolute
   // plane coordinates) and strides; the frames for an inter block, the
@@ -147,16 +140,9 @@ struct Smem {
 constexpr size_t SMEM_INTER = offsetof(Smem, bar) + sizeof(unsigned long long);
 constexpr size_t SMEM_INTRA = sizeof(Smem);
 
-// Sums / maxima over the CTA. A one-warp CTA reduces by shuffles alone; the
-// __syncwarp()s order the shared-memory writes before and after like the
-// block barriers of the general path.
+// Sums / maxima over the CTA.
 __device__ __forceinline__ long long cta_sum64(long long v, Smem &sm) {
-  if (blockDim.x == 32) __syncwarp();
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  if (blockDim.x == 32) {
-    __syncwarp();
-    return v;
-  }
   if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = v;
   __syncthreads();
   long long s = 0;
@@ -165,12 +151,7 @@ __device__ __forceinline__ long long cta_sum64(long long v, Smem &sm) {
   return s;
 }
 __device__ __forceinline__ int cta_max(int v, Smem &sm) {
-  if (blockDim.x == 32) __syncwarp();
   for (int off = 16; off > 0; off >>= 1) v = imax(v, __shfl_xor_sync(0xffffffffu, v, off));
-  if (blockDim.x == 32) {
-    __syncwarp();
-    return v;
-  }
   if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = v;
   __syncthreads();
   int m = 0;
@@ -312,19 +293,17 @@ __device__ __forceinline__ void inv_col_split(int32_t *resid, int j, int half, i
 // Levels of a candidate -> reconstruction residual (spec 7.13.3 with the
 // dequantisation of 7.12.3), into sm.resid (stride 64).
 // With rec set, the column pass adds its output straight into the
-// reconstruction (flipped for FLIPADST types) instead of storing it.
-// MAXL: the largest log2 length the instantiation handles; the sizes up to
-// 16 get their own inlined copy, so their register allocation does not
-// carry the 32- and 64-point kernels.
-template <int MAXL>
-__device__ __forceinline__ void inverse_2d_upto(Smem &sm, const int32_t *q, int txSz, int txType, int dcQ, int acQ,
-                                                uint8_t *rec, int rs, int x, int y) {
+// reconstruction (flipped for FLIPADST types) instead of storing it. Every
+// length is in it, so it is out of line: the kernel keeps its register budget,
+// and the 32- and 64-point passes spill here (1,072 bytes a thread).
+__device__ __noinline__ void inverse_2d_any(Smem &sm, const int32_t *q, int txSz, int txType, int dcQ, int acQ,
+                                            uint8_t *rec, int rs, int x, int y) {
   int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz];
   int w = 1 << lw, h = 1 << lh, th = imin(32, h);
   int rowShift = T(Transform_Row_Shift)[txSz], denom = tx::dq_denom(txSz);
   int rect = iabs(lw - lh) == 1;
   int rk = tx::row_kind(txType), ck = tx::col_kind(txType);
-  if (MAXL >= 5 && lw >= 5 && rk == tx::KIND_DCT) {
+  if (lw >= 5 && rk == tx::KIND_DCT) {
     for (int p = threadIdx.x; p < 2 * h; p += RT) {
       if (lw == 5) inv_row_split<5, 64, true>(sm.resid, q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
       else inv_row_split<6, 64, true>(sm.resid, q, p >> 1, p & 1, th, dcQ, acQ, denom, rect, rowShift);
@@ -334,13 +313,13 @@ __device__ __forceinline__ void inverse_2d_upto(Smem &sm, const int32_t *q, int 
       case 2: inv_row<2, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
       case 3: inv_row<3, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
       case 4: inv_row<4, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
-      case 5: if (MAXL >= 5) inv_row<5, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
-      default: if (MAXL >= 6) inv_row<6, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      case 5: inv_row<5, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
+      default: inv_row<6, 64, true>(sm.resid, q, i, th, dcQ, acQ, denom, rect, rk, rowShift); break;
     }
   }
   __syncthreads();
   int fud = tx::flip_ud(txType), flr = tx::flip_lr(txType);
-  if (MAXL >= 5 && lh >= 5 && ck == tx::KIND_DCT) {
+  if (lh >= 5 && ck == tx::KIND_DCT) {
     for (int p = threadIdx.x; p < 2 * w; p += RT) {
       if (lh == 5) inv_col_split<5, 64>(sm.resid, p >> 1, p & 1, w, fud, flr, rec, rs, x, y);
       else inv_col_split<6, 64>(sm.resid, p >> 1, p & 1, w, fud, flr, rec, rs, x, y);
@@ -350,26 +329,20 @@ __device__ __forceinline__ void inverse_2d_upto(Smem &sm, const int32_t *q, int 
       case 2: inv_col<2, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
       case 3: inv_col<3, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
       case 4: inv_col<4, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
-      case 5: if (MAXL >= 5) inv_col<5, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
-      default: if (MAXL >= 6) inv_col<6, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
+      case 5: inv_col<5, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
+      default: inv_col<6, 64>(sm.resid, j, w, ck, fud, flr, rec, rs, x, y); break;
     }
   }
   __syncthreads();
 }
 
-__device__ __noinline__ void inverse_2d_large(Smem &sm, const int32_t *q, int txSz, int txType, int dcQ, int acQ,
-                                              uint8_t *rec, int rs, int x, int y) {
-  inverse_2d_upto<6>(sm, q, txSz, txType, dcQ, acQ, rec, rs, x, y);
-}
-
-// Out of line: the kernel keeps its register budget.
 __device__ __forceinline__ void inverse_2d(Smem &sm, const int32_t *q, int txSz, int txType, int dcQ, int acQ,
                                            uint8_t *rec = nullptr, int rs = 0, int x = 0, int y = 0) {
   if (threadIdx.x == 0) {  // h rows of w points, then w columns of h points: 3 log2 N operations per point
     int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz];
     WORK(W_REC_INV_OPS, 3 * (1 << (lw + lh)) * (lw + lh));
   }
-  inverse_2d_large(sm, q, txSz, txType, dcQ, acQ, rec, rs, x, y);
+  inverse_2d_any(sm, q, txSz, txType, dcQ, acQ, rec, rs, x, y);
 }
 
 // The transpose of every forward matrix (slot k: kind k / 5, length 4 << k % 5).
@@ -602,7 +575,7 @@ __device__ __noinline__ long long cand_cost(const CandIn &in, Cand &cd, int type
 // candidates): the CTA's warps take them in turn, each keeping its best one's
 // scratch, and the first least cost is written out. Returns the eob.
 __device__ __noinline__ int search_types(const Ctx &c, Smem &sm, const uint8_t *sp, int ss, uint8_t *pp, int ps, int txSz, int plane,
-                                         const int *cands, int numCands, int32_t *coefOut, int *outType, long long *outCost) {
+                                         const int *cands, int numCands, int32_t *coefOut, int *outType) {
   const FrameParams *fp = c.fp;
   constexpr int WARPS = INTER_THREADS / 32;
   static_assert(2 * WARPS * sizeof(Cand) <= offsetof(Smem, sse33), "two candidates a warp in the transform scratch");
@@ -653,7 +626,6 @@ __device__ __noinline__ int search_types(const Ctx &c, Smem &sm, const uint8_t *
   }
   __syncthreads();
   *outType = eob ? type : DCT_DCT;
-  *outCost = best;
   return eob;
 }
 
@@ -726,16 +698,15 @@ __device__ int code_wht(const Ctx &c, Smem &sm, const uint8_t *src, int stride, 
 // Transform, quantise and reconstruct one inter transform block whose prediction
 // is in `rec` (code_tx_block, k_recon.h:60-173). Returns the eob.
 __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *src, int stride, uint8_t *rec, int rs, int x, int y, int txSz,
-                       int plane, const int *cands, int numCands, int32_t *coefOut, int *outType, long long *outCost) {
+                       int plane, const int *cands, int numCands, int32_t *coefOut, int *outType) {
   const FrameParams *fp = c.fp;
   int lw = T(Tx_Width_Log2)[txSz], lh = T(Tx_Height_Log2)[txSz];
   int w = 1 << lw, h = 1 << lh, tw = imin(32, w), th = imin(32, h);
   int dcQ = fp->dc_q[plane], acQ = fp->ac_q[plane];
   int tid = threadIdx.x;
   if (numCands > 1 && lw <= 4 && lh <= 4)
-    return search_types(c, sm, src + y * stride + x, stride, rec + y * rs + x, rs, txSz, plane, cands, numCands, coefOut, outType,
-                        outCost);
-  // an inter block has no depth search: a single candidate's cost is not used
+    return search_types(c, sm, src + y * stride + x, stride, rec + y * rs + x, rs, txSz, plane, cands, numCands, coefOut, outType);
+  // an inter block has no depth search: a single candidate needs no cost
   int single = numCands == 1;
   int shifts = T(Transform_Row_Shift)[txSz] + 4, rect = iabs(lw - lh) == 1;
   int denom = tx::dq_denom(txSz);
@@ -775,7 +746,6 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
       for (int k = tid; k < tw * th; k += RT) coefOut[k] = sm.q[k];
       if (nz) inverse_2d(sm, sm.q, txSz, t, dcQ, acQ, rec, rs, x, y);
       *outType = nz ? t : DCT_DCT;
-      *outCost = 0;
       return nz;
     }
     int eob = cta_max(myEob, sm);  // includes the barrier after the quantiser
@@ -832,7 +802,6 @@ __device__ __forceinline__ int code_tx(const Ctx &c, Smem &sm, const uint8_t *sr
   }
   __syncthreads();
   *outType = bestType;
-  *outCost = bestCost;
   return bestEob;
 }
 
@@ -1033,18 +1002,17 @@ __device__ __forceinline__ void edge_segs(const Ctx &c, Smem &sm, const uint8_t 
                   e.ly1 >= e.ly0 ? e.ly1 - e.ly0 + 1 : 0, 0};
 }
 
-// Stages the first NP planes of intra block sm.blk in shared memory, in one
+// Stages the planes of intra block sm.blk in shared memory, in one
 // batch of copies: the block's own samples (the reconstruction so far,
 // overwritten as it is coded), its source and its edge samples from frame
 // `edges`, complete there. cb: BlockDecoded of its corner units. The views
 // then point at the tiles.
-template <int NP>
 __device__ void stage_block(const Ctx &c, Smem &sm, const uint8_t *edges, int cb) {
   const FrameParams *fp = c.fp;
   const BlockInfo &b = sm.blk;
   int bs = b.bsize, tid = threadIdx.x;
-  CopySeg sg[4 * NP];
-  for (int p = 0; p < NP; p++) {
+  CopySeg sg[4 * 3];
+  for (int p = 0; p < 3; p++) {
     int sub = p > 0, S = sub ? TILE_C : TILE_Y, sh = sub ? 2 : 0;
     uint8_t *t = sub ? sm.tileC[p - 1] : sm.tileY, *sb = sub ? sm.srcC[p - 1] : sm.srcY;
     int lw = floor_log2(block_w(bs) >> sub), w = 1 << lw, h = block_h(bs) >> sub;
@@ -1061,17 +1029,17 @@ __device__ void stage_block(const Ctx &c, Smem &sm, const uint8_t *edges, int cb
       sm.cornerBL[p] = (cb >> (sh + 1)) & 1;
     }
   }
-  copy_segs<4 * NP>(sg);
+  copy_segs<4 * 3>(sg);
   __syncthreads();
 }
 
-// Writes planes 0 .. np - 1 of an intra block's own samples from its tiles
+// Writes an intra block's own samples from its tiles
 // to the frame (whole words: block positions and widths are multiples of 4
 // samples).
-__device__ void unstage_intra(const Ctx &c, Smem &sm, int np) {
+__device__ void unstage_intra(const Ctx &c, Smem &sm) {
   const FrameParams *fp = c.fp;
   const BlockInfo &b = sm.blk;
-  for (int p = 0; p < np; p++) {
+  for (int p = 0; p < 3; p++) {
     int sub = p > 0, S = sub ? TILE_C : TILE_Y;
     const uint8_t *t = sub ? sm.tileC[p - 1] : sm.tileY;
     int lw = floor_log2(block_w(b.bsize) >> sub) - 2, h = block_h(b.bsize) >> sub;
@@ -1084,9 +1052,10 @@ __device__ void unstage_intra(const Ctx &c, Smem &sm, int np) {
   }
 }
 
-// Every transform block of one plane of block b (code_plane, k_recon.h:190-291).
+// Every transform block of one plane of block b (code_plane, k_recon.h:190-291;
+// its cost, which no caller here uses, is not summed).
 template <bool INTER>
-__device__ long long code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
+__device__ void code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
   const FrameParams *fp = c.fp;
   BlockInfo &b = sm.blk;
   int bs = b.bsize, MiRow = b.mi_row, MiCol = b.mi_col;
@@ -1113,7 +1082,6 @@ __device__ long long code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
   } else {
     cands[numCands++] = chroma_tx_type(txSz, isInter, b.uv_mode, b.tx_type, fp->reduced_tx_set);
   }
-  long long total = 0;
   int txIdx = 0, anyNz = 0;
   int *above = sm.edge[0] + EDGE_OFF, *left = sm.edge[1] + EDGE_OFF, *etmp = sm.edge[2];
   for (int y = 0; y < num4x4H; y += stepY) {
@@ -1181,12 +1149,10 @@ __device__ long long code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
         sm.maxLumaH = startY + stepY * 4;
       }
       int t = DCT_DCT, eob = 0;
-      long long cst = 0;
       int32_t *coefOut = c.coefs + b.coef_off[plane] + txIdx * T(Tx_Width)[txSz] * T(Tx_Height)[txSz];
       if (fp->lossless) eob = code_wht(c, sm, spx, stride, px, rs, startX, startY, plane, coefOut);
       else if constexpr (INTER)
-        eob = code_tx(c, sm, spx, stride, px, rs, startX, startY, txSz, plane, cands, numCands, coefOut, &t, &cst);
-      total += cst;
+        eob = code_tx(c, sm, spx, stride, px, rs, startX, startY, txSz, plane, cands, numCands, coefOut, &t);
       if (threadIdx.x == 0 && plane == 0) {
         tx_type_set(b, txIdx, t);
         if (txIdx == 0) b.tx_type = t;
@@ -1198,7 +1164,6 @@ __device__ long long code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
   }
   if (threadIdx.x == 0) b.eob[plane] = anyNz;
   __syncthreads();
-  return total;
 }
 
 // Inter prediction of a w x h block (spec 7.11.3.4) in three steps, staged in
@@ -1887,7 +1852,7 @@ __device__ __forceinline__ void predict4(int mode, const EdgePrep &e, const int 
 }
 
 // Inverse transform of the dequantised levels in m.q, added into m.px.
-template <int MAXD, int NT, int LOW, int HIGH>
+template <int MAXD, int NT, int HIGH>
 __device__ __forceinline__ void inverse_g(PlaneMem<MAXD> &m, const Group<NT> &g, int lw, int lh, int type, int txSz, int dcQ, int acQ) {
   constexpr int RS = MAXD + 4;
   const int w = 1 << lw, h = 1 << lh, th = imin(32, h), rowShift = T(Transform_Row_Shift)[txSz], denom = tx::dq_denom(txSz);
@@ -1923,7 +1888,7 @@ __device__ __forceinline__ void inverse_g(PlaneMem<MAXD> &m, const Group<NT> &g,
 // the common sizes' registers do not carry the 32- and 64-point kernels.
 template <int MAXD, int NT>
 __device__ __noinline__ void inverse_large(PlaneMem<MAXD> &m, const Group<NT> g, int lw, int lh, int type, int txSz, int dcQ, int acQ) {
-  inverse_g<MAXD, NT, 2, MAXD == 64 ? 6 : 5>(m, g, lw, lh, type, txSz, dcQ, acQ);
+  inverse_g<MAXD, NT, MAXD == 64 ? 6 : 5>(m, g, lw, lh, type, txSz, dcQ, acQ);
 }
 
 // CfL prediction of a chroma plane (spec 7.11.5; cfl_best_alpha,
@@ -2134,7 +2099,7 @@ __device__ __forceinline__ int code_single(const Ctx &c, IntraShared &sh, PlaneM
   nz = g.any(nz);
   if (nz) {
     if (tid == 0) WORK(W_REC_INV_OPS, 3 * (1 << (lw + lh)) * (lw + lh));
-    if (lw <= 4 && lh <= 4) inverse_g<MAXD, NT, 2, 4>(m, g, lw, lh, type, txSz, dcQ, acQ);
+    if (lw <= 4 && lh <= 4) inverse_g<MAXD, NT, 4>(m, g, lw, lh, type, txSz, dcQ, acQ);
     else inverse_large<MAXD, NT>(m, g, lw, lh, type, txSz, dcQ, acQ);
   }
 #pragma unroll
@@ -2763,7 +2728,6 @@ __global__ void __launch_bounds__(INTRA_THREADS) k_recon_lossless(Ctx cg) {
   const int r0 = (sb / fp->sb_cols) * 16, c0 = (sb % fp->sb_cols) * 16;
   if (tid < (int)(sizeof(BlockInfo) / 4)) ((int *)&sm.blk)[tid] = ((const int *)(c.blocks + me))[tid];
   if (tid == 32) {
-    sm.me = me;
     sm.r0 = r0;
     sm.c0 = c0;
     sm.maxLumaW = sm.maxLumaH = 0;
@@ -2772,9 +2736,9 @@ __global__ void __launch_bounds__(INTRA_THREADS) k_recon_lossless(Ctx cg) {
   int cb = 0;
   for (int p = 0; p < 2; p++)
     for (int k = 0; k < 2; k++) cb |= corner_decoded(fp, c.blk_at, sm.blk, me, r0, c0, p, k) << (2 * p + k);
-  stage_block<3>(c, sm, c.src, cb);
+  stage_block(c, sm, c.src, cb);
   for (int p = 0; p < 3; p++) code_plane<false>(c, sm, p, TX_4X4);
-  unstage_intra(c, sm, 3);
+  unstage_intra(c, sm);
   if (tid == 0) {
     sm.blk.tx_depth = 0;
     sm.blk.interp_filter &= 0x30;

@@ -198,7 +198,9 @@ HD int ldpx(const uint8_t *p) {
 // holds for a lane, or after `limit` polls. done() reads a word that other
 // warps set, so the lanes of one poll may read different values: the warp goes
 // by the vote, never by a lane's own value, so that every lane takes part in
-// the same full-mask operations. Warp: any, ballot, pause.
+// the same full-mask operations. (In the intra feeder, voting on done() before
+// ready(), and a plain loop on the word, which is not safe: a 2560x1440 key
+// frame 4,474 and 4,440 us; this order 4,444-4,458.) Warp: any, ballot, pause.
 #if defined(__CUDACC__)
 #define WARP_FN __device__ __forceinline__
 struct FullWarp {
@@ -212,9 +214,10 @@ struct FullWarp {
 template <class Warp, class Done, class Ready>
 WARP_FN unsigned watch_ready(const Warp &warp, int limit, Done done, Ready ready) {
   for (int polls = 0; polls < limit; polls++) {
-    if (warp.any(done())) return 0;
-    unsigned r = warp.ballot(ready());
+    const unsigned r = warp.ballot(ready());
+    const bool d = warp.any(done());  // read after ready()'s loads have come: the newest value
     if (r) return r;
+    if (d) return 0;
     warp.pause();
   }
   return 0;

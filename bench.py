@@ -570,9 +570,9 @@ def int_roofline(times, counts):
 KEY_RECON_BYTES = 2 * 3133440 + 2 * 510 * 64 * 108 + 510 * 6144 * 4 + 61440 * 4
 # dram__bytes_read.sum + dram__bytes_write.sum of that launch of k_recon_blocks
 # in one ncu capture (the key frame of `bench.py --profile-frames 3
-# --profile-export`: 18.467 MB read + 1.447 MB written,
+# --profile-export`: 13.942 MB read + 0.355 MB written,
 # profiles/k_recon_blocks_1080p_turbo_3frames.md).
-KEY_RECON_DRAM_BYTES = 19914752
+KEY_RECON_DRAM_BYTES = 14297600
 
 
 # Integer-pipe figures of each stage's main kernel from the committed ncu
@@ -580,10 +580,10 @@ KEY_RECON_DRAM_BYTES = 19914752
 # and leaf frames): the ALU pipe's share of its peak and the issue slots
 # active, ranges over the captured launches.
 STAGE_NCU = {
-    "motion_search": ("k_me_level", "31-48", "27-55", "profiles/k_me_level_1080p_turbo_3frames.md"),
-    "analyze": ("k_analyze_level", "23-31", "33-42", "profiles/k_analyze_level_1080p_turbo_3frames.md"),
-    "recon": ("k_recon_inter", "22", "31-33", "profiles/k_recon_inter_1080p_turbo_3frames.md"),
-    "filter": ("k_deblock, k_cdef", "49-59", "63-67", "profiles/k_deblock_1080p_turbo_3frames.md"),
+    "motion_search": ("k_me_level", "26-40", "33-45", "profiles/k_me_level_1080p_turbo_3frames.md"),
+    "analyze": ("k_analyze_level", "20-27", "27-34", "profiles/k_analyze_level_1080p_turbo_3frames.md"),
+    "recon": ("k_recon_inter", "21-22", "29-30", "profiles/k_recon_inter_1080p_turbo_3frames.md"),
+    "filter": ("k_deblock, k_cdef", "51-63", "53-62", "profiles/k_deblock_1080p_turbo_3frames.md"),
 }
 
 

@@ -81,7 +81,6 @@ enum { RESTORE_NONE = 0, RESTORE_WIENER = 1, RESTORE_SGRPROJ = 2, RESTORE_SWITCH
 
 #define MAX_LOOP_FILTER 63
 #define MAX_TX_DEPTH 2
-#define MAX_ANGLE_DELTA 3
 #define ANGLE_STEP 3
 #define MI_SIZE 4
 #define SUBPEL_MASK 15

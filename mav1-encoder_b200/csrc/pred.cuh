@@ -52,27 +52,21 @@ HD void inter_setup(Inter *p, const uint8_t *ref, int stride, int refW, int refH
   }
 }
 
-// Vertical filter sum of output sample (r, c) before its final rounding.
-HD int inter_sum(const Inter *p, int r, int c) {
-  int xs[8];
-  for (int t = 0; t < 8; t++) xs[t] = clip3(0, p->lastX, p->ix0 + c + t);
-  int acc = 0;
-  for (int tv = 0; tv < 8; tv++) {
-    const uint8_t *row = p->ref + (size_t)clip3(0, p->lastY, p->iy0 + r + tv) * p->stride;
-    int s = 0;
-    for (int t = 0; t < 8; t++) s += p->fh[t] * (int)row[xs[t]];
-    acc += p->fv[tv] * round2(s, 3);
-  }
-  return acc;
+// The predictions take half taps (in 8 bits) for whole ones in the horizontal
+// sum: with every tap even, (2 S + 4) >> 3 = (S + 2) >> 2.
+constexpr int SUBPEL_TAPS MAV1T_Subpel_Filters_DIMS = MAV1T_Subpel_Filters;
+constexpr bool subpel_taps_halve() {
+  for (const auto &filter : SUBPEL_TAPS)
+    for (const auto &phase : filter)
+      for (int t : phase)
+        if (t % 2 || t / 2 < -128 || t / 2 > 127) return false;
+  return true;
 }
-
-// Single-reference sample: Clip1( Round2( sum, 11 ) ).
-HD int inter_pixel(const Inter *p, int r, int c) { return clip1(round2(inter_sum(p, r, c), 11)); }
-// Compound intermediate (isCompound: InterRound1 = 7, not clipped).
-HD int inter_raw(const Inter *p, int r, int c) { return round2(inter_sum(p, r, c), 7); }
+static_assert(subpel_taps_halve(), "every subpel filter tap is even and its half fits a signed byte");
 
 // The 16 single-reference samples of the 4x4 unit at (r0, c0), row-major
-// into o: inter_pixel in separable form. A horizontal sum Round2( ., 3 )
+// into o, Clip1( Round2( sum, 11 ) ) of the 8 x 8 taps in separable form. A
+// horizontal sum Round2( ., 3 )
 // depends only on its row and column, so the unit's 11 x 4 of them are
 // formed once (11 x 11 reference samples) and each output takes 8 of them;
 // at a full-sample position every filter is (0, 0, 0, 128, 0, 0, 0, 0) and

@@ -1169,7 +1169,7 @@ __device__ void code_plane(const Ctx &c, Smem &sm, int plane, int txSz) {
 // Inter prediction of a w x h block (spec 7.11.3.4) in three steps, staged in
 // shared memory: the clamped reference window (h + 7 rows of w + 7 samples),
 // the horizontal 8-tap pass of every window row (Round2 by InterRound0 = 3),
-// the vertical pass - the values inter_sum forms sample by sample
+// the vertical pass - the values the reference forms sample by sample
 // (k_inter.h:451-504). Every tap is even, so half taps (in 8 bits) give the
 // same rounded sum: (2 S + 4) >> 3 = (S + 2) >> 2, and a row's 4 sums take 8
 // byte dot products on 3 words instead of 32 loads and multiplies; the
